@@ -233,6 +233,11 @@ bool ruai_gemv_wide_eligible(const ruai_ctx* ctx, const ruai_qweight* w, uint32_
 int ruai_gemv_wide_launch(ruai_ctx* ctx, const ruai_qweight* w, const void* x, int x_dtype, uint32_t x_ld, uint32_t m, void* out,
                           const GemvEpilogue& epi, const GemvPrologue& pro);
 bool ruai_gemm_tc_eligible(const ruai_qweight* w, uint32_t m);
+// Whether ruai_gemv_launch runs these rows on the GEMM.  It alone takes a norm weight without sums of squares: its pre-kernel
+// then computes the whole RMSNorm.
+inline bool ruai_gemm_tc_takes(const ruai_ctx* ctx, const ruai_qweight* w, uint32_t m, const GemvEpilogue& e) {
+  return ctx->use_bulk && ctx->use_tc && ruai_gemm_tc_eligible(w, m) && !e.sumsq && !e.argmax_out;
+}
 int ruai_gemm_tc_launch(ruai_ctx* ctx, const ruai_qweight* w, const void* x, int x_dtype, uint32_t x_ld, uint32_t m, void* out,
                         const GemvEpilogue& epi, const GemvPrologue& pro);
 // Reads and clears the context's device status word (synchronizes the stream).

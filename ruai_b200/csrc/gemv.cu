@@ -380,7 +380,7 @@ int ruai_gemv_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x_dt
     d.w = w; d.x = x; d.x_ld = x_ld; d.out = out; d.epi = epi_in;
     return ruai_dense_launch(c, &d, 1, x_dtype, m);
   }
-  if (c->use_bulk && c->use_tc && ruai_gemm_tc_eligible(w, m) && !epi_in.sumsq && !epi_in.argmax_out)
+  if (ruai_gemm_tc_takes(c, w, m, epi_in))
     return ruai_gemm_tc_launch(c, w, x, x_dtype, x_ld, m, out, epi_in, pro);
   if (c->use_bulk && c->use_tc && ruai_gemv_wide_eligible(c, w, m)) return ruai_gemv_wide_launch(c, w, x, x_dtype, x_ld, m, out, epi_in, pro);
   if (c->use_bulk && c->use_tc && ruai_gemv_tc8_eligible(w, m) && !(epi_in.argmax_out && m > 8)) return ruai_gemv_tc8_launch(c, w, x, x_dtype, x_ld, m, out, epi_in, pro);
@@ -425,8 +425,8 @@ int ruai_gemv_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x_dt
 
 size_t ruai_gemv_xs_bytes(const ruai_qweight* w, uint32_t m) {
   const size_t groups = (w->k + 31) / 32;
-  // up to 16 rows: one 16-row tile, 2 KB per group, whole 64-k tiles; beyond: 16 KB per group and block of 128 rows
-  return m <= 16 ? ((groups + 1) & ~(size_t)1) * 2048 : (size_t)((m + 127) / 128) * groups * 16384;
+  // up to 16 rows: one 16-row tile, 2 KB per group, whole 64-k tiles; beyond: 32 KB per 64 k and block of 128 rows, and a factor per row
+  return m <= 16 ? ((groups + 1) & ~(size_t)1) * 2048 : (size_t)((m + 127) / 128) * ((groups + 1) / 2) * 32768 + (size_t)m * 4;
 }
 
 uint32_t ruai_gemv_tiles(const ruai_ctx* c, const ruai_qweight* w) {
