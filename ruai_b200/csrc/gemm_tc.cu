@@ -171,29 +171,47 @@ struct Params {
   GemvEpilogue epi;
 };
 
-// CB column blocks of 128 x NT rows of x per CTA.  Warps: 0 copies, 1 issues MMAs, 4-7 expand, 8.. drain (four per column block).
+// CB column blocks of 128 x NT rows of x per CTA.  Warps: 0 copies W, 1 and 2 issue MMAs, 3 copies x, then, with one column block,
+// four that expand and four per 64 rows that drain; with two, sixteen that do both (96 registers for twenty warps are what the
+// register file holds).  The A operand lies in tensor memory: from shared memory its reads, the writes of the expanding warps and the
+// copies together took more than the 128 bytes per clock there are (measured: a stage's MMAs 1,900 clocks instead of 1,024).  Shared
+// memory: a ring of packed stages (the scales of int4 in one of their own) and a ring of stages of x.
 template <int BITS, int CB, int NT>
 struct Tile {
   static constexpr int kCols = CB * 128;
-  static constexpr int kThreads = 256 + 128 * CB;
+  static constexpr int kDrains = CB * NT / 64;                           // draining warpgroups
+  static constexpr bool kBoth = CB == 2;                                 // the draining warps expand as well
+  static constexpr int kDrain0 = kBoth ? 4 : 8;                          // first draining warp
+  static constexpr int kExpanders = kBoth ? 4 * kDrains : 4;             // warps
+  static constexpr int kThreads = 32 * kDrain0 + 128 * kDrains;
   static constexpr uint32_t kWChunk = kCols * 16;                        // one 16-byte chunk of every column
   static constexpr int kChunks = BITS == 4 ? 2 : 4;                      // chunks per stage
   static constexpr uint32_t kWBytes = kChunks * kWChunk;
-  static constexpr uint32_t kPiece = NT * 128;                           // one piece of a stage
-  static constexpr uint32_t kSlot = 2 * kPiece + kWBytes;
-  static constexpr uint32_t kA = kCols * 128;                            // one stage of the A operand
-  static constexpr int kFit = (int)((230400 - 1024 - 2 * kA) / kSlot);
-  static constexpr int kSlots = kFit < 6 ? kFit : 6;
-  static constexpr size_t kSmem = 1024 + 2 * (size_t)kA + (size_t)kSlots * kSlot;
-  static constexpr uint32_t kTmem = 2 * CB * NT;                         // two sets of sums
-  static_assert(kSlots >= 3, "ring too short");
+  static constexpr int kWSlots = CB == 2 ? 4 : 6;
+  static constexpr uint32_t kPiece = NT * 128;                           // one piece of x of a stage
+  static constexpr uint32_t kX = 2 * kPiece;                             // both
+  // Tensor memory: three buffers of sums, then the A operand, 32 words per column block and stage.
+  static constexpr uint32_t kACol0 = 3 * NT;
+  static constexpr int kABufs = 4 / CB;
+  static constexpr uint32_t kTmem = 512;
+  static constexpr uint32_t kScale = BITS == 4 ? 2 * kCols * 4 : 0;      // scales of a stage
+  static constexpr int kScaleSlots = kWSlots + kABufs + 2;               // see the copies
+  static constexpr uint32_t kFixed = kWSlots * kWBytes + kScaleSlots * kScale;
+  static constexpr int kFit = (int)((230400 - 1024 - kFixed) / kX);
+  static constexpr int kXSlots = kFit < 8 ? kFit : 8;
+  static constexpr uint32_t off_w = kXSlots * kX, off_scale = off_w + kWSlots * kWBytes;
+  static constexpr size_t kRed = (size_t)(NT + 8) * kCols * 4;           // split k: partial sums of this CTA's rows
+  static constexpr size_t kRing = (size_t)kFixed + (size_t)kXSlots * kX;
+  static constexpr size_t kSmem = 1024 + (kRing > kRed ? kRing : kRed);
+  static_assert(kXSlots >= 3, "ring too short");
 };
 
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {  // K-major, 128-byte swizzle, 1024 bytes between 8-row blocks
   return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b),
+// A from tensor memory: lane = column of W, word c of a step holds its k positions 2 c and 2 c + 1.
+__device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b),
                "r"(idesc), "r"(accumulate)
                : "memory");
 }
@@ -202,13 +220,26 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
   return p != 0;
 }
-// 16 consecutive 32-bit columns of this thread's TMEM lane.
+// 16 consecutive 32-bit columns of this thread's TMEM lane.  The load writes its registers until the wait has returned, so the wait
+// takes them as operands: nothing that uses them can be placed ahead of it, and nothing else can be put into them.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
         "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]),
+                 "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "r"(v[0]),
+      "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]),
+      "r"(v[14]), "r"(v[15])
       : "memory");
 }
 // Two f32 multiply-adds in one instruction, each rounded like fmaf.
@@ -247,7 +278,7 @@ __device__ __forceinline__ void expand_int4(const uint4& q, uint32_t (&o)[16]) {
     o[8 + 2 * i + 1] = hfma2_bits((t & 0x00F000F0u) | 0x64006400u, 0x2C002C00u, 0xD480D480u);
   }
 }
-__device__ __forceinline__ void expand_int8(const uint4& q, uint32_t (&o)[8]) {
+__device__ __forceinline__ void expand_int8(const uint4& q, uint32_t* o) {
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {  // 1024 + 128 + value
@@ -256,20 +287,12 @@ __device__ __forceinline__ void expand_int8(const uint4& q, uint32_t (&o)[8]) {
   }
 }
 
-template <int R>
-__device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
-template <int R>
-__device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
-
 // Row factor, column scale, bias, activation, residual and store of R consecutive rows of one column (a lane per column, the
 // warp converged).  What is read is requested before the first store: the compiler cannot move loads over stores.
 template <int R>
-__device__ __forceinline__ void finish_rows(const Params& p, uint32_t end, float (&v)[R], uint32_t row, uint32_t j, bool active, float cs, float bias) {
+__device__ __forceinline__ void finish_rows(const Params& p, uint32_t end, float (&v)[R], const float (&rf)[R], uint32_t row, uint32_t j, bool active, float cs, float bias) {
   const GemvEpilogue& e = p.epi;
   const uint32_t nr = min((uint32_t)R, end - row);
-  float rf[R];
-#pragma unroll
-  for (int t = 0; t < R; ++t) rf[t] = (uint32_t)t < nr ? __ldcg(p.rowf + row + t) : 0.0f;
 #pragma unroll
   for (int t = 0; t < R; ++t) v[t] = v[t] * cs * rf[t] + bias;
   if (e.act == ACT_SWIGLU) {
@@ -323,24 +346,25 @@ __device__ __forceinline__ void finish_rows(const Params& p, uint32_t end, float
 template <int BITS, int CB, int NT>
 __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kernel(const Params p) {
   using T = Tile<BITS, CB, NT>;
-  constexpr uint32_t S = T::kSlots;
+  constexpr uint32_t XS = T::kXSlots, WS = T::kWSlots, AB = T::kABufs;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t full[S], empty[S];   // a slot's copies landed; the MMAs that read it completed
-  __shared__ __align__(8) uint64_t a_ready[2];          // A operand of a stage written (4 expanding warps)
-  __shared__ __align__(8) uint64_t acc_full[2], acc_free[2];  // a segment's sums complete; read out (4 CB warps)
-  __shared__ __align__(8) uint64_t fin;
+  __shared__ __align__(8) uint64_t x_full[XS], x_empty[XS];   // x of a stage landed; the MMAs that read it completed
+  __shared__ __align__(8) uint64_t w_full[WS], w_empty[WS];   // a packed stage (and its scales) landed; expanded (every expanding warp)
+  __shared__ __align__(8) uint64_t a_ready[AB], a_free[AB];   // A operand of a stage written; the MMAs that read it completed
+  __shared__ __align__(8) uint64_t acc_full[3], acc_free[3];  // the sums of a unit (segment, column block) complete; read out (the column block's draining warps)
+  __shared__ __align__(8) uint64_t fin[2];
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_abort;
   // swizzled operands start on 1024-byte boundaries (the same offset in every CTA of a cluster: the window bases are alike)
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  unsigned char* abuf = smem;
-  unsigned char* ring = smem + 2 * T::kA;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   if (tid == 0) {
-    for (uint32_t s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&a_ready[s], 4); mbar_init(&acc_full[s], 1); mbar_init(&acc_free[s], 4 * CB); }
-    mbar_init(&fin, 1);
+    for (uint32_t s = 0; s < XS; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], CB); }
+    for (uint32_t s = 0; s < WS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], T::kExpanders); }
+    for (uint32_t s = 0; s < AB; ++s) { mbar_init(&a_ready[s], T::kExpanders); mbar_init(&a_free[s], CB); }
+    for (int s = 0; s < 3; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_free[s], 4 * T::kDrains / CB); }
+    mbar_init(&fin[0], 1); mbar_init(&fin[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_abort = 0;
   }
@@ -356,194 +380,218 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
   auto cols_of = [&](uint32_t t) { return (t / p.row_blocks) * (uint32_t)T::kCols; };  // row blocks fastest: a tile of W comes from HBM once
   auto rows_of = [&](uint32_t t) { return (t % p.row_blocks) * (uint32_t)NT; };
 
+  // Stage `it` of this CTA: packed weights -> A operand, for one warp's columns of column block cb, groups u0 .. u1 of the stage.
+  auto expand = [&](uint32_t it, uint32_t cb, uint32_t u0, uint32_t u1) -> bool {
+    const uint32_t slot = it % WS, ab = it % AB, quarter = (uint32_t)warp & 3u;
+    if (s_abort || !mbar_wait(&w_full[slot], (it / WS) & 1u)) return false;
+    if (it >= AB && !mbar_wait(&a_free[ab], (it / AB - 1u) & 1u)) return false;
+    const unsigned char* w = smem + T::off_w + slot * T::kWBytes + (cb * 128u + quarter * 32u + lane) * 16u;
+    const uint32_t a = tmem + ((quarter * 32u) << 16) + T::kACol0 + (ab * CB + cb) * 32;
+    tc_fence_after_sync();
+    for (uint32_t u = u0; u < u1; ++u) {
+      uint32_t o[16];
+      if constexpr (BITS == 4) expand_int4(*reinterpret_cast<const uint4*>(w + u * T::kWChunk), o);
+      else {
+        const uint4 q0 = *reinterpret_cast<const uint4*>(w + 2 * u * T::kWChunk), q1 = *reinterpret_cast<const uint4*>(w + (2 * u + 1) * T::kWChunk);
+        expand_int8(q0, o);
+        expand_int8(q1, o + 8);
+      }
+      tmem_st16(a + u * 16, o);
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) { mbar_arrive(&a_ready[ab]); mbar_arrive(&w_empty[slot]); }
+    return true;
+  };
+
   if (warp < 4) {
-    if constexpr (NT == 128) setmaxnreg_dec<40>();
-    if (warp == 0 && lane == 0) {
-      // ===== copies.  Weights do not depend on the predecessor kernel: the first slots' are requested before the wait. =====
-      const uint32_t bbytes = (uint32_t)p.pieces * T::kPiece;
-      auto copy_w = [&](uint32_t t, uint32_t s, uint32_t slot) {
-        const uint32_t j0 = cols_of(t), bytes = min((uint32_t)T::kCols, p.n - j0) * 16u, c0 = s * T::kChunks;
-        const uint32_t nc = min((uint32_t)T::kChunks, p.chunks - c0);
-        unsigned char* dst = ring + slot * T::kSlot + 2 * T::kPiece;
-        mbar_expect_tx(&full[slot], nc * bytes + bbytes);
-        for (uint32_t c = 0; c < nc; ++c) bulk_load(dst + c * T::kWChunk, p.w + (size_t)(c0 + c) * p.n + j0, bytes, &full[slot]);
-      };
-      auto copy_x = [&](uint32_t t, uint32_t s, uint32_t slot) {
-        bulk_load(ring + slot * T::kSlot, p.xs + ((size_t)(t % p.row_blocks) * p.stages + s) * bbytes, bbytes, &full[slot]);
-      };
-      const uint32_t pre = min(nst, S);
-      for (uint32_t i = 0; i < pre; ++i) copy_w(tile0, s0 + i, i);
-      grid_dependency_wait();
-      grid_launch_dependents();
-      for (uint32_t i = 0; i < pre; ++i) copy_x(tile0, s0 + i, i);
-      uint32_t it = pre;
+    if (warp == 0 && elect_one()) {
+      // ===== packed weights (and their scales).  They do not depend on the predecessor kernel. =====
+      uint32_t it = 0;
       bool ok = true;
       for (uint32_t t = tile0; t < p.tiles && ok; t += stride) {
-        for (uint32_t s = t == tile0 ? s0 + pre : s0; s < s1; ++s, ++it) {
-          const uint32_t slot = it % S;
-          if (it >= S && (s_abort || !mbar_wait(&empty[slot], (it / S - 1u) & 1u))) { s_abort = 1; ok = false; break; }
-          copy_w(t, s, slot);
-          copy_x(t, s, slot);
+        const uint32_t j0 = cols_of(t), nc = min((uint32_t)T::kCols, p.n - j0);
+        for (uint32_t s = s0; s < s1; ++s, ++it) {
+          const uint32_t slot = it % WS;
+          if (it >= WS && (s_abort || !mbar_wait(&w_empty[slot], (it / WS - 1u) & 1u))) { s_abort = 1; ok = false; break; }
+          const uint32_t c0 = s * T::kChunks, chunks = min((uint32_t)T::kChunks, p.chunks - c0);
+          unsigned char* dst = smem + T::off_w + slot * T::kWBytes;
+          // int4: a chunk is a scale group.  The scales' slot is free: this packed slot is, so stage it - kWSlots is expanded, so the
+          // MMAs of stage it - kWSlots - kABufs are done, and those waited for the read-out of all but the last three units up to
+          // theirs: every stage up to it - kWSlots - kABufs - 2 has been read out (a tile's last stage may be one group).
+          mbar_expect_tx(&w_full[slot], chunks * nc * (BITS == 4 ? 20u : 16u));
+          for (uint32_t c = 0; c < chunks; ++c) {
+            bulk_load(dst + c * T::kWChunk, p.w + (size_t)(c0 + c) * p.n + j0, nc * 16u, &w_full[slot]);
+            if constexpr (BITS == 4)
+              bulk_load(smem + T::off_scale + (it % T::kScaleSlots) * T::kScale + c * T::kCols * 4, p.scale + (size_t)(c0 + c) * p.n + j0, nc * 4u, &w_full[slot]);
+          }
         }
       }
       if (s_abort)  // leave no copy in flight into shared memory that another CTA may get
-        for (uint32_t i = it > S ? it - S : 0; i < it; ++i) (void)mbar_wait(&full[i % S], (i / S) & 1u);
-    } else if (warp == 1 && elect_one()) {
-      // ===== MMAs =====
-      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((128u >> 4) << 24);  // fp16 x fp16 -> f32
-      uint32_t it = 0, seg = 0;
+        for (uint32_t i = it > WS ? it - WS : 0; i < it; ++i) (void)mbar_wait(&w_full[i % WS], (i / WS) & 1u);
+    } else if (warp == 3 && elect_one()) {
+      // ===== x =====
+      grid_dependency_wait();
+      grid_launch_dependents();
+      uint32_t it = 0;
       bool ok = true;
       for (uint32_t t = tile0; t < p.tiles && ok; t += stride) {
-        for (uint32_t s = s0; s < s1; ++s, ++it) {
-          const uint32_t slot = it % S, ab = it & 1u;
-          if (s_abort || !mbar_wait(&a_ready[ab], (it >> 1) & 1u) || !mbar_wait(&full[slot], (it / S) & 1u)) { ok = false; break; }
-          const uint64_t ad = desc_sw128(smem_u32(abuf + ab * T::kA)), bd = desc_sw128(smem_u32(ring + slot * T::kSlot));
-          if constexpr (BITS == 4) {
-            const uint32_t ng = min(2u, p.groups - 2u * s);
-            for (uint32_t u = 0; u < ng; ++u, ++seg) {
-              const uint32_t set = seg & 1u;
-              if (seg >= 2 && !mbar_wait(&acc_free[set], ((seg >> 1) - 1u) & 1u)) { ok = false; break; }
-              tc_fence_after_sync();
-#pragma unroll
-              for (uint32_t cb = 0; cb < CB; ++cb)
-                for (uint32_t pc = 0; pc < (uint32_t)p.pieces; ++pc)
+        const uint32_t bytes = (uint32_t)p.pieces * T::kPiece;
+        const unsigned char* src = p.xs + ((size_t)(t % p.row_blocks) * p.stages + s0) * bytes;
+        for (uint32_t i = 0; i < nst; ++i, ++it) {
+          const uint32_t slot = it % XS;
+          if (it >= XS && (s_abort || !mbar_wait(&x_empty[slot], (it / XS - 1u) & 1u))) { s_abort = 1; ok = false; break; }
+          mbar_expect_tx(&x_full[slot], bytes);
+          bulk_load(smem + slot * T::kX, src + (size_t)i * bytes, bytes, &x_full[slot]);
+        }
+      }
+      if (s_abort)
+        for (uint32_t i = it > XS ? it - XS : 0; i < it; ++i) (void)mbar_wait(&x_full[i % XS], (i / XS) & 1u);
+    } else if ((warp == 1 || warp == 2) && elect_one()) {
+      // ===== MMAs.  A wait behind MMAs comes back only when those have left the issue queue (measured: 90 to 260 clocks in which
+      // the tensor pipe has nothing to do), so two threads issue, each into its own sums: one per column block, or, with one
+      // column block, every other stage each. =====
+      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((128u >> 4) << 24);  // fp16 x fp16 -> f32
+      const uint64_t xd0 = desc_sw128(smem_u32(smem));
+      const uint32_t pieces = (uint32_t)p.pieces, h = (uint32_t)warp - 1u, cb = CB == 2 ? h : 0u;
+      uint32_t it = 0, unit = BITS == 4 && CB == 1 ? 0u : h;
+      bool ok = true;
+      auto sums_free = [&](uint32_t u) { return u < 3 || mbar_wait(&acc_free[u % 3], (u / 3 - 1u) & 1u); };
+      for (uint32_t t = tile0; t < p.tiles && ok; t += stride) {
+        for (uint32_t s = s0; s < s1 && ok; ++s, ++it) {
+          const uint32_t ab = it % AB, slot = it % XS, ng = BITS == 4 ? min(2u, p.groups - 2u * s) : 1u, at = (s - s0) % kSegStages;
+          const bool mine = CB == 2 || ((s - s0) & 1u) == h;
+          if (BITS == 4 && !mine) { unit += ng; continue; }
+          const bool last = at + 3 - CB >= kSegStages || s + 3 - CB >= s1;  // int8: of this thread's stages in the segment
+          if (mine) {
+            if (s_abort || !mbar_wait(&a_ready[ab], (it / AB) & 1u) || !mbar_wait(&x_full[slot], (it / XS) & 1u)) { ok = false; break; }
+            const uint32_t a = tmem + T::kACol0 + (ab * CB + cb) * 32;
+            const uint64_t xd = umma_desc_advance(xd0, slot * T::kX);
+            if constexpr (BITS == 4) {
+              for (uint32_t u = 0; u < ng; ++u, unit += CB) {
+                if (!sums_free(unit)) { ok = false; break; }
+                tc_fence_after_sync();
+                const uint32_t d = tmem + (unit % 3) * NT;
+                for (uint32_t pc = 0; pc < pieces; ++pc)
 #pragma unroll
                   for (uint32_t q = 0; q < 2; ++q)
-                    mma_f16(tmem + (set * CB + cb) * NT, umma_desc_advance(ad, cb * 16384u + u * 64u + q * 32u),
-                            umma_desc_advance(bd, pc * T::kPiece + u * 64u + q * 32u), idesc, (pc | q) != 0 ? 1u : 0u);
-              umma_commit(&acc_full[set]);
+                    mma_f16(d, a + u * 16 + q * 8, umma_desc_advance(xd, pc * T::kPiece + u * 64u + q * 32u), idesc, (pc | q) != 0 ? 1u : 0u);
+                umma_commit(&acc_full[unit % 3]);
+              }
+            } else {
+              const bool first = at < 3 - CB;
+              if (first && !sums_free(unit)) { ok = false; break; }
+              tc_fence_after_sync();
+              const uint32_t d = tmem + (unit % 3) * NT;
+              for (uint32_t pc = 0; pc < pieces; ++pc)
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q) mma_f16(d, a + q * 8, umma_desc_advance(xd, pc * T::kPiece + q * 32u), idesc, !first || (pc | q) != 0 ? 1u : 0u);
+              if (last) { umma_commit(&acc_full[unit % 3]); unit += 2; }
             }
-            if (!ok) break;
-          } else {
-            const uint32_t set = seg & 1u, at = (s - s0) % kSegStages;
-            if (at == 0 && seg >= 2 && !mbar_wait(&acc_free[set], ((seg >> 1) - 1u) & 1u)) { ok = false; break; }
-            tc_fence_after_sync();
-#pragma unroll
-            for (uint32_t cb = 0; cb < CB; ++cb)
-              for (uint32_t pc = 0; pc < (uint32_t)p.pieces; ++pc)
-#pragma unroll
-                for (uint32_t q = 0; q < 4; ++q)
-                  mma_f16(tmem + (set * CB + cb) * NT, umma_desc_advance(ad, cb * 16384u + q * 32u),
-                          umma_desc_advance(bd, pc * T::kPiece + q * 32u), idesc, (at | pc | q) != 0 ? 1u : 0u);
-            if (at == kSegStages - 1 || s + 1 == s1) { umma_commit(&acc_full[set]); ++seg; }
+            umma_commit(&x_empty[slot]);
+            umma_commit(&a_free[ab]);
+          } else if (h == 1 && at == 0 && s + 1 == s1) {  // int8, a segment of one stage: the other thread's sums are all there is
+            if (!sums_free(unit)) { ok = false; break; }
+            umma_commit(&acc_full[unit % 3]);
+            unit += 2;
           }
-          umma_commit(&empty[slot]);
         }
       }
       if (!ok) s_abort = 1;
-      umma_commit(&fin);  // nothing is left running when tensor memory is freed
-      if (!mbar_wait(&fin, 0)) s_abort = 1;
+      umma_commit(&fin[h]);  // nothing is left running when tensor memory is freed
+      if (!mbar_wait(&fin[h], 0)) s_abort = 1;
     }
     __syncwarp();
     grid_dependency_wait();
-  } else if (warp < 8) {
-    if constexpr (NT == 128) setmaxnreg_dec<CB == 2 ? 72 : 152>();
-    // ===== expanding warps: thread = column of each column block =====
-    const uint32_t c = (uint32_t)tid - 128u, xr = c & 7u;
+  } else if (warp < T::kDrain0) {
+    // ===== expanding warps (one column block) =====
     uint32_t it = 0;
     bool ok = true;
-    for (uint32_t t = tile0; t < p.tiles && ok; t += stride) {
-      for (uint32_t s = s0; s < s1; ++s, ++it) {
-        const uint32_t slot = it % S, ab = it & 1u;
-        if (s_abort || !mbar_wait(&full[slot], (it / S) & 1u)) { ok = false; break; }
-        // the A buffer was read last by the MMAs of stage it - 2, whose slot's barrier cannot have gone on: that takes this stage
-        if (it >= 2 && !mbar_wait(&empty[(it - 2) % S], ((it - 2) / S) & 1u)) { ok = false; break; }
-        const unsigned char* w = ring + slot * T::kSlot + 2 * T::kPiece + c * 16u;
-        unsigned char* a = abuf + ab * T::kA + (c >> 3) * 1024u + xr * 128u;
-#pragma unroll
-        for (uint32_t cb = 0; cb < CB; ++cb) {
-          uint4 q[T::kChunks];
-#pragma unroll
-          for (int u = 0; u < T::kChunks; ++u) q[u] = *reinterpret_cast<const uint4*>(w + u * T::kWChunk + cb * 2048u);
-#pragma unroll
-          for (int u = 0; u < T::kChunks; ++u) {
-            if constexpr (BITS == 4) {
-              uint32_t o[16];
-              expand_int4(q[u], o);
-#pragma unroll
-              for (uint32_t i = 0; i < 4; ++i)
-                *reinterpret_cast<uint4*>(a + cb * 16384u + (((4u * u + i) ^ xr) << 4)) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
-            } else {
-              uint32_t o[8];
-              expand_int8(q[u], o);
-#pragma unroll
-              for (uint32_t i = 0; i < 2; ++i)
-                *reinterpret_cast<uint4*>(a + cb * 16384u + (((2u * u + i) ^ xr) << 4)) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
-            }
-          }
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&a_ready[ab]);
-      }
-    }
+    for (uint32_t t = tile0; t < p.tiles && ok; t += stride)
+      for (uint32_t s = s0; s < s1 && ok; ++s, ++it) ok = expand(it, 0, 0, 2);
     if (!ok) s_abort = 1;
     grid_dependency_wait();
   } else {
-    if constexpr (NT == 128) setmaxnreg_inc<CB == 2 ? 200 : 232>();
-    // ===== draining warps: thread = column of one column block =====
-    grid_dependency_wait();
-    const uint32_t quarter = (uint32_t)warp & 3u, cb = (uint32_t)(warp - 8) >> 2, col = cb * 128u + quarter * 32u + lane;
-    const uint32_t lane_base = (quarter * 32u) << 16;
-    constexpr int kFinish = NT == 128 ? 8 : 16;  // rows finished together: what the registers beside the sums hold
-    unsigned long long acc[NT / 2];
-    uint32_t seg = 0;
-    auto drain = [&](unsigned long long s2) -> bool {
-      const uint32_t set = seg & 1u;
-      if (s_abort || !mbar_wait(&acc_full[set], (seg >> 1) & 1u)) return false;
+    // ===== draining warps: thread = column of one column block, 64 rows =====
+    const uint32_t dw = (uint32_t)(warp - T::kDrain0), quarter = (uint32_t)warp & 3u, cb = (dw >> 2) & (CB - 1), half = dw / (4 * CB) * 64u;
+    const uint32_t col = cb * 128u + quarter * 32u + lane, sums = tmem + ((quarter * 32u) << 16) + half;
+    constexpr int kFinish = CB == 2 ? 8 : 16;  // rows finished together: what the registers beside the sums hold
+    unsigned long long acc[32];
+    uint32_t unit = cb;
+    bool ok = true;
+    // one unit's sums into the registers, times the scale of group u of a stage
+    auto drain = [&](uint32_t scale_slot, uint32_t u, bool none) -> bool {
+      const uint32_t set = unit % 3;
+      if (s_abort || !mbar_wait(&acc_full[set], (unit / 3) & 1u)) return false;
       tc_fence_after_sync();
-      const uint32_t at = tmem + lane_base + (set * CB + cb) * NT;
+      float sv = 1.0f;
+      if constexpr (BITS == 4)  // a column past the matrix reads what an earlier tile left: it is never stored
+        sv = *reinterpret_cast<const float*>(smem + T::off_scale + scale_slot * T::kScale + (u * T::kCols + col) * 4u);
+      const unsigned long long s2 = pair_of(sv);
+      const uint32_t at = sums + set * NT;
 #pragma unroll
-      for (int c = 0; c < NT / 16; ++c) {
+      for (int c = 0; c < 4; ++c) {
         uint32_t d[16];
         tmem_ld16(at + 16 * c, d);
-        tmem_ld_wait();
-        if (c == NT / 16 - 1) {  // the set may be overwritten
+        if (c == 3) {  // the buffer may be overwritten
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_free[set]);
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) fma2(acc[8 * c + i], d[2 * i], d[2 * i + 1], s2);
+        for (int i = 0; i < 8; ++i)
+          if (!none) fma2(acc[8 * c + i], d[2 * i], d[2 * i + 1], s2);
       }
-      ++seg;
+      unit += CB;
       return true;
     };
-    bool ok = true;
-    for (uint32_t t = tile0; t < p.tiles && ok; t += stride) {
-      const uint32_t j = cols_of(t) + col, row0 = rows_of(t);
-      const bool active = j < p.n;
-#pragma unroll
-      for (int i = 0; i < NT / 2; ++i) acc[i] = 0ull;
+    // what stage s (number it of this CTA) completes
+    auto drain_stage = [&](uint32_t it, uint32_t s) -> bool {
       if constexpr (BITS == 4) {
-        const uint32_t g0 = 2 * s0, g1 = min(p.groups, 2 * s1);
-        float sc[4];  // the column's scales, four groups ahead
-        auto scale_at = [&](uint32_t g) { return active && g < g1 ? __ldg(p.scale + (size_t)g * p.n + j) : 0.0f; };
+        const uint32_t ng = min(2u, p.groups - 2u * s);
+#pragma unroll 1
+        for (uint32_t u = 0; u < ng; ++u)
+          if (!drain(it % T::kScaleSlots, u, false)) return false;
+      } else if ((s - s0) % kSegStages == kSegStages - 1 || s + 1 == s1) {
+        // one column block: both issuing threads' sums, of which the second has none in a segment of one stage
+#pragma unroll 1
+        for (uint32_t u = 0; u < 3 - CB; ++u)
+          if (!drain(0, 0, u == 1 && (s - s0) % kSegStages == 0)) return false;
+      }
+      return true;
+    };
+    uint32_t it = 0;
+    if constexpr (T::kBoth) ok = expand(0, cb, half / 64u, half / 64u + 1);
+    grid_dependency_wait();
+    for (uint32_t t = tile0; t < p.tiles && ok; t += stride) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) sc[q] = scale_at(g0 + q);
-        for (uint32_t g = g0; g < g1 && ok; g += 4) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (g + q >= g1) break;
-            const unsigned long long s2 = pair_of(sc[q]);
-            sc[q] = scale_at(g + q + 4);
-            if (!drain(s2)) { ok = false; break; }
-          }
+      for (int i = 0; i < 32; ++i) acc[i] = 0ull;
+#pragma unroll 1
+      for (uint32_t s = s0; s < s1 && ok; ++s, ++it) {
+        if constexpr (T::kBoth) {  // the next stage (the next tile's first) is ready before this one's sums are read
+          if (s + 1 < s1 || t + stride < p.tiles) ok = expand(it + 1, cb, half / 64u, half / 64u + 1);
         }
-      } else {
-        for (uint32_t s = 0; s < nst; s += kSegStages)
-          if (!drain(pair_of(1.0f))) { ok = false; break; }
+        ok = ok && drain_stage(it, s);
       }
       if (!ok) break;
       if (p.splits > 1) break;  // one tile per cluster: see below
+      const uint32_t j = cols_of(t) + col, row0 = rows_of(t) + half;
+      const bool active = j < p.n;
+      // everything the epilogue reads is requested ahead of its first store: loads between stores wait behind them (measured: 63,000
+      // clocks for an epilogue that read the rows' factors in groups of eight)
       const float cs = BITS == 8 && active ? __ldg(p.scale + j) : 1.0f, bias = p.epi.bias && active ? __ldg(p.epi.bias + j) : 0.0f;
+      const float rfl[2] = {row0 + lane < p.m ? __ldcg(p.rowf + row0 + lane) : 0.0f, row0 + 32u + lane < p.m ? __ldcg(p.rowf + row0 + 32u + lane) : 0.0f};
 #pragma unroll
-      for (int r = 0; r < NT; r += kFinish) {
+      for (int r = 0; r < 64; r += kFinish) {
         if (row0 + r >= p.m) break;
-        float v[kFinish];
+        float v[kFinish], rf[kFinish];
 #pragma unroll
-        for (int i = 0; i < kFinish / 2; ++i) { v[2 * i] = low_of(acc[r / 2 + i]); v[2 * i + 1] = high_of(acc[r / 2 + i]); }
-        finish_rows<kFinish>(p, p.m, v, row0 + r, j, active, cs, bias);
+        for (int i = 0; i < kFinish; ++i) {
+          v[i] = (i & 1) ? high_of(acc[(r + i) / 2]) : low_of(acc[(r + i) / 2]);
+          rf[i] = __shfl_sync(0xFFFFFFFFu, rfl[r / 32], (r + i) % 32);
+        }
+        finish_rows<kFinish>(p, p.m, v, rf, row0 + r, j, active, cs, bias);
       }
     }
     if (!ok) s_abort = 1;
@@ -555,32 +603,34 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
       const bool active = j < p.n;
       __syncwarp();
       cluster_sync_all();  // every CTA is through with its operands
-      uint32_t owner = 0, at = 0;
+      uint32_t owner = half / rows_per, at = half % rows_per;
 #pragma unroll
-      for (int r = 0; r < NT; ++r) {
+      for (int r = 0; r < 64; ++r) {
         st_cluster_f32(red + ((size_t)split * rows_per + at) * T::kCols + col, owner, (r & 1) ? high_of(acc[r / 2]) : low_of(acc[r / 2]));
         if (++at == rows_per) { at = 0; ++owner; }
       }
+      __syncwarp();
       cluster_sync_all();
       if (!s_abort) {
         const float cs = BITS == 8 && active ? __ldg(p.scale + j) : 1.0f, bias = p.epi.bias && active ? __ldg(p.epi.bias + j) : 0.0f;
         const uint32_t first = split * rows_per, last = min(first + rows_per, (uint32_t)NT);
-        for (uint32_t r = first; r < last; r += 8) {
+        // eight rows at a time, in turn over the warpgroups of a column block
+        for (uint32_t r = first + half / 8u; r < last; r += NT / 8u) {
           if (row0 + r >= p.m) break;
-          float v[8];
+          float v[8], rf[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = 0.0f;
+          for (uint32_t i = 0; i < 8; ++i) { v[i] = 0.0f; rf[i] = row0 + r + i < p.m ? __ldcg(p.rowf + row0 + r + i) : 0.0f; }
           for (uint32_t q = 0; q < p.splits; ++q) {
 #pragma unroll
             for (uint32_t i = 0; i < 8; ++i)
               if (r + i < last) v[i] += red[((size_t)q * rows_per + (r - first) + i) * T::kCols + col];
           }
-          finish_rows<8>(p, min(p.m, row0 + last), v, row0 + r, j, active, cs, bias);
+          finish_rows<8>(p, min(p.m, row0 + last), v, rf, row0 + r, j, active, cs, bias);
         }
       }
     }
   }
-  if (p.splits > 1 && warp < 8) {  // the draining warps' two
+  if (p.splits > 1 && warp < T::kDrain0) {  // the draining warps' two
     __syncwarp();
     cluster_sync_all();
     cluster_sync_all();
