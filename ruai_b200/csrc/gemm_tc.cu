@@ -5,17 +5,18 @@
 //   - the activations are scaled by a power of two per row and split once, by a small pre-kernel, into two fp16 pieces
 //     x = hi + lo (22 significant bits; bf16 and fp16 activations are one piece, exactly) stored as the tensor core's B
 //     operand: K-major with the 128-byte swizzle, so that a stage of 64 k is one bulk copy;
-//   - packed tiles of W (the chunk layout of pack.cu) ride in the same ring of bulk copies; four warps expand them to fp16
-//     (int4 and int8 values are exact) into the A operand, same swizzle;
+//   - packed tiles of W (the chunk layout of pack.cu) come through a ring of bulk copies of their own and are expanded to fp16
+//     (int4 and int8 values are exact) in tensor memory, the A operand;
 //   - `tcgen05.mma kind::f16`, D[128 columns of W][rows of x], both pieces into the same f32 sums in tensor memory;
 //   - draining warps (thread = column of W) read the sums of every segment out and add them in f32 registers: int4: a segment
 //     is a scale group of 32 k, times scale[g, j] (cpu.rs:1045-1063); int8: four stages, so that the tensor core's own
 //     additions stay short, with the column scale at the end (cpu.rs:903-920).
-// What bounds it: the tensor pipe.  A CTA of 256 columns x 128 rows needs 16 MMAs of 64 clocks per stage (measured: one thread
-// issues M 128, N 128, K 16 every 64 clocks, N 64 every 48 from swizzled shared memory; from the unswizzled layout that an
-// earlier version used a stage took twice as long), while its four expanding and eight draining warps need about 900 issue slots
-// per scheduler.  256 columns, because every B byte is then used twice: with 128 the copies of B alone ask the L2 for 64 bytes
-// per clock and SM.  Three tile shapes and a split of k over a cluster cover the sizes that leave that tile's grid small.
+// What bounds it: int8, the tensor pipe and the power limit (4096 x 4096 x 14336: 0.82 ms, 1.18 PFLOP/s counting both pieces, where
+// cuBLAS sustains 1.40; 1.48 ms int4 and 1.45 int8 with unswizzled operands, which take twice as long); int4, the issue slots of the
+// warps that expand and drain (1.29 ms: per scheduler and stage about 900 of the 1,037 clocks that its MMAs take).  A CTA of 256
+// columns x 128 rows needs 16 MMAs of 64 clocks per stage.  256 columns, because every byte of x is then used twice: with 128 the
+// copies of x alone ask the L2 for 64 bytes per clock and SM.  Three tile shapes and a split of k over a cluster cover the sizes that
+// leave that tile's grid small (64 x 2048 x 2048 int8: 41 us before, 20 CTAs; 11 now).
 // Every mbarrier wait is bounded.
 #include "common.cuh"
 #include "gemv_epilogue.cuh"
@@ -677,12 +678,11 @@ cudaError_t launch(ruai_ctx* c, const Params& p) {
 
 struct Shape { uint32_t cb, nt, splits; };
 
-// The tile and the number of splits of k: a model of the launch in clocks.  A stage costs what its MMAs take (16 x 64 clocks,
-// 8 x 64, 8 x 48) or, with one piece, what expanding and draining take; a wave of CTAs costs a fixed part and one for the
-// epilogue; a split adds the exchange.
-Shape choose(const ruai_ctx* c, uint32_t m, uint32_t n, uint32_t stages, int pieces) {
-  struct Cand { uint32_t cb, nt; double stage2, stage1, epilogue; };
-  const Cand cand[3] = {{2, 128, 1100, 750, 6000}, {1, 128, 620, 480, 5000}, {1, 64, 440, 360, 3000}};
+// The tile and the number of splits of k: a model of the launch in microseconds, fitted to launches of 37 to 2000 rows of the 1.1B and
+// 8B shapes' Linears with every tile and 1 .. 8 splits (the choice is within 5 % of the best of them; a wrong one costs up to 2 x).
+Shape choose(const ruai_ctx* c, uint32_t m, uint32_t n, uint32_t stages, int bits, int pieces) {
+  struct Cand { uint32_t cb, nt; double stage4, stage8, split; };  // a stage of int4 and int8; what a split adds
+  const Cand cand[3] = {{2, 128, 1.55, 1.0, 7.0}, {1, 128, 0.80, 0.55, 6.0}, {1, 64, 0.62, 0.45, 3.5}};
   Shape best = {1, 64, 1};
   double best_t = 1e300;
   for (const Cand& d : cand) {
@@ -690,11 +690,11 @@ Shape choose(const ruai_ctx* c, uint32_t m, uint32_t n, uint32_t stages, int pie
     for (uint32_t s = 1; s <= 8; ++s) {
       const uint32_t per = (stages + s - 1) / s;
       if (s > 1 && (per < 2 || (s - 1) * per >= stages)) continue;
-      // clusters do not fill every SM: groups of SMs are not multiples of their size
-      const uint32_t room = s > 1 ? (uint32_t)c->sm_count * 15u / 16u / s : (uint32_t)c->sm_count;
+      // a cluster lies within one group of SMs: not every SM is reached (measured: sixteen clusters of 8 take two waves)
+      const uint32_t sms = (uint32_t)c->sm_count, room = s == 1 ? sms : s >= 7 ? sms / 10u : sms * 15u / 16u / s;
       if (room == 0) continue;
-      const double waves = (double)((tiles + room - 1) / room);
-      const double t = 4000.0 + waves * ((s > 1 ? 4000.0 : 0.0) + per * (pieces == 2 ? d.stage2 : d.stage1) + d.epilogue / s) + (s > 1 ? 2500.0 : 0.0);
+      const double waves = (double)((tiles + room - 1) / room), stage = (bits == 4 ? d.stage4 : d.stage8) * (pieces == 2 ? 1.0 : 0.8);
+      const double t = 4.0 + waves * (per * stage + 1.0 + (s > 1 ? d.split : 0.0));
       if (t < best_t) { best_t = t; best = {d.cb, d.nt, s}; }
     }
   }
@@ -718,7 +718,7 @@ int ruai_gemm_tc_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x
   const uint32_t groups = (w->k + 31) / 32, stages = (groups + 1) / 2;
   // fp16 and bf16 activations are one fp16 piece (bf16: after the row's scaling); not when a norm multiplies them
   const int pieces = x_dtype == RUAI_F32 || pro.norm_w ? 2 : 1;
-  Shape sh = choose(c, m, w->n, stages, pieces);
+  Shape sh = choose(c, m, w->n, stages, w->bits, pieces);
   if (c->force_splits >= 1 && c->force_splits <= 8) {
     sh.splits = c->force_splits;
     while (sh.splits > 1 && (sh.splits - 1) * ((stages + sh.splits - 1) / sh.splits) >= stages) --sh.splits;
