@@ -6,10 +6,9 @@
 //       y = y + (x @ A @ B) * scale    (A [k, r], B [r, n], scale = alpha / r)
 //       y = y + bias
 //   Backward of Tensor::matmul_int8 / matmul_int4 (src/nn/ops.rs:705-709, 731-734): the weights are frozen, the
-//   only gradient is dx = g @ dequant(W)^T.  The reference materialises the f32 [k, n] weight for it; here the
-//   packed weight is read once per row of g and dequantised in registers.
-// These are training-side kernels (a handful of rows, run once per step), written for correctness and coalesced
-// reads, not tuned like the decode path.
+//   only gradient is dx = g @ dequant(W)^T.  The reference materialises the f32 [k, n] weight for it; here tiles of
+//   the packed weight are dequantised in shared memory.
+// All in f32.
 #include "common.cuh"
 
 namespace {
@@ -28,7 +27,8 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return t;
 }
 
-// dx[i, rows of chunk c] = sum_j g[i, j] * scale * q[row, j]; chunk layout (pack.cu).  grid (chunks, m).
+// dx[i, rows of chunk c] = sum_j g[i, j] * scale * q[row, j]; chunk layout (pack.cu): few rows, each reading the packed weight
+// once for itself.  grid (chunks, m).
 template <int BITS>
 __global__ void __launch_bounds__(kThreads) grad_input_chunk_kernel(const uint4* __restrict__ w, const float* __restrict__ scale, const float* __restrict__ g,
                                                                     uint32_t k, uint32_t n, float* __restrict__ dx) {
@@ -64,7 +64,131 @@ __global__ void __launch_bounds__(kThreads) grad_input_chunk_kernel(const uint4*
   }
 }
 
-// The same for int4 weights kept in the reference layout (groups other than 32): one packed row (two rows of k)
+// dx[i, r] = sum_j g[i, j] * scale * q[r, j] for the chunk layout (pack.cu): an f32 matrix product on tiles of 64 rows of g x 64 rows of
+// W, 16 columns of W at a time through two shared-memory buffers; W is dequantised once per tile instead of once per row of g.  A thread
+// owns 8 x 4 results; g is kept twice side by side, so that packed multiply-adds (two f32 in one instruction, each rounded like fmaf)
+// need no shuffling: five 16-byte reads from shared memory per 16 of them.  The columns are shared out over gridDim.z CTAs for about
+// four CTAs per SM; the shares are added in a fixed order by sum_shares_kernel.  Bound by f32 multiply-adds and their operands'
+// reads: 256 x 2048 x 2048 int4 114 us (a row of g at a time, as before: 344 us).
+// Up to here a row at a time is faster (us, k x n): 16 rows int4 2048 x 2048 27 against 26, int8 22 against 26; 4096 x 4096 80 and 65
+// against 80; 24 rows 39 and 32 against 28, 116 and 95 against 84.
+constexpr uint32_t kGradFewRows = 18;
+constexpr int kGradTile = 64, kGradCols = 16, kGradThreads = 128, kGradPad = kGradTile + 4;
+
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+template <int BITS>
+__global__ void __launch_bounds__(kGradThreads) grad_input_kernel(const uint4* __restrict__ w, const float* __restrict__ scale, const float* __restrict__ g,
+                                                                  uint32_t m, uint32_t k, uint32_t n, uint32_t chunks, uint32_t cols_per_share, float* __restrict__ out) {
+  constexpr int kChunkRows = BITS == 4 ? 32 : 16, kTileChunks = kGradTile / kChunkRows;
+  constexpr int kLoads = kTileChunks * kGradCols / kGradThreads > 0 ? kTileChunks * kGradCols / kGradThreads : 1;  // chunks per thread and step
+  constexpr uint32_t kGHalf = kGradCols / 2;
+  __shared__ __align__(16) float2 gs[2][kGradCols][kGradTile];
+  __shared__ __align__(16) float ws[2][kGradCols][kGradPad];
+  const uint32_t tid = threadIdx.x, c0 = blockIdx.x * kTileChunks, i0 = blockIdx.y * kGradTile;
+  const uint32_t j_begin = blockIdx.z * cols_per_share, j_end = min(n, j_begin + cols_per_share);
+  const uint32_t wj = tid % kGradCols, wc = tid / kGradCols;  // this thread's column and first chunk of a step
+  const uint32_t gi = tid / 2, gj = (tid % 2) * kGHalf;       // its row of g and the first of its columns
+  uint4 q[kLoads];
+  float sc[kLoads], gv[kGHalf];
+  auto load = [&](uint32_t j0) {
+#pragma unroll
+    for (int l = 0; l < kLoads; ++l) {
+      const uint32_t c = c0 + wc + l * (kGradThreads / kGradCols), j = j0 + wj;
+      const bool in = wc < (uint32_t)kTileChunks && c < chunks && j < j_end;
+      q[l] = in ? __ldg(&w[(size_t)c * n + j]) : make_uint4(0, 0, 0, 0);
+      sc[l] = in ? __ldg(&scale[BITS == 4 ? (size_t)c * n + j : (size_t)j]) : 0.0f;
+    }
+#pragma unroll
+    for (uint32_t t = 0; t < kGHalf; ++t) gv[t] = i0 + gi < m && j0 + gj + t < j_end ? __ldg(&g[(size_t)(i0 + gi) * n + j0 + gj + t]) : 0.0f;
+  };
+  auto store = [&](int b) {
+    if (wc < (uint32_t)kTileChunks) {
+#pragma unroll
+      for (int l = 0; l < kLoads; ++l) {
+        float* dst = &ws[b][wj][(wc + l * (kGradThreads / kGradCols)) * kChunkRows];
+        const uint32_t words[4] = {q[l].x, q[l].y, q[l].z, q[l].w};
+#pragma unroll
+        for (int wi = 0; wi < 4; ++wi) {
+          float lo[4], hi[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const uint32_t byte = (words[wi] >> (8 * t)) & 0xFFu;
+            if (BITS == 4) {  // low nibble: row 4 wi + t, high nibble: row 16 + 4 wi + t, stored value + 8
+              lo[t] = sc[l] * (float)((int)(byte & 0xFu) - 8);
+              hi[t] = sc[l] * (float)((int)(byte >> 4) - 8);
+            } else {
+              lo[t] = sc[l] * (float)(int)(int8_t)byte;
+            }
+          }
+          *reinterpret_cast<float4*>(dst + 4 * wi) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+          if (BITS == 4) *reinterpret_cast<float4*>(dst + 16 + 4 * wi) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+        }
+      }
+    }
+#pragma unroll
+    for (uint32_t t = 0; t < kGHalf; ++t) gs[b][gj + t][gi] = make_float2(gv[t], gv[t]);
+  };
+  const uint32_t tr = (tid / 16) * 8, tk = (tid % 16) * 4;  // this thread's 8 rows of g x 4 rows of W
+  // sums of 32 columns, added up separately: the rounding error grows with the longer of two short chains
+  unsigned long long acc[8][2], sum[8][2];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) { acc[r][0] = acc[r][1] = 0ull; sum[r][0] = sum[r][1] = 0ull; }
+  if (j_begin < j_end) {
+    load(j_begin);
+    store(0);
+  }
+  __syncthreads();
+  int b = 0;
+  for (uint32_t j0 = j_begin; j0 < j_end; j0 += kGradCols, b ^= 1) {
+    const bool more = j0 + kGradCols < j_end;
+    if (more) load(j0 + kGradCols);
+#pragma unroll 8
+    for (int j = 0; j < kGradCols; ++j) {
+      const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(&ws[b][j][tk]);
+#pragma unroll
+      for (int r = 0; r < 8; r += 2) {
+        const ulonglong2 gp = *reinterpret_cast<const ulonglong2*>(&gs[b][j][tr + r]);
+        fma2(acc[r][0], gp.x, wv.x); fma2(acc[r][1], gp.x, wv.y);
+        fma2(acc[r + 1][0], gp.y, wv.x); fma2(acc[r + 1][1], gp.y, wv.y);
+      }
+    }
+    if (b == 1 || !more) {
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[r][t]) : "l"(acc[r][t]));
+          acc[r][t] = 0ull;
+        }
+    }
+    if (more) store(b ^ 1);
+    __syncthreads();
+  }
+  float* dst = out + (size_t)blockIdx.z * m * k;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const uint32_t row = i0 + tr + r;
+    if (row >= m) break;
+#pragma unroll
+    for (uint32_t t = 0; t < 4; ++t) {
+      const uint32_t kk = c0 * kChunkRows + tk + t;
+      if (kk < k) dst[(size_t)row * k + kk] = __uint_as_float((uint32_t)(sum[r][t / 2] >> (32 * (t & 1))));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kThreads) sum_shares_kernel(const float* __restrict__ part, size_t count, uint32_t shares, float* __restrict__ out) {
+  const size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x;
+  if (i >= count) return;
+  float v = part[i];
+  for (uint32_t s = 1; s < shares; ++s) v += part[(size_t)s * count + i];
+  out[i] = v;
+}
+
+// dx for int4 weights kept in the reference layout (groups other than 32): one packed row (two rows of k)
 // per block.  grid (k / 2, m).
 __global__ void __launch_bounds__(kThreads) grad_input_ref4_kernel(const int8_t* __restrict__ q, const float* __restrict__ scale, const float* __restrict__ g,
                                                                    uint32_t k, uint32_t n, uint32_t group, float* __restrict__ dx) {
@@ -83,24 +207,43 @@ __global__ void __launch_bounds__(kThreads) grad_input_ref4_kernel(const int8_t*
   if (threadIdx.x == 0) { dx[(size_t)i * k + 2 * r] = t0; dx[(size_t)i * k + 2 * r + 1] = t1; }
 }
 
-// t[i, r0 .. r0+7] = sum_p x[i, p] * A[p, r]; grid (m, ceil(rank / 8)).
-__global__ void __launch_bounds__(kThreads) lora_xa_kernel(const float* __restrict__ x, const float* __restrict__ a, uint32_t k, uint32_t rank,
+// t[i, r0 .. r0+7] = sum_p x[i, p] * A[p, r] for kXaRows rows of x, which read A once between them; grid (ceil(m / kXaRows), ceil(rank / 8)).
+constexpr int kXaRows = 4;
+__global__ void __launch_bounds__(kThreads) lora_xa_kernel(const float* __restrict__ x, const float* __restrict__ a, uint32_t m, uint32_t k, uint32_t rank,
                                                            float* __restrict__ t) {
-  __shared__ float red[kThreads / 32];
-  const uint32_t i = blockIdx.x, r0 = blockIdx.y * 8;
-  float acc[8];
+  __shared__ float red[kThreads / 32][8 * kXaRows];
+  const uint32_t i0 = blockIdx.x * kXaRows, r0 = blockIdx.y * 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float acc[kXaRows][8];
 #pragma unroll
-  for (int u = 0; u < 8; ++u) acc[u] = 0.0f;
+  for (int i = 0; i < kXaRows; ++i)
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc[i][u] = 0.0f;
   for (uint32_t p = threadIdx.x; p < k; p += kThreads) {
-    const float xv = x[(size_t)i * k + p];
+    float av[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (r0 + u < rank) acc[u] = fmaf(xv, a[(size_t)p * rank + r0 + u], acc[u]);
+    for (uint32_t u = 0; u < 8; ++u) av[u] = r0 + u < rank ? a[(size_t)p * rank + r0 + u] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < kXaRows; ++i) {
+      const float xv = i0 + i < m ? x[(size_t)(i0 + i) * k + p] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc[i][u] = fmaf(xv, av[u], acc[i][u]);
+    }
   }
 #pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const float s = block_sum(acc[u], red);
-    if (threadIdx.x == 0 && r0 + u < rank) t[(size_t)i * rank + r0 + u] = s;
+  for (int i = 0; i < kXaRows; ++i)
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      float v = acc[i][u];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+      if (lane == 0) red[warp][8 * i + u] = v;
+    }
+  __syncthreads();
+  if (threadIdx.x < 8 * kXaRows) {
+    const uint32_t i = i0 + threadIdx.x / 8, r = r0 + threadIdx.x % 8;
+    float v = 0.0f;
+    for (int w = 0; w < kThreads / 32; ++w) v += red[w][threadIdx.x];  // fixed order
+    if (i < m && r < rank) t[(size_t)i * rank + r] = v;
   }
 }
 
@@ -125,9 +268,33 @@ RUAI_API int ruai_matmul_q_grad_input(ruai_ctx* c, const float* g_dev, const rua
   if (m > 65535u) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "ruai_matmul_q_grad_input: %u rows exceed 65535", m);
   DeviceGuard g(c->ordinal);
   if (w->layout == QL_CHUNK16) {
-    const dim3 grid(w->chunks, m);
-    if (w->bits == 4) grad_input_chunk_kernel<4><<<grid, kThreads, 0, c->stream>>>((const uint4*)w->data, w->scale, g_dev, w->k, w->n, dx_dev);
-    else grad_input_chunk_kernel<8><<<grid, kThreads, 0, c->stream>>>((const uint4*)w->data, w->scale, g_dev, w->k, w->n, dx_dev);
+    if (m <= kGradFewRows) {
+      const dim3 grid(w->chunks, m);
+      if (w->bits == 4) grad_input_chunk_kernel<4><<<grid, kThreads, 0, c->stream>>>((const uint4*)w->data, w->scale, g_dev, w->k, w->n, dx_dev);
+      else grad_input_chunk_kernel<8><<<grid, kThreads, 0, c->stream>>>((const uint4*)w->data, w->scale, g_dev, w->k, w->n, dx_dev);
+      RUAI_CUDA(c, cudaGetLastError());
+      return RUAI_OK;
+    }
+    const uint32_t row_tiles = (m + kGradTile - 1) / kGradTile, k_tiles = (w->k + kGradTile - 1) / kGradTile, steps = (w->n + kGradCols - 1) / kGradCols;
+    // about four CTAs per SM, four steps at least for each
+    uint32_t shares = 4u * (uint32_t)c->sm_count / (row_tiles * k_tiles);
+    if (shares > steps / 4) shares = steps / 4;
+    if (shares < 1) shares = 1;
+    const uint32_t cols = (steps + shares - 1) / shares * kGradCols;
+    shares = (w->n + cols - 1) / cols;
+    float* dst = dx_dev;
+    if (shares > 1) {
+      RUAI_TRY(ruai_ctx_reserve(c, (size_t)shares * m * w->k * sizeof(float), 0));
+      dst = c->partial;
+    }
+    const dim3 grid(k_tiles, row_tiles, shares);
+    if (w->bits == 4) grad_input_kernel<4><<<grid, kGradThreads, 0, c->stream>>>((const uint4*)w->data, w->scale, g_dev, m, w->k, w->n, w->chunks, cols, dst);
+    else grad_input_kernel<8><<<grid, kGradThreads, 0, c->stream>>>((const uint4*)w->data, w->scale, g_dev, m, w->k, w->n, w->chunks, cols, dst);
+    if (shares > 1) {
+      RUAI_CUDA(c, cudaGetLastError());
+      const size_t count = (size_t)m * w->k;
+      sum_shares_kernel<<<(unsigned)((count + kThreads - 1) / kThreads), kThreads, 0, c->stream>>>(dst, count, shares, dx_dev);
+    }
   } else {
     if (w->k / 2 > 65535u * 32768u) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "k too large");
     grad_input_ref4_kernel<<<dim3(w->k / 2, m), kThreads, 0, c->stream>>>((const int8_t*)w->data, w->scale, g_dev, w->k, w->n, w->group, dx_dev);
@@ -147,7 +314,7 @@ RUAI_API int ruai_linear_lora_forward(ruai_ctx* c, const float* x_dev, const rua
   RUAI_TRY(ruai_matmul_q(c, RUAI_F32, x_dev, w, nullptr, out_dev, m));
   RUAI_TRY(ruai_ctx_reserve(c, (size_t)m * rank * sizeof(float), 0));
   float* t = c->partial;
-  lora_xa_kernel<<<dim3(m, (rank + 7) / 8), kThreads, 0, c->stream>>>(x_dev, lora_a_dev, w->k, rank, t);
+  lora_xa_kernel<<<dim3((m + kXaRows - 1) / kXaRows, (rank + 7) / 8), kThreads, 0, c->stream>>>(x_dev, lora_a_dev, m, w->k, rank, t);
   RUAI_CUDA(c, cudaGetLastError());
   lora_add_kernel<<<dim3((w->n + 255) / 256, m), 256, 0, c->stream>>>(out_dev, t, lora_b_dev, bias_dev_or_null, w->n, rank, scale);
   RUAI_CUDA(c, cudaGetLastError());

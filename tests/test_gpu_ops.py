@@ -384,3 +384,39 @@ def test_lora_forward_matches_checker(dev, m, k, n, rank, bits):
     zero = np.zeros((rank, n), np.float32)
     got = nn.linear_lora_forward(T(x), qw, T(a), T(zero), scale).numpy()
     assert np.array_equal(got, nn._matmul_q(T(x), qw).numpy())
+
+
+# ---- the GEMM's tiles: edges of rows, columns and k, every split of k ----
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("m,k,n", [(17, 64, 128), (64, 96, 132), (65, 4160, 300), (128, 2016, 256), (129, 544, 516), (300, 1504, 1500), (513, 224, 2564)])
+def test_gemm_tiles_against_float64(dev, m, k, n, bits):
+    """Both fp16 pieces of x carry 22 bits, sums are f32: errors below 2^-20 of the sum of the products' magnitudes."""
+    if bits == 8:
+        k -= 7  # a ragged last chunk
+    q, s, qw = _qw(dev, bits, k, n, 31)
+    wd = q.astype(np.float64) * s if bits == 8 else qw.dequant().astype(np.float64)
+    x = oracle.synth_normal(31, m, (m, k), 1.0) * np.exp2(np.arange(m) % 40 - 20).astype(np.float32)[:, None]  # rows of very different size
+    want, mag = x.astype(np.float64) @ wd, np.abs(x).astype(np.float64) @ np.abs(wd)
+    xt = nn.Tensor.from_numpy(dev, x)
+    try:
+        for splits in (0, 1, 2, 3, 5, 7, 8):
+            dev.force_splits(splits)
+            got = nn._matmul_q(xt, qw).numpy().astype(np.float64)
+            assert (np.abs(got - want) <= 2.0 ** -20 * mag + 1e-30).all(), (splits, (np.abs(got - want) / mag).max())
+    finally:
+        dev.force_splits(0)
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("m,k,n", [(7, 32, 16), (18, 64, 40), (19, 96, 17), (63, 96, 17), (65, 160, 300), (200, 2048, 1000)])
+def test_grad_input_tiles_against_float64(dev, m, k, n, bits):
+    """f32 sums of n terms, each rounded three times: errors below (n + 3) 2^-24 of the sum of the magnitudes."""
+    if bits == 8:
+        k -= 5
+    q, s, qw = _qw(dev, bits, k, n, 32)
+    wd = q.astype(np.float64) * s if bits == 8 else qw.dequant().astype(np.float64)
+    g = oracle.synth_normal(32, m, (m, n), 1.0)
+    want, mag = g.astype(np.float64) @ wd.T, np.abs(g).astype(np.float64) @ np.abs(wd).T
+    got = nn.matmul_q_grad_input(nn.Tensor.from_numpy(dev, g), qw).numpy().astype(np.float64)
+    assert (np.abs(got - want) <= (n + 3) * 2.0 ** -24 * mag + 1e-30).all()
