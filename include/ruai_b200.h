@@ -82,7 +82,8 @@ int ruai_ctx_inject_copy_shortfall(ruai_ctx* ctx, unsigned bytes);
  * on a list of shapes.  No counterpart in the reference. */
 int ruai_ctx_force_splits(ruai_ctx* ctx, unsigned splits);
 
-/* Device memory for callers without their own allocator (cuda.rs:288-300). */
+/* Device memory for callers without their own allocator (cuda.rs:288-300).  Blocks given back are kept for later calls (512 MB a device
+ * at most) and given out again when no stream of the device can still use them; memory of ruai_malloc goes back through ruai_free. */
 int ruai_malloc(ruai_ctx* ctx, size_t bytes, void** out_dev);
 int ruai_free(ruai_ctx* ctx, void* ptr_dev);
 int ruai_memcpy_h2d(ruai_ctx* ctx, void* dst_dev, const void* src_host, size_t bytes);

@@ -98,6 +98,9 @@ struct DeviceGuard {
   }
 };
 
+// cudaMalloc that gives the blocks kept by ruai_free back before it fails.
+cudaError_t ruai_device_malloc(void** out, size_t bytes);
+
 // Grows the split-K scratch when a launch needs more (never inside a graph capture).
 int ruai_ctx_reserve(ruai_ctx* ctx, size_t partial_bytes, size_t counters);
 

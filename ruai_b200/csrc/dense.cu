@@ -618,7 +618,7 @@ int ruai_dense_alloc(ruai_ctx* c, uint32_t n, uint32_t k, uint32_t bits, ruai_qw
   w->ctx = c; w->k = k; w->n = n; w->bits = bits; w->layout = QL_DENSE;
   w->ld = (k + 7) & ~7u;
   w->data_bytes = (size_t)n * w->ld * (bits / 8);
-  cudaError_t e = cudaMalloc(&w->data, w->data_bytes);
+  cudaError_t e = ruai_device_malloc((void**)&w->data, w->data_bytes);
   if (e == cudaSuccess) e = cudaMemsetAsync(w->data, 0, w->data_bytes, c->stream);
   if (e != cudaSuccess) {
     if (w->data) cudaFree(w->data);
@@ -752,7 +752,7 @@ RUAI_API int ruai_pack_dense(ruai_ctx* c, const float* w, uint32_t n, uint32_t k
   RUAI_TRY(ruai_dense_alloc(c, n, k, bits, &q));
   float* tmp = nullptr;
   int rc = RUAI_OK;
-  cudaError_t e = cudaMalloc(&tmp, (size_t)n * k * sizeof(float));
+  cudaError_t e = ruai_device_malloc((void**)&tmp, (size_t)n * k * sizeof(float));
   if (e == cudaSuccess) e = cudaMemcpyAsync(tmp, w, (size_t)n * k * sizeof(float), cudaMemcpyDefault, c->stream);
   if (e == cudaSuccess) rc = ruai_dense_put(c, q, tmp, n, k, 0, 1, 0);
   if (e == cudaSuccess && rc == RUAI_OK) e = cudaStreamSynchronize(c->stream);

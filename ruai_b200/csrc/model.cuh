@@ -12,7 +12,7 @@ struct DevBuf {
   size_t bytes = 0;
   int alloc(ruai_ctx* c, size_t n) {
     release();
-    RUAI_CUDA(c, cudaMalloc(&p, n ? n : 1));
+    RUAI_CUDA(c, ruai_device_malloc((void**)&p, n ? n : 1));
     bytes = n;
     return RUAI_OK;
   }

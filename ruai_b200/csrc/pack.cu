@@ -108,7 +108,7 @@ bool is_device_ptr(const void* p) {
 int stage_in(ruai_ctx* c, const void* src, size_t bytes, void** dev, bool* owned) {
   if (is_device_ptr(src)) { *dev = const_cast<void*>(src); *owned = false; return RUAI_OK; }
   *owned = true;
-  RUAI_CUDA(c, cudaMalloc(dev, bytes ? bytes : 1));
+  RUAI_CUDA(c, ruai_device_malloc((void**)dev, bytes ? bytes : 1));
   RUAI_CUDA(c, cudaMemcpyAsync(*dev, src, bytes, cudaMemcpyHostToDevice, c->stream));
   return RUAI_OK;
 }
@@ -146,7 +146,7 @@ static int make_qweight(ruai_ctx* c, const int8_t* q, const float* scale, uint32
   };
   if ((rc = stage_in(c, q, q_bytes, &qd, &qo)) != RUAI_OK) return fail(rc);
   if ((rc = stage_in(c, scale, w->scale_bytes, &sd, &so)) != RUAI_OK) return fail(rc);
-  if (cudaMalloc(&w->data, w->data_bytes) != cudaSuccess || cudaMalloc(&w->scale, w->scale_bytes) != cudaSuccess)
+  if (ruai_device_malloc((void**)&w->data, w->data_bytes) != cudaSuccess || ruai_device_malloc((void**)&w->scale, w->scale_bytes) != cudaSuccess)
     return fail(ruai_fail(c, RUAI_ERR_CUDA, "repack: out of device memory (%zu bytes)", w->data_bytes + w->scale_bytes));
   cudaMemcpyAsync(w->scale, sd, w->scale_bytes, cudaMemcpyDeviceToDevice, c->stream);
   dim3 grid((n + 127) / 128, w->chunks ? w->chunks : 1);
@@ -198,7 +198,7 @@ RUAI_API int ruai_unpack(ruai_ctx* c, const ruai_qweight* w, int8_t* q_out, floa
   const size_t q_bytes = w->bits == 8 ? (size_t)w->k * w->n : (size_t)(w->k / 2) * w->n;
   const bool q_dev = is_device_ptr(q_out), s_dev = is_device_ptr(scale_out);
   int8_t* qd = q_out;
-  if (!q_dev) RUAI_CUDA(c, cudaMalloc(&qd, q_bytes));
+  if (!q_dev) RUAI_CUDA(c, ruai_device_malloc((void**)&qd, q_bytes));
   dim3 grid((w->n + 127) / 128, w->chunks ? w->chunks : 1);
   if (w->layout == QL_REFERENCE) cudaMemcpyAsync(qd, w->data, q_bytes, cudaMemcpyDeviceToDevice, c->stream);
   else if (w->bits == 8) unpack8_kernel<<<grid, 128, 0, c->stream>>>((const uint4*)w->data, w->k, w->n, qd);

@@ -105,7 +105,7 @@ int ruai_sample_device(ruai_ctx* c, const float* logits_dev, uint32_t vocab, flo
     cudaFree(c->sample_buf);
     c->sample_buf = nullptr;
     c->sample_bytes = 0;
-    RUAI_CUDA(c, cudaMalloc(&c->sample_buf, need));
+    RUAI_CUDA(c, ruai_device_malloc((void**)&c->sample_buf, need));
     c->sample_bytes = need;
   }
   unsigned char* base = static_cast<unsigned char*>(c->sample_buf);

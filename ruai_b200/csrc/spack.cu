@@ -43,7 +43,7 @@ int ruai_sweight_create(ruai_ctx* c, const ruai_qweight* w, ruai_sweight* out) {
   out->bytes = (size_t)out->ntiles * out->nblk * out->rec_bytes;
   out->colscale = w->bits == 8 ? w->scale : nullptr;
   if (out->nblk > 65535u || out->ntiles > 65535u) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "weight [%u, %u] is too large for the tile-stream layout", w->k, w->n);
-  RUAI_CUDA(c, cudaMalloc(&out->data, out->bytes));
+  RUAI_CUDA(c, ruai_device_malloc((void**)&out->data, out->bytes));
   const dim3 grid(out->nblk, out->ntiles);
   if (w->bits == 4) stream4_kernel<<<grid, kStreamTileCols, 0, c->stream>>>((const uint4*)w->data, w->scale, w->n, out->nblk, out->data);
   else stream8_kernel<<<grid, kStreamTileCols, 0, c->stream>>>((const uint4*)w->data, w->n, w->chunks, out->nblk, out->data);

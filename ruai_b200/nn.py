@@ -9,6 +9,7 @@ gpt2.rs).  Every computation is a call into libruai_b200.so through its C ABI;
 nothing here computes on the host.
 """
 import ctypes as C
+import math
 
 import numpy as np
 
@@ -73,7 +74,7 @@ class Tensor:
 
     def __init__(self, dev, shape, np_dtype, rdtype=None):
         self.dev, self.shape, self.np_dtype, self.rdtype = dev, tuple(int(s) for s in shape), np.dtype(np_dtype), rdtype
-        self.nbytes = int(np.prod(self.shape, dtype=np.int64)) * self.np_dtype.itemsize
+        self.nbytes = math.prod(self.shape) * self.np_dtype.itemsize
         p = C.c_void_p()
         dev.check(dev.L.ruai_malloc(dev.ctx, self.nbytes, C.byref(p)))
         self.ptr = p
@@ -188,7 +189,7 @@ def _matmul_q(x, w, bias=None):
         raise TypeError("matmul_int8/int4: activations must be a float tensor")
     if x.shape[-1] != w.k:
         raise ValueError(f"inner dims differ ({x.shape} @ int{w.bits} [{w.k}, {w.n}])")
-    m = int(np.prod(x.shape[:-1], dtype=np.int64))
+    m = math.prod(x.shape[:-1])
     out = Tensor(x.dev, x.shape[:-1] + (w.n,), x.np_dtype, x.rdtype)
     x.dev.check(x.dev.L.ruai_matmul_q(x.dev.ctx, x.rdtype, x.ptr, w.h, bias.ptr if bias is not None else None, out.ptr, m))
     return out
@@ -198,7 +199,7 @@ def matmul_q_grad_input(g, w):
     """Gradient of `matmul_int8` / `matmul_int4` with respect to the activations (ops.rs:705-709, 731-734): g @ dequant(W)^T."""
     if g.rdtype != F32 or g.shape[-1] != w.n:
         raise ValueError(f"gradient must be f32 [..., {w.n}]")
-    m = int(np.prod(g.shape[:-1], dtype=np.int64))
+    m = math.prod(g.shape[:-1])
     out = Tensor(g.dev, g.shape[:-1] + (w.k,), np.float32, F32)
     g.dev.check(g.dev.L.ruai_matmul_q_grad_input(g.dev.ctx, g.ptr, w.h, out.ptr, m))
     return out
@@ -211,7 +212,7 @@ def linear_lora_forward(x, w, lora_a, lora_b, scale, bias=None):
     rank = lora_a.shape[1]
     if lora_a.shape != (w.k, rank) or lora_b.shape != (rank, w.n):
         raise ValueError("lora_a must be [k, rank] and lora_b [rank, n]")
-    m = int(np.prod(x.shape[:-1], dtype=np.int64))
+    m = math.prod(x.shape[:-1])
     out = Tensor(x.dev, x.shape[:-1] + (w.n,), np.float32, F32)
     x.dev.check(x.dev.L.ruai_linear_lora_forward(x.dev.ctx, x.ptr, w.h, lora_a.ptr, lora_b.ptr, rank, float(scale),
                                                  bias.ptr if bias is not None else None, out.ptr, m))
@@ -240,7 +241,7 @@ def matmul_q_stream(x, w, repeat=1):
         raise TypeError("matmul_q_stream: activations must be f32")
     if x.shape[-1] != w.k:
         raise ValueError(f"inner dims differ ({x.shape} @ int{w.bits} [{w.k}, {w.n}])")
-    m = int(np.prod(x.shape[:-1], dtype=np.int64))
+    m = math.prod(x.shape[:-1])
     out = Tensor(x.dev, x.shape[:-1] + (w.n,), np.float32, F32)
     x.dev.check(x.dev.L.ruai_matmul_q_stream(x.dev.ctx, x.ptr, w.h, out.ptr, m, repeat))
     return out

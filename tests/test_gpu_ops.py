@@ -420,3 +420,15 @@ def test_grad_input_tiles_against_float64(dev, m, k, n, bits):
     want, mag = g.astype(np.float64) @ wd.T, np.abs(g).astype(np.float64) @ np.abs(wd).T
     got = nn.matmul_q_grad_input(nn.Tensor.from_numpy(dev, g), qw).numpy().astype(np.float64)
     assert (np.abs(got - want) <= (n + 3) * 2.0 ** -24 * mag + 1e-30).all()
+
+
+def test_freed_tensors_are_reused_only_after_a_wait(dev):
+    """Blocks freed while their context's stream still works on them do not come back before that work is done."""
+    q, s, qw = _qw(dev, 8, 2048, 2048, 33)
+    xs = [nn.Tensor.from_numpy(dev, oracle.synth_normal(33, i, (256, 2048), 1.0)) for i in range(3)]
+    want = [nn._matmul_q(x, qw).numpy() for x in xs]
+    for r in range(120):  # results are dropped while queued, so that their memory goes round several times
+        i = r % 3
+        for j in range(3):
+            nn._matmul_q(xs[j], qw)
+        assert np.array_equal(nn._matmul_q(xs[i], qw).numpy(), want[i])
