@@ -19,6 +19,7 @@
 // leave that tile's grid small (64 x 2048 x 2048 int8: 41 us before, 20 CTAs; 11 now).
 // Every mbarrier wait is bounded.
 #include "common.cuh"
+#include "gemm_tile.cuh"
 #include "gemv_epilogue.cuh"
 #include "pipeline.cuh"
 
@@ -170,41 +171,6 @@ struct Params {
   void* out;
   int* status;
   GemvEpilogue epi;
-};
-
-// CB column blocks of 128 x NT rows of x per CTA.  Warps: 0 copies W, 1 and 2 issue MMAs, 3 copies x, then, with one column block,
-// four that expand and four per 64 rows that drain; with two, sixteen that do both (96 registers for twenty warps are what the
-// register file holds).  The A operand lies in tensor memory: from shared memory its reads, the writes of the expanding warps and the
-// copies together took more than the 128 bytes per clock there are (measured: a stage's MMAs 1,900 clocks instead of 1,024).  Shared
-// memory: a ring of packed stages (the scales of int4 in one of their own) and a ring of stages of x.
-template <int BITS, int CB, int NT>
-struct Tile {
-  static constexpr int kCols = CB * 128;
-  static constexpr int kDrains = CB * NT / 64;                           // draining warpgroups
-  static constexpr bool kBoth = CB == 2;                                 // the draining warps expand as well
-  static constexpr int kDrain0 = kBoth ? 4 : 8;                          // first draining warp
-  static constexpr int kExpanders = kBoth ? 4 * kDrains : 4;             // warps
-  static constexpr int kThreads = 32 * kDrain0 + 128 * kDrains;
-  static constexpr uint32_t kWChunk = kCols * 16;                        // one 16-byte chunk of every column
-  static constexpr int kChunks = BITS == 4 ? 2 : 4;                      // chunks per stage
-  static constexpr uint32_t kWBytes = kChunks * kWChunk;
-  static constexpr int kWSlots = CB == 2 ? 4 : 6;
-  static constexpr uint32_t kPiece = NT * 128;                           // one piece of x of a stage
-  static constexpr uint32_t kX = 2 * kPiece;                             // both
-  // Tensor memory: three buffers of sums, then the A operand, 32 words per column block and stage.
-  static constexpr uint32_t kACol0 = 3 * NT;
-  static constexpr int kABufs = 4 / CB;
-  static constexpr uint32_t kTmem = 512;
-  static constexpr uint32_t kScale = BITS == 4 ? 2 * kCols * 4 : 0;      // scales of a stage
-  static constexpr int kScaleSlots = kWSlots + kABufs + 2;               // see the copies
-  static constexpr uint32_t kFixed = kWSlots * kWBytes + kScaleSlots * kScale;
-  static constexpr int kFit = (int)((230400 - 1024 - kFixed) / kX);
-  static constexpr int kXSlots = kFit < 8 ? kFit : 8;
-  static constexpr uint32_t off_w = kXSlots * kX, off_scale = off_w + kWSlots * kWBytes;
-  static constexpr size_t kRed = (size_t)(NT + 8) * kCols * 4;           // split k: partial sums of this CTA's rows
-  static constexpr size_t kRing = (size_t)kFixed + (size_t)kXSlots * kX;
-  static constexpr size_t kSmem = 1024 + (kRing > kRed ? kRing : kRed);
-  static_assert(kXSlots >= 3, "ring too short");
 };
 
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {  // K-major, 128-byte swizzle, 1024 bytes between 8-row blocks
@@ -418,9 +384,7 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
           if (it >= WS && (s_abort || !mbar_wait(&w_empty[slot], (it / WS - 1u) & 1u))) { s_abort = 1; ok = false; break; }
           const uint32_t c0 = s * T::kChunks, chunks = min((uint32_t)T::kChunks, p.chunks - c0);
           unsigned char* dst = smem + T::off_w + slot * T::kWBytes;
-          // int4: a chunk is a scale group.  The scales' slot is free: this packed slot is, so stage it - kWSlots is expanded, so the
-          // MMAs of stage it - kWSlots - kABufs are done, and those waited for the read-out of all but the last three units up to
-          // theirs: every stage up to it - kWSlots - kABufs - 2 has been read out (a tile's last stage may be one group).
+          // int4: a chunk is a scale group.  That the scales' slot is free as well: see Tile::kScaleSlots.
           mbar_expect_tx(&w_full[slot], chunks * nc * (BITS == 4 ? 20u : 16u));
           for (uint32_t c = 0; c < chunks; ++c) {
             bulk_load(dst + c * T::kWChunk, p.w + (size_t)(c0 + c) * p.n + j0, nc * 16u, &w_full[slot]);

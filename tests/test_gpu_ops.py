@@ -408,6 +408,18 @@ def test_gemm_tiles_against_float64(dev, m, k, n, bits):
         dev.force_splits(0)
 
 
+@pytest.mark.parametrize("m,n", [(88320, 384), (88320, 300)])
+def test_gemm_of_one_group_over_many_tiles(dev, m, n):
+    """k of one scale group and a dozen column blocks per CTA: the scales' ring goes round with one group per stage."""
+    q, s, qw = _qw(dev, 4, 32, n, 34)
+    x = oracle.synth_normal(34, 1, (m, 32), 1.0)
+    got = nn._matmul_q(nn.Tensor.from_numpy(dev, x), qw).numpy()
+    rows = np.r_[0:m:37, m - 1]
+    wd = qw.dequant().astype(np.float64)
+    want, mag = x[rows].astype(np.float64) @ wd, np.abs(x[rows]).astype(np.float64) @ np.abs(wd)
+    assert (np.abs(got[rows] - want) <= 2.0 ** -20 * mag + 1e-30).all()
+
+
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("m,k,n", [(7, 32, 16), (18, 64, 40), (19, 96, 17), (63, 96, 17), (65, 160, 300), (200, 2048, 1000)])
 def test_grad_input_tiles_against_float64(dev, m, k, n, bits):
