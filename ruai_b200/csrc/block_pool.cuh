@@ -1,0 +1,185 @@
+// Device memory of ruai_malloc / ruai_free (ctx.cu): blocks given back are kept for later requests of their size.  Host code that needs
+// nothing but the CUDA runtime's interface, so that it can be run against a stand-in for it.
+//
+// A program makes a tensor per call and drops it soon after; cudaMalloc and cudaFree between launches cost more than most Linears
+// (int8 2048 x 2048, one row: 7 us on the device of 25 a call; 4096 x 14336 results: 0.9 ms of mapping and unmapping).  Freed blocks
+// are kept for the next request of their size class.  cudaFree waits for the device, so a block may be freed while a kernel on ANY
+// stream still uses it; here it is set aside, and given out only after its context's stream and then the device have been waited for,
+// once for all the blocks set aside until then, when so many of the wanted class lie waiting that it pays.
+// At most kKeptBytes are kept per device; they are given back when memory runs short and with the device's last context.
+#pragma once
+#include <cuda_runtime_api.h>
+
+#include <cstddef>
+#include <list>
+#include <map>
+#include <mutex>
+#include <unordered_map>
+
+namespace block_pool {
+
+constexpr size_t kKeptBytes = 512ull << 20;
+constexpr int kDevices = 64;
+
+using Blocks = std::map<size_t, std::list<void*>>;  // by size class
+
+struct Pool {  // of a device
+  std::unordered_map<void*, size_t> live;  // blocks handed out, by size class
+  Blocks clean;                            // nothing on the device uses them
+  std::map<const void*, Blocks> aside;     // freed through a context since its last device-wide wait
+  size_t bytes = 0;                        // in clean and aside
+  int contexts = 0;
+};
+struct State {
+  std::mutex lock;  // held for bookkeeping, not for a wait or a call that maps or unmaps memory
+  Pool device[kDevices];
+};
+inline State& state() {
+  static State* s = new State;  // never destroyed: the driver may be gone before static destructors run
+  return *s;
+}
+using Lock = std::lock_guard<std::mutex>;
+inline Pool& of(int ordinal) { return state().device[ordinal]; }
+inline bool pooled(int ordinal) { return ordinal >= 0 && ordinal < kDevices; }
+
+inline size_t size_class(size_t bytes) {
+  if (bytes > (1ull << 20)) return (bytes + (2ull << 20) - 1) / (2ull << 20) * (2ull << 20);
+  size_t c = 512;
+  while (c < bytes) c *= 2;
+  return c;
+}
+
+inline void merge(Blocks& to, Blocks& from) {
+  for (auto& kv : from) to[kv.first].splice(to[kv.first].end(), kv.second);
+  from.clear();
+}
+
+// Waits for the context's stream and the device and makes the blocks set aside through the context before that clean.  The wait is
+// cudaFree's, which other threads' captures allow as they allow any cudaFree.
+inline bool settle(Pool& p, const void* context, cudaStream_t stream) {
+  Blocks moved;
+  {
+    Lock l(state().lock);
+    moved.swap(p.aside[context]);
+  }
+  void* dummy = nullptr;
+  const bool ok = cudaStreamSynchronize(stream) == cudaSuccess && cudaMalloc(&dummy, 512) == cudaSuccess && cudaFree(dummy) == cudaSuccess;
+  if (!ok) (void)cudaGetLastError();
+  Lock l(state().lock);
+  merge(ok ? p.clean : p.aside[context], moved);
+  return ok;
+}
+
+inline void trim(Pool& p) {
+  Blocks out;
+  {
+    Lock l(state().lock);
+    merge(out, p.clean);
+    for (auto& kv : p.aside) merge(out, kv.second);
+    p.bytes = 0;
+  }
+  for (auto& kv : out)
+    for (void* q : kv.second) cudaFree(q);  // waits for the device
+}
+
+inline void* take(Pool& p, size_t cls) {
+  Lock l(state().lock);
+  auto it = p.clean.find(cls);
+  if (it == p.clean.end() || it->second.empty()) return nullptr;
+  void* q = it->second.back();
+  it->second.pop_back();
+  p.bytes -= cls;
+  p.live[q] = cls;
+  return q;
+}
+
+// A context of the device more; the device's last one to go gives the kept memory back, and each what was set aside through it.
+inline void attach(const void*, int ordinal, cudaStream_t) {
+  if (!pooled(ordinal)) return;
+  Lock l(state().lock);
+  ++of(ordinal).contexts;
+}
+inline void detach(const void* context, int ordinal) {
+  if (!pooled(ordinal)) return;
+  Pool& p = of(ordinal);
+  Blocks out;
+  bool last;
+  {
+    Lock l(state().lock);
+    out.swap(p.aside[context]);
+    p.aside.erase(context);
+    for (auto& kv : out) p.bytes -= kv.first * kv.second.size();
+    last = --p.contexts == 0;
+  }
+  for (auto& kv : out)
+    for (void* q : kv.second) cudaFree(q);
+  if (last) trim(p);
+}
+
+// cudaMalloc on the current device that gives the kept blocks back before it reports that memory has run out.
+inline cudaError_t device_malloc(void** out, size_t bytes) {
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  int ordinal = 0;
+  if (cudaGetDevice(&ordinal) != cudaSuccess || !pooled(ordinal)) return e;
+  Pool& p = of(ordinal);
+  {
+    Lock l(state().lock);
+    if (p.bytes == 0) return e;
+  }
+  (void)cudaGetLastError();
+  trim(p);
+  return cudaMalloc(out, bytes);
+}
+
+// A block for a context on its stream; the device is current.
+inline cudaError_t allocate(const void* context, int ordinal, cudaStream_t stream, size_t bytes, void** out) {
+  if (!pooled(ordinal) || bytes > kKeptBytes / 2) return device_malloc(out, bytes ? bytes : 1);
+  Pool& p = of(ordinal);
+  const size_t cls = size_class(bytes);
+  if ((*out = take(p, cls)) != nullptr) return cudaSuccess;
+  size_t waiting = 0;
+  {
+    Lock l(state().lock);
+    auto& mine = p.aside[context];
+    auto it = mine.find(cls);
+    if (it != mine.end()) waiting = it->second.size();
+  }
+  // Until then new ones are mapped, which costs hundreds of microseconds for a large block: two of those do.
+  if (waiting >= 32 || (waiting * cls >= (4ull << 20) && (waiting >= 2 || cls >= (64ull << 20)))) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) (void)cudaGetLastError();
+    if (st == cudaStreamCaptureStatusNone && settle(p, context, stream) && (*out = take(p, cls)) != nullptr) return cudaSuccess;
+  }
+  const cudaError_t e = device_malloc(out, cls);
+  if (e != cudaSuccess) return e;
+  Lock l(state().lock);
+  p.live[*out] = cls;
+  return cudaSuccess;
+}
+
+// Frees a block on behalf of a context, whose device is current.
+inline cudaError_t give_back(const void* context, int ordinal, cudaStream_t stream, void* q) {
+  bool kept = false, full = false;
+  if (q && pooled(ordinal)) {
+    Pool& p = of(ordinal);
+    Lock l(state().lock);
+    auto it = p.live.find(q);
+    if (it != p.live.end()) {
+      const size_t cls = it->second;
+      p.live.erase(it);
+      p.aside[context][cls].push_back(q);
+      p.bytes += cls;
+      full = p.bytes > kKeptBytes;
+      kept = true;
+    }
+  }
+  if (kept) {
+    if (full) trim(of(ordinal));  // of sizes no longer asked for, most of it
+    return cudaSuccess;
+  }
+  const cudaError_t e = cudaStreamSynchronize(stream);
+  return e != cudaSuccess ? e : cudaFree(q);
+}
+
+}  // namespace block_pool

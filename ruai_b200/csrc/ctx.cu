@@ -1,11 +1,8 @@
 // Context, device memory and timing entry points.
 #include <cstdlib>
 #include <cstring>
-#include <map>
-#include <mutex>
-#include <unordered_map>
-#include <vector>
 
+#include "block_pool.cuh"
 #include "common.cuh"
 
 thread_local std::string g_ruai_global_err;
@@ -20,9 +17,6 @@ int ruai_fail(ruai_ctx* ctx, int code, const char* fmt, ...) {
   g_ruai_global_err = buf;
   return code;
 }
-
-static void ruai_pool_forget(ruai_ctx* c);
-static void ruai_pool_contexts(int ordinal, int change);  // the device's last context gives the kept memory back
 
 RUAI_API const char* ruai_version(void) { return "ruai_b200 0.1 (sm_100a)"; }
 
@@ -71,7 +65,7 @@ RUAI_API int ruai_ctx_create(int ordinal, void* stream_or_null, ruai_ctx** out) 
   }
   int rc = ruai_ctx_reserve(c, 8u << 20, 4096);
   if (rc != RUAI_OK) { g_ruai_global_err = c->err; delete c; return rc; }
-  ruai_pool_contexts(ordinal, 1);
+  block_pool::attach(c, ordinal, c->stream);
   *out = c;
   return RUAI_OK;
 }
@@ -80,7 +74,6 @@ RUAI_API int ruai_ctx_destroy(ruai_ctx* c) {
   if (!c) return RUAI_OK;
   DeviceGuard g(c->ordinal);
   cudaStreamSynchronize(c->stream);
-  ruai_pool_forget(c);
   cudaFree(c->partial);
   cudaFree(c->counters);
   cudaFree(c->status);
@@ -89,7 +82,7 @@ RUAI_API int ruai_ctx_destroy(ruai_ctx* c) {
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
   if (c->own_stream) cudaStreamDestroy(c->stream);
-  ruai_pool_contexts(c->ordinal, -1);
+  block_pool::detach(c, c->ordinal);
   delete c;
   return RUAI_OK;
 }
@@ -138,182 +131,20 @@ RUAI_API int ruai_ctx_synchronize(ruai_ctx* c) {
   return ruai_ctx_check_status(c);
 }
 
-// ---- ruai_malloc / ruai_free ----------------------------------------------------------------
-//
-// A program makes a tensor per call and drops it soon after; cudaMalloc and cudaFree between launches cost more than most Linears
-// (int8 2048 x 2048, one row: 7 us on the device of 25 a call; 4096 x 14336 results: 0.9 ms of mapping and unmapping).  Freed blocks
-// are kept for the next request of their size class.  cudaFree waits for the device, so a block may be freed while a kernel on ANY
-// stream still uses it; here it is set aside, and given out only after its context's stream and then the device have been waited for,
-// once for all the blocks set aside until then, when so many of the wanted class lie waiting that it pays.
-// At most kPoolBytes are kept per device; they are given back when memory runs short and with the device's last context.
-namespace {
-
-constexpr size_t kPoolBytes = 512ull << 20;
-constexpr int kPoolDevices = 64;
-
-struct Pool {
-  std::mutex lock;
-  std::unordered_map<void*, size_t> live;         // blocks handed out, by size class
-  std::map<size_t, std::vector<void*>> clean;     // nothing on the device uses them
-  std::map<ruai_ctx*, std::map<size_t, std::vector<void*>>> aside;  // freed through a context since its last device-wide wait
-  size_t bytes = 0;                               // in clean and aside
-  int contexts = 0;
-};
-Pool& pool_of(int ordinal) {
-  static Pool* pools = new Pool[kPoolDevices];  // never destroyed: the driver may be gone before static destructors run
-  return pools[ordinal];
-}
-bool pooled(int ordinal) { return ordinal >= 0 && ordinal < kPoolDevices; }
-
-size_t size_class(size_t bytes) {
-  if (bytes > (1ull << 20)) return (bytes + (2ull << 20) - 1) / (2ull << 20) * (2ull << 20);
-  size_t c = 512;
-  while (c < bytes) c *= 2;
-  return c;
-}
-// Waits for the context's stream and the device and makes the blocks set aside through the context before that clean.  The wait is
-// cudaFree's, which other threads' captures allow as they allow any cudaFree.
-bool pool_settle(ruai_ctx* c, Pool& p) {
-  std::map<size_t, std::vector<void*>> moved;
-  {
-    std::lock_guard<std::mutex> g(p.lock);
-    moved.swap(p.aside[c]);
-  }
-  void* dummy = nullptr;
-  const bool ok = cudaStreamSynchronize(c->stream) == cudaSuccess && cudaMalloc(&dummy, 512) == cudaSuccess && cudaFree(dummy) == cudaSuccess;
-  if (!ok) (void)cudaGetLastError();
-  std::lock_guard<std::mutex> g(p.lock);
-  for (auto& kv : moved) {
-    std::vector<void*>& to = ok ? p.clean[kv.first] : p.aside[c][kv.first];
-    to.insert(to.end(), kv.second.begin(), kv.second.end());
-  }
-  return ok;
-}
-void pool_trim(Pool& p) {
-  std::vector<void*> out;
-  {
-    std::lock_guard<std::mutex> g(p.lock);
-    auto all = [&](std::map<size_t, std::vector<void*>>& m) {
-      for (auto& kv : m) out.insert(out.end(), kv.second.begin(), kv.second.end());
-      m.clear();
-    };
-    all(p.clean);
-    for (auto& kv : p.aside) all(kv.second);
-    p.bytes = 0;
-  }
-  for (void* q : out) cudaFree(q);  // waits for the device
-}
-void* pool_take(Pool& p, size_t cls) {
-  std::lock_guard<std::mutex> g(p.lock);
-  auto it = p.clean.find(cls);
-  if (it == p.clean.end() || it->second.empty()) return nullptr;
-  void* q = it->second.back();
-  it->second.pop_back();
-  p.bytes -= cls;
-  p.live[q] = cls;
-  return q;
-}
-
-}  // namespace
-
-// What was set aside through a context that goes is freed.
-static void ruai_pool_forget(ruai_ctx* c) {
-  if (!pooled(c->ordinal)) return;
-  Pool& p = pool_of(c->ordinal);
-  std::map<size_t, std::vector<void*>> moved;
-  {
-    std::lock_guard<std::mutex> g(p.lock);
-    auto it = p.aside.find(c);
-    if (it == p.aside.end()) return;
-    moved.swap(it->second);
-    p.aside.erase(it);
-    for (auto& kv : moved) p.bytes -= kv.first * kv.second.size();
-  }
-  for (auto& kv : moved)
-    for (void* q : kv.second) cudaFree(q);
-}
-
-static void ruai_pool_contexts(int ordinal, int change) {
-  if (!pooled(ordinal)) return;
-  Pool& p = pool_of(ordinal);
-  bool last;
-  {
-    std::lock_guard<std::mutex> g(p.lock);
-    p.contexts += change;
-    last = p.contexts == 0;
-  }
-  if (last) pool_trim(p);
-}
-
-// cudaMalloc on the current device that gives the kept blocks back before it reports that memory has run out.
-cudaError_t ruai_device_malloc(void** out, size_t bytes) {
-  cudaError_t e = cudaMalloc(out, bytes);
-  if (e != cudaErrorMemoryAllocation) return e;
-  int ordinal = 0;
-  if (cudaGetDevice(&ordinal) != cudaSuccess || !pooled(ordinal)) return e;
-  Pool& p = pool_of(ordinal);
-  {
-    std::lock_guard<std::mutex> g(p.lock);
-    if (p.bytes == 0) return e;
-  }
-  (void)cudaGetLastError();
-  pool_trim(p);
-  return cudaMalloc(out, bytes);
-}
+cudaError_t ruai_device_malloc(void** out, size_t bytes) { return block_pool::device_malloc(out, bytes); }
 
 RUAI_API int ruai_malloc(ruai_ctx* c, size_t bytes, void** out) {
   if (!c || !out) return ruai_fail(c, RUAI_ERR_ARG, "ruai_malloc: NULL argument");
   DeviceGuard g(c->ordinal);
   *out = nullptr;
-  if (!pooled(c->ordinal) || bytes > kPoolBytes / 2) {
-    RUAI_CUDA(c, ruai_device_malloc(out, bytes ? bytes : 1));
-    return RUAI_OK;
-  }
-  Pool& p = pool_of(c->ordinal);
-  const size_t cls = size_class(bytes);
-  if ((*out = pool_take(p, cls)) != nullptr) return RUAI_OK;
-  size_t waiting = 0;
-  {
-    std::lock_guard<std::mutex> l(p.lock);
-    auto& mine = p.aside[c];
-    auto it = mine.find(cls);
-    if (it != mine.end()) waiting = it->second.size();
-  }
-  // Until then new ones are mapped, which costs hundreds of microseconds for a large block: two of those do.
-  if (waiting >= 32 || (waiting * cls >= (4ull << 20) && (waiting >= 2 || cls >= (64ull << 20)))) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) (void)cudaGetLastError();
-    if (st == cudaStreamCaptureStatusNone && pool_settle(c, p) && (*out = pool_take(p, cls)) != nullptr) return RUAI_OK;
-  }
-  RUAI_CUDA(c, ruai_device_malloc(out, cls));
-  std::lock_guard<std::mutex> l(p.lock);
-  p.live[*out] = cls;
+  RUAI_CUDA(c, block_pool::allocate(c, c->ordinal, c->stream, bytes, out));
   return RUAI_OK;
 }
 
 RUAI_API int ruai_free(ruai_ctx* c, void* p) {
   if (!c) return ruai_fail(nullptr, RUAI_ERR_ARG, "ctx is NULL");
   DeviceGuard g(c->ordinal);
-  bool kept = false, full = false;
-  if (p && pooled(c->ordinal)) {
-    Pool& pool = pool_of(c->ordinal);
-    std::lock_guard<std::mutex> l(pool.lock);
-    auto it = pool.live.find(p);
-    if (it != pool.live.end()) {
-      const size_t cls = it->second;
-      pool.live.erase(it);
-      pool.aside[c][cls].push_back(p);
-      pool.bytes += cls;
-      full = pool.bytes > kPoolBytes;
-      kept = true;
-    }
-  }
-  if (kept) {
-    if (full) pool_trim(pool_of(c->ordinal));  // of sizes no longer asked for, most of it
-    return RUAI_OK;
-  }
-  RUAI_CUDA(c, cudaStreamSynchronize(c->stream));
-  RUAI_CUDA(c, cudaFree(p));
+  RUAI_CUDA(c, block_pool::give_back(c, c->ordinal, c->stream, p));
   return RUAI_OK;
 }
 

@@ -1,0 +1,139 @@
+// Runs block_pool.cuh against a stand-in for the CUDA runtime: addresses without memory behind them, streams that can be capturing,
+// and work that goes on until the device is waited for.  One scenario per run; exit status 0: it held.
+#include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+#include <functional>
+#include <set>
+#include <string>
+#include <vector>
+
+#include "../ruai_b200/csrc/block_pool.cuh"
+
+#define CHECK(c)                                                     \
+  do {                                                               \
+    if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); std::exit(1); } \
+  } while (0)
+
+namespace fake {
+std::mutex lock;
+std::map<char*, size_t> memory;      // what the driver has handed out
+std::vector<std::pair<char*, size_t>> freed;  // addresses to hand out again, last first
+size_t limit = ~(size_t)0, used = 0, waits = 0;
+std::set<cudaStream_t> capturing, spoiled;
+std::set<void*> busy;                // work that is still going on reads or writes it
+std::function<void()> during_wait;
+char* next = (char*)0x1000000;
+cudaStream_t stream(int i) { return (cudaStream_t)(size_t)(16 + i); }
+}  // namespace fake
+
+extern "C" {
+cudaError_t cudaMalloc(void** out, size_t bytes) {
+  std::lock_guard<std::mutex> g(fake::lock);
+  if (fake::used + bytes > fake::limit) return cudaErrorMemoryAllocation;
+  char* at = fake::next;
+  auto same = std::find_if(fake::freed.rbegin(), fake::freed.rend(), [&](auto& f) { return f.second >= bytes; });
+  if (same != fake::freed.rend()) { at = same->first; fake::freed.erase(std::next(same).base()); }
+  else fake::next += (bytes + 4095) / 4096 * 4096;
+  fake::memory[at] = bytes;
+  fake::used += bytes;
+  *out = at;
+  return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {  // may wait for the device, or not
+  std::lock_guard<std::mutex> g(fake::lock);
+  if (!p) return cudaSuccess;
+  auto it = fake::memory.find((char*)p);
+  if (it == fake::memory.end()) return cudaErrorInvalidValue;
+  fake::used -= it->second;
+  fake::freed.push_back(*it);
+  fake::memory.erase(it);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+  if (fake::capturing.count(s)) { fake::spoiled.insert(s); return cudaErrorStreamCaptureUnsupported; }
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceSynchronize(void) {
+  ++fake::waits;
+  if (fake::during_wait) { auto f = fake::during_wait; fake::during_wait = nullptr; f(); }
+  fake::busy.clear();
+  return cudaSuccess;
+}
+cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* st) {
+  *st = fake::capturing.count(s) ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+  return cudaSuccess;
+}
+cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+}
+
+using namespace block_pool;
+
+struct Context {  // what ctx.cu makes of a ruai_ctx
+  int ordinal;
+  cudaStream_t stream;
+  explicit Context(int i, int ordinal_ = 0) : ordinal(ordinal_), stream(fake::stream(i)) { attach(this, ordinal, stream); }
+  ~Context() { detach(this, ordinal); }
+  void* get(size_t bytes) {
+    void* p = nullptr;
+    return allocate(this, ordinal, stream, bytes, &p) == cudaSuccess ? p : nullptr;
+  }
+  cudaError_t put(void* p) { return give_back(this, ordinal, stream, p); }
+};
+constexpr size_t MB = 1 << 20;
+
+// Requests of this size until one comes from the blocks kept.
+void* reused(Context& c, size_t bytes) {
+  std::set<void*> seen;
+  for (int i = 0; i < 200; ++i) {
+    void* p = c.get(bytes);
+    CHECK(p);
+    if (!seen.insert(p).second) return p;
+    c.put(p);
+  }
+  return nullptr;
+}
+
+int main(int argc, char** argv) {
+  const std::string what = argc > 1 ? argv[1] : "";
+  if (what == "reuse") {
+    Context c(0);
+    for (size_t bytes : {size_t(1), size_t(4096), MB, 3 * MB, 200 * MB}) CHECK(reused(c, bytes));
+    const size_t used = fake::used;
+    CHECK(c.put(c.get(300 * MB)) == cudaSuccess && fake::used == used);  // too large to be kept
+  } else if (what == "last context") {
+    {
+      Context a(0);
+      { Context b(1); b.put(b.get(MB)); a.put(a.get(4 * MB)); }
+      a.put(a.get(MB));
+    }
+    CHECK(fake::memory.empty());
+  } else if (what == "limit") {
+    Context c(0);
+    std::vector<void*> all;
+    for (int i = 0; i < 40; ++i) all.push_back(c.get(32 * MB));
+    for (void* p : all) {
+      CHECK(c.put(p) == cudaSuccess);
+      size_t kept = 0;
+      for (auto& m : fake::memory) kept += m.second;
+      size_t out = 0;
+      for (void* q : all) out += q > p ? 32 * MB : 0;
+      CHECK(kept - out <= kKeptBytes);
+    }
+  } else if (what == "out of memory") {
+    Context c(0);
+    fake::limit = 300 * MB;
+    std::vector<void*> all;
+    for (int i = 0; i < 8; ++i) all.push_back(c.get(32 * MB));
+    for (void* p : all) c.put(p);
+    CHECK(c.get(250 * MB));                       // what is kept makes room
+    CHECK(!c.get(250 * MB));
+    void* p = nullptr;
+    CHECK(device_malloc(&p, 40 * MB) == cudaSuccess);
+  } else {
+    std::printf("no scenario \"%s\"\n", what.c_str());
+    return 2;
+  }
+  return 0;
+}
