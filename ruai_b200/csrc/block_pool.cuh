@@ -7,6 +7,8 @@
 // stream still uses it; here it is set aside, and given out only after its context's stream and then the device have been waited for,
 // once for all the blocks set aside until then, when so many of the wanted class lie waiting that it pays.
 // At most kKeptBytes are kept per device; they are given back when memory runs short and with the device's last context.
+// While a stream of the device's contexts is being captured, nothing is kept or given out: a graph uses its memory whenever it is
+// replayed, which no wait sees, so what is freed then is for the driver to refuse, as cudaFree after a wait for the stream does.
 #pragma once
 #include <cuda_runtime_api.h>
 
@@ -28,7 +30,7 @@ struct Pool {  // of a device
   Blocks clean;                            // nothing on the device uses them
   std::map<const void*, Blocks> aside;     // freed through a context since its last device-wide wait
   size_t bytes = 0;                        // in clean and aside
-  int contexts = 0;
+  std::map<const void*, cudaStream_t> contexts;
 };
 struct State {
   std::mutex lock;  // held for bookkeeping, not for a wait or a call that maps or unmaps memory
@@ -82,6 +84,20 @@ inline void trim(Pool& p) {
     for (void* q : kv.second) cudaFree(q);  // waits for the device
 }
 
+// Whether a stream of the device's contexts is being captured, or cannot be asked.  The lock is held, so that none of them goes meanwhile.
+inline bool capturing(const Pool& p) {
+  bool any = false;
+  for (auto& kv : p.contexts) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(kv.second, &st) != cudaSuccess) {
+      (void)cudaGetLastError();
+      any = true;
+    }
+    any = any || st != cudaStreamCaptureStatusNone;
+  }
+  return any;
+}
+
 inline void* take(Pool& p, size_t cls) {
   Lock l(state().lock);
   auto it = p.clean.find(cls);
@@ -94,10 +110,10 @@ inline void* take(Pool& p, size_t cls) {
 }
 
 // A context of the device more; the device's last one to go gives the kept memory back, and each what was set aside through it.
-inline void attach(const void*, int ordinal, cudaStream_t) {
+inline void attach(const void* context, int ordinal, cudaStream_t stream) {
   if (!pooled(ordinal)) return;
   Lock l(state().lock);
-  ++of(ordinal).contexts;
+  of(ordinal).contexts[context] = stream;
 }
 inline void detach(const void* context, int ordinal) {
   if (!pooled(ordinal)) return;
@@ -109,7 +125,8 @@ inline void detach(const void* context, int ordinal) {
     out.swap(p.aside[context]);
     p.aside.erase(context);
     for (auto& kv : out) p.bytes -= kv.first * kv.second.size();
-    last = --p.contexts == 0;
+    p.contexts.erase(context);
+    last = p.contexts.empty();
   }
   for (auto& kv : out)
     for (void* q : kv.second) cudaFree(q);
@@ -137,19 +154,20 @@ inline cudaError_t allocate(const void* context, int ordinal, cudaStream_t strea
   if (!pooled(ordinal) || bytes > kKeptBytes / 2) return device_malloc(out, bytes ? bytes : 1);
   Pool& p = of(ordinal);
   const size_t cls = size_class(bytes);
-  if ((*out = take(p, cls)) != nullptr) return cudaSuccess;
   size_t waiting = 0;
+  bool captured;
   {
     Lock l(state().lock);
+    captured = capturing(p);
     auto& mine = p.aside[context];
     auto it = mine.find(cls);
     if (it != mine.end()) waiting = it->second.size();
   }
-  // Until then new ones are mapped, which costs hundreds of microseconds for a large block: two of those do.
-  if (waiting >= 32 || (waiting * cls >= (4ull << 20) && (waiting >= 2 || cls >= (64ull << 20)))) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) (void)cudaGetLastError();
-    if (st == cudaStreamCaptureStatusNone && settle(p, context, stream) && (*out = take(p, cls)) != nullptr) return cudaSuccess;
+  if (!captured) {
+    if ((*out = take(p, cls)) != nullptr) return cudaSuccess;
+    // Until then new ones are mapped, which costs hundreds of microseconds for a large block: two of those do.
+    if (waiting >= 32 || (waiting * cls >= (4ull << 20) && (waiting >= 2 || cls >= (64ull << 20))))
+      if (settle(p, context, stream) && (*out = take(p, cls)) != nullptr) return cudaSuccess;
   }
   const cudaError_t e = device_malloc(out, cls);
   if (e != cudaSuccess) return e;
@@ -165,7 +183,7 @@ inline cudaError_t give_back(const void* context, int ordinal, cudaStream_t stre
     Pool& p = of(ordinal);
     Lock l(state().lock);
     auto it = p.live.find(q);
-    if (it != p.live.end()) {
+    if (it != p.live.end() && !capturing(p)) {
       const size_t cls = it->second;
       p.live.erase(it);
       p.aside[context][cls].push_back(q);
@@ -178,8 +196,25 @@ inline cudaError_t give_back(const void* context, int ordinal, cudaStream_t stre
     if (full) trim(of(ordinal));  // of sizes no longer asked for, most of it
     return cudaSuccess;
   }
-  const cudaError_t e = cudaStreamSynchronize(stream);
-  return e != cudaSuccess ? e : cudaFree(q);
+  cudaError_t e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) return e;
+  size_t cls = 0;
+  if (pooled(ordinal)) {  // no longer this file's: forgotten before another thread can be given the address
+    Pool& p = of(ordinal);
+    Lock l(state().lock);
+    auto it = p.live.find(q);
+    if (it != p.live.end()) {
+      cls = it->second;
+      p.live.erase(it);
+    }
+  }
+  e = cudaFree(q);
+  if (e != cudaSuccess && cls) {
+    Pool& p = of(ordinal);
+    Lock l(state().lock);
+    p.live[q] = cls;
+  }
+  return e;
 }
 
 }  // namespace block_pool

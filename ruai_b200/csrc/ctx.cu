@@ -74,6 +74,7 @@ RUAI_API int ruai_ctx_destroy(ruai_ctx* c) {
   if (!c) return RUAI_OK;
   DeviceGuard g(c->ordinal);
   cudaStreamSynchronize(c->stream);
+  block_pool::detach(c, c->ordinal);  // before its stream goes
   cudaFree(c->partial);
   cudaFree(c->counters);
   cudaFree(c->status);
@@ -82,7 +83,6 @@ RUAI_API int ruai_ctx_destroy(ruai_ctx* c) {
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
   if (c->own_stream) cudaStreamDestroy(c->stream);
-  block_pool::detach(c, c->ordinal);
   delete c;
   return RUAI_OK;
 }

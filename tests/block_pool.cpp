@@ -131,6 +131,34 @@ int main(int argc, char** argv) {
     CHECK(!c.get(250 * MB));
     void* p = nullptr;
     CHECK(device_malloc(&p, 40 * MB) == cudaSuccess);
+  } else if (what == "free in a capture") {       // the graph goes on using the block after the capture
+    Context c(0);
+    void* p = c.get(4096);
+    fake::capturing.insert(c.stream);
+    CHECK(c.put(p) != cudaSuccess);
+    CHECK(fake::spoiled.count(c.stream));
+    fake::capturing.clear();
+    for (int i = 0; i < 100; ++i) {
+      void* q = c.get(4096);
+      CHECK(q != p && c.put(q) == cudaSuccess);
+    }
+    CHECK(c.put(p) == cudaSuccess);               // after the capture it is a block like any other
+  } else if (what == "capture of another context") {
+    Context a(0), b(1);
+    void* p = a.get(4096);
+    fake::capturing.insert(b.stream);
+    CHECK(a.put(p) == cudaSuccess && !fake::memory.count((char*)p));  // to the driver, which may refuse it
+    fake::capturing.clear();
+    CHECK(a.put(a.get(4096)) == cudaSuccess && !fake::memory.empty());
+  } else if (what == "request in a capture") {
+    Context c(0);
+    std::vector<void*> all;
+    for (int i = 0; i < 40; ++i) all.push_back(c.get(4096));
+    for (void* q : all) c.put(q);
+    c.put(reused(c, 4096));
+    const size_t used = fake::used;
+    fake::capturing.insert(c.stream);
+    CHECK(c.get(4096) && fake::used > used);      // the driver's answer, whatever it is
   } else {
     std::printf("no scenario \"%s\"\n", what.c_str());
     return 2;
