@@ -17,6 +17,7 @@
 #include <map>
 #include <mutex>
 #include <unordered_map>
+#include <utility>
 
 namespace block_pool {
 
@@ -25,8 +26,12 @@ constexpr int kDevices = 64;
 
 using Blocks = std::map<size_t, std::list<void*>>;  // by size class
 
+struct Block {
+  size_t cls;
+  int ordinal;
+  bool kept;  // in clean or aside, not with a caller
+};
 struct Pool {  // of a device
-  std::unordered_map<void*, size_t> live;  // blocks handed out, by size class
   Blocks clean;                            // nothing on the device uses them
   std::map<const void*, Blocks> aside;     // freed through a context since its last device-wide wait
   size_t bytes = 0;                        // in clean and aside
@@ -34,6 +39,9 @@ struct Pool {  // of a device
 };
 struct State {
   std::mutex lock;  // held for bookkeeping, not for a wait or a call that maps or unmaps memory
+  // Every block of this file's making that has not gone back to the driver: a block may come back through a context of another device, and
+  // one that lies here must not come back a second time (the driver counts it as allocated, so cudaFree would take it).
+  std::unordered_map<void*, Block> blocks;
   Pool device[kDevices];
 };
 inline State& state() {
@@ -49,6 +57,11 @@ inline size_t size_class(size_t bytes) {
   size_t c = 512;
   while (c < bytes) c *= 2;
   return c;
+}
+
+inline void forget(const Blocks& all) {  // the lock is held, the blocks are about to be freed
+  for (auto& kv : all)
+    for (void* q : kv.second) state().blocks.erase(q);
 }
 
 inline void merge(Blocks& to, Blocks& from) {
@@ -79,6 +92,7 @@ inline void trim(Pool& p) {
     merge(out, p.clean);
     for (auto& kv : p.aside) merge(out, kv.second);
     p.bytes = 0;
+    forget(out);
   }
   for (auto& kv : out)
     for (void* q : kv.second) cudaFree(q);  // waits for the device
@@ -105,7 +119,7 @@ inline void* take(Pool& p, size_t cls) {
   void* q = it->second.back();
   it->second.pop_back();
   p.bytes -= cls;
-  p.live[q] = cls;
+  state().blocks.at(q).kept = false;
   return q;
 }
 
@@ -125,6 +139,7 @@ inline void detach(const void* context, int ordinal) {
     out.swap(p.aside[context]);
     p.aside.erase(context);
     for (auto& kv : out) p.bytes -= kv.first * kv.second.size();
+    forget(out);
     p.contexts.erase(context);
     last = p.contexts.empty();
   }
@@ -151,7 +166,13 @@ inline cudaError_t device_malloc(void** out, size_t bytes) {
 
 // A block for a context on its stream; the device is current.
 inline cudaError_t allocate(const void* context, int ordinal, cudaStream_t stream, size_t bytes, void** out) {
-  if (!pooled(ordinal) || bytes > kKeptBytes / 2) return device_malloc(out, bytes ? bytes : 1);
+  if (!pooled(ordinal) || bytes > kKeptBytes / 2) {
+    const cudaError_t e = device_malloc(out, bytes ? bytes : 1);
+    if (e != cudaSuccess) return e;
+    Lock l(state().lock);
+    state().blocks.erase(*out);  // left by a caller that gave a block of ours to cudaFree itself
+    return cudaSuccess;
+  }
   Pool& p = of(ordinal);
   const size_t cls = size_class(bytes);
   size_t waiting = 0;
@@ -172,47 +193,40 @@ inline cudaError_t allocate(const void* context, int ordinal, cudaStream_t strea
   const cudaError_t e = device_malloc(out, cls);
   if (e != cudaSuccess) return e;
   Lock l(state().lock);
-  p.live[*out] = cls;
+  state().blocks[*out] = {cls, ordinal, false};
   return cudaSuccess;
 }
 
 // Frees a block on behalf of a context, whose device is current.
 inline cudaError_t give_back(const void* context, int ordinal, cudaStream_t stream, void* q) {
   bool kept = false, full = false;
-  if (q && pooled(ordinal)) {
-    Pool& p = of(ordinal);
+  {
     Lock l(state().lock);
-    auto it = p.live.find(q);
-    if (it != p.live.end() && !capturing(p)) {
-      const size_t cls = it->second;
-      p.live.erase(it);
-      p.aside[context][cls].push_back(q);
-      p.bytes += cls;
-      full = p.bytes > kKeptBytes;
-      kept = true;
+    auto it = state().blocks.find(q);
+    if (it != state().blocks.end()) {
+      if (it->second.kept) return cudaErrorInvalidValue;  // freed already: cudaFree's answer
+      if (it->second.ordinal == ordinal && !capturing(of(ordinal))) {
+        Pool& p = of(ordinal);
+        p.aside[context][it->second.cls].push_back(q);
+        p.bytes += it->second.cls;
+        it->second.kept = kept = true;
+        full = p.bytes > kKeptBytes;
+      }
     }
   }
-  if (kept) {
-    if (full) trim(of(ordinal));  // of sizes no longer asked for, most of it
-    return cudaSuccess;
-  }
+  if (full) trim(of(ordinal));  // of sizes no longer asked for, most of it
+  if (kept) return cudaSuccess;
   cudaError_t e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return e;
-  size_t cls = 0;
-  if (pooled(ordinal)) {  // no longer this file's: forgotten before another thread can be given the address
-    Pool& p = of(ordinal);
+  std::unordered_map<void*, Block>::node_type entry;
+  {
     Lock l(state().lock);
-    auto it = p.live.find(q);
-    if (it != p.live.end()) {
-      cls = it->second;
-      p.live.erase(it);
-    }
+    entry = state().blocks.extract(q);  // before another thread can be given the address
   }
   e = cudaFree(q);
-  if (e != cudaSuccess && cls) {
-    Pool& p = of(ordinal);
+  if (e != cudaSuccess && entry) {
     Lock l(state().lock);
-    p.live[q] = cls;
+    state().blocks.insert(std::move(entry));
   }
   return e;
 }

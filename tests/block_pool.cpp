@@ -159,6 +159,31 @@ int main(int argc, char** argv) {
     const size_t used = fake::used;
     fake::capturing.insert(c.stream);
     CHECK(c.get(4096) && fake::used > used);      // the driver's answer, whatever it is
+  } else if (what == "freed twice") {
+    Context c(0), d(1);
+    void* p = c.get(4096);
+    CHECK(c.put(p) == cudaSuccess);
+    CHECK(c.put(p) != cudaSuccess && d.put(p) != cudaSuccess && fake::memory.count((char*)p));
+    CHECK(reused(c, 4096));                       // the same once it is clean
+    std::vector<void*> all;
+    for (int i = 0; i < 40; ++i) all.push_back(c.get(4096));
+    for (void* q : all) CHECK(c.put(q) == cudaSuccess);
+    for (void* q : all) CHECK(c.put(q) != cudaSuccess && fake::memory.count((char*)q));
+    CHECK(c.put((void*)0x10) != cudaSuccess);  // not allocated at all: cudaFree's error
+  } else if (what == "freed through another device") {
+    Context a(0, 0), b(1, 1);
+    void* p = a.get(4096);
+    CHECK(b.put(p) == cudaSuccess && !fake::memory.count((char*)p));
+    void* q = nullptr;
+    CHECK(cudaMalloc(&q, 4096) == cudaSuccess && q == p);  // another owner of the address
+    CHECK(a.put(q) == cudaSuccess && !fake::memory.count((char*)q));
+  } else if (what == "address of a block that cudaFree took") {
+    Context c(0);
+    void* p = c.get(4 * MB);
+    cudaFree(p);
+    fake::freed = {{(char*)p, 300 * MB}};
+    void* q = c.get(300 * MB);
+    CHECK(q == p && c.put(q) == cudaSuccess && !fake::memory.count((char*)q));
   } else {
     std::printf("no scenario \"%s\"\n", what.c_str());
     return 2;

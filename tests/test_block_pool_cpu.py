@@ -18,6 +18,7 @@ def program(tmp_path_factory):
 @pytest.mark.parametrize("scenario", [
     "reuse", "last context", "limit", "out of memory",
     "free in a capture", "capture of another context", "request in a capture",
+    "freed twice", "freed through another device", "address of a block that cudaFree took",
 ])
 def test_scenario(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=60)
