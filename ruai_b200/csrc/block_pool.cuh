@@ -34,7 +34,8 @@ struct Block {
 struct Pool {  // of a device
   Blocks clean;                            // nothing on the device uses them
   std::map<const void*, Blocks> aside;     // freed through a context since its last device-wide wait
-  size_t bytes = 0;                        // in clean and aside
+  size_t bytes = 0;                        // in clean, in aside and on the way from one to the other
+  std::mutex settling;                     // held while blocks are on that way: whoever wants all that is kept waits for them; taken before the lock
   std::map<const void*, cudaStream_t> contexts;
 };
 struct State {
@@ -72,6 +73,7 @@ inline void merge(Blocks& to, Blocks& from) {
 // Waits for the context's stream and the device and makes the blocks set aside through the context before that clean.  The wait is
 // cudaFree's, which other threads' captures allow as they allow any cudaFree.
 inline bool settle(Pool& p, const void* context, cudaStream_t stream) {
+  Lock way(p.settling);
   Blocks moved;
   {
     Lock l(state().lock);
@@ -86,12 +88,13 @@ inline bool settle(Pool& p, const void* context, cudaStream_t stream) {
 }
 
 inline void trim(Pool& p) {
+  Lock way(p.settling);
   Blocks out;
   {
     Lock l(state().lock);
     merge(out, p.clean);
     for (auto& kv : p.aside) merge(out, kv.second);
-    p.bytes = 0;
+    for (auto& kv : out) p.bytes -= kv.first * kv.second.size();
     forget(out);
   }
   for (auto& kv : out)

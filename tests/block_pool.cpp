@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <functional>
+#include <future>
 #include <set>
 #include <string>
 #include <vector>
@@ -24,6 +25,12 @@ std::set<cudaStream_t> capturing, spoiled;
 std::set<void*> busy;                // work that is still going on reads or writes it
 std::function<void()> during_wait;
 char* next = (char*)0x1000000;
+void wait() {
+  if (!during_wait) return;
+  auto f = during_wait;
+  during_wait = nullptr;
+  f();
+}
 cudaStream_t stream(int i) { return (cudaStream_t)(size_t)(16 + i); }
 }  // namespace fake
 
@@ -51,12 +58,13 @@ cudaError_t cudaFree(void* p) {  // may wait for the device, or not
   return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+  fake::wait();
   if (fake::capturing.count(s)) { fake::spoiled.insert(s); return cudaErrorStreamCaptureUnsupported; }
   return cudaSuccess;
 }
 cudaError_t cudaDeviceSynchronize(void) {
   ++fake::waits;
-  if (fake::during_wait) { auto f = fake::during_wait; fake::during_wait = nullptr; f(); }
+  fake::wait();
   fake::busy.clear();
   return cudaSuccess;
 }
@@ -184,6 +192,31 @@ int main(int argc, char** argv) {
     fake::freed = {{(char*)p, 300 * MB}};
     void* q = c.get(300 * MB);
     CHECK(q == p && c.put(q) == cudaSuccess && !fake::memory.count((char*)q));
+  } else if (what == "trim during a wait" || what == "out of memory during a wait") {
+    Context a(0), b(1);
+    std::vector<void*> mine, others;
+    for (int i = 0; i < 4; ++i) mine.push_back(a.get(4 * MB));
+    for (int i = 0; i < 20; ++i) others.push_back(b.get(32 * MB));
+    for (void* p : mine) a.put(p);
+    std::future<bool> other;
+    fake::during_wait = [&] {
+      other = std::async(std::launch::async, [&] {
+        if (what == "trim during a wait") {
+          for (void* p : others) b.put(p);        // beyond the limit
+          return true;
+        }
+        fake::limit = fake::used;
+        void* p = nullptr;
+        return device_malloc(&p, 4096) == cudaSuccess;  // there is memory kept
+      });
+      other.wait_for(std::chrono::milliseconds(300));
+    };
+    void* p = a.get(4 * MB);                      // waits for the device
+    CHECK(other.valid() && other.get());
+    fake::limit = ~(size_t)0;
+    size_t out = p ? 4 * MB : 0;
+    if (what != "trim during a wait") out += 20 * 32 * MB + 4096;
+    CHECK(of(0).bytes == fake::used - out);
   } else {
     std::printf("no scenario \"%s\"\n", what.c_str());
     return 2;
