@@ -3,9 +3,10 @@
 //
 // A program makes a tensor per call and drops it soon after; cudaMalloc and cudaFree between launches cost more than most Linears
 // (int8 2048 x 2048, one row: 7 us on the device of 25 a call; 4096 x 14336 results: 0.9 ms of mapping and unmapping).  Freed blocks
-// are kept for the next request of their size class.  cudaFree waits for the device, so a block may be freed while a kernel on ANY
-// stream still uses it; here it is set aside, and given out only after its context's stream and then the device have been waited for,
-// once for all the blocks set aside until then, when so many of the wanted class lie waiting that it pays.
+// are kept for the next request of their size class.  A block may be freed while a kernel on ANY stream still uses it, as cudaFree lets a
+// caller do; it is set aside, and given out only after a cudaDeviceSynchronize, once for all the blocks set aside until then, when so
+// many of the wanted class lie waiting that it pays.  (A cudaFree in its place would do as a wait only by a side effect that CUDA does not
+// promise.  Where a capture forbids the wait it forbids the cudaMalloc that a request would come to otherwise.)
 // At most kKeptBytes are kept per device; they are given back when memory runs short and with the device's last context.
 // While a stream of the device's contexts is being captured, nothing is kept or given out: a graph uses its memory whenever it is
 // replayed, which no wait sees, so what is freed then is for the driver to refuse, as cudaFree after a wait for the stream does.
@@ -33,7 +34,7 @@ struct Block {
 };
 struct Pool {  // of a device
   Blocks clean;                            // nothing on the device uses them
-  std::map<const void*, Blocks> aside;     // freed through a context since its last device-wide wait
+  Blocks aside;                            // freed since the last device-wide wait
   size_t bytes = 0;                        // in clean, in aside and on the way from one to the other
   std::mutex settling;                     // held while blocks are on that way: whoever wants all that is kept waits for them; taken before the lock
   std::map<const void*, cudaStream_t> contexts;
@@ -70,20 +71,19 @@ inline void merge(Blocks& to, Blocks& from) {
   from.clear();
 }
 
-// Waits for the context's stream and the device and makes the blocks set aside through the context before that clean.  The wait is
-// cudaFree's, which other threads' captures allow as they allow any cudaFree.
-inline bool settle(Pool& p, const void* context, cudaStream_t stream) {
+// Waits for the device and makes the blocks set aside before that clean.
+inline bool settle(Pool& p) {
   Lock way(p.settling);
   Blocks moved;
   {
     Lock l(state().lock);
-    moved.swap(p.aside[context]);
+    moved.swap(p.aside);
   }
-  void* dummy = nullptr;
-  const bool ok = cudaStreamSynchronize(stream) == cudaSuccess && cudaMalloc(&dummy, 512) == cudaSuccess && cudaFree(dummy) == cudaSuccess;
+  if (moved.empty()) return true;  // another thread has just waited
+  const bool ok = cudaDeviceSynchronize() == cudaSuccess;
   if (!ok) (void)cudaGetLastError();
   Lock l(state().lock);
-  merge(ok ? p.clean : p.aside[context], moved);
+  merge(ok ? p.clean : p.aside, moved);
   return ok;
 }
 
@@ -93,12 +93,14 @@ inline void trim(Pool& p) {
   {
     Lock l(state().lock);
     merge(out, p.clean);
-    for (auto& kv : p.aside) merge(out, kv.second);
+    merge(out, p.aside);
     for (auto& kv : out) p.bytes -= kv.first * kv.second.size();
     forget(out);
   }
+  if (out.empty()) return;
+  if (cudaDeviceSynchronize() != cudaSuccess) (void)cudaGetLastError();
   for (auto& kv : out)
-    for (void* q : kv.second) cudaFree(q);  // waits for the device
+    for (void* q : kv.second) cudaFree(q);
 }
 
 // Whether a stream of the device's contexts is being captured, or cannot be asked.  The lock is held, so that none of them goes meanwhile.
@@ -126,7 +128,7 @@ inline void* take(Pool& p, size_t cls) {
   return q;
 }
 
-// A context of the device more; the device's last one to go gives the kept memory back, and each what was set aside through it.
+// A context of the device more; the device's last one to go gives the kept memory back.
 inline void attach(const void* context, int ordinal, cudaStream_t stream) {
   if (!pooled(ordinal)) return;
   Lock l(state().lock);
@@ -135,19 +137,12 @@ inline void attach(const void* context, int ordinal, cudaStream_t stream) {
 inline void detach(const void* context, int ordinal) {
   if (!pooled(ordinal)) return;
   Pool& p = of(ordinal);
-  Blocks out;
   bool last;
   {
     Lock l(state().lock);
-    out.swap(p.aside[context]);
-    p.aside.erase(context);
-    for (auto& kv : out) p.bytes -= kv.first * kv.second.size();
-    forget(out);
     p.contexts.erase(context);
     last = p.contexts.empty();
   }
-  for (auto& kv : out)
-    for (void* q : kv.second) cudaFree(q);
   if (last) trim(p);
 }
 
@@ -167,8 +162,8 @@ inline cudaError_t device_malloc(void** out, size_t bytes) {
   return cudaMalloc(out, bytes);
 }
 
-// A block for a context on its stream; the device is current.
-inline cudaError_t allocate(const void* context, int ordinal, cudaStream_t stream, size_t bytes, void** out) {
+// A block on a device, which is current.
+inline cudaError_t allocate(int ordinal, size_t bytes, void** out) {
   if (!pooled(ordinal) || bytes > kKeptBytes / 2) {
     const cudaError_t e = device_malloc(out, bytes ? bytes : 1);
     if (e != cudaSuccess) return e;
@@ -183,15 +178,14 @@ inline cudaError_t allocate(const void* context, int ordinal, cudaStream_t strea
   {
     Lock l(state().lock);
     captured = capturing(p);
-    auto& mine = p.aside[context];
-    auto it = mine.find(cls);
-    if (it != mine.end()) waiting = it->second.size();
+    auto it = p.aside.find(cls);
+    if (it != p.aside.end()) waiting = it->second.size();
   }
   if (!captured) {
     if ((*out = take(p, cls)) != nullptr) return cudaSuccess;
     // Until then new ones are mapped, which costs hundreds of microseconds for a large block: two of those do.
     if (waiting >= 32 || (waiting * cls >= (4ull << 20) && (waiting >= 2 || cls >= (64ull << 20))))
-      if (settle(p, context, stream) && (*out = take(p, cls)) != nullptr) return cudaSuccess;
+      if (settle(p) && (*out = take(p, cls)) != nullptr) return cudaSuccess;
   }
   const cudaError_t e = device_malloc(out, cls);
   if (e != cudaSuccess) return e;
@@ -200,8 +194,8 @@ inline cudaError_t allocate(const void* context, int ordinal, cudaStream_t strea
   return cudaSuccess;
 }
 
-// Frees a block on behalf of a context, whose device is current.
-inline cudaError_t give_back(const void* context, int ordinal, cudaStream_t stream, void* q) {
+// Frees a block on behalf of a context of a device, which is current, on its stream.
+inline cudaError_t give_back(int ordinal, cudaStream_t stream, void* q) {
   bool kept = false, full = false;
   {
     Lock l(state().lock);
@@ -210,7 +204,7 @@ inline cudaError_t give_back(const void* context, int ordinal, cudaStream_t stre
       if (it->second.kept) return cudaErrorInvalidValue;  // freed already: cudaFree's answer
       if (it->second.ordinal == ordinal && !capturing(of(ordinal))) {
         Pool& p = of(ordinal);
-        p.aside[context][it->second.cls].push_back(q);
+        p.aside[it->second.cls].push_back(q);
         p.bytes += it->second.cls;
         it->second.kept = kept = true;
         full = p.bytes > kKeptBytes;

@@ -137,14 +137,14 @@ RUAI_API int ruai_malloc(ruai_ctx* c, size_t bytes, void** out) {
   if (!c || !out) return ruai_fail(c, RUAI_ERR_ARG, "ruai_malloc: NULL argument");
   DeviceGuard g(c->ordinal);
   *out = nullptr;
-  RUAI_CUDA(c, block_pool::allocate(c, c->ordinal, c->stream, bytes, out));
+  RUAI_CUDA(c, block_pool::allocate(c->ordinal, bytes, out));
   return RUAI_OK;
 }
 
 RUAI_API int ruai_free(ruai_ctx* c, void* p) {
   if (!c) return ruai_fail(nullptr, RUAI_ERR_ARG, "ctx is NULL");
   DeviceGuard g(c->ordinal);
-  RUAI_CUDA(c, block_pool::give_back(c, c->ordinal, c->stream, p));
+  RUAI_CUDA(c, block_pool::give_back(c->ordinal, c->stream, p));
   return RUAI_OK;
 }
 

@@ -49,6 +49,7 @@ cudaError_t cudaMalloc(void** out, size_t bytes) {
 }
 cudaError_t cudaFree(void* p) {  // may wait for the device, or not
   std::lock_guard<std::mutex> g(fake::lock);
+  if (fake::busy.count(p)) { std::printf("memory in use goes back to the driver\n"); std::exit(1); }
   if (!p) return cudaSuccess;
   auto it = fake::memory.find((char*)p);
   if (it == fake::memory.end()) return cudaErrorInvalidValue;
@@ -85,9 +86,9 @@ struct Context {  // what ctx.cu makes of a ruai_ctx
   ~Context() { detach(this, ordinal); }
   void* get(size_t bytes) {
     void* p = nullptr;
-    return allocate(this, ordinal, stream, bytes, &p) == cudaSuccess ? p : nullptr;
+    return allocate(ordinal, bytes, &p) == cudaSuccess ? p : nullptr;
   }
-  cudaError_t put(void* p) { return give_back(this, ordinal, stream, p); }
+  cudaError_t put(void* p) { return give_back(ordinal, stream, p); }
 };
 constexpr size_t MB = 1 << 20;
 
@@ -217,6 +218,27 @@ int main(int argc, char** argv) {
     size_t out = p ? 4 * MB : 0;
     if (what != "trim during a wait") out += 20 * 32 * MB + 4096;
     CHECK(of(0).bytes == fake::used - out);
+  } else if (what == "used by another stream") {  // nothing but a wait for the whole device ends that use
+    Context a(0), b(1);
+    for (size_t bytes : {size_t(4096), 4 * MB, 64 * MB}) {
+      void* p = a.get(bytes);
+      fake::busy.insert(p);
+      CHECK(a.put(p) == cudaSuccess);
+      for (int i = 0; i < 200; ++i) {
+        void* q = (i & 1 ? a : b).get(bytes);
+        CHECK(!fake::busy.count(q));
+        a.put(q);
+      }
+      CHECK(fake::busy.empty());
+    }
+  } else if (what == "limit with work going on") {
+    Context c(0);
+    std::vector<void*> all;
+    for (int i = 0; i < 40; ++i) all.push_back(c.get(32 * MB));
+    for (void* p : all) {
+      fake::busy.insert(p);
+      c.put(p);
+    }
   } else {
     std::printf("no scenario \"%s\"\n", what.c_str());
     return 2;
