@@ -17,6 +17,7 @@
 #include <list>
 #include <map>
 #include <mutex>
+#include <new>
 #include <unordered_map>
 #include <utility>
 
@@ -67,8 +68,12 @@ inline void forget(const Blocks& all) {  // the lock is held, the blocks are abo
 }
 
 inline void merge(Blocks& to, Blocks& from) {
-  for (auto& kv : from) to[kv.first].splice(to[kv.first].end(), kv.second);
-  from.clear();
+  while (!from.empty()) {  // of nodes that exist: nothing here can throw
+    auto node = from.extract(from.begin());
+    auto it = to.find(node.key());
+    if (it == to.end()) to.insert(std::move(node));
+    else it->second.splice(it->second.end(), node.mapped());
+  }
 }
 
 // Waits for the device and makes the blocks set aside before that clean.
@@ -129,10 +134,16 @@ inline void* take(Pool& p, size_t cls) {
 }
 
 // A context of the device more; the device's last one to go gives the kept memory back.
-inline void attach(const void* context, int ordinal, cudaStream_t stream) {
-  if (!pooled(ordinal)) return;
-  Lock l(state().lock);
-  of(ordinal).contexts[context] = stream;
+// false: the host is out of memory.  (Callers of the C interface cannot catch what the containers throw.)
+inline bool attach(const void* context, int ordinal, cudaStream_t stream) {
+  if (!pooled(ordinal)) return true;
+  try {
+    Lock l(state().lock);
+    of(ordinal).contexts[context] = stream;
+  } catch (const std::bad_alloc&) {
+    return false;
+  }
+  return true;
 }
 inline void detach(const void* context, int ordinal) {
   if (!pooled(ordinal)) return;
@@ -189,8 +200,11 @@ inline cudaError_t allocate(int ordinal, size_t bytes, void** out) {
   }
   const cudaError_t e = device_malloc(out, cls);
   if (e != cudaSuccess) return e;
-  Lock l(state().lock);
-  state().blocks[*out] = {cls, ordinal, false};
+  try {
+    Lock l(state().lock);
+    state().blocks[*out] = {cls, ordinal, false};
+  } catch (const std::bad_alloc&) {  // not in the book: its ruai_free is cudaFree's
+  }
   return cudaSuccess;
 }
 
@@ -204,10 +218,13 @@ inline cudaError_t give_back(int ordinal, cudaStream_t stream, void* q) {
       if (it->second.kept) return cudaErrorInvalidValue;  // freed already: cudaFree's answer
       if (it->second.ordinal == ordinal && !capturing(of(ordinal))) {
         Pool& p = of(ordinal);
-        p.aside[it->second.cls].push_back(q);
-        p.bytes += it->second.cls;
-        it->second.kept = kept = true;
-        full = p.bytes > kKeptBytes;
+        try {
+          p.aside[it->second.cls].push_back(q);
+          p.bytes += it->second.cls;
+          it->second.kept = kept = true;
+          full = p.bytes > kKeptBytes;
+        } catch (const std::bad_alloc&) {  // then it goes back to the driver
+        }
       }
     }
   }

@@ -65,7 +65,10 @@ RUAI_API int ruai_ctx_create(int ordinal, void* stream_or_null, ruai_ctx** out) 
   }
   int rc = ruai_ctx_reserve(c, 8u << 20, 4096);
   if (rc != RUAI_OK) { g_ruai_global_err = c->err; delete c; return rc; }
-  block_pool::attach(c, ordinal, c->stream);
+  if (!block_pool::attach(c, ordinal, c->stream)) {
+    ruai_ctx_destroy(c);
+    return ruai_fail(nullptr, RUAI_ERR_CUDA, "ruai_ctx_create: out of host memory");
+  }
   *out = c;
   return RUAI_OK;
 }

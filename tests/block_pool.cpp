@@ -9,6 +9,8 @@
 #include <string>
 #include <vector>
 
+#include <new>
+
 #include "../ruai_b200/csrc/block_pool.cuh"
 
 #define CHECK(c)                                                     \
@@ -16,7 +18,22 @@
     if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); std::exit(1); } \
   } while (0)
 
+// Operator new that can be told to fail.
+static bool host_memory_out = false;
+void* operator new(size_t n) {
+  void* p = host_memory_out ? nullptr : std::malloc(n ? n : 1);
+  if (!p) throw std::bad_alloc();
+  return p;
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
+
 namespace fake {
+struct Host {  // the stand-in's own containers are not what fails
+  bool was = host_memory_out;
+  Host() { host_memory_out = false; }
+  ~Host() { host_memory_out = was; }
+};
 std::mutex lock;
 std::map<char*, size_t> memory;      // what the driver has handed out
 std::vector<std::pair<char*, size_t>> freed;  // addresses to hand out again, last first
@@ -36,6 +53,7 @@ cudaStream_t stream(int i) { return (cudaStream_t)(size_t)(16 + i); }
 
 extern "C" {
 cudaError_t cudaMalloc(void** out, size_t bytes) {
+  const fake::Host h;
   std::lock_guard<std::mutex> g(fake::lock);
   if (fake::used + bytes > fake::limit) return cudaErrorMemoryAllocation;
   char* at = fake::next;
@@ -48,6 +66,7 @@ cudaError_t cudaMalloc(void** out, size_t bytes) {
   return cudaSuccess;
 }
 cudaError_t cudaFree(void* p) {  // may wait for the device, or not
+  const fake::Host h;
   std::lock_guard<std::mutex> g(fake::lock);
   if (fake::busy.count(p)) { std::printf("memory in use goes back to the driver\n"); std::exit(1); }
   if (!p) return cudaSuccess;
@@ -82,7 +101,7 @@ using namespace block_pool;
 struct Context {  // what ctx.cu makes of a ruai_ctx
   int ordinal;
   cudaStream_t stream;
-  explicit Context(int i, int ordinal_ = 0) : ordinal(ordinal_), stream(fake::stream(i)) { attach(this, ordinal, stream); }
+  explicit Context(int i, int ordinal_ = 0) : ordinal(ordinal_), stream(fake::stream(i)) { CHECK(attach(this, ordinal, stream)); }
   ~Context() { detach(this, ordinal); }
   void* get(size_t bytes) {
     void* p = nullptr;
@@ -239,6 +258,16 @@ int main(int argc, char** argv) {
       fake::busy.insert(p);
       c.put(p);
     }
+  } else if (what == "host memory out") {         // what a C caller could not catch
+    Context c(0);
+    void *p = c.get(4096), *q = c.get(8192);
+    host_memory_out = true;
+    void* r = c.get(4096);
+    const bool attached = attach(&p, 0, c.stream);
+    const cudaError_t first = c.put(p), second = c.put(r);
+    host_memory_out = false;
+    CHECK(r && !attached && first == cudaSuccess && second == cudaSuccess);
+    CHECK(!fake::memory.count((char*)p) && !fake::memory.count((char*)r) && c.put(q) == cudaSuccess);
   } else {
     std::printf("no scenario \"%s\"\n", what.c_str());
     return 2;

@@ -21,6 +21,7 @@ def program(tmp_path_factory):
     "freed twice", "freed through another device", "address of a block that cudaFree took",
     "trim during a wait", "out of memory during a wait",
     "used by another stream", "limit with work going on",
+    "host memory out",
 ])
 def test_scenario(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=60)
