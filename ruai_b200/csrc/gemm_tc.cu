@@ -2,12 +2,19 @@
 //
 // Replaces the reference's "dequantize the whole weight to f32, cast, cuBLAS" route for m > 16
 // (src/nn/backend/cuda.rs:812-826) with one kernel that keeps the weight packed in HBM:
-//   - the activations are scaled by a power of two per row and split once, by a small pre-kernel, into two fp16 pieces
-//     x = hi + lo (22 significant bits; bf16 and fp16 activations are one piece, exactly) stored as the tensor core's B
-//     operand: K-major with the 128-byte swizzle, so that a stage of 64 k is one bulk copy;
-//   - packed tiles of W (the chunk layout of pack.cu) come through a ring of bulk copies of their own and are expanded to fp16
-//     (int4 and int8 values are exact) in tensor memory, the A operand;
-//   - `tcgen05.mma kind::f16`, D[128 columns of W][rows of x], both pieces into the same f32 sums in tensor memory;
+//   - the activations are stored once, by a small pre-kernel, as the tensor core's B operand: K-major with the 128-byte swizzle,
+//     so that a stage of 64 k is one bulk copy.  f32 is scaled by a power of two per row and split into two fp16 pieces, 22
+//     significant bits; fp16 is one piece as it is; so is bf16 for int4 (scaled to fp16 for int8).  What small elements keep is
+//     set by fp16's quantum of 2^-24, by their distance from the row's largest element:
+//       int4, x = hi + 2^-12 lo: 22 bits down to 2^-28, then a quantum of 2^-50 of the largest (17 bits at 2^-33);
+//       int8, x = hi + lo: 22 bits down to 2^-16, then a quantum of 2^-38 (17 bits at 2^-21); bf16 exact down to 2^-31.
+//     It shows only in a column whose weights for the large elements are all zero, since f32 sums have a quantum of 2^-24 of
+//     theirs.  (Zeros are common in int4.  For int8 the same form costs 13 to 15 %: its sums cannot stay in tensor memory over
+//     several stages then; 4096 x 4096 x 14336 835 -> 941 us, and 690 -> 764 with bf16 expanded weights);
+//   - packed tiles of W (the chunk layout of pack.cu) come through a ring of bulk copies of their own and are expanded to fp16 or
+//     bf16 (int4 and int8 values are exact) in tensor memory, the A operand;
+//   - `tcgen05.mma kind::f16`, D[128 columns of W][rows of x], both pieces into the same f32 sums in tensor memory; int4: the lo
+//     products first, the first hi product scales them by 2^-12 (exact);
 //   - draining warps (thread = column of W) read the sums of every segment out and add them in f32 registers: int4: a segment
 //     is a scale group of 32 k, times scale[g, j] (cpu.rs:1045-1063); int8: four stages, so that the tensor core's own
 //     additions stay short, with the column scale at the end (cpu.rs:903-920).
@@ -28,6 +35,7 @@ namespace gemm_tc {
 using namespace pipe;
 
 constexpr int kSegStages = 4;    // int8: stages per segment
+constexpr int kLoShift = 12;     // int4: lo pieces are stored times 2^12.  Hi pieces below 2^15 leave out 2^3 at most: they stay below 2^15 too
 
 // ---- activations -> fp16 pieces in B-operand layout --------------------------------------------------
 // xs[row block of NT][stage][piece][row / 8][row % 8][8 chunks of 8 k, at chunk ^ (row % 8)]; the k of every four are stored in
@@ -35,6 +43,8 @@ constexpr int kSegStages = 4;    // int8: stages per segment
 struct SplitParams {
   const void* x;
   int x_dtype, pieces, vec;
+  int raw;               // one piece, fp16 or bf16 as it is
+  float lo_scale;
   uint32_t x_ld, m, k, stages, nt;
   const float* norm_w;   // RMSNorm folded in: x * norm_w
   const float* sumsq;    // [tiles][m] sums of squares of the row, or NULL: this kernel takes them (row_norm)
@@ -70,6 +80,9 @@ __device__ __forceinline__ void load8(const SplitParams& p, uint32_t row, uint32
   }
 }
 
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {  // of values that are bf16
+  return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
+}
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
   const __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&h);
@@ -88,7 +101,7 @@ __global__ void __launch_bounds__(kSplitThreads) xsplit_kernel(const SplitParams
       if (k0 + t < p.k) v[t] *= p.norm_w[k0 + t];
   };
   float f = 1.0f, back = 1.0f;
-  if (p.x_dtype != RUAI_F16 || p.norm_w) {  // the row's largest magnitude (and its sum of squares)
+  if (!p.raw) {  // the row's largest magnitude (and its sum of squares)
     float mx = 0.0f, ss = 0.0f;
     for (uint32_t c = tid; c * 8u < p.k; c += kSplitThreads) {
       float v[8];
@@ -111,8 +124,8 @@ __global__ void __launch_bounds__(kSplitThreads) xsplit_kernel(const SplitParams
     mx = 0.0f; ss = 0.0f;
 #pragma unroll
     for (int w = 0; w < kSplitThreads / 32; ++w) { mx = fmaxf(mx, red[0][w]); ss += red[1][w]; }
-    // scaled by 2^e the largest magnitude lies in [2^14, 2^15): both pieces of everything down to 2^-28 of it are normal fp16
-    // numbers or exact, and nothing overflows.  Zero and infinite rows stay as they are.
+    // scaled by 2^e the largest magnitude lies in [2^14, 2^15): nothing overflows, and hi pieces are normal fp16 numbers down to
+    // 2^-28 of it.  Zero and infinite rows stay as they are.
     const int ex = (int)((__float_as_uint(mx) >> 23) & 0xFFu) - 127;
     if (mx > 0.0f && ex < 128) {
       const int e = min(14 - ex, 126);
@@ -128,6 +141,7 @@ __global__ void __launch_bounds__(kSplitThreads) xsplit_kernel(const SplitParams
   }
   if (tid == 0) p.rowf[row] = back;
   const uint32_t r = row % p.nt, piece = p.nt * 128u;
+  const bool bf = p.raw && p.x_dtype == RUAI_BF16;
   unsigned char* base = p.xs + (size_t)(row / p.nt) * p.stages * p.pieces * piece + (r >> 3) * 1024u + (r & 7u) * 128u;
   for (uint32_t c = tid; c < chunks; c += kSplitThreads) {
     float v[8];
@@ -139,14 +153,14 @@ __global__ void __launch_bounds__(kSplitThreads) xsplit_kernel(const SplitParams
     for (int t = 0; t < 8; ++t) v[t] *= f;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      h[2 * q] = pack_half2(v[4 * q], v[4 * q + 2]);
-      h[2 * q + 1] = pack_half2(v[4 * q + 1], v[4 * q + 3]);
+      h[2 * q] = bf ? pack_bf16(v[4 * q], v[4 * q + 2]) : pack_half2(v[4 * q], v[4 * q + 2]);
+      h[2 * q + 1] = bf ? pack_bf16(v[4 * q + 1], v[4 * q + 3]) : pack_half2(v[4 * q + 1], v[4 * q + 3]);
     }
     unsigned char* dst = base + (size_t)(c >> 3) * p.pieces * piece + (((c & 7u) ^ (r & 7u)) << 4);
     *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
     if (p.pieces == 2) {
 #pragma unroll
-      for (int t = 0; t < 8; ++t) lo[t] = v[t] - __half2float(__float2half_rn(v[t]));
+      for (int t = 0; t < 8; ++t) lo[t] = (v[t] - __half2float(__float2half_rn(v[t]))) * p.lo_scale;
       uint32_t l[4];
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
@@ -180,6 +194,12 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {  // K-major, 128
 __device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b),
                "r"(idesc), "r"(accumulate)
+               : "memory");
+}
+// The same onto sums of lo pieces, which it brings to the hi pieces' scale.
+__device__ __forceinline__ void mma_f16_after_lo(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t}" ::"r"(d), "r"(a), "l"(b),
+               "r"(idesc), "n"(kLoShift)
                : "memory");
 }
 __device__ __forceinline__ bool elect_one() {
@@ -243,6 +263,19 @@ __device__ __forceinline__ void expand_int4(const uint4& q, uint32_t (&o)[16]) {
     o[2 * i + 1] = hsub2_bits((t & 0x000F000Fu) | 0x64006400u, 0x64086408u);      // rows 4i + 1, 4i + 3
     o[8 + 2 * i] = hfma2_bits((w[i] & 0x00F000F0u) | 0x64006400u, 0x2C002C00u, 0xD480D480u);  // 1024 + 16 u: / 16, - 72
     o[8 + 2 * i + 1] = hfma2_bits((t & 0x00F000F0u) | 0x64006400u, 0x2C002C00u, 0xD480D480u);
+  }
+}
+// The same to bf16: 128 + u has the bit pattern 0x4300 | u for u < 128.
+__device__ __forceinline__ void expand_int4_bf16(const uint4& q, uint32_t (&o)[16]) {
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w}, offset = 0x43084308u;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const uint32_t u = ((w[i] >> (8 * (n & 1) + 4 * (n >> 1))) & 0x000F000Fu) | 0x43004300u;
+      const __nv_bfloat162 r = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&u), *reinterpret_cast<const __nv_bfloat162*>(&offset));
+      o[(n >> 1) * 8 + 2 * i + (n & 1)] = *reinterpret_cast<const uint32_t*>(&r);
+    }
   }
 }
 __device__ __forceinline__ void expand_int8(const uint4& q, uint32_t* o) {
@@ -310,7 +343,7 @@ __device__ __forceinline__ void finish_rows(const Params& p, uint32_t end, float
   }
 }
 
-template <int BITS, int CB, int NT>
+template <int BITS, int CB, int NT, bool BF>  // BF: both operands in bf16 (one piece)
 __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kernel(const Params p) {
   using T = Tile<BITS, CB, NT>;
   constexpr uint32_t XS = T::kXSlots, WS = T::kWSlots, AB = T::kABufs;
@@ -357,7 +390,8 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
     tc_fence_after_sync();
     for (uint32_t u = u0; u < u1; ++u) {
       uint32_t o[16];
-      if constexpr (BITS == 4) expand_int4(*reinterpret_cast<const uint4*>(w + u * T::kWChunk), o);
+      if constexpr (BF) expand_int4_bf16(*reinterpret_cast<const uint4*>(w + u * T::kWChunk), o);
+      else if constexpr (BITS == 4) expand_int4(*reinterpret_cast<const uint4*>(w + u * T::kWChunk), o);
       else {
         const uint4 q0 = *reinterpret_cast<const uint4*>(w + 2 * u * T::kWChunk), q1 = *reinterpret_cast<const uint4*>(w + (2 * u + 1) * T::kWChunk);
         expand_int8(q0, o);
@@ -417,7 +451,7 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
       // ===== MMAs.  A wait behind MMAs comes back only when those have left the issue queue (measured: 90 to 260 clocks in which
       // the tensor pipe has nothing to do), so two threads issue, each into its own sums: one per column block, or, with one
       // column block, every other stage each. =====
-      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((128u >> 4) << 24);  // fp16 x fp16 -> f32
+      constexpr uint32_t idesc = (1u << 4) | (BF ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(NT >> 3) << 17) | ((128u >> 4) << 24);  // fp16 x fp16 or bf16 x bf16 -> f32
       const uint64_t xd0 = desc_sw128(smem_u32(smem));
       const uint32_t pieces = (uint32_t)p.pieces, h = (uint32_t)warp - 1u, cb = CB == 2 ? h : 0u;
       uint32_t it = 0, unit = BITS == 4 && CB == 1 ? 0u : h;
@@ -437,11 +471,16 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
               for (uint32_t u = 0; u < ng; ++u, unit += CB) {
                 if (!sums_free(unit)) { ok = false; break; }
                 tc_fence_after_sync();
-                const uint32_t d = tmem + (unit % 3) * NT;
-                for (uint32_t pc = 0; pc < pieces; ++pc)
-#pragma unroll
-                  for (uint32_t q = 0; q < 2; ++q)
-                    mma_f16(d, a + u * 16 + q * 8, umma_desc_advance(xd, pc * T::kPiece + u * 64u + q * 32u), idesc, (pc | q) != 0 ? 1u : 0u);
+                const uint32_t d = tmem + (unit % 3) * NT, au = a + u * 16;
+                const uint64_t xu = umma_desc_advance(xd, u * 64u);
+                if (pieces == 2) {
+                  mma_f16(d, au, umma_desc_advance(xu, T::kPiece), idesc, 0u);
+                  mma_f16(d, au + 8, umma_desc_advance(xu, T::kPiece + 32u), idesc, 1u);
+                  mma_f16_after_lo(d, au, xu, idesc);
+                } else {
+                  mma_f16(d, au, xu, idesc, 0u);
+                }
+                mma_f16(d, au + 8, umma_desc_advance(xu, 32u), idesc, 1u);
                 umma_commit(&acc_full[unit % 3]);
               }
             } else {
@@ -606,12 +645,12 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
   if (warp == 2) tmem_dealloc(tmem, T::kTmem);
 }
 
-template <int BITS, int CB, int NT>
+template <int BITS, int CB, int NT, bool BF>
 cudaError_t launch(ruai_ctx* c, const Params& p) {
   using T = Tile<BITS, CB, NT>;
   static bool attr_done[64] = {};
   if (!attr_done[c->ordinal & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BITS, CB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BITS, CB, NT, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmem);
     if (e != cudaSuccess) return e;
     attr_done[c->ordinal & 63] = true;
   }
@@ -637,10 +676,15 @@ cudaError_t launch(ruai_ctx* c, const Params& p) {
   cfg.attrs = attr;
   cfg.numAttrs = na;
   c->launches++;
-  return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BITS, CB, NT>, p);
+  return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BITS, CB, NT, BF>, p);
 }
 
 struct Shape { uint32_t cb, nt, splits; };
+
+template <int BITS, bool BF>
+cudaError_t launch_tile(ruai_ctx* c, const Params& p, const Shape& sh) {
+  return sh.cb == 2 ? launch<BITS, 2, 128, BF>(c, p) : sh.nt == 128 ? launch<BITS, 1, 128, BF>(c, p) : launch<BITS, 1, 64, BF>(c, p);
+}
 
 // The tile and the number of splits of k: a model of the launch in microseconds, fitted to launches of 37 to 2000 rows of the 1.1B and
 // 8B shapes' Linears with every tile and 1 .. 8 splits (the choice is within 5 % of the best of them; a wrong one costs up to 2 x).
@@ -680,7 +724,7 @@ int ruai_gemm_tc_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x
   if (epi.sumsq || epi.argmax_out) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "the prefill GEMM has no fused sum of squares / argmax");
   if ((m + 127u) / 128u > 65535u) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "m too large");
   const uint32_t groups = (w->k + 31) / 32, stages = (groups + 1) / 2;
-  // fp16 and bf16 activations are one fp16 piece (bf16: after the row's scaling); not when a norm multiplies them
+  // fp16 and bf16 activations are one piece; not when a norm multiplies them
   const int pieces = x_dtype == RUAI_F32 || pro.norm_w ? 2 : 1;
   Shape sh = choose(c, m, w->n, stages, w->bits, pieces);
   if (c->force_splits >= 1 && c->force_splits <= 8) {
@@ -695,6 +739,8 @@ int ruai_gemm_tc_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x
   sp.x = x; sp.x_dtype = x_dtype; sp.pieces = pieces; sp.x_ld = x_ld; sp.m = m; sp.k = w->k; sp.stages = stages; sp.nt = sh.nt;
   sp.vec = ((uintptr_t)x & 15u) == 0 && x_ld % (x_dtype == RUAI_F32 ? 4u : 8u) == 0 ? 1 : 0;
   sp.norm_w = pro.norm_w; sp.sumsq = pro.sumsq; sp.tiles = pro.tiles; sp.row_norm = pro.norm_w && !pro.sumsq ? 1 : 0; sp.eps = pro.eps;
+  sp.raw = pieces == 1 && (x_dtype == RUAI_F16 || w->bits == 4) ? 1 : 0;
+  sp.lo_scale = w->bits == 4 ? (float)(1 << kLoShift) : 1.0f;
   sp.xs = reinterpret_cast<unsigned char*>(c->partial);
   sp.rowf = reinterpret_cast<float*>(sp.xs + xs_bytes);
   RUAI_CUDA(c, ruai_launch(c, xsplit_kernel, dim3(m), dim3(kSplitThreads), 0, true, sp));
@@ -703,11 +749,7 @@ int ruai_gemm_tc_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x
   p.stages = stages; p.splits = sh.splits; p.stages_per_split = (stages + sh.splits - 1) / sh.splits;
   p.row_blocks = row_blocks; p.tiles = row_blocks * col_tiles; p.pieces = pieces;
   p.out = out; p.status = c->status; p.epi = epi;
-  cudaError_t e;
-  if (w->bits == 8)
-    e = sh.cb == 2 ? launch<8, 2, 128>(c, p) : sh.nt == 128 ? launch<8, 1, 128>(c, p) : launch<8, 1, 64>(c, p);
-  else
-    e = sh.cb == 2 ? launch<4, 2, 128>(c, p) : sh.nt == 128 ? launch<4, 1, 128>(c, p) : launch<4, 1, 64>(c, p);
+  const cudaError_t e = w->bits == 8 ? launch_tile<8, false>(c, p, sh) : sp.raw && x_dtype == RUAI_BF16 ? launch_tile<4, true>(c, p, sh) : launch_tile<4, false>(c, p, sh);
   if (e != cudaSuccess) return ruai_fail(c, RUAI_ERR_CUDA, "prefill GEMM launch failed: %s", cudaGetErrorString(e));
   return RUAI_OK;
 }

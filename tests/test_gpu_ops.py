@@ -408,6 +408,26 @@ def test_gemm_tiles_against_float64(dev, m, k, n, bits):
         dev.force_splits(0)
 
 
+@pytest.mark.parametrize("dtype,bits,ratio,quantum", [("f32", 4, 28, 2.0 ** -50), ("f32", 8, 20, 2.0 ** -38), ("bf16", 4, 100, 0.0), ("bf16", 8, 28, 0.0), ("f16", 4, 14, 0.0), ("f16", 8, 14, 0.0)])
+@pytest.mark.parametrize("m,k,n", [(37, 544, 300), (150, 1504, 516)])
+def test_gemm_small_elements_beside_large_ones(dev, m, k, n, dtype, bits, ratio, quantum):
+    """Every row has elements 2^ratio times the others whose weights are zero: what the others keep is seen alone.  A scaled row's pieces
+    round to half their quantum of the row's largest; 16-bit elements are exact, and the output is rounded to their type."""
+    w = oracle.synth_normal(35, k * 65537 + n, (k, n))
+    w[5::97] = 0.0
+    q, s = oracle.quantize_int8(w) if bits == 8 else oracle.quantize_int4(w, 32)
+    qw = nn.QWeight.int8(dev, q, s) if bits == 8 else nn.QWeight.int4(dev, q, s, 32)
+    wd = q.astype(np.float64) * s if bits == 8 else qw.dequant().astype(np.float64)
+    x = oracle.synth_normal(35, m, (m, k), 1.0)
+    x = np.where(np.abs(x) < 0.5, 0.5, x).astype(np.float32)  # none further below the row's largest than stated
+    x[:, 5::97] = 2.0 ** ratio
+    xf, got = run_matmul(dev, x, qw, dtype)
+    want, mag = xf.astype(np.float64) @ wd, np.abs(xf).astype(np.float64) @ np.abs(wd)
+    bound = 2.0 ** -20 * mag + 0.5 * quantum * np.abs(xf).max(1, keepdims=True).astype(np.float64) * np.abs(wd).sum(0)
+    bound += {"f32": 0.0, "f16": 2.0 ** -11, "bf16": 2.0 ** -8}[dtype] * np.abs(want) + 1e-7
+    assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
+
+
 @pytest.mark.parametrize("m,n", [(88320, 384), (88320, 300)])
 def test_gemm_of_one_group_over_many_tiles(dev, m, n):
     """k of one scale group and a dozen column blocks per CTA: the scales' ring goes round with one group per stage."""
