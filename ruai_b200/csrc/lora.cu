@@ -69,7 +69,8 @@ __global__ void __launch_bounds__(kThreads) grad_input_chunk_kernel(const uint4*
 // owns 8 x 4 results; g is kept twice side by side, so that packed multiply-adds (two f32 in one instruction, each rounded like fmaf)
 // need no shuffling: five 16-byte reads from shared memory per 16 of them.  The columns are shared out over gridDim.z CTAs for about
 // four CTAs per SM; the shares are added in a fixed order by sum_shares_kernel.  Bound by f32 multiply-adds and their operands'
-// reads: 256 x 2048 x 2048 int4 114 us (a row of g at a time, as before: 344 us).
+// reads: 256 x 2048 x 2048 int4 115 us (a row of g at a time: 344 us).  The sums' additions are a fifth of the multiply-adds and
+// within what the reads leave free: four CTAs per SM (128 registers) 115 us, three with 158 registers 123.
 // Up to here a row at a time is faster (us, k x n): 16 rows int4 2048 x 2048 27 against 26, int8 22 against 26; 4096 x 4096 80 and 65
 // against 80; 24 rows 39 and 32 against 28, 116 and 95 against 84.
 constexpr uint32_t kGradFewRows = 18;
@@ -79,8 +80,19 @@ __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(b), "l"(0xBF800000BF800000ull), "l"(a));
+  return r;
+}
+
 template <int BITS>
-__global__ void __launch_bounds__(kGradThreads) grad_input_kernel(const uint4* __restrict__ w, const float* __restrict__ scale, const float* __restrict__ g,
+__global__ void __launch_bounds__(kGradThreads, 4) grad_input_kernel(const uint4* __restrict__ w, const float* __restrict__ scale, const float* __restrict__ g,
                                                                   uint32_t m, uint32_t k, uint32_t n, uint32_t chunks, uint32_t cols_per_share, float* __restrict__ out) {
   constexpr int kChunkRows = BITS == 4 ? 32 : 16, kTileChunks = kGradTile / kChunkRows;
   constexpr int kLoads = kTileChunks * kGradCols / kGradThreads > 0 ? kTileChunks * kGradCols / kGradThreads : 1;  // chunks per thread and step
@@ -132,40 +144,52 @@ __global__ void __launch_bounds__(kGradThreads) grad_input_kernel(const uint4* _
     for (uint32_t t = 0; t < kGHalf; ++t) gs[b][gj + t][gi] = make_float2(gv[t], gv[t]);
   };
   const uint32_t tr = (tid / 16) * 8, tk = (tid % 16) * 4;  // this thread's 8 rows of g x 4 rows of W
-  // sums of 32 columns, added up separately: the rounding error grows with the longer of two short chains
+  // Sums of a step's 16 columns, added up; what an addition leaves out (exactly, where the sum so far is the larger) starts the next step's
+  // sum, so that the rounding error is that of a chain of 16 however long the share is.  An infinite sum leaves a NaN out: where a sum is
+  // not finite in the end, the CTA starts over without.
   unsigned long long acc[8][2], sum[8][2];
+  for (bool plain = false;; plain = true) {
 #pragma unroll
-  for (int r = 0; r < 8; ++r) { acc[r][0] = acc[r][1] = 0ull; sum[r][0] = sum[r][1] = 0ull; }
-  if (j_begin < j_end) {
-    load(j_begin);
-    store(0);
-  }
-  __syncthreads();
-  int b = 0;
-  for (uint32_t j0 = j_begin; j0 < j_end; j0 += kGradCols, b ^= 1) {
-    const bool more = j0 + kGradCols < j_end;
-    if (more) load(j0 + kGradCols);
-#pragma unroll 8
-    for (int j = 0; j < kGradCols; ++j) {
-      const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(&ws[b][j][tk]);
-#pragma unroll
-      for (int r = 0; r < 8; r += 2) {
-        const ulonglong2 gp = *reinterpret_cast<const ulonglong2*>(&gs[b][j][tr + r]);
-        fma2(acc[r][0], gp.x, wv.x); fma2(acc[r][1], gp.x, wv.y);
-        fma2(acc[r + 1][0], gp.y, wv.x); fma2(acc[r + 1][1], gp.y, wv.y);
-      }
+    for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = sum[r][0] = sum[r][1] = 0ull;
+    if (j_begin < j_end) {
+      load(j_begin);
+      store(0);
     }
-    if (b == 1 || !more) {
+    __syncthreads();
+    int b = 0;
+    for (uint32_t j0 = j_begin; j0 < j_end; j0 += kGradCols, b ^= 1) {
+      const bool more = j0 + kGradCols < j_end;
+      if (more) load(j0 + kGradCols);
+#pragma unroll 8
+      for (int j = 0; j < kGradCols; ++j) {
+        const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(&ws[b][j][tk]);
+#pragma unroll
+        for (int r = 0; r < 8; r += 2) {
+          const ulonglong2 gp = *reinterpret_cast<const ulonglong2*>(&gs[b][j][tr + r]);
+          fma2(acc[r][0], gp.x, wv.x); fma2(acc[r][1], gp.x, wv.y);
+          fma2(acc[r + 1][0], gp.y, wv.x); fma2(acc[r + 1][1], gp.y, wv.y);
+        }
+      }
 #pragma unroll
       for (int r = 0; r < 8; ++r)
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[r][t]) : "l"(acc[r][t]));
-          acc[r][t] = 0ull;
+          const unsigned long long now = add2(sum[r][t], acc[r][t]);
+          acc[r][t] = plain ? 0ull : sub2(acc[r][t], sub2(now, sum[r][t]));
+          sum[r][t] = now;
         }
+      if (more) store(b ^ 1);
+      __syncthreads();
     }
-    if (more) store(b ^ 1);
-    __syncthreads();
+    bool finite = true;
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        sum[r][t] = add2(sum[r][t], acc[r][t]);
+        finite = finite && isfinite(__uint_as_float((uint32_t)sum[r][t])) && isfinite(__uint_as_float((uint32_t)(sum[r][t] >> 32)));
+      }
+    if (plain || !__syncthreads_or(!finite)) break;
   }
   float* dst = out + (size_t)blockIdx.z * m * k;
 #pragma unroll
@@ -183,9 +207,19 @@ __global__ void __launch_bounds__(kGradThreads) grad_input_kernel(const uint4* _
 __global__ void __launch_bounds__(kThreads) sum_shares_kernel(const float* __restrict__ part, size_t count, uint32_t shares, float* __restrict__ out) {
   const size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x;
   if (i >= count) return;
-  float v = part[i];
-  for (uint32_t s = 1; s < shares; ++s) v += part[(size_t)s * count + i];
-  out[i] = v;
+  float v = 0.0f, low = 0.0f;  // low: what the additions leave out
+  for (uint32_t s0 = 0; s0 < shares; s0 += 8) {
+    float a[8];  // requested together
+#pragma unroll
+    for (uint32_t t = 0; t < 8; ++t) a[t] = s0 + t < shares ? __ldcg(part + (size_t)(s0 + t) * count + i) : 0.0f;
+#pragma unroll
+    for (uint32_t t = 0; t < 8; ++t) {
+      const float now = __fadd_rn(v, a[t]);
+      low += __fsub_rn(a[t], __fsub_rn(now, v));
+      v = now;
+    }
+  }
+  out[i] = isfinite(low) ? v + low : v;  // an infinite sum leaves no number out
 }
 
 // dx for int4 weights kept in the reference layout (groups other than 32): one packed row (two rows of k)

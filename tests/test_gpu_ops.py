@@ -454,6 +454,40 @@ def test_grad_input_tiles_against_float64(dev, m, k, n, bits):
     assert (np.abs(got - want) <= (n + 3) * 2.0 ** -24 * mag + 1e-30).all()
 
 
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("m,k,n", [(19, 512, 512), (256, 2048, 2048), (64, 2048, 4096), (512, 4096, 1500), (40, 1024, 600)])
+def test_grad_input_error_does_not_grow_with_the_columns(dev, m, k, n, bits):
+    """Sums of 16 terms whose additions' rests are carried on: sixteen roundings of a growing sum, sqrt(16 / 2) 2^-24 / sqrt(3) = 0.97e-7 of
+    the result in the 2-norm at the most (each rounding uniform within half a unit in the last place)."""
+    q, s, qw = _qw(dev, bits, k, n, 36)
+    wd = (q * s).astype(np.float64) if bits == 8 else qw.dequant().astype(np.float64)
+    g = oracle.synth_normal(36, m, (m, n), 1.0)
+    want = g.astype(np.float64) @ wd.T
+    got = nn.matmul_q_grad_input(nn.Tensor.from_numpy(dev, g), qw).numpy().astype(np.float64)
+    assert np.linalg.norm(got - want) <= 1.0e-7 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("m,k,n", [(19, 64, 2000), (65, 4096, 300), (600, 4096, 80)])
+def test_grad_input_infinities_and_nans(dev, m, k, n, bits):
+    """A row with an infinity sums to infinities, one with a NaN or with both infinities to NaN; the other rows are what they were."""
+    q, s, qw = _qw(dev, bits, k, n, 37)
+    g = oracle.synth_normal(37, m, (m, n), 1.0)
+    T = lambda v: nn.matmul_q_grad_input(nn.Tensor.from_numpy(dev, v), qw).numpy()
+    plain = T(g)
+    bad = g.copy()
+    bad[0, 3], bad[1, n - 1], bad[2, 7], bad[m - 1, 5], bad[m - 1, n - 5] = np.inf, -np.inf, np.nan, np.inf, -np.inf
+    bad[3, 0] = bad[3, 1] = 3e38  # overflows, or not, by the weights' signs
+    got = T(bad)
+    wd = (q * s).astype(np.float64) if bits == 8 else qw.dequant().astype(np.float64)
+    with np.errstate(invalid="ignore", over="ignore"):
+        want = bad[[0, 1, 2, m - 1]].astype(np.float64) @ wd.T
+    for row, w in zip(got[[0, 1, 2, m - 1]], want):
+        assert np.array_equal(np.isnan(row), np.isnan(w)) and np.array_equal(row[np.isinf(w)], w[np.isinf(w)].astype(np.float32))
+    others = np.r_[4:m - 1]
+    assert np.allclose(got[others], plain[others], rtol=1e-5, atol=1e-6)
+
+
 def test_freed_tensors_are_reused_only_after_a_wait(dev):
     """Blocks freed while their context's stream still works on them do not come back before that work is done."""
     q, s, qw = _qw(dev, 8, 2048, 2048, 33)
