@@ -101,6 +101,10 @@ struct DeviceGuard {
 // cudaMalloc that gives the blocks kept by ruai_free back before it fails.
 cudaError_t ruai_device_malloc(void** out, size_t bytes);
 
+// What a context's scratch holds from the start: what the input gradient's shares need at the most (four CTAs per SM with 16 KB of sums
+// each, 9.7 MB), so that it never grows for them.
+constexpr size_t kScratchBytes = 10u << 20;
+
 // Grows the split-K scratch when a launch needs more (never inside a graph capture).
 int ruai_ctx_reserve(ruai_ctx* ctx, size_t partial_bytes, size_t counters);
 

@@ -63,7 +63,7 @@ RUAI_API int ruai_ctx_create(int ordinal, void* stream_or_null, ruai_ctx** out) 
     delete c;
     return ruai_fail(nullptr, RUAI_ERR_CUDA, "cannot allocate the status word");
   }
-  int rc = ruai_ctx_reserve(c, 8u << 20, 4096);
+  int rc = ruai_ctx_reserve(c, kScratchBytes, 4096);
   if (rc != RUAI_OK) { g_ruai_global_err = c->err; delete c; return rc; }
   if (!block_pool::attach(c, ordinal, c->stream)) {
     ruai_ctx_destroy(c);

@@ -313,12 +313,21 @@ RUAI_API int ruai_matmul_q_grad_input(ruai_ctx* c, const float* g_dev, const rua
     // about four CTAs per SM, four steps at least for each
     uint32_t shares = 4u * (uint32_t)c->sm_count / (row_tiles * k_tiles);
     if (shares > steps / 4) shares = steps / 4;
+    // Their sums lie in the scratch as every context has it from the start: a call neither allocates nor waits.  A graph would keep the
+    // scratch's address, which a later call of another kind may change, so nothing is shared out in a capture.
+    const size_t out_bytes = (size_t)m * w->k * sizeof(float);
+    if (shares > kScratchBytes / out_bytes) shares = (uint32_t)(kScratchBytes / out_bytes);
+    if (shares > 1) {
+      cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+      RUAI_CUDA(c, cudaStreamIsCapturing(c->stream, &st));
+      if (st != cudaStreamCaptureStatusNone) shares = 1;
+    }
     if (shares < 1) shares = 1;
     const uint32_t cols = (steps + shares - 1) / shares * kGradCols;
     shares = (w->n + cols - 1) / cols;
     float* dst = dx_dev;
     if (shares > 1) {
-      RUAI_TRY(ruai_ctx_reserve(c, (size_t)shares * m * w->k * sizeof(float), 0));
+      RUAI_TRY(ruai_ctx_reserve(c, shares * out_bytes, 0));
       dst = c->partial;
     }
     const dim3 grid(k_tiles, row_tiles, shares);

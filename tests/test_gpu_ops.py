@@ -1,4 +1,6 @@
 """GPU parity of the op-level C ABI (quantizer, repack, dequant, quantized matmul) against the CPU checker."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -486,6 +488,72 @@ def test_grad_input_infinities_and_nans(dev, m, k, n, bits):
         assert np.array_equal(np.isnan(row), np.isnan(w)) and np.array_equal(row[np.isinf(w)], w[np.isinf(w)].astype(np.float32))
     others = np.r_[4:m - 1]
     assert np.allclose(got[others], plain[others], rtol=1e-5, atol=1e-6)
+
+
+class Capturing:
+    """A context on a stream of its own, whose work can be captured into a graph."""
+
+    def __init__(self):
+        self.cu = C.CDLL("libcuda.so.1")
+        self.stream, self.graph, self.exec = C.c_void_p(), C.c_void_p(), C.c_void_p()
+        assert self.cu.cuStreamCreate(C.byref(self.stream), 1) == 0  # not ordered with the legacy stream
+        self.dev = nn.Device.__new__(nn.Device)
+        self.dev.ordinal, self.dev.L, self.dev.ctx = 0, nn._lib.load(), C.c_void_p()
+        nn._lib.check(self.dev.L.ruai_ctx_create(0, self.stream, C.byref(self.dev.ctx)))
+
+    def begin(self):
+        assert self.cu.cuStreamBeginCapture_v2(self.stream, 1) == 0  # of this thread
+
+    def end(self):
+        return self.cu.cuStreamEndCapture(self.stream, C.byref(self.graph))
+
+    def replay(self):
+        if not self.exec:
+            assert self.cu.cuGraphInstantiateWithFlags(C.byref(self.exec), self.graph, C.c_ulonglong(0)) == 0
+        assert self.cu.cuGraphLaunch(self.exec, self.stream) == 0
+        self.dev.synchronize()
+
+    def close(self):
+        if self.exec:
+            self.cu.cuGraphExecDestroy(self.exec)
+        if self.graph:
+            self.cu.cuGraphDestroy(self.graph)
+        nn._lib.check(self.dev.L.ruai_ctx_destroy(self.dev.ctx))
+        assert self.cu.cuStreamDestroy_v2(self.stream) == 0
+
+
+@pytest.fixture()
+def capturing(dev):
+    c = Capturing()
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("m,k,n", [(256, 4096, 1024), (300, 1800, 1024), (20, 64, 300)])
+def test_grad_input_in_a_graph(dev, capturing, m, k, n):
+    """The gradient can be captured on a fresh context, and its graph replayed after the context's scratch has moved."""
+    d = capturing.dev
+    q, s, qw = _qw(d, 8, k, n, 38)
+    wd = (q * s).astype(np.float64)
+    gs = [oracle.synth_normal(38, i, (m, n), 1.0) for i in (1, 2)]
+    g, dx = nn.Tensor.from_numpy(d, gs[0]), nn.Tensor(d, (m, k), np.float32, nn.F32)
+    capturing.begin()
+    rc = d.L.ruai_matmul_q_grad_input(d.ctx, g.ptr, qw.h, dx.ptr, m)
+    assert capturing.end() == 0 and rc == 0
+
+    def check(v):
+        want = v.astype(np.float64) @ wd.T
+        assert np.linalg.norm(dx.numpy() - want) <= 1.0e-7 * np.linalg.norm(want)
+
+    capturing.replay()
+    check(gs[0])
+    _, _, big = _qw(d, 8, 4096, 256, 39)
+    nn._matmul_q(nn.Tensor.from_numpy(d, np.full((1000, 4096), 3.0, np.float32)), big)  # its scratch is larger than a context's first
+    d.check(d.L.ruai_memcpy_h2d(d.ctx, g.ptr, np.ascontiguousarray(gs[1]).ctypes.data_as(C.c_void_p), g.nbytes))
+    capturing.replay()
+    check(gs[1])
+    for t in (g, dx, qw, big):
+        t.free()
 
 
 def test_freed_tensors_are_reused_only_after_a_wait(dev):
