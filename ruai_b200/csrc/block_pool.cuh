@@ -231,16 +231,20 @@ inline cudaError_t give_back(int ordinal, cudaStream_t stream, void* q) {
   if (full) trim(of(ordinal));  // of sizes no longer asked for, most of it
   if (kept) return cudaSuccess;
   cudaError_t e = cudaStreamSynchronize(stream);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();  // it is reported here, and not by the next launch's check as well
+    return e;
+  }
   std::unordered_map<void*, Block>::node_type entry;
   {
     Lock l(state().lock);
     entry = state().blocks.extract(q);  // before another thread can be given the address
   }
   e = cudaFree(q);
-  if (e != cudaSuccess && entry) {
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
     Lock l(state().lock);
-    state().blocks.insert(std::move(entry));
+    if (entry) state().blocks.insert(std::move(entry));
   }
   return e;
 }

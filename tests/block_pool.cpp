@@ -41,6 +41,7 @@ size_t limit = ~(size_t)0, used = 0, waits = 0;
 std::set<cudaStream_t> capturing, spoiled;
 std::set<void*> busy;                // work that is still going on reads or writes it
 std::function<void()> during_wait;
+cudaError_t last = cudaSuccess;
 char* next = (char*)0x1000000;
 void wait() {
   if (!during_wait) return;
@@ -71,7 +72,7 @@ cudaError_t cudaFree(void* p) {  // may wait for the device, or not
   if (fake::busy.count(p)) { std::printf("memory in use goes back to the driver\n"); std::exit(1); }
   if (!p) return cudaSuccess;
   auto it = fake::memory.find((char*)p);
-  if (it == fake::memory.end()) return cudaErrorInvalidValue;
+  if (it == fake::memory.end()) return fake::last = cudaErrorInvalidValue;
   fake::used -= it->second;
   fake::freed.push_back(*it);
   fake::memory.erase(it);
@@ -79,7 +80,7 @@ cudaError_t cudaFree(void* p) {  // may wait for the device, or not
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
   fake::wait();
-  if (fake::capturing.count(s)) { fake::spoiled.insert(s); return cudaErrorStreamCaptureUnsupported; }
+  if (fake::capturing.count(s)) { fake::spoiled.insert(s); return fake::last = cudaErrorStreamCaptureUnsupported; }
   return cudaSuccess;
 }
 cudaError_t cudaDeviceSynchronize(void) {
@@ -92,7 +93,11 @@ cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* st) {
   *st = fake::capturing.count(s) ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
   return cudaSuccess;
 }
-cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaGetLastError(void) {
+  const cudaError_t e = fake::last;
+  fake::last = cudaSuccess;
+  return e;
+}
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 }
 
@@ -164,7 +169,7 @@ int main(int argc, char** argv) {
     void* p = c.get(4096);
     fake::capturing.insert(c.stream);
     CHECK(c.put(p) != cudaSuccess);
-    CHECK(fake::spoiled.count(c.stream));
+    CHECK(fake::spoiled.count(c.stream) && fake::last == cudaSuccess);  // the error is reported once
     fake::capturing.clear();
     for (int i = 0; i < 100; ++i) {
       void* q = c.get(4096);
@@ -197,7 +202,7 @@ int main(int argc, char** argv) {
     for (int i = 0; i < 40; ++i) all.push_back(c.get(4096));
     for (void* q : all) CHECK(c.put(q) == cudaSuccess);
     for (void* q : all) CHECK(c.put(q) != cudaSuccess && fake::memory.count((char*)q));
-    CHECK(c.put((void*)0x10) != cudaSuccess);  // not allocated at all: cudaFree's error
+    CHECK(c.put((void*)0x10) != cudaSuccess && fake::last == cudaSuccess);  // not allocated at all: cudaFree's error
   } else if (what == "freed through another device") {
     Context a(0, 0), b(1, 1);
     void* p = a.get(4096);

@@ -566,3 +566,18 @@ def test_freed_tensors_are_reused_only_after_a_wait(dev):
         for j in range(3):
             nn._matmul_q(xs[j], qw)
         assert np.array_equal(nn._matmul_q(xs[i], qw).numpy(), want[i])
+
+
+def test_memory_freed_in_a_capture_or_twice_is_refused(dev, capturing):
+    d = capturing.dev
+    p, q = C.c_void_p(), C.c_void_p()
+    d.check(d.L.ruai_malloc(d.ctx, 4096, C.byref(p)))
+    capturing.begin()
+    assert d.L.ruai_free(d.ctx, p) == nn._lib.ERR_CUDA
+    assert capturing.end() != 0 and not capturing.graph  # as a wait for the capturing stream ends it
+    d.check(d.L.ruai_free(d.ctx, p))
+    assert d.L.ruai_free(d.ctx, p) == nn._lib.ERR_CUDA and dev.L.ruai_free(dev.ctx, p) == nn._lib.ERR_CUDA
+    d.check(d.L.ruai_malloc(d.ctx, 4096, C.byref(q)))
+    d.check(d.L.ruai_free(d.ctx, q))
+    y = nn._matmul_q(nn.Tensor.from_numpy(dev, np.ones((3, 64), np.float32)), _qw(dev, 8, 64, 48, 44)[2])  # no error is left over for the next launch
+    assert np.isfinite(y.numpy()).all()
