@@ -351,7 +351,8 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
   __shared__ __align__(8) uint64_t x_full[XS], x_empty[XS];   // x of a stage landed; the MMAs that read it completed
   __shared__ __align__(8) uint64_t w_full[WS], w_empty[WS];   // a packed stage (and its scales) landed; expanded (every expanding warp)
   __shared__ __align__(8) uint64_t a_ready[AB], a_free[AB];   // A operand of a stage written; the MMAs that read it completed
-  __shared__ __align__(8) uint64_t acc_full[3], acc_free[3];  // the sums of a unit (segment, column block) complete; read out (the column block's draining warps)
+  // the sums of a unit (segment, column block) complete; read out (the column block's draining warps): of unit u at u % T::kUnitBars
+  __shared__ __align__(8) uint64_t acc_full[T::kUnitBars], acc_free[T::kUnitBars];
   __shared__ __align__(8) uint64_t fin[2];
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_abort;
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
     for (uint32_t s = 0; s < XS; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], CB); }
     for (uint32_t s = 0; s < WS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], T::kExpanders); }
     for (uint32_t s = 0; s < AB; ++s) { mbar_init(&a_ready[s], T::kExpanders); mbar_init(&a_free[s], CB); }
-    for (int s = 0; s < 3; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_free[s], 4 * T::kDrains / CB); }
+    for (uint32_t s = 0; s < T::kUnitBars; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_free[s], 4 * T::kDrains / CB); }
     mbar_init(&fin[0], 1); mbar_init(&fin[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_abort = 0;
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
       const uint32_t pieces = (uint32_t)p.pieces, h = (uint32_t)warp - 1u, cb = CB == 2 ? h : 0u;
       uint32_t it = 0, unit = BITS == 4 && CB == 1 ? 0u : h;
       bool ok = true;
-      auto sums_free = [&](uint32_t u) { return u < 3 || mbar_wait(&acc_free[u % 3], (u / 3 - 1u) & 1u); };
+      auto sums_free = [&](uint32_t u) { return u < 3 || mbar_wait(&acc_free[(u - 3) % T::kUnitBars], ((u - 3) / T::kUnitBars) & 1u); };
       for (uint32_t t = tile0; t < p.tiles && ok; t += stride) {
         for (uint32_t s = s0; s < s1 && ok; ++s, ++it) {
           const uint32_t ab = it % AB, slot = it % XS, ng = BITS == 4 ? min(2u, p.groups - 2u * s) : 1u, at = (s - s0) % kSegStages;
@@ -481,7 +482,7 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
                   mma_f16(d, au, xu, idesc, 0u);
                 }
                 mma_f16(d, au + 8, umma_desc_advance(xu, 32u), idesc, 1u);
-                umma_commit(&acc_full[unit % 3]);
+                umma_commit(&acc_full[unit % T::kUnitBars]);
               }
             } else {
               const bool first = at < 3 - CB;
@@ -491,13 +492,13 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
               for (uint32_t pc = 0; pc < pieces; ++pc)
 #pragma unroll
                 for (uint32_t q = 0; q < 4; ++q) mma_f16(d, a + q * 8, umma_desc_advance(xd, pc * T::kPiece + q * 32u), idesc, !first || (pc | q) != 0 ? 1u : 0u);
-              if (last) { umma_commit(&acc_full[unit % 3]); unit += 2; }
+              if (last) { umma_commit(&acc_full[unit % T::kUnitBars]); unit += 2; }
             }
             umma_commit(&x_empty[slot]);
             umma_commit(&a_free[ab]);
           } else if (h == 1 && at == 0 && s + 1 == s1) {  // int8, a segment of one stage: the other thread's sums are all there is
             if (!sums_free(unit)) { ok = false; break; }
-            umma_commit(&acc_full[unit % 3]);
+            umma_commit(&acc_full[unit % T::kUnitBars]);
             unit += 2;
           }
         }
@@ -527,7 +528,7 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
     // one unit's sums into the registers, times the scale of group u of a stage
     auto drain = [&](uint32_t scale_slot, uint32_t u, bool none) -> bool {
       const uint32_t set = unit % 3;
-      if (s_abort || !mbar_wait(&acc_full[set], (unit / 3) & 1u)) return false;
+      if (s_abort || !mbar_wait(&acc_full[unit % T::kUnitBars], (unit / T::kUnitBars) & 1u)) return false;
       tc_fence_after_sync();
       float sv = 1.0f;
       if constexpr (BITS == 4)  // a column past the matrix reads what an earlier tile left: it is never stored
@@ -541,7 +542,7 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
         if (c == 3) {  // the buffer may be overwritten
           tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&acc_free[set]);
+          if (lane == 0) mbar_arrive(&acc_free[unit % T::kUnitBars]);
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i)

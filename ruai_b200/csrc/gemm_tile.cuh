@@ -26,6 +26,12 @@ struct Tile {
   static constexpr uint32_t kPiece = NT * 128;                           // one piece of x of a stage
   static constexpr uint32_t kX = 2 * kPiece;                             // both
   // Tensor memory: three buffers of sums, then the A operand, 32 words per column block and stage.
+  // A wait for a phase of a barrier by its parity also returns while the phase before is open, so whoever waits must know that one to be
+  // over.  The buffers are used in turn, but by two issuing threads and two column blocks' draining warps: with a barrier per buffer one
+  // party meets every other phase only.  With six, units u and u + 6 of a barrier belong to the same column block, or to the same
+  // issuing thread; and where two threads take stages in turn (int4, one column block), a thread's units are at most five apart and
+  // the read-out goes in order, so that the phase before its own (unit u - 9) is over.
+  static constexpr uint32_t kUnitBars = 6;
   static constexpr uint32_t kACol0 = 3 * NT;
   static constexpr int kABufs = 4 / CB;
   static constexpr uint32_t kTmem = 512;

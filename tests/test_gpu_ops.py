@@ -430,6 +430,23 @@ def test_gemm_small_elements_beside_large_ones(dev, m, k, n, dtype, bits, ratio,
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
 
 
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("m,k,n", [(2000, 576, 3072), (2000, 576, 960), (4000, 1120, 1536), (3000, 4096, 2560)])
+def test_gemm_again_and_again(dev, m, k, n, bits):
+    """Several tiles per CTA, of an odd number of stages among others: every run gives the same bits, and the status stays clean."""
+    q, s, qw = _qw(dev, bits, k, n, 45)
+    wd = q.astype(np.float64) * s if bits == 8 else qw.dequant().astype(np.float64)
+    x = oracle.synth_normal(45, m, (m, k), 1.0)
+    xt = nn.Tensor.from_numpy(dev, x)
+    first = nn._matmul_q(xt, qw).numpy()
+    want, mag = x.astype(np.float64) @ wd, np.abs(x).astype(np.float64) @ np.abs(wd)
+    assert (np.abs(first - want) <= 2.0 ** -20 * mag + 1e-30).all()
+    for _ in range(12):
+        ys = [nn._matmul_q(xt, qw) for _ in range(8)]
+        dev.synchronize()
+        assert all(np.array_equal(y.numpy(), first) for y in ys[::3])
+
+
 @pytest.mark.parametrize("m,n", [(88320, 384), (88320, 300)])
 def test_gemm_of_one_group_over_many_tiles(dev, m, n):
     """k of one scale group and a dozen column blocks per CTA: the scales' ring goes round with one group per stage."""
