@@ -81,6 +81,9 @@ int ruai_ctx_inject_copy_shortfall(ruai_ctx* ctx, unsigned bytes);
  * of a few f32 additions.  `python -m ruai_b200.sweep_splits` uses it to compare the cost model with every fixed split
  * on a list of shapes.  No counterpart in the reference. */
 int ruai_ctx_force_splits(ruai_ctx* ctx, unsigned splits);
+/* The same for the tile of the many-row GEMM: `cols` columns of the weight (256 or 128) x `rows` rows of x (128, or 64 with 128
+ * columns); 0, 0 gives the choice back. */
+int ruai_ctx_force_tile(ruai_ctx* ctx, unsigned cols, unsigned rows);
 
 /* Device memory for callers without their own allocator (cuda.rs:288-300).  Blocks given back are kept for later calls (512 MB a device
  * at most) and given out again when no stream of the device can still use them; memory of ruai_malloc goes back through ruai_free. */

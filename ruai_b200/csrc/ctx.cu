@@ -189,6 +189,16 @@ RUAI_API int ruai_ctx_force_splits(ruai_ctx* c, unsigned splits) {
   return RUAI_OK;
 }
 
+// Tuning knob: the tile of the prefill GEMM (0, 0 = the chooser decides).
+RUAI_API int ruai_ctx_force_tile(ruai_ctx* c, unsigned cols, unsigned rows) {
+  if (!c) return ruai_fail(c, RUAI_ERR_ARG, "NULL argument");
+  if (!((cols == 0 && rows == 0) || (cols == 256 && rows == 128) || (cols == 128 && (rows == 128 || rows == 64))))
+    return ruai_fail(c, RUAI_ERR_ARG, "tile %u x %u: 0 x 0 (automatic), 256 x 128, 128 x 128 or 128 x 64", cols, rows);
+  c->force_cols = cols;
+  c->force_rows = rows;
+  return RUAI_OK;
+}
+
 // Profiling hooks, present only in builds made with RUAI_B200_TRACE=1 (never in the library as shipped).
 #ifdef RUAI_B200_TRACE
 RUAI_API int ruai_debug_force_splits(ruai_ctx* c, unsigned splits) {  // also the profiling bits above the count

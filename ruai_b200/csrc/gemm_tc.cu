@@ -695,6 +695,7 @@ Shape choose(const ruai_ctx* c, uint32_t m, uint32_t n, uint32_t stages, int bit
   Shape best = {1, 64, 1};
   double best_t = 1e300;
   for (const Cand& d : cand) {
+    if (c->force_cols && (c->force_cols != d.cb * 128 || c->force_rows != d.nt)) continue;
     const uint32_t tiles = ((n + d.cb * 128 - 1) / (d.cb * 128)) * ((m + d.nt - 1) / d.nt);
     for (uint32_t s = 1; s <= 8; ++s) {
       const uint32_t per = (stages + s - 1) / s;

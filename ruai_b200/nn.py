@@ -60,6 +60,10 @@ class Device:
         """Fix the split-k count of the tensor-core GEMVs (1..8), or 0 to let the library choose."""
         self.check(self.L.ruai_ctx_force_splits(self.ctx, splits))
 
+    def force_tile(self, cols, rows):
+        """Fix the tile of the many-row GEMM (256 x 128, 128 x 128 or 128 x 64), or 0, 0 to let the library choose."""
+        self.check(self.L.ruai_ctx_force_tile(self.ctx, cols, rows))
+
     def timer_start(self):
         self.check(self.L.ruai_timer_start(self.ctx))
 

@@ -430,6 +430,50 @@ def test_gemm_small_elements_beside_large_ones(dev, m, k, n, dtype, bits, ratio,
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
 
 
+TILES = [(256, 128), (128, 128), (128, 64)]
+
+
+def _against_float64(dev, dtype, bits, m, k, n, seed):
+    """Sums in f32 of products that hold 22 bits of x: errors below 2^-20 of the sum of the products' magnitudes, and the rounding of a
+    16-bit output."""
+    if bits == 8:
+        k -= 7  # a ragged last chunk
+    q, s, qw = _qw(dev, bits, k, n, seed)
+    wd = q.astype(np.float64) * s if bits == 8 else qw.dequant().astype(np.float64)
+    x, bias = oracle.synth_normal(seed, m, (m, k), 1.0), oracle.synth_normal(seed, 1, (n,))
+    xf, got = run_matmul(dev, x, qw, dtype, bias)
+    want, mag = xf.astype(np.float64) @ wd + bias, np.abs(xf).astype(np.float64) @ np.abs(wd) + np.abs(bias)
+    bound = 2.0 ** -20 * mag + {"f32": 0.0, "f16": 2.0 ** -11, "bf16": 2.0 ** -8}[dtype] * np.abs(want) + 1e-7
+    assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("tile", TILES)
+@pytest.mark.parametrize("m,k,n", [(17, 64, 128), (64, 96, 132), (129, 544, 516), (300, 1504, 1500), (513, 224, 2564),
+                                   # several tiles per CTA, of three, one and four stages: the rings and barriers go on from tile to tile
+                                   (2053, 160, 4900), (1700, 64, 6404), (2053, 256, 4900)])
+def test_gemm_every_tile(dev, tile, m, k, n, bits):
+    try:
+        dev.force_tile(*tile)
+        _against_float64(dev, "f32", bits, m, k, n, 41)
+        with pytest.raises(nn.RuaiError, match="tile"):
+            dev.force_tile(256, 64)
+    finally:
+        dev.force_tile(0, 0)
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("tile", TILES)
+@pytest.mark.parametrize("m,k,n", [(17, 96, 132), (37, 1504, 1500), (129, 544, 516), (513, 224, 2564), (2053, 160, 4900)])
+def test_gemm_half_precision_activations(dev, tile, m, k, n, dtype, bits):
+    try:
+        dev.force_tile(*tile)
+        _against_float64(dev, dtype, bits, m, k, n, 42)
+    finally:
+        dev.force_tile(0, 0)
+
+
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("m,k,n", [(2000, 576, 3072), (2000, 576, 960), (4000, 1120, 1536), (3000, 4096, 2560)])
 def test_gemm_again_and_again(dev, m, k, n, bits):
@@ -573,16 +617,49 @@ def test_grad_input_in_a_graph(dev, capturing, m, k, n):
         t.free()
 
 
-def test_freed_tensors_are_reused_only_after_a_wait(dev):
-    """Blocks freed while their context's stream still works on them do not come back before that work is done."""
+def test_results_while_their_memory_goes_round(dev):
+    """Results dropped while they are queued, on one stream: their blocks come back several times."""
     q, s, qw = _qw(dev, 8, 2048, 2048, 33)
     xs = [nn.Tensor.from_numpy(dev, oracle.synth_normal(33, i, (256, 2048), 1.0)) for i in range(3)]
     want = [nn._matmul_q(x, qw).numpy() for x in xs]
-    for r in range(120):  # results are dropped while queued, so that their memory goes round several times
+    for r in range(120):
         i = r % 3
         for j in range(3):
             nn._matmul_q(xs[j], qw)
         assert np.array_equal(nn._matmul_q(xs[i], qw).numpy(), want[i])
+
+
+def test_freed_tensors_are_reused_only_after_a_wait(dev):
+    """A tensor freed through its own context while another context's stream has yet to read it: its block comes back to the first one only
+    after that read."""
+    other = nn.Device(0)
+    m, k, n = 2048, 4096, 4096
+    _, _, qw = _qw(other, 8, k, n, 43)
+    data = oracle.synth_normal(43, 1, (m, k), 1.0)
+    xs = [nn.Tensor.from_numpy(dev, data) for _ in range(3)]  # 32 MB each
+    out, busy = (nn.Tensor(other, (m, n), np.float32, nn.F32) for _ in range(2))
+
+    def product(x, y):
+        other.check(other.L.ruai_matmul_q(other.ctx, nn.F32, x.ptr, qw.h, None, y.ptr, m))
+
+    product(xs[0], out)
+    want = out.numpy()
+    other.check(other.L.ruai_memcpy_h2d(other.ctx, out.ptr, np.zeros_like(want).ctypes.data_as(C.c_void_p), out.nbytes))
+    for _ in range(150):  # about 20 ms
+        product(xs[0], busy)
+    product(xs[1], out)
+    freed = {t.ptr.value for t in xs[1:]}
+    for t in xs[1:]:
+        t.free()
+    again = [nn.Tensor(dev, (m, k), np.float32, nn.F32) for _ in range(2)]
+    for t in again:
+        dev.check(dev.L.ruai_memcpy_h2d(dev.ctx, t.ptr, np.full_like(data, np.nan).ctypes.data_as(C.c_void_p), t.nbytes))
+    got = out.numpy()
+    assert {t.ptr.value for t in again} == freed  # they did come back
+    assert np.array_equal(got, want)
+    for t in (out, busy, qw):
+        t.free()
+    nn._lib.check(other.L.ruai_ctx_destroy(other.ctx))
 
 
 def test_memory_freed_in_a_capture_or_twice_is_refused(dev, capturing):
