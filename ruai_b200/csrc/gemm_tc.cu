@@ -688,7 +688,9 @@ cudaError_t launch_tile(ruai_ctx* c, const Params& p, const Shape& sh) {
 }
 
 // The tile and the number of splits of k: a model of the launch in microseconds, fitted to launches of 37 to 2000 rows of the 1.1B and
-// 8B shapes' Linears with every tile and 1 .. 8 splits (the choice is within 5 % of the best of them; a wrong one costs up to 2 x).
+// 8B shapes' Linears with every tile and 1 .. 8 splits.  Over 17 to 2000 rows of those and the 135M shape's (`python -m
+// ruai_b200.sweep_splits`) the choice is within 5 % of the best tile and split at 115 of 132 sizes, the worst 1.19 times the best (a wrong
+// one costs up to 2 x).
 Shape choose(const ruai_ctx* c, uint32_t m, uint32_t n, uint32_t stages, int bits, int pieces) {
   struct Cand { uint32_t cb, nt; double stage4, stage8, split; };  // a stage of int4 and int8; what a split adds
   const Cand cand[3] = {{2, 128, 1.55, 1.0, 7.0}, {1, 128, 0.80, 0.55, 6.0}, {1, 64, 0.62, 0.45, 3.5}};
