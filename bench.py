@@ -48,9 +48,9 @@ OTHER_WORKLOADS = ["llama3-8b-int8-b1", "llama3-8b-int4-b16", "llama3-8b-int8-b1
 ARITHMETIC = ("f32 in and out; inside the GEMV the activations are block fixed point (int4 weights: 21 bits per group of 32; "
               "int8 weights: 28 bits per row of a CTA's slice), products exact in tcgen05 kind::i8, one f32 scale multiply-add "
               "per group, split-k sums met in 64-bit fixed point")
-# steps of 5..16 sequences (and prefill-sized row counts): another arithmetic
-ARITHMETIC_WIDE = ("f32 in and out; inside the Linears the activations are two bf16 pieces x = hi + lo (16 significant bits), the int4 / "
-                   "int8 weights exact in bf16, products and sums in f32 in tcgen05 kind::f16, one f32 scale multiply-add per group "
+# steps of 5..16 sequences and prefill-sized row counts: other arithmetics
+ARITHMETIC_WIDE = ("f32 in and out; inside the Linears the activations are two bf16 pieces x = hi + lo (16 significant bits; from 17 rows on "
+                   "two fp16 pieces under a power of two per row, 22 bits), the int4 / int8 weights exact, products and sums in f32 in tcgen05 kind::f16, one f32 scale multiply-add per group "
                    "(int8: per column); Linears below 4M weights keep the block-fixed-point kernels")
 
 

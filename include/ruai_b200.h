@@ -85,8 +85,13 @@ int ruai_ctx_force_splits(ruai_ctx* ctx, unsigned splits);
  * columns); 0, 0 gives the choice back. */
 int ruai_ctx_force_tile(ruai_ctx* ctx, unsigned cols, unsigned rows);
 
-/* Device memory for callers without their own allocator (cuda.rs:288-300).  Blocks given back are kept for later calls (512 MB a device
- * at most) and given out again when no stream of the device can still use them; memory of ruai_malloc goes back through ruai_free. */
+/* Device memory for callers without their own allocator (cuda.rs:288-300).  Blocks of up to 256 MB that are given back are kept for later
+ * calls, 512 MB a device at most, and given out again after a wait for every stream of the device.  They go back to the driver when an
+ * allocation of this library runs out of memory and with the device's last context; other allocators of the process do not see them.
+ * Memory of ruai_malloc goes back through ruai_free, by any context.  ruai_free does not wait for the block's users and so reports no
+ * error of their work, unless the driver already knows of it; a second free of a block is refused.  While a stream of one of the device's
+ * contexts is being captured nothing is kept or given out: ruai_free then waits for the context's stream and frees, which fails for the
+ * capturing stream itself and ends its capture, and ruai_malloc allocates. */
 int ruai_malloc(ruai_ctx* ctx, size_t bytes, void** out_dev);
 int ruai_free(ruai_ctx* ctx, void* ptr_dev);
 int ruai_memcpy_h2d(ruai_ctx* ctx, void* dst_dev, const void* src_host, size_t bytes);
@@ -137,16 +142,21 @@ int ruai_pack_dense(ruai_ctx* ctx, const float* w, uint32_t n, uint32_t k, uint3
  * x_dtype, bias_dev_or_null is f32 [n].  Sums, scales and bias are f32.  The
  * products run on the tensor cores with the weights exact: up to 4 rows the
  * activations as block fixed point of 21 (int4) or 28 (int8) bits, results
- * within 1e-4 * (1 + |y|) of the reference's CPU path (tests/devices.rs); from
- * 5 rows on (Linears of 4M weights and more) and in the many-row GEMM the
- * activations as two bf16 pieces (16 significant bits): max-abs 1e-2, 1e-3 of
- * the output's scale, and all but about 1e-4 of the outputs inside the 1e-4.
- * A non-finite activation makes its row of the output non-finite.           */
+ * within 1e-4 * (1 + |y|) of the reference's CPU path (tests/devices.rs); 5
+ * to 16 rows (Linears of 4M weights and more) the activations as two bf16
+ * pieces (16 significant bits): max-abs 1e-2, 1e-3 of the output's scale, and
+ * all but about 1e-4 of the outputs inside the 1e-4; from 17 rows on f32
+ * activations as two fp16 pieces under one power of two per row: 22 bits,
+ * errors below 2^-20 of sum |x| |w|.  Elements far below their row's largest
+ * keep fewer: int4 22 bits down to 2^-28 of it, then a quantum of 2^-50 of it;
+ * int8 22 bits down to 2^-16, then a quantum of 2^-38.  f16 activations are
+ * exact; bf16 ones too for int4, and for int8 down to 2^-31 of the row's
+ * largest.  A non-finite activation makes its row of the output non-finite.  */
 int ruai_matmul_q(ruai_ctx* ctx, int x_dtype, const void* x_dev, const ruai_qweight* w,
                   const float* bias_dev_or_null, void* out_dev, uint32_t m);
 /* Backward of `Tensor::matmul_int8` / `matmul_int4` (ops.rs:705-709, 731-734): the weights are frozen, the only
- * gradient is dx[m,k] = g[m,n] @ dequant(W)^T.  The reference materialises the f32 weight for it; here the packed
- * weight is read once per row of g.  f32 in, f32 out, m <= 65535.                                                   */
+ * gradient is dx[m,k] = g[m,n] @ dequant(W)^T.  The reference materialises the f32 weight for it; here tiles of the
+ * packed weight are dequantised on the way (up to 18 rows: once per row of g).  f32 in, f32 out, m <= 65535.        */
 int ruai_matmul_q_grad_input(ruai_ctx* ctx, const float* g_dev, const ruai_qweight* w, float* dx_dev, uint32_t m);
 /* `Linear::forward` of a quantized layer with a LoRA adapter (layers.rs:169-190; add_lora 84-97), QLoRA-style:
  * out = matmul_q(x) + (x @ A @ B) * scale + bias, A [k,rank], B [rank,n] row-major f32, scale = alpha / rank,

@@ -69,10 +69,11 @@ __global__ void __launch_bounds__(kThreads) grad_input_chunk_kernel(const uint4*
 // owns 8 x 4 results; g is kept twice side by side, so that packed multiply-adds (two f32 in one instruction, each rounded like fmaf)
 // need no shuffling: five 16-byte reads from shared memory per 16 of them.  The columns are shared out over gridDim.z CTAs for about
 // four CTAs per SM; the shares are added in a fixed order by sum_shares_kernel.  Bound by f32 multiply-adds and their operands'
-// reads: 256 x 2048 x 2048 int4 115 us (a row of g at a time: 344 us).  The sums' additions are a fifth of the multiply-adds and
-// within what the reads leave free: four CTAs per SM (128 registers) 115 us, three with 158 registers 123.
-// Up to here a row at a time is faster (us, k x n): 16 rows int4 2048 x 2048 27 against 26, int8 22 against 26; 4096 x 4096 80 and 65
-// against 80; 24 rows 39 and 32 against 28, 116 and 95 against 84.
+// reads: 256 x 2048 x 2048 int4 116 us (a row of g at a time: 344 us).  The sums' additions are a fifth of the multiply-adds and
+// within what the reads leave free: four CTAs per SM (128 registers) 116 us, three with 158 registers 123.
+// Up to here a row at a time is as fast or faster, taken together (us, rows | tiles): 16 rows, 2048 x 2048 int4 28.7 | 28.8, int8 22.6 |
+// 28.8, 4096 x 4096 79 | 84 and 64 | 82; 20 rows 33.8 | 29.0, 27.4 | 28.8, 98 | 86, 78 | 84.  Small weights favour the rows for longer
+// (512 x 512 int4, 24 rows: 10.3 | 12.4), flat ones the tiles sooner (k 2048, n 512 int4, 14 rows: 17.4 | 14.4).
 constexpr uint32_t kGradFewRows = 18;
 constexpr int kGradTile = 64, kGradCols = 16, kGradThreads = 128, kGradPad = kGradTile + 4;
 

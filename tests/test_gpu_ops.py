@@ -200,9 +200,9 @@ def test_matmul_grid_8b_widths(dev, m, k, n, bits):
         q, s = oracle.quantize_int4(w, 32)
         qw, want = nn.QWeight.int4(dev, q, s, 32), oracle.matmul_int4(x, q, s)
     _, y = run_matmul(dev, x, qw, "f32")
-    # Quantized-Linear outputs: max-abs 1e-2 and 1e-3 relative to the output's scale.  (The rows-by-the-hundred GEMM
-    # carries the activations as two bf16 pieces, 16 significant bits; over k = 14336 a handful of the 524288 outputs
-    # miss the 1e-4 * (1 + |y|) of tests/devices.rs by up to 4e-4, which the smaller shapes above all meet.)
+    # Quantized-Linear outputs: max-abs 1e-2 and 1e-3 relative to the output's scale, all but a sliver inside the 1e-4 * (1 + |y|)
+    # of tests/devices.rs: what two bf16 pieces of the activations need.  The GEMM's pieces hold 22 bits and stay well inside;
+    # test_gemm_every_tile has their bound.
     err = np.abs(want.astype(np.float64) - y).max()
     assert err <= 1e-2 and err <= 1e-3 * np.abs(want).max(), (err, np.abs(want).max())
     loose = ~(np.abs(want - y) <= 1e-4 * (1 + np.abs(want)))
@@ -305,7 +305,7 @@ def test_matmul_non_finite_activations_propagate(dev, bits, m):
         xb[0, 1234] = bad
         _, y = run_matmul(dev, xb, qw, "f32")
         assert not np.isfinite(y[0]).any(), bad
-        if m > 1:  # (five rows and more: activations as two bf16 pieces, see test_matmul_five_to_sixteen_rows)
+        if m > 1:  # (5 to 16 rows: activations as two bf16 pieces, see test_matmul_five_to_sixteen_rows)
             same(want[1:], y[1:], 1e-4 if m < 5 else 3e-4)
 
 
