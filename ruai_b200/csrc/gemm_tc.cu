@@ -20,7 +20,7 @@
 //     additions stay short, with the column scale at the end (cpu.rs:903-920).
 // What bounds it: int8, the tensor pipe and the power limit (4096 x 4096 x 14336: 0.82 ms, 1.18 PFLOP/s counting both pieces, where
 // cuBLAS sustains 1.40; 1.48 ms int4 and 1.45 int8 with unswizzled operands, which take twice as long); int4, the issue slots of the
-// warps that expand and drain (1.29 ms: per scheduler and stage about 900 of the 1,037 clocks that its MMAs take).  A CTA of 256
+// warps that expand and drain (1.23 to 1.25 ms: per scheduler and stage about 900 of the 1,037 clocks that its MMAs take).  A CTA of 256
 // columns x 128 rows needs 16 MMAs of 64 clocks per stage.  256 columns, because every byte of x is then used twice: with 128 the
 // copies of x alone ask the L2 for 64 bytes per clock and SM.  Three tile shapes and a split of k over a cluster cover the sizes that
 // leave that tile's grid small (64 x 2048 x 2048 int8: 41 us before, 20 CTAs; 11 now).
