@@ -15,6 +15,8 @@
 
 namespace {
 
+constexpr int kAttnWarps = 8;  // at the most
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
@@ -157,74 +159,70 @@ __global__ void rope_kv_kernel(float* __restrict__ qkv, uint32_t qkv_ld, uint32_
 // scaled_dot_product_attention over the cache (functional.rs:264-296, llama.rs:248-277):
 // softmax(q k^T / sqrt(hd) + causal mask) v.  The `rep` query heads of one KV head are
 // handled by one CTA so the cached rows are read once (the reference's [B, H_kv, rep*T, hd]
-// view, llama.rs:264-268).  Keys are split over gridDim.z CTAs; a CTA brings its keys and
-// values into shared memory with bulk copies, 64 at a time, requested before the
-// grid-dependency wait in the fused step.
-//   scores : warp (block of 32 keys, head): one key per lane, the lane walks its key row
-//            starting at its own 16-byte column (no bank conflicts, no cross-lane sums);
-//            block maximum and sum by shuffles.
-//   values : thread (head, element): sums p * V over the chunk's keys, rows read conflict-free.
-// Every thread keeps a running (max, sum, weighted value) for its outputs across chunks; the
-// splits are merged by the last CTA to arrive.
+// view, llama.rs:264-268).
 // With p.fuse (single new token per sequence) the kernel also does apply_rope
 // (functional.rs:197-204) on q and on the new key and appends the new key / value to the
 // cache (KvBuf::append, transformer.rs:27-53): the last key split owns the new position.
-
-// SUB: warps per (32 keys, query head).  2 (more warps than the work needs, to hide each other's latencies) for grids of
-// about one CTA per SM; 1 for large grids, where two or three smaller CTAs per SM hide them instead.
-template <int REP, int SUB>
-__global__ void __launch_bounds__(kAttnChunkKeys * REP * SUB) attention_kernel(const AttnParams p) {
-  constexpr int kThreads = kAttnChunkKeys * REP * SUB, kBlocks = kAttnChunkKeys / 32, kParts = REP * SUB;
-  extern __shared__ __align__(128) float sm[];  // K chunk | V chunk | q [REP][hd] | new k | new v | probs | stats | parts | merge
-  __shared__ __align__(8) uint64_t kv_bar;
-  __shared__ unsigned s_last;
-  const uint32_t hd = p.hd, half = hd / 2;
-  float* ks = sm;
-  float* vs = ks + (size_t)kAttnChunkKeys * hd;
-  float* qs = vs + (size_t)kAttnChunkKeys * hd;
-  float* knew = qs + REP * hd;
-  float* vnew = knew + hd;
-  float* probs = vnew + hd;                       // [kBlocks][REP][32]
-  float* bmax = probs + kBlocks * REP * 32;       // [kBlocks + 1][REP]: block maxima; the last row is the new key's score
-  float* bsum = bmax + (kBlocks + 1) * REP;       // [kBlocks][REP]
-  float* part = bsum + kBlocks * REP;             // [kParts][REP heads][64 keys] partial scores
-  float* mg = part + kParts * REP * kAttnChunkKeys;  // split merge: [64][REP] weights, [64][REP] sums, [REP]
-  const uint32_t bk = blockIdx.x, b = bk / p.KV, kvh = bk % p.KV, t = blockIdx.y, split = blockIdx.z;
+//
+// Every warp works alone on keys of its own, 32 / LPK at a time, which it copies into its part of shared memory itself (in the fused
+// step requested before the grid-dependency wait).  Scores: LPK lanes per key, a part of the head dimension each, against all REP
+// query heads (key rows padded by four floats: no bank conflicts; the queries are broadcast); running softmax per head over the
+// warp's lanes; values: a lane per four elements, all heads at once.  So a cached element is read from shared memory once per warp,
+// and nothing but the warps' results meets at a barrier.  Keys are split over a cluster of gridDim.z CTAs as well; the first one
+// merges the results, through distributed shared memory.
+// Bound by HBM where there are many sequences (64 of 260 keys, 4 key heads of 64 with 8 query heads each: 52 us a launch with the
+// warps of a CTA at 64 keys in turn, four barriers for them and every key and value read once per head; 25 us now, 5 at the
+// bandwidth), by latency where there is one (1024 keys: 8 to 9 us before and now).
+template <int REP, int LPK>  // lanes per key: 1, 2 or 4 for head dimensions up to 64, 128, 256, so that a warp's copy stays below 17 KB
+__global__ void __launch_bounds__(kAttnWarps * 32) attention_kernel(const AttnParams p) {
+  constexpr int kJ = LPK == 4 ? 2 : 1, kRepPad = REP == 3 ? 4 : REP, kKeys = 32 / LPK;
+  extern __shared__ __align__(128) float sm[];
+  __shared__ __align__(8) uint64_t bars[kAttnWarps];
+  __shared__ float s_m[kAttnWarps][REP], s_l[kAttnWarps][REP];
+  const uint32_t hd = p.hd, half = hd / 2, nq4 = hd / 4, kstride = hd + 4, warps = blockDim.x / 32, ns = gridDim.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t per_warp = max((uint32_t)kKeys * (kstride + hd), REP * hd);  // floats: keys, then values; at the end the warp's sums
+  float* ks = sm + (size_t)warp * per_warp;
+  float* vs = ks + kKeys * kstride;
+  float* qs = sm + (size_t)warps * per_warp;                 // [REP][hd]
+  float* knew = qs + REP * hd;                               // [hd], then the new value
+  float* vnew = knew + hd;
+  float* probs = vnew + hd + warp * kKeys * kRepPad;         // [kKeys][kRepPad] per warp
+  float* cl = vnew + hd + warps * kKeys * kRepPad;           // the cluster's results: [ns][REP][hd + 4]
+  const uint32_t bk = blockIdx.x, b = bk / p.KV, kvh = bk % p.KV, t = blockIdx.y, split = blockIdx.z;
   float* kbase = p.kcache + ((size_t)b * p.KV + kvh) * p.cap * hd;
   float* vbase = p.vcache + ((size_t)b * p.KV + kvh) * p.cap * hd;
-  if (tid == 0) {
-    pipe::mbar_init(&kv_bar, 1);
+  uint64_t* bar = &bars[warp];
+  if (lane == 0) {
+    pipe::mbar_init(bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncthreads();
-  uint32_t past = 0, pos = 0, n_keys = 0, n_cached = 0, k0 = 0, k1 = 0;
+  __syncwarp();
+  if (ns > 1) pipe::cluster_arrive();  // waited for ahead of the first store into another CTA
+  uint32_t pos = 0, k0 = 0, k1 = 0;  // this warp's keys
   bool over = false;
   auto plan = [&]() {
-    past = (uint32_t)*p.len;
-    pos = past + t;
-    n_keys = pos + 1;  // causal_mask_offset, functional.rs:238-247
-    n_cached = p.fuse ? n_keys - 1 : n_keys;
+    pos = (uint32_t)*p.len + t;  // causal_mask_offset, functional.rs:238-247
     // The host grows the cache before the step, so a position at or past the capacity means the device's position
     // word is not the host's: touch nothing of the cache, leave an error for the host (the step's output is void).
     over = pos >= p.cap;
-    if (over) n_cached = 0;
-    const uint32_t per = (n_cached + gridDim.z - 1) / gridDim.z;
-    k0 = min(n_cached, split * per);
-    k1 = min(n_cached, k0 + per);
+    const uint32_t n = over ? 0u : p.fuse ? pos : pos + 1;
+    const uint32_t shares = ns * warps, share = split * warps + warp;
+    k0 = (uint32_t)((uint64_t)n * share / shares);
+    k1 = (uint32_t)((uint64_t)n * (share + 1) / shares);
   };
-  auto fetch_chunk = [&](uint32_t c0) {  // one thread
-    const uint32_t nk = min((uint32_t)kAttnChunkKeys, k1 - c0);
-    const uint32_t bytes = nk * hd * 4u;
-    pipe::mbar_expect_tx(&kv_bar, 2u * bytes);
-    pipe::bulk_load(ks, kbase + (size_t)c0 * hd, bytes, &kv_bar);
-    pipe::bulk_load(vs, vbase + (size_t)c0 * hd, bytes, &kv_bar);
+  auto fetch = [&](uint32_t c0) {  // the whole warp: a lane per key
+    const uint32_t nk = min((uint32_t)kKeys, k1 - c0);
+    if (lane == 0) pipe::mbar_expect_tx(bar, nk * hd * 8u);
+    __syncwarp();
+    if ((uint32_t)lane < nk) pipe::bulk_load(ks + lane * kstride, kbase + (size_t)(c0 + lane) * hd, hd * 4u, bar);
+    if (lane == 0) pipe::bulk_load(vs, vbase + (size_t)c0 * hd, nk * hd * 4u, bar);
   };
   // In the fused single-token step the cached rows were written by earlier steps, and the position by the
   // previous step's last kernel: both are safe to read while the predecessor (the q/k/v GEMV) still runs.
   if (p.fuse) {
     plan();
-    if (tid == 0 && k1 > k0) fetch_chunk(k0);
+    if (k1 > k0) fetch(k0);
   }
   if (tid == 0) trace_min(p.trace, 0);
   grid_dependency_wait();
@@ -232,277 +230,176 @@ __global__ void __launch_bounds__(kAttnChunkKeys * REP * SUB) attention_kernel(c
   grid_launch_dependents();
   if (!p.fuse) {
     plan();
-    if (tid == 0 && k1 > k0) fetch_chunk(k0);
+    if (k1 > k0) fetch(k0);
   }
-  const bool owns_new = p.fuse && split == gridDim.z - 1;
+  const bool owns_new = p.fuse && split == ns - 1;
   if (over && tid == 0 && p.status) atomicCAS(p.status, 0, 5);
   const float* row = p.q + (size_t)(b * p.T + t) * p.q_ld;
-  const float* qrow = row + (size_t)kvh * REP * hd;
   const bool rot = p.fuse && p.table != nullptr;
-  for (uint32_t i = tid; i < REP * hd; i += kThreads) {
-    float v = qrow[i];
-    if (rot) {
-      const uint32_t r = i / hd, e = i % hd, f = e < half ? e : e - half;
-      const float2 cs = p.table[(size_t)pos * half + f];
-      const float x1 = qrow[r * hd + f], x2 = qrow[r * hd + f + half];
-      v = e < half ? x1 * cs.x + (-x2) * cs.y : x2 * cs.x + x1 * cs.y;
+  for (uint32_t i = tid; i < (REP + (owns_new ? 2 : 0)) * half; i += blockDim.x) {  // pairs (e, e + half) of the queries, the new key, the new value
+    const uint32_t r = i / half, e = i % half;
+    const float* src = row + (r < REP ? ((size_t)kvh * REP + r) * hd : r == REP ? p.k_off + (size_t)kvh * hd : p.v_off + (size_t)kvh * hd);
+    float x1 = src[e], x2 = src[e + half];
+    if (rot && r <= REP) {
+      const float2 cs = p.table[(size_t)pos * half + e];
+      const float y1 = x1 * cs.x + (-x2) * cs.y;
+      x2 = x2 * cs.x + x1 * cs.y;
+      x1 = y1;
     }
-    qs[i] = v;
-  }
-  if (owns_new) {
-    const float* kr = row + p.k_off + (size_t)kvh * hd;
-    const float* vr = row + p.v_off + (size_t)kvh * hd;
-    for (uint32_t e = tid; e < hd; e += kThreads) {
-      float kvv = kr[e];
-      if (rot) {
-        const uint32_t f = e < half ? e : e - half;
-        const float2 cs = p.table[(size_t)pos * half + f];
-        const float x1 = kr[f], x2 = kr[f + half];
-        kvv = e < half ? x1 * cs.x + (-x2) * cs.y : x2 * cs.x + x1 * cs.y;
-      }
-      const float vv = vr[e];
-      knew[e] = kvv;
-      vnew[e] = vv;
-      if (!over) {
-        kbase[(size_t)pos * hd + e] = kvv;
-        vbase[(size_t)pos * hd + e] = vv;
-      }
+    float* dst = qs + r * hd;  // the new key and value lie behind the queries
+    dst[e] = x1; dst[e + half] = x2;
+    if (r >= REP && !over) {
+      float* cache = (r == REP ? kbase : vbase) + (size_t)pos * hd;
+      cache[e] = x1; cache[e + half] = x2;
     }
   }
   __syncthreads();
-  // ---- thread roles ----
-  // partial scores: warp (key block, part of the head dimension), lane = key, all REP heads at once
-  // softmax stats : warp (key block, head), lane = key
-  // values        : thread (key group, head, 4 consecutive elements)
-  const uint32_t nq4 = hd / 4;
-  const int wblk = warp / kParts, wpart = warp % kParts, wr = wpart;  // wr: the head, for the warps with wpart < REP
-  const uint32_t cper = (nq4 + kParts - 1) / kParts;
-  const uint32_t c_lo = min(nq4, (uint32_t)wpart * cper), c_hi = min(nq4, c_lo + cper), ncols = c_hi - c_lo;
-  const uint32_t vthreads = REP * nq4;                 // threads that cover one full set of outputs
-  const uint32_t G = max(1u, (uint32_t)kThreads / vthreads);  // key groups in the value phase
-  const uint32_t vg = tid / vthreads, vrem = tid % vthreads, vr = vrem / nq4, vc = vrem % nq4;
-  const bool vact = (uint32_t)tid < G * vthreads;
-  float run_m = -INFINITY, run_l = 0.0f;
-  float4 run_o = make_float4(0.f, 0.f, 0.f, 0.f);
+  // values: lanes of a row, rows side by side
+  const uint32_t lanes = nq4 <= 8 ? 8 : nq4 <= 16 ? 16 : 32, groups = 32 / lanes, vg = lane / lanes, vc = lane % lanes;
+  float m[REP], l[REP];  // l: this lane's part
+  float4 o[kJ][REP];
+#pragma unroll
+  for (int r = 0; r < REP; ++r) {
+    m[r] = -INFINITY; l[r] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kJ; ++j) o[j][r] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (owns_new && warp == 0) {  // the token's own key is the first one
+#pragma unroll
+    for (int r = 0; r < REP; ++r) {
+      float a = 0.0f;
+      for (uint32_t e = lane; e < hd; e += 32) a = fmaf(qs[r * hd + e], knew[e], a);
+      m[r] = warp_sum(a) * p.scale;
+      l[r] = lane == 0 ? 1.0f : 0.0f;
+#pragma unroll
+      for (int j = 0; j < kJ; ++j)
+        if (vg == 0 && vc + 32u * j < nq4) o[j][r] = reinterpret_cast<const float4*>(vnew)[vc + 32u * j];
+    }
+  }
   uint32_t phase = 0;
   bool ok = true;
-  for (uint32_t c0 = k0; c0 < k1 || (c0 == k0 && owns_new); c0 += kAttnChunkKeys) {
-    const bool have_keys = c0 < k1;
+  const uint32_t key = lane % kKeys, share = nq4 / LPK;  // this lane's key, and of it `share` 16-byte columns (the last lanes: the rest)
+  const uint32_t q_lo = (lane / kKeys) * share, q_hi = lane / kKeys == LPK - 1 ? nq4 : q_lo + share;
+  for (uint32_t c0 = k0; c0 < k1; c0 += kKeys) {
     if (c0 != k0) {
-      __syncthreads();  // everyone is done with the previous chunk
-      if (tid == 0) fetch_chunk(c0);
+      __syncwarp();  // the lanes are done with the last keys
+      fetch(c0);
     }
-    if (have_keys) {
-      // the whole CTA leaves together if the copy did not arrive for any of its threads: the barriers below are for all
-      const bool got = pipe::mbar_wait(&kv_bar, phase & 1u);
-      if (__syncthreads_or(!got)) { ok = false; break; }
-      ++phase;
-    }
-    const uint32_t c1 = have_keys ? min(k1, c0 + kAttnChunkKeys) : c0;
-    const uint32_t nkeys = c1 - c0;
-    // ---- partial scores: this lane's key against this warp's columns of every head ----
-    {
-      const uint32_t key = wblk * 32 + lane;
-      const float4* krow = reinterpret_cast<const float4*>(ks + (size_t)(key < nkeys ? key : 0) * hd);
-      const float4* q4 = reinterpret_cast<const float4*>(qs);
-      float acc[REP][2];
+    ok = __all_sync(0xFFFFFFFFu, pipe::mbar_wait(bar, phase & 1u));
+    if (!ok) break;
+    ++phase;
+    const uint32_t nk = min((uint32_t)kKeys, k1 - c0);
+    const bool valid = key < nk;
+    float a0[REP], a1[REP];
 #pragma unroll
-      for (int r = 0; r < REP; ++r) { acc[r][0] = 0.0f; acc[r][1] = 0.0f; }
-      auto dot4 = [](const float4& a, const float4& b2, float s) {
-        s = fmaf(a.x, b2.x, s); s = fmaf(a.y, b2.y, s); s = fmaf(a.z, b2.z, s); return fmaf(a.w, b2.w, s);
-      };
-      if (ncols > 0) {
-        // each lane starts at its own column: the eight lanes of a quarter warp read eight different 16-byte columns
-        uint32_t cc = c_lo + lane % ncols;
-        uint32_t it = 0;
-        for (; it + 2 <= ncols; it += 2) {
-          const uint32_t ca = cc, cb = ca + 1 == c_hi ? c_lo : ca + 1;
-          const float4 ka = krow[ca], kb = krow[cb];
+    for (int r = 0; r < REP; ++r) { a0[r] = 0.0f; a1[r] = 0.0f; }
+    const float4* kr = reinterpret_cast<const float4*>(ks + (valid ? key : 0u) * kstride);
+    const float4* q4 = reinterpret_cast<const float4*>(qs);
+#pragma unroll 4
+    for (uint32_t c = q_lo; c < q_hi; ++c) {
+      const float4 kv = kr[c];
+#pragma unroll
+      for (int r = 0; r < REP; ++r) {
+        const float4 qv = q4[r * nq4 + c];
+        a0[r] = fmaf(qv.x, kv.x, a0[r]); a1[r] = fmaf(qv.y, kv.y, a1[r]); a0[r] = fmaf(qv.z, kv.z, a0[r]); a1[r] = fmaf(qv.w, kv.w, a1[r]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < REP; ++r) {
+      float a = a0[r] + a1[r];
+#pragma unroll
+      for (int off = kKeys; off < 32; off <<= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, off);
+      const float s = valid ? a * p.scale : -INFINITY;
+      const float m_new = fmaxf(m[r], warp_max(s)), pr = valid ? expf(s - m_new) : 0.0f, corr = m[r] == -INFINITY ? 0.0f : expf(m[r] - m_new);
+      l[r] = fmaf(l[r], corr, lane < kKeys ? pr : 0.0f);
+      m[r] = m_new;
+#pragma unroll
+      for (int j = 0; j < kJ; ++j) { o[j][r].x *= corr; o[j][r].y *= corr; o[j][r].z *= corr; o[j][r].w *= corr; }
+      if (lane < kKeys) probs[lane * kRepPad + r] = pr;
+    }
+    __syncwarp();
+#pragma unroll 2
+    for (uint32_t k = vg; k < nk; k += groups) {
+      float pr[kRepPad];
+      if constexpr (kRepPad >= 4) {
+#pragma unroll
+        for (int r = 0; r < kRepPad; r += 4) *reinterpret_cast<float4*>(pr + r) = *reinterpret_cast<const float4*>(probs + k * kRepPad + r);
+      } else {
+#pragma unroll
+        for (int r = 0; r < kRepPad; ++r) pr[r] = probs[k * kRepPad + r];
+      }
+#pragma unroll
+      for (int j = 0; j < kJ; ++j) {
+        if (vc + 32u * j < nq4) {
+          const float4 v = reinterpret_cast<const float4*>(vs + (size_t)k * hd)[vc + 32u * j];
 #pragma unroll
           for (int r = 0; r < REP; ++r) {
-            acc[r][0] = dot4(q4[r * nq4 + ca], ka, acc[r][0]);
-            acc[r][1] = dot4(q4[r * nq4 + cb], kb, acc[r][1]);
+            o[j][r].x = fmaf(pr[r], v.x, o[j][r].x); o[j][r].y = fmaf(pr[r], v.y, o[j][r].y); o[j][r].z = fmaf(pr[r], v.z, o[j][r].z); o[j][r].w = fmaf(pr[r], v.w, o[j][r].w);
           }
-          cc = cb + 1 == c_hi ? c_lo : cb + 1;
-        }
-        if (it < ncols) {
-          const float4 ka = krow[cc];
-#pragma unroll
-          for (int r = 0; r < REP; ++r) acc[r][0] = dot4(q4[r * nq4 + cc], ka, acc[r][0]);
         }
       }
-#pragma unroll
-      for (int r = 0; r < REP; ++r) part[(wpart * REP + r) * kAttnChunkKeys + key] = acc[r][0] + acc[r][1];
-    }
-    __syncthreads();
-    // ---- scores of (key block, head): sum of the parts, block maximum and sum by shuffles ----
-    if (wpart < REP) {
-      const uint32_t key = wblk * 32 + lane;
-      const bool valid = key < nkeys;
-      float sc = 0.0f;
-#pragma unroll
-      for (int pt = 0; pt < kParts; ++pt) sc += part[(pt * REP + wr) * kAttnChunkKeys + key];
-      const float sv = valid ? sc * p.scale : -INFINITY;
-      float bm = sv;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, off));
-      const float pr = valid ? expf(sv - bm) : 0.0f;
-      float bs = pr;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) bs += __shfl_xor_sync(0xFFFFFFFFu, bs, off);
-      probs[(wblk * REP + wr) * 32 + lane] = pr;
-      if (lane == 0) { bmax[wblk * REP + wr] = bm; bsum[wblk * REP + wr] = bs; }
-      // the token's own key: one more score per head, computed by the first block's warps on the first chunk
-      if (owns_new && c0 == k0 && wblk == 0) {
-        float a = 0.0f;
-        for (uint32_t e = lane; e < hd; e += 32) a = fmaf(qs[wr * hd + e], knew[e], a);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, off);
-        if (lane == 0) bmax[kBlocks * REP + wr] = a * p.scale;
-      }
-    }
-    __syncthreads();
-    // ---- weighted values: this thread's four elements over its group's keys ----
-    if (vact) {
-      const bool with_new = owns_new && c0 == k0;
-      float M = run_m;
-#pragma unroll
-      for (int bl = 0; bl < kBlocks; ++bl) M = fmaxf(M, bmax[bl * REP + vr]);
-      const float snew = with_new ? bmax[kBlocks * REP + vr] : -INFINITY;
-      M = fmaxf(M, snew);
-      const float cr = expf(run_m - M);  // 0 on the first chunk
-      float L = run_l * cr;
-      float4 O = make_float4(run_o.x * cr, run_o.y * cr, run_o.z * cr, run_o.w * cr);
-#pragma unroll
-      for (int bl = 0; bl < kBlocks; ++bl) {
-        const float bm = bmax[bl * REP + vr];
-        if (bm != -INFINITY) {
-          const float cb = expf(bm - M);
-          L = fmaf(bsum[bl * REP + vr], cb, L);
-          const uint32_t nb = min(32u, nkeys - min(nkeys, (uint32_t)bl * 32u));
-          const float* pp = probs + (bl * REP + vr) * 32;
-          const float4* vp = reinterpret_cast<const float4*>(vs + (size_t)bl * 32 * hd) + vc;
-          float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-          uint32_t kk = vg;
-          for (; kk + G < nb; kk += 2 * G) {  // two keys per step: independent reads and sums
-            const float p0 = pp[kk], p1 = pp[kk + G];
-            const float4 v0 = vp[(size_t)kk * nq4], v1 = vp[(size_t)(kk + G) * nq4];
-            a0.x = fmaf(p0, v0.x, a0.x); a0.y = fmaf(p0, v0.y, a0.y); a0.z = fmaf(p0, v0.z, a0.z); a0.w = fmaf(p0, v0.w, a0.w);
-            a1.x = fmaf(p1, v1.x, a1.x); a1.y = fmaf(p1, v1.y, a1.y); a1.z = fmaf(p1, v1.z, a1.z); a1.w = fmaf(p1, v1.w, a1.w);
-          }
-          if (kk < nb) {
-            const float p0 = pp[kk];
-            const float4 v0 = vp[(size_t)kk * nq4];
-            a0.x = fmaf(p0, v0.x, a0.x); a0.y = fmaf(p0, v0.y, a0.y); a0.z = fmaf(p0, v0.z, a0.z); a0.w = fmaf(p0, v0.w, a0.w);
-          }
-          O.x = fmaf(a0.x + a1.x, cb, O.x); O.y = fmaf(a0.y + a1.y, cb, O.y); O.z = fmaf(a0.z + a1.z, cb, O.z); O.w = fmaf(a0.w + a1.w, cb, O.w);
-        }
-      }
-      if (with_new) {
-        const float cn = expf(snew - M);
-        L += cn;
-        if (vg == 0) {
-          const float4 vn = reinterpret_cast<const float4*>(vnew)[vc];
-          O.x = fmaf(cn, vn.x, O.x); O.y = fmaf(cn, vn.y, O.y); O.z = fmaf(cn, vn.z, O.z); O.w = fmaf(cn, vn.w, O.w);
-        }
-      }
-      run_m = M; run_l = L; run_o = O;
     }
   }
-  if (!ok && p.status && tid == 0) atomicExch(p.status, 3);
-  // ---- the key groups' sums come together in group 0 (through the K staging area, no longer needed) ----
-  if (G > 1) {
-    __syncthreads();
-    float4* comb = reinterpret_cast<float4*>(ks);
-    if (vact && vg > 0) comb[(vg - 1) * vthreads + vrem] = run_o;
-    __syncthreads();
-    if (vact && vg == 0) {
-      for (uint32_t g2 = 1; g2 < G; ++g2) {
-        const float4 o2 = comb[(g2 - 1) * vthreads + vrem];
-        run_o.x += o2.x; run_o.y += o2.y; run_o.z += o2.z; run_o.w += o2.w;
+  if (!ok && p.status && lane == 0) atomicCAS(p.status, 0, 3);
+  // ---- this warp's result, over its lanes, into its part of shared memory: [REP][hd] ----
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < REP; ++r) {
+    const float lt = warp_sum(l[r]);
+    if (lane == 0) { s_m[warp][r] = m[r]; s_l[warp][r] = lt; }
+#pragma unroll
+    for (int j = 0; j < kJ; ++j) {
+      for (uint32_t off = lanes; off < 32; off <<= 1) {
+        o[j][r].x += __shfl_xor_sync(0xFFFFFFFFu, o[j][r].x, off); o[j][r].y += __shfl_xor_sync(0xFFFFFFFFu, o[j][r].y, off);
+        o[j][r].z += __shfl_xor_sync(0xFFFFFFFFu, o[j][r].z, off); o[j][r].w += __shfl_xor_sync(0xFFFFFFFFu, o[j][r].w, off);
       }
+      if (vg == 0 && vc + 32u * j < nq4) reinterpret_cast<float4*>(ks)[r * nq4 + vc + 32u * j] = o[j][r];
     }
-  }
-  // ---- this CTA's result: straight out, or into the split scratch ----
-  const uint32_t stride = hd + 4;  // a row of sums, then its maximum and total; 16-byte aligned rows
-  const bool writer = vact && vg == 0;
-  float* sc = p.scratch + ((((size_t)bk * p.T + t) * gridDim.z + split) * REP) * stride;
-  if (writer) {
-    if (gridDim.z == 1) {
-      float* o = p.out + (size_t)(b * p.T + t) * p.out_ld + ((size_t)kvh * REP + vr) * hd + 4 * vc;
-      const float inv = 1.0f / run_l;
-      o[0] = run_o.x * inv; o[1] = run_o.y * inv; o[2] = run_o.z * inv; o[3] = run_o.w * inv;
-    } else {
-      *reinterpret_cast<float4*>(sc + (size_t)vr * stride + 4 * vc) = run_o;
-      if (vc == 0) { sc[(size_t)vr * stride + hd] = run_m; sc[(size_t)vr * stride + hd + 1] = run_l; }
-    }
-  }
-  if (gridDim.z == 1) { if (tid == 0) trace_max(p.trace, 2); return; }
-  // ---- merge the key splits: last CTA to arrive ----
-  __threadfence();
-  __syncthreads();
-  unsigned* counter = p.counters + (size_t)bk * p.T + t;
-  if (tid == 0) {
-    const unsigned a = atomicAdd(counter, 1u);
-    s_last = a == gridDim.z - 1 ? 1u : 0u;
   }
   __syncthreads();
-  if (!s_last) { if (tid == 0) trace_max(p.trace, 2); return; }
-  __threadfence();
-  if (tid == 0) *counter = 0;
-  const float* base = p.scratch + (((size_t)bk * p.T + t) * gridDim.z) * REP * stride;
-  const uint32_t ns = gridDim.z;  // <= 64
-  float* wgt = mg;                // [ns][REP] max, then coefficient
-  float* lsum = mg + 64 * REP;    // [ns][REP]
-  // the splits' sums for this thread's elements are requested first; the weights are worked out while they travel
-  float4 part_o[8];
-  if (writer) {
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      part_o[u] = (uint32_t)u < ns ? __ldcg(reinterpret_cast<const float4*>(base + ((size_t)u * REP + vr) * stride + 4 * vc)) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  for (uint32_t i = tid; i < ns * REP; i += kThreads) {
-    const float* src = base + (size_t)i * stride;  // i = s * REP + r
-    wgt[i] = __ldcg(src + hd);
-    lsum[i] = __ldcg(src + hd + 1);
-  }
-  __syncthreads();
-  float* inv = lsum + 64 * REP;   // [REP] 1 / total
-  if (warp < REP) {  // one warp per head: the lanes share the splits (ns <= 64)
-    const uint32_t r = warp;
-    const float m0 = (uint32_t)lane < ns ? wgt[lane * REP + r] : -INFINITY;
-    const float m1 = (uint32_t)lane + 32 < ns ? wgt[(lane + 32) * REP + r] : -INFINITY;
-    float M = fmaxf(m0, m1);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, off));
-    const float c0 = m0 == -INFINITY ? 0.0f : expf(m0 - M), c1 = m1 == -INFINITY ? 0.0f : expf(m1 - M);
-    float L = 0.0f;
-    if ((uint32_t)lane < ns) { L = lsum[lane * REP + r] * c0; wgt[lane * REP + r] = c0; }
-    if ((uint32_t)lane + 32 < ns) { L = fmaf(lsum[(lane + 32) * REP + r], c1, L); wgt[(lane + 32) * REP + r] = c1; }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xFFFFFFFFu, L, off);
-    if (lane == 0) inv[r] = 1.0f / L;
-  }
-  __syncthreads();
-  if (writer) {
+  if (ns > 1) pipe::cluster_wait();
+  // ---- the warps' results together; several CTAs: to the first one of the cluster ----
+  float* out = p.out + (size_t)(b * p.T + t) * p.out_ld + (size_t)kvh * REP * hd;
+  for (uint32_t i = tid; i < REP * nq4; i += blockDim.x) {
+    const uint32_t r = i / nq4, c = i % nq4;
+    float M = -INFINITY, L = 0.0f;
+    for (uint32_t w = 0; w < warps; ++w) M = fmaxf(M, s_m[w][r]);
     float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (uint32_t s0 = 0; s0 < ns; s0 += 8) {
-      if (s0 > 0) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          part_o[u] = s0 + u < ns ? __ldcg(reinterpret_cast<const float4*>(base + ((size_t)(s0 + u) * REP + vr) * stride + 4 * vc)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (s0 + u < ns) {
-          const float w = wgt[(s0 + u) * REP + vr];
-          O.x = fmaf(part_o[u].x, w, O.x); O.y = fmaf(part_o[u].y, w, O.y); O.z = fmaf(part_o[u].z, w, O.z); O.w = fmaf(part_o[u].w, w, O.w);
+    for (uint32_t w = 0; w < warps; ++w) {
+      const float f = s_m[w][r] == -INFINITY ? 0.0f : expf(s_m[w][r] - M);
+      const float4 v = reinterpret_cast<const float4*>(sm + (size_t)w * per_warp)[i];
+      L = fmaf(s_l[w][r], f, L);
+      O.x = fmaf(v.x, f, O.x); O.y = fmaf(v.y, f, O.y); O.z = fmaf(v.z, f, O.z); O.w = fmaf(v.w, f, O.w);
+    }
+    if (ns == 1) {
+      const float inv = 1.0f / L;
+      reinterpret_cast<float4*>(out)[i] = make_float4(O.x * inv, O.y * inv, O.z * inv, O.w * inv);
+    } else {
+      float* dst = cl + ((size_t)split * REP + r) * (hd + 4);
+      pipe::st_cluster_f4(dst + 4 * c, 0, O);
+      if (c == 0) { pipe::st_cluster_f32(dst + hd, 0, M); pipe::st_cluster_f32(dst + hd + 1, 0, L); }
+    }
+  }
+  if (ns > 1) {
+    pipe::cluster_sync_all();
+    if (split == 0) {
+      for (uint32_t i = tid; i < REP * nq4; i += blockDim.x) {
+        const uint32_t r = i / nq4, c = i % nq4;
+        const float* src = cl + (size_t)r * (hd + 4);
+        const uint32_t step = REP * (hd + 4);
+        float M = -INFINITY, L = 0.0f;
+        for (uint32_t s = 0; s < ns; ++s) M = fmaxf(M, src[s * step + hd]);
+        float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (uint32_t s = 0; s < ns; ++s) {
+          const float ms = src[s * step + hd], f = ms == -INFINITY ? 0.0f : expf(ms - M);
+          const float4 v = *reinterpret_cast<const float4*>(src + s * step + 4 * c);
+          L = fmaf(src[s * step + hd + 1], f, L);
+          O.x = fmaf(v.x, f, O.x); O.y = fmaf(v.y, f, O.y); O.z = fmaf(v.z, f, O.z); O.w = fmaf(v.w, f, O.w);
         }
+        const float inv = 1.0f / L;
+        reinterpret_cast<float4*>(out)[i] = make_float4(O.x * inv, O.y * inv, O.z * inv, O.w * inv);
       }
     }
-    float* o = p.out + (size_t)(b * p.T + t) * p.out_ld + ((size_t)kvh * REP + vr) * hd + 4 * vc;
-    const float iv = inv[vr];
-    o[0] = O.x * iv; o[1] = O.y * iv; o[2] = O.z * iv; o[3] = O.w * iv;
   }
   if (tid == 0) trace_max(p.trace, 2);
 }
@@ -573,22 +470,49 @@ __global__ void take_rows_kernel(const float* __restrict__ x, const int32_t* __r
   for (uint32_t i = threadIdx.x; i < d; i += blockDim.x) y[(size_t)blockIdx.x * d + i] = src[i];
 }
 
-template <int REP, int SUB>
-cudaError_t launch_attn_sub(ruai_ctx* c, const AttnParams& p, dim3 grid, size_t smem) {
+constexpr size_t kAttnSmemMax = 227 * 1024 - 1024;
+
+uint32_t attn_keys(uint32_t hd) { return hd <= 64 ? 32 : hd <= 128 ? 16 : 8; }  // of a warp at a time
+size_t attn_smem(uint32_t rep, uint32_t hd, uint32_t warps, uint32_t splits) {
+  const size_t pad = rep == 3 ? 4 : rep, keys = attn_keys(hd);
+  return ((size_t)warps * std::max(keys * (2 * hd + 4), (size_t)rep * hd) + (rep + 2) * (size_t)hd + warps * keys * pad +
+          (splits > 1 ? (size_t)splits * rep * (hd + 4) : 0)) * sizeof(float);
+}
+
+template <int REP, int LPK>
+cudaError_t launch_attn(ruai_ctx* c, const AttnParams& p, dim3 grid, uint32_t warps, size_t smem) {
   static bool attr_done[64] = {};
   if (!attr_done[c->ordinal & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(attention_kernel<REP, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(attention_kernel<REP, LPK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemMax);
     if (e != cudaSuccess) return e;
     attr_done[c->ordinal & 63] = true;
   }
-  return ruai_launch(c, attention_kernel<REP, SUB>, grid, dim3(kAttnChunkKeys * REP * SUB), smem, true, p);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(warps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (c->use_pdl) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (grid.z > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = 1;
+    attr[na].val.clusterDim.y = 1;
+    attr[na++].val.clusterDim.z = grid.z;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  c->launches++;
+  return cudaLaunchKernelEx(&cfg, attention_kernel<REP, LPK>, p);
 }
 template <int REP>
-cudaError_t launch_attn(ruai_ctx* c, const AttnParams& p, dim3 grid, size_t smem_per_sub) {
-  // smem_per_sub: bytes without the partial scores; those take REP * REP * SUB * 64 floats more
-  const bool big = (size_t)grid.x * grid.y * grid.z > 2u * (size_t)c->sm_count;
-  const size_t parts = (size_t)REP * REP * kAttnChunkKeys * sizeof(float);
-  return big ? launch_attn_sub<REP, 1>(c, p, grid, smem_per_sub + parts) : launch_attn_sub<REP, 2>(c, p, grid, smem_per_sub + 2 * parts);
+cudaError_t launch_attn(ruai_ctx* c, const AttnParams& p, dim3 grid, uint32_t warps, size_t smem) {
+  const uint32_t keys = attn_keys(p.hd);
+  return keys == 32 ? launch_attn<REP, 1>(c, p, grid, warps, smem) : keys == 16 ? launch_attn<REP, 2>(c, p, grid, warps, smem) : launch_attn<REP, 4>(c, p, grid, warps, smem);
 }
 
 }  // namespace
@@ -624,22 +548,33 @@ int ruai_rope_kv(ruai_ctx* c, float* qkv, uint32_t qkv_ld, uint32_t k_off, uint3
   return RUAI_OK;
 }
 
-int ruai_attention(ruai_ctx* c, const AttnParams& p_in, uint32_t B, uint32_t rep, uint32_t splits) {
+int ruai_attention(ruai_ctx* c, const AttnParams& p_in, uint32_t B, uint32_t rep) {
   AttnParams p = p_in;
   p.trace = ruai_trace_slot(c);
   if (p.hd % 4 || p.hd > 256) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "head_dim %u must be a multiple of 4 and at most 256", p.hd);
-  constexpr size_t kb = kAttnChunkKeys / 32;
-  const size_t floats = 2 * (size_t)kAttnChunkKeys * p.hd + (size_t)rep * p.hd + 2 * (size_t)p.hd + kb * rep * 32 + (kb + 1) * rep + kb * rep +
-                        128 * (size_t)rep + rep;  // + the partial scores, added per variant at the launch
-  const size_t smem = floats * sizeof(float);
+  // Warps per CTA and CTAs per item: the numbers with the shortest launch, from the steps that a warp then takes one after the other
+  // and the rounds of CTAs that the grid takes.
+  uint32_t warps = 4, splits = 1;
+  double best = 1e30;
+  for (uint32_t w = 4; w <= (uint32_t)kAttnWarps; w *= 2)
+    for (uint32_t s = 1; s <= 8; s *= 2) {
+      const size_t smem = attn_smem(rep, p.hd, w, s);
+      if (smem > kAttnSmemMax) break;
+      const uint32_t shares = s * w * attn_keys(p.hd), steps = (p.cap + shares - 1) / shares;
+      const uint64_t places = (uint64_t)c->sm_count * std::max<size_t>(1, std::min<size_t>(32 / w, kAttnSmemMax / (smem + 1024)));
+      const uint64_t rounds = ((uint64_t)B * p.KV * p.T * s + places - 1) / places;
+      const double t = rounds * (2.0 + 1.2 * steps) + 0.1 * w + (s > 1 ? 0.6 + 0.1 * s : 0.0);
+      if (t < best) { best = t; splits = s; warps = w; }
+    }
+  const size_t smem = attn_smem(rep, p.hd, warps, splits);
   const dim3 grid(B * p.KV, p.T, splits);
   cudaError_t e;
   switch (rep) {
-    case 1: e = launch_attn<1>(c, p, grid, smem); break;
-    case 2: e = launch_attn<2>(c, p, grid, smem); break;
-    case 3: e = launch_attn<3>(c, p, grid, smem); break;
-    case 4: e = launch_attn<4>(c, p, grid, smem); break;
-    case 8: e = launch_attn<8>(c, p, grid, smem); break;
+    case 1: e = launch_attn<1>(c, p, grid, warps, smem); break;
+    case 2: e = launch_attn<2>(c, p, grid, warps, smem); break;
+    case 3: e = launch_attn<3>(c, p, grid, warps, smem); break;
+    case 4: e = launch_attn<4>(c, p, grid, warps, smem); break;
+    case 8: e = launch_attn<8>(c, p, grid, warps, smem); break;
     default: return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "%u query heads per KV head (supported: 1, 2, 3, 4, 8)", rep);
   }
   if (e != cudaSuccess) return ruai_fail(c, RUAI_ERR_CUDA, "attention launch: %s", cudaGetErrorString(e));

@@ -2,8 +2,6 @@
 #pragma once
 #include "common.cuh"
 
-constexpr int kAttnChunkKeys = 64;  // keys (and values) staged in shared memory at a time
-
 struct AttnParams {
   const float* q;       // [B*T, q_ld]; the rep query heads of KV head g at column g*rep*hd
   uint32_t q_ld;
@@ -19,8 +17,6 @@ struct AttnParams {
   float scale;          // 1/sqrt(hd)
   float* out;           // [B*T, out_ld]
   uint32_t out_ld;
-  float* scratch;       // split merge: [B*KV*T][splits][rep][hd+2]
-  unsigned* counters;   // [B*KV*T], zero between launches
   int* status;          // context status word (bounded waits)
   unsigned long long* trace;  // debug timeline slot
   // ruai_attention_prefill only.  Values of another width than the keys (0: as wide): rows of vd floats in the cache, of
@@ -51,7 +47,7 @@ int ruai_layer_norm(ruai_ctx* c, const float* x, const float* w, const float* b,
 int ruai_rope_table(ruai_ctx* c, const float* inv_freq, uint32_t half, uint32_t max_pos, float2* table);
 int ruai_rope_kv(ruai_ctx* c, float* qkv, uint32_t qkv_ld, uint32_t k_off, uint32_t v_off, const float2* table, const int32_t* len, uint32_t rows,
                  uint32_t T, uint32_t Hq, uint32_t KV, uint32_t hd, uint32_t cap, float* kcache, float* vcache);
-int ruai_attention(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep, uint32_t splits);
+int ruai_attention(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep);
 // Many query positions at once, queries in tiles (attn_prefill.cu).  1: launched; 0: not taken for this shape; < 0: error.
 int ruai_attention_prefill(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep);
 // Whether heads of these widths, each with keys of its own (rep 1, one map), fit it.

@@ -410,19 +410,6 @@ int ensure_cache(ruai_model* m, uint32_t B, uint32_t need) {
   return RUAI_OK;
 }
 
-uint32_t attn_splits(const ruai_model* m, uint32_t B, uint32_t T) {
-  if (T > 1) return 1;
-  // one chunk of 64 keys per CTA where the capacity allows it (a single round trip to memory per CTA); with many
-  // (sequence, KV head) items there are CTAs enough without it, and fewer splits mean fewer partial results to merge
-  // (measured, 8B shape, 1024 positions: 16 sequences 5.65 -> 5.49 ms with two chunks per CTA, 128 sequences 27.2 -> 26.1
-  // with two splits in all)
-  const uint32_t by_len = (m->cap + kAttnChunkKeys - 1) / kAttnChunkKeys;
-  const uint32_t items = B * m->KVl;
-  if (items >= 512) return std::max(1u, std::min(by_len, 2u));
-  if (B >= 5) return std::max(1u, std::min((by_len + 1) / 2, 64u));
-  return std::max(1u, std::min(by_len, 64u));
-}
-
 int ensure_activations(ruai_model* m, uint32_t rows, uint32_t out_rows, uint32_t B, uint32_t T) {
   ruai_ctx* c = m->ctx;
   if (m->hy) return hybrid_reserve(m, rows, out_rows, B, T);
@@ -449,19 +436,6 @@ int ensure_activations(ruai_model* m, uint32_t rows, uint32_t out_rows, uint32_t
     RUAI_CUDA(c, cudaStreamSynchronize(c->stream));
     RUAI_TRY(m->logits.alloc(c, (size_t)out_rows * m->Vl * sizeof(float)));
     m->logit_rows = out_rows;
-    drop_graph(m);
-  }
-  const uint32_t splits = attn_splits(m, B, T);
-  const uint32_t rep = m->Hl / m->KVl;
-  const size_t need = (size_t)B * m->KVl * T * splits * rep * (m->hd + 4) * sizeof(float);
-  const size_t cnt = (size_t)B * m->KVl * T * sizeof(unsigned);
-  if (need > m->attn_scratch.bytes || cnt > m->attn_counters.bytes) {
-    RUAI_CUDA(c, cudaStreamSynchronize(c->stream));
-    RUAI_TRY(m->attn_scratch.reserve(c, need));
-    if (cnt > m->attn_counters.bytes) {
-      RUAI_TRY(m->attn_counters.alloc(c, cnt));
-      RUAI_CUDA(c, cudaMemsetAsync(m->attn_counters.p, 0, cnt, c->stream));
-    }
     drop_graph(m);
   }
   return RUAI_OK;
@@ -494,7 +468,6 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
   const uint32_t nql = m->Hl * hd, nkvl = m->KVl * hd, nqkv = nql + 2 * nkvl, rep = m->Hl / m->KVl;
   int32_t* len = m->d_len.as<int32_t>();
   float *x = m->x.as<float>(), *qkv = m->qkv.as<float>(), *att = m->att.as<float>(), *hb = m->hbuf.as<float>();
-  const uint32_t splits = attn_splits(m, B, T);
   const bool tp = m->world > 1;
   // RMSNorm rides in the prologue of the GEMV that consumes it: the producer of x (embedding, o_proj, down_proj)
   // leaves per-tile sums of squares.  LayerNorm (GPT-2) and the sharded model (x is produced by the exchange
@@ -525,11 +498,11 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
     ap.q = qkv; ap.q_ld = nqkv; ap.kcache = Ly.kc.as<float>(); ap.vcache = Ly.vc.as<float>(); ap.len = len;
     ap.fuse = fuse ? 1 : 0; ap.table = table; ap.k_off = nql; ap.v_off = nql + nkvl;
     ap.T = T; ap.KV = m->KVl; ap.hd = hd; ap.cap = m->cap; ap.scale = 1.0f / sqrtf((float)hd);
-    ap.out = att; ap.out_ld = nql; ap.scratch = m->attn_scratch.as<float>(); ap.counters = m->attn_counters.as<unsigned>(); ap.status = c->status;
+    ap.out = att; ap.out_ld = nql; ap.status = c->status;
     {
       const int took = ruai_attention_prefill(c, ap, B, rep);  // many query positions: queries in tiles
       if (took < 0) return RUAI_ERR_CUDA;
-      if (took == 0) RUAI_TRY(ruai_attention(c, ap, B, rep, splits));
+      if (took == 0) RUAI_TRY(ruai_attention(c, ap, B, rep));
     }
     GemvEpilogue eo;
     eo.bias = Ly.o.bias.as<float>();
@@ -843,7 +816,7 @@ RUAI_API int ruai_model_destroy(ruai_model* m) {
   ruai_sweight_free(&m->head.sw);
   for (DevBuf* b : {&m->ps.layers, &m->ps.x, &m->ps.ss, &m->ps.acc, &m->ps.poison, &m->ps.att_part, &m->ps.arg_slots, &m->ps.sync}) b->release();
   for (DevBuf* b : {&m->embed, &m->wpe, &m->final_w, &m->final_b, &m->rope_table, &m->d_ids, &m->d_len, &m->d_err, &m->x, &m->xn, &m->qkv, &m->att,
-                    &m->hbuf, &m->xl, &m->logits, &m->attn_scratch, &m->attn_counters, &m->sumsq, &m->arg_slots, &m->arg_counter})
+                    &m->hbuf, &m->xl, &m->logits, &m->sumsq, &m->arg_slots, &m->arg_counter})
     b->release();
   m->d_rows.release();
   hybrid_destroy(m);

@@ -201,6 +201,66 @@ def test_attention_geometries(dev, H, KV, hd, B):
         tok = np.argmax(want, axis=1).astype(np.int32).reshape(B, 1)
 
 
+def _pointed(dev, H, KV, hd, B):
+    """One layer whose queries and keys are large, so that few keys carry the weight of a row: the model, and its logits [B, T, V] in float64."""
+    V, d, ff, rng = 41, 64, 32, np.random.default_rng(H * 1000 + hd + B)
+    gm = nn.Llama(dev, nn.LlamaConfig(V, d, ff, 1, H, KV, hd, 700, 1e-5, 10000.0, 0))
+    shapes = {0: (d, H * hd, 0.3), 1: (d, KV * hd, 0.3), 2: (d, KV * hd, 0.3), 3: (H * hd, d, 0.1), 4: (d, ff, 0.02), 5: (d, ff, 0.02), 6: (ff, d, 0.02), T_LMHEAD: (d, V, 0.1)}
+    w = {}
+    for t, (k, n, std) in shapes.items():
+        f = (rng.standard_normal((k, n)) * std).astype(np.float32)
+        gm.set_f32(t, f)
+        q, sc = oracle.quantize_int8(f)
+        w[t] = q.astype(np.float64) * sc
+    embed = rng.standard_normal((V, d)).astype(np.float32)
+    gm.set_f32(0x10000000, embed)
+    for t in (0x50000000, 0x52000000, 0x40000000):
+        gm.set_f32(t, np.ones(d, np.float32))
+    gm.quantize_int8()
+    inv = np.float32(10000.0) ** (-np.arange(0, hd, 2, dtype=np.float32) / np.float32(hd))
+
+    def rms(x):
+        return x / np.sqrt((x * x).mean(-1, keepdims=True) + 1e-5)
+
+    def logits(ids):
+        T = ids.shape[1]
+        angle = np.arange(T)[:, None] * inv.astype(np.float64)
+        cos, sin = np.concatenate([np.cos(angle)] * 2, 1), np.concatenate([np.sin(angle)] * 2, 1)
+        turn = lambda t: t * cos + np.concatenate([-t[..., hd // 2:], t[..., :hd // 2]], -1) * sin
+        x = embed[ids].astype(np.float64)
+        heads = lambda t, n: t.reshape(B, T, n, hd).transpose(0, 2, 1, 3)
+        h = rms(x)
+        q, k, v = turn(heads(h @ w[0], H)), turn(heads(h @ w[1], KV)), heads(h @ w[2], KV)
+        k, v = np.repeat(k, H // KV, 1), np.repeat(v, H // KV, 1)
+        s = np.where(np.tril(np.ones((T, T), bool)), q @ k.transpose(0, 1, 3, 2) / np.sqrt(hd), -np.inf)
+        p = np.exp(s - s.max(-1, keepdims=True))
+        x = x + ((p / p.sum(-1, keepdims=True)) @ v).transpose(0, 2, 1, 3).reshape(B, T, H * hd) @ w[3]
+        h = rms(x)
+        g = h @ w[4]
+        return rms(x + (g / (1 + np.exp(-g)) * (h @ w[5])) @ w[6]) @ w[T_LMHEAD]
+
+    return gm, logits, rng
+
+
+@pytest.mark.parametrize("H,KV,hd", [(1, 1, 64), (4, 2, 128), (6, 2, 64), (8, 2, 8), (8, 1, 64), (2, 2, 256), (8, 1, 256), (3, 1, 80)])
+@pytest.mark.parametrize("B,lengths", [(1, (1, 9, 31, 33, 64, 127, 129, 600)), (3, (63, 130)), (40, (32, 65))])
+def test_attention_against_float64(dev, H, KV, hd, B, lengths):
+    """A prompt at once, in two portions, and a step of one token after it: keys shared out over warps and CTAs, tiles of 64 keys, rows of
+    128.  Scores of up to 40 in f32 (and in the matrix products' 22 bits): 40 * 2^-22 of a weight, and as much again for the rest."""
+    gm, logits, rng = _pointed(dev, H, KV, hd, B)
+    for n in lengths:
+        ids = rng.integers(0, 41, (B, n + 1)).astype(np.int32)
+        want = logits(ids)
+        near = lambda got, ref: np.abs(got - ref).max() <= 2e-5 * np.abs(want).max()
+        gm.cache_clear()
+        assert near(gm.forward_cached(ids[:, :n], all_positions=True), want[:, :n]), n
+        assert near(gm.forward_cached(ids[:, n:]), want[:, -1]), n
+        gm.cache_clear()
+        gm.forward_cached(ids[:, :n // 3 + 1], want_logits=False)
+        if n // 3 < n:
+            assert near(gm.forward_cached(ids[:, n // 3 + 1:], all_positions=True), want[:, n // 3 + 1:]), n
+
+
 def test_errors_mirror_the_reference_asserts(dev):
     _, gm = build(dev, llama_cfg(**dict(TINY_LLAMA, max_pos=8)), 5, 8)
     with pytest.raises(nn.RuaiError, match="exceeds max_position_embeddings"):
