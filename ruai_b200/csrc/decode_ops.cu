@@ -112,46 +112,34 @@ __global__ void rope_table_kernel(const float* __restrict__ inv_freq, uint32_t h
 
 // apply_rope (functional.rs:197-204) on q in place and on k while appending k, v to the
 // cache (KvBuf::append, transformer.rs:27-53).  qkv row layout: [q heads | k heads | v heads].
-// grid (B*T, Hq + KV); thread i < hd/2 handles the pair (i, i + hd/2).
-__global__ void rope_kv_kernel(float* __restrict__ qkv, uint32_t qkv_ld, uint32_t k_off, uint32_t v_off, const float2* __restrict__ table,
+// A CTA per token, a thread per pair (i, i + hd/2) of a head.
+constexpr int kRopeThreads = 256;
+__global__ void __launch_bounds__(kRopeThreads) rope_kv_kernel(float* __restrict__ qkv, uint32_t qkv_ld, uint32_t k_off, uint32_t v_off, const float2* __restrict__ table,
                                const int32_t* __restrict__ len, uint32_t T, uint32_t Hq, uint32_t KV, uint32_t hd, uint32_t cap,
                                float* __restrict__ kcache, float* __restrict__ vcache, int* __restrict__ status) {
   grid_dependency_wait();
   grid_launch_dependents();
-  const uint32_t r = blockIdx.x, b = r / T, t = r % T, head = blockIdx.y, half = hd / 2;
+  const uint32_t r = blockIdx.x, b = r / T, t = r % T, half = hd / 2;
   const uint32_t pos = (uint32_t)*len + t;
   float* row = qkv + (size_t)r * qkv_ld;
-  if (head < Hq) {
-    if (!table) return;
-    float* q = row + (size_t)head * hd;
-    for (uint32_t i = threadIdx.x; i < half; i += blockDim.x) {
-      const float2 cs = table[(size_t)pos * half + i];
-      const float x1 = q[i], x2 = q[i + half];
-      q[i] = x1 * cs.x + (-x2) * cs.y;
-      q[i + half] = x2 * cs.x + x1 * cs.y;
-    }
-  } else {
-    const uint32_t h = head - Hq;
-    if (pos >= cap) {  // never write past the cache (see attention_kernel)
-      if (threadIdx.x == 0 && status) atomicCAS(status, 0, 5);
-      return;
-    }
-    const float* k = row + k_off + (size_t)h * hd;
-    const float* v = row + v_off + (size_t)h * hd;
-    float* kd = kcache + (((size_t)b * KV + h) * cap + pos) * hd;
-    float* vd = vcache + (((size_t)b * KV + h) * cap + pos) * hd;
-    for (uint32_t i = threadIdx.x; i < half; i += blockDim.x) {
-      const float x1 = k[i], x2 = k[i + half];
-      if (table) {
-        const float2 cs = table[(size_t)pos * half + i];
-        kd[i] = x1 * cs.x + (-x2) * cs.y;
-        kd[i + half] = x2 * cs.x + x1 * cs.y;
-      } else {
-        kd[i] = x1;
-        kd[i + half] = x2;
-      }
-      vd[i] = v[i];
-      vd[i + half] = v[i + half];
+  const bool over = pos >= cap;  // never write past the cache (see attention_kernel)
+  if (over && threadIdx.x == 0 && status) atomicCAS(status, 0, 5);
+  const uint32_t begin = table ? 0u : Hq * half, end = (over ? Hq : Hq + KV) * half;
+#pragma unroll 4
+  for (uint32_t p = begin + threadIdx.x; p < end; p += kRopeThreads) {
+    const uint32_t head = p / half, i = p % half;
+    const bool key = head >= Hq;
+    float* src = key ? row + k_off + (size_t)(head - Hq) * hd : row + (size_t)head * hd;
+    const float x1 = src[i], x2 = src[i + half];
+    const float2 cs = table ? table[(size_t)pos * half + i] : make_float2(1.0f, 0.0f);
+    const size_t at = key ? (((size_t)b * KV + head - Hq) * cap + pos) * hd : 0;
+    float* dst = key ? kcache + at : src;
+    dst[i] = table ? x1 * cs.x + (-x2) * cs.y : x1;
+    dst[i + half] = table ? x2 * cs.x + x1 * cs.y : x2;
+    if (key) {
+      const float* v = row + v_off + (size_t)(head - Hq) * hd;
+      vcache[at + i] = v[i];
+      vcache[at + i + half] = v[i + half];
     }
   }
 }
@@ -542,8 +530,7 @@ int ruai_rope_table(ruai_ctx* c, const float* inv_freq, uint32_t half, uint32_t 
 
 int ruai_rope_kv(ruai_ctx* c, float* qkv, uint32_t qkv_ld, uint32_t k_off, uint32_t v_off, const float2* table, const int32_t* len, uint32_t rows,
                  uint32_t T, uint32_t Hq, uint32_t KV, uint32_t hd, uint32_t cap, float* kcache, float* vcache) {
-  const unsigned threads = hd / 2 >= 64 ? 64 : 32;
-  RUAI_CUDA(c, ruai_launch(c, rope_kv_kernel, dim3(rows, Hq + KV), dim3(threads), 0, true, qkv, qkv_ld, k_off, v_off, table, len, T, Hq, KV, hd, cap,
+  RUAI_CUDA(c, ruai_launch(c, rope_kv_kernel, dim3(rows), dim3(kRopeThreads), 0, true, qkv, qkv_ld, k_off, v_off, table, len, T, Hq, KV, hd, cap,
                            kcache, vcache, c->status));
   return RUAI_OK;
 }
