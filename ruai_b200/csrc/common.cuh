@@ -17,6 +17,8 @@
 // Number of SMs of the target part; grids are sized in multiples of it.
 constexpr int kSmCountB200 = 148;
 
+constexpr uint32_t kPinnedWords = 1024;
+
 struct ruai_ctx {
   int ordinal = 0;
   cudaStream_t stream = nullptr;
@@ -38,6 +40,7 @@ struct ruai_ctx {
   unsigned long long* trace = nullptr;  // debug: per-launch [first entry, first past the dependency wait, last exit] in ns
   unsigned trace_slots = 0, trace_seq = 0;
   int* status = nullptr;  // device word: 0 ok, 3 / 4 = a bounded wait inside a kernel ran out (mbarrier / grid barrier), 5 = cache position out of range
+  int32_t* pinned = nullptr;  // kPinnedWords words of pinned host memory: what a step leaves for the host
   unsigned long long launches = 0;
   // persistent kernels (pstep.cu)
   unsigned spin_limit = 1u << 20;  // polls of a bounded device-side wait (about a second)
@@ -250,6 +253,8 @@ int ruai_gemm_tc_launch(ruai_ctx* ctx, const ruai_qweight* w, const void* x, int
                         const GemvEpilogue& epi, const GemvPrologue& pro);
 // Reads and clears the context's device status word (synchronizes the stream).
 int ruai_ctx_check_status(ruai_ctx* ctx);
+// What a status word that has been read means; clears it on the device.
+int ruai_ctx_status_result(ruai_ctx* ctx, int status);
 
 // y = x @ W for m rows; x is [m, k] (row stride x_ld) in x_dtype.
 int ruai_gemv_launch(ruai_ctx* ctx, const ruai_qweight* w, const void* x, int x_dtype, uint32_t x_ld, uint32_t m, void* out,

@@ -63,6 +63,11 @@ RUAI_API int ruai_ctx_create(int ordinal, void* stream_or_null, ruai_ctx** out) 
     delete c;
     return ruai_fail(nullptr, RUAI_ERR_CUDA, "cannot allocate the status word");
   }
+  if (cudaHostAlloc(&c->pinned, kPinnedWords * sizeof(int32_t), cudaHostAllocDefault) != cudaSuccess) {
+    cudaFree(c->status);
+    delete c;
+    return ruai_fail(nullptr, RUAI_ERR_CUDA, "cannot allocate pinned memory");
+  }
   int rc = ruai_ctx_reserve(c, kScratchBytes, 4096);
   if (rc != RUAI_OK) { g_ruai_global_err = c->err; delete c; return rc; }
   if (!block_pool::attach(c, ordinal, c->stream)) {
@@ -81,6 +86,7 @@ RUAI_API int ruai_ctx_destroy(ruai_ctx* c) {
   cudaFree(c->partial);
   cudaFree(c->counters);
   cudaFree(c->status);
+  cudaFreeHost(c->pinned);
   cudaFree(c->ps_sync);
   cudaFree(c->sample_buf);
   cudaEventDestroy(c->ev0);
@@ -118,6 +124,10 @@ int ruai_ctx_check_status(ruai_ctx* c) {
   int st = 0;
   RUAI_CUDA(c, cudaMemcpyAsync(&st, c->status, sizeof st, cudaMemcpyDeviceToHost, c->stream));
   RUAI_CUDA(c, cudaStreamSynchronize(c->stream));
+  return ruai_ctx_status_result(c, st);
+}
+
+int ruai_ctx_status_result(ruai_ctx* c, int st) {
   if (st == 0) return RUAI_OK;
   cudaMemsetAsync(c->status, 0, sizeof(int), c->stream);
   if (c->ps_sync) {  // a persistent launch that gave up leaves its barrier count undefined: start over

@@ -575,19 +575,28 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
 
 int pstep_reset(ruai_model* m);
 
-int check_device_status(ruai_model* m) {
-  int32_t e = 0;
-  RUAI_CUDA(m->ctx, cudaMemcpyAsync(&e, m->d_err.p, sizeof e, cudaMemcpyDeviceToHost, m->ctx->stream));
-  RUAI_CUDA(m->ctx, cudaStreamSynchronize(m->ctx->stream));
+// Waits for the step; its error words and the first n token ids come back with it, through pinned memory, so that the host waits once:
+// a copy into pageable memory is a wait of its own.
+int read_back(ruai_model* m, int32_t* ids_host, uint32_t n) {
+  ruai_ctx* c = m->ctx;
+  int32_t* h = c->pinned;  // the model's error word, the context's, the ids
+  const bool staged = n + 2 <= kPinnedWords;
+  RUAI_CUDA(c, cudaMemcpyAsync(h, m->d_err.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+  RUAI_CUDA(c, cudaMemcpyAsync(h + 1, c->status, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+  if (n) RUAI_CUDA(c, cudaMemcpyAsync(staged ? h + 2 : ids_host, m->d_ids.p, (size_t)n * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+  RUAI_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (n && staged) memcpy(ids_host, h + 2, (size_t)n * sizeof(int32_t));
+  const int32_t e = h[0], status = h[1];
   if (e == 0) {
-    const int rc = ruai_ctx_check_status(m->ctx);
+    const int rc = ruai_ctx_status_result(c, status);
     if (rc != RUAI_OK) pstep_reset(m);  // a step that gave up leaves its accumulators and barrier count undefined
     return rc;
   }
-  cudaMemsetAsync(m->d_err.p, 0, sizeof(int32_t), m->ctx->stream);
+  cudaMemsetAsync(m->d_err.p, 0, sizeof(int32_t), c->stream);
   if (e == 1) return model_fail(m, RUAI_ERR_ARG, "token id out of range [0, %u)", m->V);
   return model_fail(m, RUAI_ERR_TIMEOUT, "tensor-parallel exchange timed out waiting for a peer (status %d)", e);
 }
+int check_device_status(ruai_model* m) { return read_back(m, nullptr, 0); }
 
 // ---- the persistent decode step (pstep.cu) ---------------------------------------------------
 
@@ -1122,11 +1131,7 @@ RUAI_API int ruai_model_decode_step(ruai_model* m, const int32_t* ids_dev, uint3
     m->len_dirty = false;
   }
   RUAI_TRY(run_decode_graph(m, B));
-  if (next_host) {
-    RUAI_CUDA(c, cudaMemcpyAsync(next_host, m->d_ids.p, (size_t)B * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-    return check_device_status(m);
-  }
-  return RUAI_OK;
+  return next_host ? read_back(m, next_host, B) : RUAI_OK;
 }
 
 // Times `iters` passes over every quantized Linear of the model (the weight-streaming
@@ -1251,13 +1256,11 @@ static int generate_impl(ruai_model* m, const int32_t* prompt, uint32_t T, uint3
       m->len_dirty = false;
       RUAI_TRY(issue_step(m, 1, Tn, HeadRows(), true));
       m->len += Tn;
-      RUAI_CUDA(c, cudaMemcpyAsync(&next, m->d_ids.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-      RUAI_TRY(check_device_status(m));
+      RUAI_TRY(read_back(m, &next, 1));
     }
     if (sampler) {  // the step left the argmax in d_ids; the sampled token replaces it there
       RUAI_TRY(ruai_sample_device(c, m->logits.as<float>(), m->V, sampler->temperature, sampler->top_k, sampler->top_p, &sampler->state, m->d_ids.as<int32_t>()));
-      RUAI_CUDA(c, cudaMemcpyAsync(&next, m->d_ids.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-      RUAI_TRY(check_device_status(m));
+      RUAI_TRY(read_back(m, &next, 1));
     }
     on_device = true;
     ids.push_back(next);
