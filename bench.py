@@ -399,8 +399,8 @@ def run_workload(nn, dev, name, K, W, regions, rank=0, world=1, dist=None, local
         achieved = lin_bytes / (lin_ms / 1000.0) / 1e9
         traffic = None
         try:
-            # DRAM bytes per algorithmic byte from one ncu capture per kernel family (narrow: up to 4 rows; 16-row tile: 5..16)
-            with open(os.path.join(ROOT, "profiles", "gemv_traffic.json" if B <= 4 else "gemv_wide_traffic.json")) as f:
+            # DRAM bytes per algorithmic byte from one ncu capture per kernel family (one row; 2..4 rows; 16-row tile: 5..16)
+            with open(os.path.join(ROOT, "profiles", "gemv_dot_traffic.json" if B == 1 else "gemv_traffic.json" if B <= 4 else "gemv_wide_traffic.json")) as f:
                 tr = json.load(f).get(f"int{bits}")
                 if tr and B <= 16:
                     traffic = tr["dram_bytes_per_algorithmic_byte"] * lin_bytes / lin_launches
@@ -410,10 +410,10 @@ def run_workload(nn, dev, name, K, W, regions, rank=0, world=1, dist=None, local
             kname = "gemm_tc_kernel (tcgen05 kind::f16 dequant GEMM, every Linear of the model)"
         elif B >= 5:
             kname = f"gemv_wide_kernel<{bits}> + xsplit16_kernel (tcgen05 kind::f16, one 16-row tile, weights streamed once; Linears of 4M weights and more)"
-        elif bits == 4:
-            kname = f"gemv_tc_int4_kernel<rows<={min(B, 8)}> (tcgen05 kind::i8 fused dequant GEMV; the int8 head runs gemv_tc_int8_kernel)"
+        elif B == 1:
+            kname = f"gemv_dot::row_kernel<{bits}> (dp4a fused dequant GEMV, every Linear of the model; the head in int8)"
         else:
-            kname = f"gemv_tc_int8_kernel<rows<={min(B, 8)}> (tcgen05 kind::i8 fused dequant GEMV, every Linear of the model)"
+            kname = f"gemv_tc_int{bits}_kernel<rows<={min(B, 8)}> (tcgen05 kind::i8 fused dequant GEMV; small Linears on gemv_dot::rows_kernel)"
         res["roofline"] = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                            "peak_source": peak_src + " hbm_gbs", "traffic": traffic, "bytes_per_launch": lin_bytes / lin_launches,
                            "us_per_launch": 1000.0 * lin_ms / lin_launches, "launches_timed": lin_launches * iters, "per_gpu": True,

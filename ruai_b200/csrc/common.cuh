@@ -219,6 +219,7 @@ struct GemvEpilogue {
 // rstd = 1/sqrt(sum(x^2) * (1/k) + eps), the sum given as per-tile partial sums [tiles][m].
 struct GemvPrologue {
   const float* norm_w = nullptr;  // f32 [k]; NULL: x is used as it is
+  const float* norm_b = nullptr;  // f32 [k]: LayerNorm (functional.rs:137-146) in the place of RMSNorm; gemv_dot.cu only
   const float* sumsq = nullptr;
   uint32_t tiles = 0;
   float eps = 0.0f;
@@ -227,8 +228,16 @@ struct GemvPrologue {
 
 constexpr int kGemvTileCols = 256;      // columns per CTA of gemv.cu, and per sumsq / argmax tile it writes
 constexpr int kGemvBulkTileCols = 128;  // the same for gemv_bulk.cu
-// Number of sumsq / argmax tiles a GEMV over `w` writes (depends on which kernel serves it).
-uint32_t ruai_gemv_tiles(const ruai_ctx* ctx, const ruai_qweight* w);
+constexpr int kGemvDotTileCols = 8;     // the narrowest of gemv_dot.cu
+constexpr uint32_t kGemvDotPickRows = 8;  // rows up to which its greedy pick is fused, with a slot per row and CTA (two per SM)
+// Number of sumsq / argmax tiles a GEMV over `w` and m rows writes (depends on which kernel serves it).
+uint32_t ruai_gemv_tiles(const ruai_ctx* ctx, const ruai_qweight* w, uint32_t m);
+// The dot-product kernel (gemv_dot.cu): whether it runs m rows of w, and the sumsq tiles it then writes.  It works the norm of its
+// input out by itself (the prologue's sumsq is not used).
+bool ruai_gemv_dot_takes(const ruai_ctx* ctx, const ruai_qweight* w, uint32_t m);
+uint32_t ruai_gemv_dot_tiles(const ruai_ctx* ctx, const ruai_qweight* w, uint32_t m);
+int ruai_gemv_dot_launch(ruai_ctx* ctx, const ruai_qweight* w, const void* x, int x_dtype, uint32_t x_ld, uint32_t m, void* out,
+                         const GemvEpilogue& epi, const GemvPrologue& pro);
 bool ruai_gemv_bulk_eligible(const ruai_qweight* w);
 int ruai_gemv_bulk_launch(ruai_ctx* ctx, const ruai_qweight* w, const void* x, int x_dtype, uint32_t x_ld, uint32_t m, void* out,
                           const GemvEpilogue& epi, const GemvPrologue& pro);

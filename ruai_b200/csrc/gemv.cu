@@ -380,6 +380,7 @@ int ruai_gemv_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x_dt
     d.w = w; d.x = x; d.x_ld = x_ld; d.out = out; d.epi = epi_in;
     return ruai_dense_launch(c, &d, 1, x_dtype, m);
   }
+  if (ruai_gemv_dot_takes(c, w, m)) return ruai_gemv_dot_launch(c, w, x, x_dtype, x_ld, m, out, epi_in, pro);
   if (ruai_gemm_tc_takes(c, w, m, epi_in))
     return ruai_gemm_tc_launch(c, w, x, x_dtype, x_ld, m, out, epi_in, pro);
   if (c->use_bulk && c->use_tc && ruai_gemv_wide_eligible(c, w, m)) return ruai_gemv_wide_launch(c, w, x, x_dtype, x_ld, m, out, epi_in, pro);
@@ -429,7 +430,8 @@ size_t ruai_gemv_xs_bytes(const ruai_qweight* w, uint32_t m) {
   return m <= 16 ? ((groups + 1) & ~(size_t)1) * 2048 : (size_t)((m + 127) / 128) * ((groups + 1) / 2) * 32768 + (size_t)m * 4;
 }
 
-uint32_t ruai_gemv_tiles(const ruai_ctx* c, const ruai_qweight* w) {
+uint32_t ruai_gemv_tiles(const ruai_ctx* c, const ruai_qweight* w, uint32_t m) {
+  if (ruai_gemv_dot_takes(c, w, m)) return ruai_gemv_dot_tiles(c, w, m);
   const uint32_t t = c->use_bulk && ruai_gemv_bulk_eligible(w) ? kGemvBulkTileCols : kGemvTileCols;
   return (w->n + t - 1) / t;
 }

@@ -1,5 +1,5 @@
 // Fused dequantize + GEMV on the tensor cores (tcgen05, accumulators in tensor memory) for
-// int4 group-32 weights and up to sixteen rows of activations (eight per CTA): the decode hot path.
+// int4 group-32 weights and two to sixteen rows of activations (eight per CTA): what gemv_dot.cu leaves of the decode hot path.
 //
 // Why tensor cores for a memory-bound kernel: at full HBM speed one SM has to consume about
 // 46 int4 weights per clock.  On the CUDA cores every weight costs a byte permute, a
@@ -533,14 +533,14 @@ int ruai_gemv_tc_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x
   if (epi.sumsq && epi.act == ACT_SWIGLU) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "sum of squares with the SwiGLU epilogue");
   if (epi.argmax_out && epi.act == ACT_SWIGLU) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "argmax with the SwiGLU epilogue");
   // up to 8 rows per CTA; 9..16 rows run as two row tiles (the second pass over the weights mostly hits the L2)
-  const int mt = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : 8;
+  const int mt = m <= 2 ? 2 : m <= 4 ? 4 : 8;
   const uint32_t row_tiles = (m + mt - 1) / mt;
   if (epi.argmax_out && row_tiles != 1) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "fused argmax needs a single row tile");
   const uint32_t col_tiles = (w->n + kCols - 1) / kCols;
   // Split k over a cluster of up to 8 CTAs.  A launch is a link in a chain of dependent kernels, so what counts is its
   // latency.  Measured on the 8B shapes, in microseconds: about 5.5 per wave of CTAs that is fixed, 0.45 per stage
   // (more with more rows) and 0.15 per CTA of the cluster for the reduction.
-  const double per_stage = 0.45 * (mt == 1 ? 1.0 : mt == 2 ? 1.4 : mt == 4 ? 2.0 : 3.2);
+  const double per_stage = 0.45 * (mt == 2 ? 1.4 : mt == 4 ? 2.0 : 3.2);
   uint32_t splits = 1;
   bool small = false;  // the three-CTAs-per-SM variant
   double best = 1e30;
@@ -575,8 +575,7 @@ int ruai_gemv_tc_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x
   const dim3 grid(col_tiles, splits, row_tiles);
   // few CTAs per SM: spend the free registers on a deeper weight queue
   const bool deep = !(c->force_splits & 256u);
-  cudaError_t e = mt == 1 ? (deep && !small ? launch_one<1, 4>(c, p, grid) : launch_one<1, 2>(c, p, grid))
-                : mt == 2 ? (deep && !small ? launch_one<2, 4>(c, p, grid) : launch_one<2, 2>(c, p, grid))
+  cudaError_t e = mt == 2 ? (deep && !small ? launch_one<2, 4>(c, p, grid) : launch_one<2, 2>(c, p, grid))
                 : mt == 4 ? launch_one<4, 2>(c, p, grid)
                           : launch_one<8, 2>(c, p, grid);
   if (e != cudaSuccess) return ruai_fail(c, RUAI_ERR_CUDA, "tensor-core gemv launch failed: %s", cudaGetErrorString(e));

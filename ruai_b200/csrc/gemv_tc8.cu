@@ -429,7 +429,7 @@ int ruai_gemv_tc8_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int 
   if (epi.act == ACT_SWIGLU && (w->n & 1)) return ruai_fail(c, RUAI_ERR_SHAPE, "SwiGLU epilogue needs an even column count, got %u", w->n);
   if (epi.out_ld == 0) epi.out_ld = epi.act == ACT_SWIGLU ? w->n / 2 : w->n;
   if (epi.sumsq && epi.act == ACT_SWIGLU) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "sum of squares with the SwiGLU epilogue");
-  const int mt = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : 8;
+  const int mt = m <= 2 ? 2 : m <= 4 ? 4 : 8;
   const uint32_t row_tiles = (m + mt - 1) / mt;
   if (epi.argmax_out && (row_tiles != 1 || epi.act == ACT_SWIGLU)) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "fused argmax needs a single row tile");
   const uint32_t col_tiles = (w->n + kCols - 1) / kCols;
@@ -461,8 +461,7 @@ int ruai_gemv_tc8_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int 
   p.pro.trace = ruai_trace_slot(c);
   const dim3 grid(col_tiles, splits, row_tiles);
   const bool deep = mt <= 2 && slice_k >= 4096;  // a long slice of k and a small digit buffer: the deeper ring pays
-  cudaError_t e = mt == 1 ? (deep ? launch_one<1, kStagesLong>(c, p, grid, slice_k) : launch_one<1, kStagesShort>(c, p, grid, slice_k))
-                : mt == 2 ? (deep ? launch_one<2, kStagesLong>(c, p, grid, slice_k) : launch_one<2, kStagesShort>(c, p, grid, slice_k))
+  cudaError_t e = mt == 2 ? (deep ? launch_one<2, kStagesLong>(c, p, grid, slice_k) : launch_one<2, kStagesShort>(c, p, grid, slice_k))
                 : mt == 4 ? launch_one<4, kStagesShort>(c, p, grid, slice_k) : launch_one<8, kStagesShort>(c, p, grid, slice_k);
   if (e != cudaSuccess) return ruai_fail(c, RUAI_ERR_CUDA, "int8 tensor-core gemv launch failed: %s", cudaGetErrorString(e));
   return RUAI_OK;

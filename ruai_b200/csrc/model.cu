@@ -423,8 +423,9 @@ int ensure_activations(ruai_model* m, uint32_t rows, uint32_t out_rows, uint32_t
     RUAI_TRY(m->att.alloc(c, (size_t)rows * m->Hl * m->hd * sizeof(float)));
     RUAI_TRY(m->hbuf.alloc(c, (size_t)rows * m->fl * sizeof(float)));
     RUAI_TRY(m->xl.alloc(c, (size_t)rows * m->d * sizeof(float)));
-    RUAI_TRY(m->sumsq.alloc(c, (size_t)rows * ((m->d + kGemvBulkTileCols - 1) / kGemvBulkTileCols) * sizeof(float)));
-    RUAI_TRY(m->arg_slots.alloc(c, (size_t)16 * ((m->Vl + kGemvBulkTileCols - 1) / kGemvBulkTileCols) * sizeof(int2)));
+    RUAI_TRY(m->sumsq.alloc(c, (size_t)rows * ((m->d + kGemvDotTileCols - 1) / kGemvDotTileCols) * sizeof(float)));
+    const size_t slots = std::max<size_t>(16 * ((m->Vl + kGemvBulkTileCols - 1) / kGemvBulkTileCols), kGemvDotPickRows * 2 * (size_t)c->sm_count);
+    RUAI_TRY(m->arg_slots.alloc(c, slots * sizeof(int2)));
     if (!m->arg_counter.p) {
       RUAI_TRY(m->arg_counter.alloc(c, sizeof(unsigned)));
       RUAI_CUDA(c, cudaMemsetAsync(m->arg_counter.p, 0, sizeof(unsigned), c->stream));
@@ -448,9 +449,10 @@ int ensure_activations(ruai_model* m, uint32_t rows, uint32_t out_rows, uint32_t
 int normed_linear(ruai_model* m, const ruai_qweight* w, const float* x, const float* nw, const float* nb, uint32_t rows, float* out, const GemvEpilogue& e) {
   ruai_ctx* c = m->ctx;
   float* xn = m->xn.as<float>();
-  if (m->llama && ruai_gemm_tc_takes(c, w, rows, e)) {
+  const bool dot = ruai_gemv_dot_takes(c, w, rows);
+  if (dot || (m->llama && ruai_gemm_tc_takes(c, w, rows, e))) {
     GemvPrologue pr;
-    pr.norm_w = nw; pr.eps = m->eps;
+    pr.norm_w = nw; pr.norm_b = nb; pr.eps = m->llama ? m->eps : 1e-5f;
     return ruai_gemv_launch(c, w, x, RUAI_F32, m->d, rows, out, e, pr);
   }
   if (m->llama) RUAI_TRY(ruai_rms_norm(c, x, nw, rows, m->d, m->eps, xn));
@@ -474,8 +476,9 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
   // kernel) keep the standalone norm kernels.
   // decode-sized steps on the chunk-layout kernels; sharded: only where the exchange kernel can supply the sum of squares
   const bool fold = m->llama && (m->bits == 8 || m->group == 32) && rows <= 16 && (!tp || ruai_tp_allreduce_gives_sumsq(rows, d));
-  float* ss = fold ? m->sumsq.as<float>() : nullptr;
-  const uint32_t d_tiles = tp ? 1u : ruai_gemv_tiles(c, m->layers[0].o.w);  // o_proj and down_proj both write [.., d]; sharded: the exchange writes one tile
+  auto dot = [&](const Lin& l) { return ruai_gemv_dot_takes(c, l.w, rows); };
+  // the sums of squares are for the kernels that do not work them out themselves
+  float* ss = fold && !(dot(m->layers[0].qkv) && dot(m->layers[0].up) && dot(m->head)) ? m->sumsq.as<float>() : nullptr;
   uint32_t ss_tiles = 1;
   RUAI_TRY(ruai_embed(c, m->d_ids.as<int32_t>(), m->embed.as<float>(), m->llama ? nullptr : m->wpe.as<float>(), len, rows, T, d, m->V, x,
                       m->d_err.as<int>(), ss));
@@ -483,7 +486,7 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
     Layer& Ly = m->layers[l];
     GemvEpilogue e;
     e.bias = Ly.qkv.bias.as<float>();
-    if (fold) {
+    if (fold && !dot(Ly.qkv)) {
       GemvPrologue pr;
       pr.norm_w = Ly.n1w.as<float>(); pr.sumsq = ss; pr.tiles = ss_tiles; pr.eps = m->eps;
       RUAI_TRY(ruai_gemv_launch(c, Ly.qkv.w, x, RUAI_F32, d, rows, qkv, e, pr));
@@ -515,11 +518,11 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
       RUAI_TRY(ruai_gemv_launch(c, Ly.o.w, att, RUAI_F32, nql, rows, m->tp.local_partial(), eo));
       RUAI_TRY(ruai_tp_allreduce_add(c, &m->tp, x, rows, d, m->d_err.as<int>(), ss));
     }
-    ss_tiles = d_tiles;
+    if (!tp) ss_tiles = ruai_gemv_tiles(c, Ly.o.w, rows);  // sharded: the exchange writes one tile
     GemvEpilogue eu;
     eu.bias = Ly.up.bias.as<float>();
     eu.act = m->llama ? ACT_SWIGLU : ACT_GELU;
-    if (fold) {
+    if (fold && !dot(Ly.up)) {
       GemvPrologue pr;
       pr.norm_w = Ly.n2w.as<float>(); pr.sumsq = ss; pr.tiles = ss_tiles; pr.eps = m->eps;
       RUAI_TRY(ruai_gemv_launch(c, Ly.up.w, x, RUAI_F32, d, rows, hb, eu, pr));
@@ -533,6 +536,7 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
       ed.sumsq = ss;
       GemvPrologue pd;
       RUAI_TRY(ruai_gemv_launch(c, Ly.down.w, hb, RUAI_F32, m->fl, rows, x, ed, pd));
+      ss_tiles = ruai_gemv_tiles(c, Ly.down.w, rows);
     } else {
       RUAI_TRY(ruai_gemv_launch(c, Ly.down.w, hb, RUAI_F32, m->fl, rows, m->tp.local_partial(), ed));
       RUAI_TRY(ruai_tp_allreduce_add(c, &m->tp, x, rows, d, m->d_err.as<int>(), ss));
@@ -551,12 +555,12 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
   GemvEpilogue eh;
   // the pick rides in the head GEMV's epilogue where that runs as one row tile on a tensor-core kernel (up to 4 rows, or
   // 5..16 on the 16-row tile); otherwise the separate argmax kernel beats the CUDA-core kernel that could fuse it
-  const bool fused_pick = want_argmax && !tp && (out_rows <= 8 || (c->use_bulk && c->use_tc && ruai_gemv_wide_eligible(c, m->head.w, out_rows)));
+  const bool fused_pick = want_argmax && !tp && (out_rows <= kGemvDotPickRows || (c->use_bulk && c->use_tc && ruai_gemv_wide_eligible(c, m->head.w, out_rows)));
   if (fused_pick) {
     eh.argmax_out = m->d_ids.as<int32_t>(); eh.argmax_slots = m->arg_slots.as<int2>(); eh.argmax_counter = m->arg_counter.as<unsigned>();
     eh.len_ptr = len; eh.len_add = (int32_t)T;
   }
-  if (fold && !some) {
+  if (fold && !some && !dot(m->head)) {
     GemvPrologue pr;
     pr.norm_w = m->final_w.as<float>(); pr.sumsq = ss; pr.tiles = ss_tiles; pr.eps = m->eps;
     RUAI_TRY(ruai_gemv_launch(c, m->head.w, hx, RUAI_F32, d, out_rows, m->logits.as<float>(), eh, pr));

@@ -1,12 +1,13 @@
 """Compares the split-k cost model of the tensor-core GEMVs with every fixed split, and the many-row GEMM's choice of tile and split with
 every fixed one, shape by shape.
 
-    python -m ruai_b200.sweep_splits [rows ...]          (default rows: 1 4; needs a B200)
+    python -m ruai_b200.sweep_splits [rows ...]          (default rows: 2 4; needs a B200)
 
 Per shape and row count: `ruai_matmul_q` timed with CUDA events over copies of the weight that together exceed the L2
 (so every launch streams from HBM), six rounds, once with the library's choice and once each with 1, 2, 4 and 8 splits
 fixed through `ruai_ctx_force_splits`.  Prints microseconds per launch and the ratio choice / best.  The int8 kernel
-only lets the count be raised above its own choice, so its fixed columns mostly repeat the choice.
+only lets the count be raised above its own choice, so its fixed columns mostly repeat the choice; one row, and few rows of
+small weights, run on the dot-product kernel, which has no split.
 
 From 17 rows on: the choice, each tile with its best split of 1, 2, 3, 4, 6 and 8 (`ruai_ctx_force_tile`), the best of them, choice / best.
 """
@@ -69,4 +70,4 @@ def main(rows):
 
 
 if __name__ == "__main__":
-    main([int(a) for a in sys.argv[1:]] or [1, 4])
+    main([int(a) for a in sys.argv[1:]] or [2, 4])

@@ -388,6 +388,33 @@ def test_lora_forward_matches_checker(dev, m, k, n, rank, bits):
     assert np.array_equal(got, nn._matmul_q(T(x), qw).numpy())
 
 
+# ---- few rows on the dot-product units: edges of the tiles of columns, of the warps' ranges of k, of the blocks of one exponent ----
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("k,n,rows", [(32, 4, (1, 2, 8)), (64, 8, (1, 3, 16)), (96, 36, (1, 4, 9)), (544, 132, (1, 2, 3, 4, 8, 13, 16)), (1056, 1300, (1, 2, 5, 16)),
+                                      (1536, 1664, (2, 4, 8, 16)), (2080, 2500, (1,)), (4128, 4900, (1,)), (4096, 4736, (1,)), (14336, 96, (1,))])
+def test_few_rows_against_float64(dev, k, n, rows, bits, dtype):
+    """x is rounded to half of 2^-22 (int8: 2^-27) of the largest magnitude of its block of 32 (128) at the most, the sums are f32: errors
+    below that, summed over the block's weights, and 2^-20 of the sum of the products' magnitudes."""
+    if bits == 8:  # a ragged last chunk, rows of x that are not aligned, an odd number of columns
+        k -= 5
+        n -= 1
+    q, s, qw = _qw(dev, bits, k, n, 51)
+    wd = q.astype(np.float64) * s if bits == 8 else qw.dequant().astype(np.float64)
+    bias = oracle.synth_normal(51, 1, (n,))
+    for m in rows:
+        x = oracle.synth_normal(51, m, (m, k), 1.0) * np.exp2(np.arange(k) // 32 % 23 - 11).astype(np.float32)  # blocks of very different size
+        xf, got = run_matmul(dev, x, qw, dtype, bias)
+        want, mag = xf.astype(np.float64) @ wd + bias, np.abs(xf).astype(np.float64) @ np.abs(wd) + np.abs(bias)
+        # int8: a block of one exponent is 128 consecutive k of a warp's range: no larger than twice 128 neighbours
+        lo, hi = (0, 32) if bits == 4 else (224, 256)
+        top = np.stack([np.abs(xf[:, max(0, i - lo):i + hi]).max(1) for i in range(0, k, 32)], 1)
+        rounding = np.repeat(top, 32, 1)[:, :k].astype(np.float64) @ np.abs(wd) * 2.0 ** (-22 if bits == 4 else -27)
+        bound = rounding + 2.0 ** -20 * mag + (2.0 ** -8 * np.abs(want) if dtype == "bf16" else 0.0) + 1e-30
+        assert (np.abs(got - want) <= bound).all(), (m, (np.abs(got - want) / bound).max())
+
+
 # ---- the GEMM's tiles: edges of rows, columns and k, every split of k ----
 
 @pytest.mark.parametrize("bits", [8, 4])
