@@ -21,6 +21,9 @@
 // The same kernel serves windows with kept first positions (chunks nothing of which a tile sees are not read), values of
 // another width than the keys, and two score maps per head over the same values (MAPS = 2: half of the warps own the
 // rows of each map; the maps meet in shared memory at the end).
+//
+// Prompts of 96 tokens and more go to attn_prefill_tc.cu (the line is explained there); this one keeps shorter ones, keys that lie
+// apart, sinks and gates.
 #include "common.cuh"
 #include "decode_ops.cuh"
 #include "pipeline.cuh"
@@ -296,6 +299,7 @@ int ruai_attention_prefill(ruai_ctx* c, const AttnParams& p_in, uint32_t B, uint
   if (p.vd == 0) p.vd = p.hd;
   if (p.vd_out == 0) p.vd_out = p.vd;
   if (p.fuse || p.T < 8 || !widths_fit(p.hd, p.vd) || p.maps > 2 || (p.k_pos && p.maps != 1)) return 0;
+  if (const int took = ruai_attention_prefill_tc(c, p, B, rep_in)) return took;
   // query heads per CTA; other counts are shared out over several CTAs
   uint32_t rep = 1;
   for (uint32_t r : {8u, 4u, 3u, 2u})

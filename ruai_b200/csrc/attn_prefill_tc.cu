@@ -1,0 +1,638 @@
+// Causal attention over the KV cache for many query positions on the tensor cores (tcgen05): what attn_prefill.cu computes, with
+// both products as matrix instructions at f32's precision.
+//
+// Precision.  Every f32 operand is scaled by a power of two (a query row's own; one per tile of 64 keys for the keys and one for the
+// values; 2^14 for the probabilities) so that its largest magnitude lies below 2^15, and split into two fp16 pieces,
+// x = hi + 2^-12 lo: 22 bits down to 2^-28 of the largest, then a quantum of 2^-50 of it.  A product takes three of the four products
+// of pieces; the lo ones go first and the first hi one scales them by 2^-12 (exact).  The tensor core adds a tile's 64 keys (a
+// score's head dimension) only: sums over tiles, the running softmax and its exponentials are f32 in registers.  Infinities and NaN
+// stay what they are in hi (lo is 0 there) and make the rows that see them non-finite.
+//
+// Keys that lie apart (latent attention spread out) stay on attn_prefill.cu: the decoder that has them may follow them with a choice of
+// experts, which the smallest change of rounding turns where two scores are close.
+//
+// attn_split_kernel writes the pieces of keys and values once, in the form the tensor core reads (K-major, 128-byte swizzle; values
+// transposed), so that a tile is one bulk copy for each of the query tiles that see it.
+//
+// attn_tc_kernel: a CTA owns 128 rows (queries x the query heads of a KV head, of one score map).  One thread copies tiles, one issues
+// the MMAs (scores of tile t + 1 ahead of the values of tile t), and 4 CS warps are the softmax: thread = row and a CS-th of the
+// tile's keys, and of the output's columns.  Scores lie in tensor memory twice, probabilities (the A operand of the second product)
+// and a tile's weighted values once; the latter are read out and added up in registers while the next tile's scores are made.
+// Two score maps per head: a CTA each, their rows through scratch to attn_maps_kernel, which combines and norms them.
+// Every mbarrier wait is bounded.
+//
+// What bounds it: the softmax warps' issue slots (scores read out, scaled, exponentials, split into pieces, and a tile's values read out
+// and added up), not the MMAs, of which three f16 products of 128 x 64 x 128 take some 600 clocks a tile.  2000 tokens of the 8B shape
+// (32 heads of 128, 8 of keys): 180 to 200 us a layer and 23 for the split, where the f32 units took 1541; two maps of 128 with values of
+// 256, 2048 tokens: 227 us, 69 for the maps and 23 for the split, before 1843.  Two warps per row and tile (CS = 2) where the values are at
+// most 64 wide, else four: the registers that hold the output then leave room for the products' read-out.
+#include <algorithm>
+
+#include "common.cuh"
+#include "decode_ops.cuh"
+#include "pipeline.cuh"
+
+namespace {
+
+using namespace pipe;
+
+constexpr int kKeys = 64;      // keys per tile
+constexpr int kRows = 128;     // rows per CTA: the MMA's M
+constexpr int kControl = 2;    // warps that do not own rows: copies, MMAs
+constexpr int kLoShift = 12;
+constexpr float kLoScale = 4096.0f;
+constexpr uint32_t kSmemMax = 227 * 1024 - 1024 - 5120;  // what a CTA can have, less the alignment of operands and the static part
+
+struct Pieces {
+  unsigned char* k;   // [B * KV][tiles][map][piece][block of 64 elements][64 keys][128 bytes]
+  unsigned char* v;   // [B * KV][tiles][piece][vdp][128 bytes: 64 keys]
+  float* factor;      // [B * KV][tiles][2]: what a tile's scores and weighted values are multiplied by
+  float* maps;        // [B * T][heads][2][vd]: two score maps per head
+  uint32_t tiles, blocks, vdp, kslots, vslots, tmem, rep, b0;
+};
+
+__device__ __forceinline__ uint32_t magnitude(float v) {  // of a finite number, as ordered bits; 0 for the others
+  const uint32_t a = __float_as_uint(v) & 0x7FFFFFFFu;
+  return a < 0x7F800000u ? a : 0u;
+}
+// The power of two that brings the largest magnitude (bits) into [2^14, 2^15), and its inverse.
+__device__ __forceinline__ void scale_of(uint32_t largest, float& f, float& back) {
+  const int ex = (int)(largest >> 23) - 127;
+  const int e = largest ? min(14 - ex, 126) : 0;
+  f = __uint_as_float((uint32_t)(e + 127) << 23);
+  back = __uint_as_float((uint32_t)(127 - e) << 23);
+}
+__device__ __forceinline__ uint32_t half2_bits(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+// Two numbers as packed hi and lo pieces.
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+  hi = half2_bits(a, b);
+  const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  lo = half2_bits((a - h.x) * kLoScale, (b - h.y) * kLoScale);
+}
+__device__ __forceinline__ void split2_any(float a, float b, uint32_t& hi, uint32_t& lo) {  // the same where infinities and NaN may come
+  hi = half2_bits(a, b);
+  const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  const float x = magnitude(a) || a == 0.0f ? (a - h.x) * kLoScale : 0.0f, y = magnitude(b) || b == 0.0f ? (b - h.y) * kLoScale : 0.0f;
+  lo = half2_bits(x, y);
+}
+
+__device__ __forceinline__ uint32_t block_max(uint32_t v, uint32_t* red) {
+  v = __reduce_max_sync(0xFFFFFFFFu, v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  for (uint32_t w = 0; w < blockDim.x / 32; ++w) v = max(v, red[w]);
+  return v;
+}
+
+constexpr int kSplitThreads = 256;
+
+// grid (tiles, sequences * KV): 64 keys and their values.
+__global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const AttnParams p, const Pieces s) {
+  extern __shared__ float vs[];  // [64][vd + 1]
+  __shared__ uint32_t red[kSplitThreads / 32];
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const uint32_t tile = blockIdx.x, k0 = tile * kKeys, tid = threadIdx.x, n = (uint32_t)*p.len + p.T;
+  if (k0 >= n || n > p.cap) return;  // beyond the cache: the attention kernel reports it
+  const uint32_t nk = min((uint32_t)kKeys, n - k0), hd = p.hd, vd = p.vd, krow = p.maps * hd;
+  const uint32_t b = s.b0 + blockIdx.y / p.KV, kvh = blockIdx.y % p.KV;
+  const size_t bk = (size_t)b * p.KV + kvh;
+  const float* kbase = p.kcache + bk * p.cap * krow;
+  const float* vbase = p.vcache + bk * p.cap * vd;
+  auto key4 = [&](uint32_t k, uint32_t e) { return *reinterpret_cast<const float4*>(kbase + (size_t)(k0 + k) * krow + e); };  // of key k0 + k
+  auto mag4 = [](const float4& v) { return max(max(magnitude(v.x), magnitude(v.y)), max(magnitude(v.z), magnitude(v.w))); };
+  uint32_t km = 0, vm = 0;
+  for (uint32_t i = tid; i < nk * (krow / 4); i += kSplitThreads) km = max(km, mag4(key4(i / (krow / 4), 4 * (i % (krow / 4)))));
+  for (uint32_t i = tid; i < kKeys * (vd / 4); i += kSplitThreads) {
+    const uint32_t k = i / (vd / 4), e = 4 * (i % (vd / 4));
+    const float4 v = k < nk ? *reinterpret_cast<const float4*>(vbase + (size_t)(k0 + k) * vd + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float* d = vs + k * (vd + 1) + e;
+    d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+    vm = max(vm, mag4(v));
+  }
+  km = block_max(km, red);
+  vm = block_max(vm, red);
+  float kf, kback, vf, vback;
+  scale_of(km, kf, kback);
+  scale_of(vm, vf, vback);
+  const size_t at = (size_t)blockIdx.y * s.tiles + tile;
+  if (tid == 0) {
+    s.factor[2 * at] = kback * (p.scale * 1.44269504088896341f);  // scores in powers of two
+    s.factor[2 * at + 1] = vback * (1.0f / 16384.0f);
+  }
+  const uint32_t piece = s.blocks * (kKeys * 128);
+  unsigned char* kd = s.k + at * p.maps * 2 * piece;
+  for (uint32_t i = tid; i < p.maps * kKeys * s.blocks * 8; i += kSplitThreads) {  // (map, key, chunk of eight elements)
+    const uint32_t c = i % (s.blocks * 8), k = i / (s.blocks * 8) % kKeys, map = i / (kKeys * s.blocks * 8);
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t e = 8 * c + 4 * h;
+      const float4 v = k < nk && e < hd ? key4(k, map * hd + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+      split2_any(v.x * kf, v.y * kf, hi[2 * h], lo[2 * h]);
+      split2_any(v.z * kf, v.w * kf, hi[2 * h + 1], lo[2 * h + 1]);
+    }
+    unsigned char* dst = kd + map * 2 * piece + (c >> 3) * (kKeys * 128) + k * 128 + (((c ^ k) & 7u) << 4);
+    *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(dst + piece) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+  unsigned char* vdst = s.v + at * 2 * s.vdp * 128;
+  for (uint32_t i = tid; i < s.vdp * 8; i += kSplitThreads) {  // (column of the values, chunk of eight keys)
+    const uint32_t c = i & 7u, r = i >> 3;
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const float a = r < vd ? vs[(8 * c + 2 * h) * (vd + 1) + r] : 0.0f, d = r < vd ? vs[(8 * c + 2 * h + 1) * (vd + 1) + r] : 0.0f;
+      split2_any(a * vf, d * vf, hi[h], lo[h]);
+    }
+    unsigned char* dst = vdst + r * 128 + (((c ^ r) & 7u) << 4);
+    *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(dst + s.vdp * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+
+__device__ __forceinline__ bool elect_one() {  // (a lane that the compiler knows to be one issues an MMA in 10 clocks, `lane == 0` in 45)
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {  // K-major, 128-byte swizzle, 1024 bytes between 8-row blocks
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+// D (+)= A B, fp16 x fp16 -> f32; A in shared memory (SS) or in tensor memory (TS).  after_lo: the sums so far are of lo pieces.
+__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
+               "r"(accumulate)
+               : "memory");
+}
+__device__ __forceinline__ void mma_ss_after_lo(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
+               "n"(kLoShift)
+               : "memory");
+}
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc),
+               "r"(accumulate)
+               : "memory");
+}
+__device__ __forceinline__ void mma_ts_after_lo(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc),
+               "n"(kLoShift)
+               : "memory");
+}
+// 16 consecutive 32-bit columns of this thread's lane of tensor memory.  The load writes its registers until the wait has returned, so
+// the wait takes them as operands.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]),
+                 "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+               "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
+__device__ __forceinline__ float exp2_of(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// Two f32 operations in one instruction, each rounded like fmaf and a product.
+__device__ __forceinline__ unsigned long long pair_of(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(__float_as_uint(a)), "r"(__float_as_uint(b)));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// Tensor memory: scores [2][64 columns], probabilities (hi 32 columns, lo 32), weighted values.
+constexpr uint32_t kProbCol = 2 * kKeys, kValueCol = kProbCol + kKeys;
+
+// CS: warps that share a row (keys of a tile, columns of the output).  OC: columns of the output per thread.
+template <int CS, int OC>
+__global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 ? 2 : 1) attn_tc_kernel(const AttnParams p, const Pieces s) {
+  constexpr int kSoftWarps = 4 * CS, SC = kKeys / CS;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t q_ready, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_free[2], p_ready, o_full, fin;
+  __shared__ uint32_t s_tmem;
+  __shared__ volatile int s_abort;
+  __shared__ float s_max[2][CS][kRows];  // a tile's row maxima by part; at the end the row sums
+  __shared__ float s_qback[kRows];
+  unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // swizzled operands start on 1024-byte boundaries
+  const uint32_t q_piece = s.blocks * (kRows * 128), k_piece = s.blocks * (kKeys * 128), k_slot = 2 * k_piece, v_piece = s.vdp * 128, v_slot = 2 * v_piece;
+  const uint32_t off_k = 2 * q_piece, off_v = off_k + s.kslots * k_slot;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t hd = p.hd, vd = p.vd, rep = s.rep, qt = kRows / rep;  // queries per CTA
+  const uint32_t bk = blockIdx.y, b = s.b0 + bk / p.KV, kvh = bk % p.KV, map = blockIdx.z;
+  const uint32_t q0 = (gridDim.x - 1u - blockIdx.x) * qt;  // the tiles with the most keys first: they are the long ones
+  const uint32_t head0 = kvh * rep;
+
+  if (tid == 0) {
+    mbar_init(&q_ready, kSoftWarps); mbar_init(&p_ready, kSoftWarps); mbar_init(&o_full, 1); mbar_init(&fin, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&s_free[i], kSoftWarps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    s_abort = 0;
+  }
+  __syncwarp();
+  if (warp == 1) tmem_alloc(&s_tmem, s.tmem);
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = s_tmem;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const uint32_t past = (uint32_t)*p.len, nq = min(qt, p.T - q0);
+  uint32_t kmax = past + q0 + nq;  // keys 0 .. kmax - 1 are seen by the tile's last query
+  const bool over = past + p.T > p.cap;  // the device's position is not the host's: touch nothing beyond the cache, tell the host
+  if (over) {
+    kmax = 0;
+    if (tid == 0 && p.status) atomicCAS(p.status, 0, 5);
+  }
+  // tiles that hold a kept first position, then those from the first query's window on
+  const uint32_t all_tiles = (kmax + kKeys - 1) / kKeys, first = past + q0;
+  const uint32_t lo = p.window && first + 1u > p.window ? first + 1u - p.window : 0u;
+  const uint32_t kept_tiles = (min(p.keep, kmax) + kKeys - 1) / kKeys, lo_tile = min(max(lo / kKeys, kept_tiles), all_tiles);
+  const uint32_t ntiles = kept_tiles + all_tiles - lo_tile;
+  auto tile_at = [&](uint32_t i) { return i < kept_tiles ? i : lo_tile + (i - kept_tiles); };
+
+  if (warp < kControl) {
+    if (warp == 0 && elect_one()) {
+      // ===== copies =====
+      const unsigned char* kbase = s.k + (size_t)bk * s.tiles * p.maps * k_slot + map * k_slot;
+      const unsigned char* vbase = s.v + (size_t)bk * s.tiles * v_slot;
+      // the keys of tile i, then the values of tile i - 1: keys are needed sooner and freed sooner
+      uint32_t k = 0, v = 0;  // requested
+      for (uint32_t i = 0; i <= ntiles && !s_abort && ntiles; ++i) {
+        if (i < ntiles) {
+          const uint32_t slot = i % s.kslots;
+          if (i >= s.kslots && !mbar_wait(&k_empty[slot], (i / s.kslots - 1u) & 1u)) { s_abort = 1; break; }
+          mbar_expect_tx(&k_full[slot], k_slot);
+          bulk_load(smem + off_k + slot * k_slot, kbase + (size_t)tile_at(i) * p.maps * k_slot, k_slot, &k_full[slot]);
+          ++k;
+        }
+        if (i > 0) {
+          const uint32_t slot = v % s.vslots;
+          if (v >= s.vslots && !mbar_wait(&v_empty[slot], (v / s.vslots - 1u) & 1u)) { s_abort = 1; break; }
+          mbar_expect_tx(&v_full[slot], v_slot);
+          bulk_load(smem + off_v + slot * v_slot, vbase + (size_t)tile_at(v) * v_slot, v_slot, &v_full[slot]);
+          ++v;
+        }
+      }
+      // leave no copy in flight into shared memory that another CTA may get, whoever gives up
+      for (uint32_t u = k > s.kslots ? k - s.kslots : 0; u < k; ++u) (void)mbar_wait(&k_full[u % s.kslots], (u / s.kslots) & 1u);
+      for (uint32_t u = v > s.vslots ? v - s.vslots : 0; u < v; ++u) (void)mbar_wait(&v_full[u % s.vslots], (u / s.vslots) & 1u);
+    } else if (warp == 1 && elect_one()) {
+      // ===== MMAs: the scores of tile i, then the weighted values of tile i - 1 =====
+      const uint32_t idesc_s = (1u << 4) | ((uint32_t)(kKeys >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+      const uint32_t idesc_v = (1u << 4) | ((s.vdp >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+      const uint64_t qd = desc_sw128(smem_u32(smem)), kd = desc_sw128(smem_u32(smem + off_k)), vd0 = desc_sw128(smem_u32(smem + off_v));
+      const uint32_t steps = (hd + 15) / 16;
+      bool ok = ntiles == 0 || mbar_wait(&q_ready, 0);
+      for (uint32_t i = 0; i <= ntiles && ok && ntiles; ++i) {
+        if (i < ntiles) {
+          const uint32_t ks = i % s.kslots, sb = i & 1u, d = tmem + sb * kKeys;
+          if (s_abort || !mbar_wait(&k_full[ks], (i / s.kslots) & 1u) || (i >= 2 && !mbar_wait(&s_free[sb], (i / 2 - 1u) & 1u))) { ok = false; break; }
+          tc_fence_after_sync();
+          const uint64_t kt = umma_desc_advance(kd, ks * k_slot);
+          auto at_q = [&](uint32_t e) { return umma_desc_advance(qd, (e >> 2) * (kRows * 128) + (e & 3u) * 32u); };
+          auto at_k = [&](uint32_t e) { return umma_desc_advance(kt, (e >> 2) * (kKeys * 128) + (e & 3u) * 32u); };
+          for (uint32_t e = 0; e < steps; ++e) {
+            mma_ss(d, at_q(e), umma_desc_advance(at_k(e), k_piece), idesc_s, e != 0 ? 1u : 0u);
+            mma_ss(d, umma_desc_advance(at_q(e), q_piece), at_k(e), idesc_s, 1u);
+          }
+          mma_ss_after_lo(d, at_q(0), at_k(0), idesc_s);
+          for (uint32_t e = 1; e < steps; ++e) mma_ss(d, at_q(e), at_k(e), idesc_s, 1u);
+          umma_commit(&k_empty[ks]);
+          umma_commit(&s_full[sb]);
+        }
+        if (i > 0) {
+          const uint32_t t = i - 1, vs = t % s.vslots, d = tmem + kValueCol, ph = tmem + kProbCol, pl = ph + kKeys / 2;
+          if (s_abort || !mbar_wait(&v_full[vs], (t / s.vslots) & 1u) || !mbar_wait(&p_ready, t & 1u)) { ok = false; break; }
+          tc_fence_after_sync();
+          const uint64_t vt = umma_desc_advance(vd0, vs * v_slot);
+#pragma unroll
+          for (uint32_t e = 0; e < kKeys / 16; ++e) {
+            mma_ts(d, ph + e * 8, umma_desc_advance(vt, v_piece + e * 32u), idesc_v, e != 0 ? 1u : 0u);
+            mma_ts(d, pl + e * 8, umma_desc_advance(vt, e * 32u), idesc_v, 1u);
+          }
+          mma_ts_after_lo(d, ph, vt, idesc_v);
+#pragma unroll
+          for (uint32_t e = 1; e < kKeys / 16; ++e) mma_ts(d, ph + e * 8, umma_desc_advance(vt, e * 32u), idesc_v, 1u);
+          umma_commit(&v_empty[vs]);
+          umma_commit(&o_full);
+        }
+      }
+      if (!ok) s_abort = 1;
+      umma_commit(&fin);  // nothing is left running when tensor memory is freed
+      if (!mbar_wait(&fin, 0)) s_abort = 1;
+    }
+    __syncwarp();
+  } else {
+    // ===== softmax: thread = row, part `cp` of a tile's keys and of the output's columns =====
+    const uint32_t quarter = (uint32_t)warp & 3u, cp = (uint32_t)(warp - kControl) >> 2, row = quarter * 32u + lane;
+    // queries as pieces: a warp's rows of shared memory, one row at a time, a lane per four elements
+    for (uint32_t r = warp - kControl; r < (uint32_t)kRows; r += kSoftWarps) {
+      const uint32_t qi = r / rep, h = r % rep;
+      const bool in = r < qt * rep && qi < nq;
+      const float* src = p.q + (size_t)(b * p.T + q0 + qi) * p.q_ld + (size_t)((head0 + h) * p.maps + map) * hd;
+      float4 v[2];
+      uint32_t mx = 0;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const uint32_t e = 4 * (lane + 32 * j);
+        v[j] = in && e < hd ? *reinterpret_cast<const float4*>(src + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+        mx = max(mx, max(max(magnitude(v[j].x), magnitude(v[j].y)), max(magnitude(v[j].z), magnitude(v[j].w))));
+      }
+      mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+      float f, back;
+      scale_of(mx, f, back);
+      if (lane == 0) s_qback[r] = back;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const uint32_t e = 4 * (lane + 32 * j);
+        if (e < s.blocks * 64) {
+          uint2 hi, lo2;
+          split2_any(v[j].x * f, v[j].y * f, hi.x, lo2.x);
+          split2_any(v[j].z * f, v[j].w * f, hi.y, lo2.y);
+          unsigned char* dst = smem + (e >> 6) * (kRows * 128) + r * 128 + ((((e & 63u) >> 3) ^ (r & 7u)) << 4) + (e & 4u) * 2u;
+          *reinterpret_cast<uint2*>(dst) = hi;
+          *reinterpret_cast<uint2*>(dst + q_piece) = lo2;
+        }
+      }
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&q_ready);
+    asm volatile("bar.sync 8, %0;" ::"n"(kSoftWarps * 32) : "memory");  // the rows' factors
+
+    const float qback = s_qback[row];
+    const uint32_t qi = row / rep, h = row % rep;
+    const uint32_t qpos = past + q0 + min(qi, nq - 1u);  // the last key this row's query sees (rows without a query: any)
+    const uint32_t qlo = p.window && qpos + 1u > p.window ? qpos + 1u - p.window : 0u;  // the first but for the kept ones
+    const uint32_t lanes = (quarter * 32u) << 16;
+    float m_run = -INFINITY, l_run = 0.0f, corr_prev = 0.0f, vf_prev = 0.0f;
+    unsigned long long sums[OC / 2];  // pairs of columns
+#pragma unroll
+    for (int j = 0; j < OC / 2; ++j) sums[j] = 0ull;
+    // A warp whose wait ran out walks on without waiting, so that a quarter's warps meet at every barrier below.
+    bool ok = true;
+    auto wait = [&](uint64_t* bar, uint32_t parity) {  // the same answer for the whole warp
+      if (ok) ok = __all_sync(0xFFFFFFFFu, !s_abort && mbar_wait(bar, parity));
+      if (!ok) s_abort = 1;
+      tc_fence_after_sync();
+    };
+    // the weighted values of tile t: out of tensor memory, onto the sums
+    auto drain = [&](uint32_t t) {
+      wait(&o_full, t & 1u);
+      const bool same = __all_sync(0xFFFFFFFFu, corr_prev == 1.0f);  // no row's maximum has grown
+      const unsigned long long v2 = pair_of(vf_prev, vf_prev), c2 = pair_of(corr_prev, corr_prev);
+#pragma unroll
+      for (int c = 0; c < OC; c += 16) {
+        uint32_t d[16];
+        tmem_ld16(tmem + lanes + kValueCol + cp * OC + c, d);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const unsigned long long add = pair_of(__uint_as_float(d[2 * j]), __uint_as_float(d[2 * j + 1]));
+          sums[c / 2 + j] = fma2(add, v2, same ? sums[c / 2 + j] : mul2(sums[c / 2 + j], c2));
+        }
+      }
+    };
+    const float* factor = s.factor + (size_t)bk * s.tiles * 2;
+    float2 fac = ntiles ? *reinterpret_cast<const float2*>(factor + 2 * tile_at(0)) : make_float2(0.f, 0.f);
+    for (uint32_t i = 0; i < ntiles; ++i) {
+      const uint32_t sb = i & 1u, key0 = tile_at(i) * kKeys + cp * SC;  // this thread's first key
+      const float2 cur = fac;
+      if (i + 1 < ntiles) fac = *reinterpret_cast<const float2*>(factor + 2 * tile_at(i + 1));
+      wait(&s_full[sb], (i >> 1) & 1u);
+      float sc[SC];
+#pragma unroll
+      for (int c = 0; c < SC; c += 16) {
+        uint32_t d[16];
+        tmem_ld16(tmem + lanes + sb * kKeys + cp * SC + c, d);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) sc[c + j] = __uint_as_float(d[j]);
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_free[sb]);
+      // which of the keys the row sees: bit j = key0 + j in [qlo, qpos], or below keep
+      auto below = [&](uint32_t n) { return n <= key0 ? 0u : n - key0 >= 32u ? 0xFFFFFFFFu : (1u << (n - key0)) - 1u; };
+      const uint32_t all = SC == 32 ? 0xFFFFFFFFu : (1u << (SC & 31)) - 1u;
+      const uint32_t seen = below(qpos + 1u) & (~below(qlo) | below(p.keep)) & all;
+      const bool whole = __all_sync(0xFFFFFFFFu, seen == all);
+      if (!whole) {
+#pragma unroll
+        for (int j = 0; j < SC; ++j) sc[j] = (seen >> j) & 1u ? sc[j] : -INFINITY;
+      }
+      const float f = qback * cur.x;
+      float mx = sc[0];
+#pragma unroll
+      for (int j = 1; j < SC; ++j) mx = fmaxf(mx, sc[j]);
+      mx = mx == -INFINITY ? mx : mx * f;  // (f may be 0)
+      s_max[sb][cp][row] = mx;
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + quarter), "n"(CS * 32) : "memory");
+#pragma unroll
+      for (int c = 0; c < CS; ++c) mx = fmaxf(mx, s_max[sb][c][row]);
+      const float m_new = fmaxf(m_run, mx), m_use = m_new == -INFINITY ? 0.0f : m_new;
+      const float corr = m_run == -INFINITY ? 0.0f : exp2_of(m_run - m_new);
+      float sum = 0.0f;
+#pragma unroll
+      for (int j = 0; j < SC; ++j) {
+        const float e = exp2_of(fmaf(sc[j], f, -m_use));
+        sc[j] = whole || ((seen >> j) & 1u) ? e : 0.0f;
+        sum += sc[j];
+      }
+      l_run = fmaf(l_run, corr, sum);
+      m_run = m_new;
+      if (i > 0) drain(i - 1);  // also: the probabilities of tile i - 1 have been read
+      corr_prev = corr;
+      vf_prev = cur.y;
+#pragma unroll
+      for (int c = 0; c < SC; c += 16) {
+        uint32_t hi[8], lo2[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) split2(sc[c + 2 * j] * 16384.0f, sc[c + 2 * j + 1] * 16384.0f, hi[j], lo2[j]);
+        tmem_st8(tmem + lanes + kProbCol + (cp * SC + c) / 2, hi);
+        tmem_st8(tmem + lanes + kProbCol + kKeys / 2 + (cp * SC + c) / 2, lo2);
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_ready);
+    }
+    if (ntiles) drain(ntiles - 1);
+    // the parts' row sums
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + quarter), "n"(CS * 32) : "memory");
+    s_max[0][cp][row] = l_run;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + quarter), "n"(CS * 32) : "memory");
+    float l = 0.0f, o[OC];
+#pragma unroll
+    for (int c = 0; c < CS; ++c) l += s_max[0][c][row];
+#pragma unroll
+    for (int j = 0; j < OC; ++j) o[j] = __uint_as_float((uint32_t)(sums[j / 2] >> (32 * (j & 1))));
+    if (!over && !s_abort && row < qt * rep && qi < nq) {
+      const size_t token = (size_t)b * p.T + q0 + qi;
+      const uint32_t c0 = cp * OC;
+      const float inv = 1.0f / l;
+      if (p.maps == 2) {
+        float* dst = s.maps + (((token - (size_t)s.b0 * p.T) * (p.KV * rep) + head0 + h) * 2 + map) * vd;
+#pragma unroll
+        for (int j = 0; j < OC; j += 4)
+          if (c0 + j < vd) *reinterpret_cast<float4*>(dst + c0 + j) = make_float4(o[j] * inv, o[j + 1] * inv, o[j + 2] * inv, o[j + 3] * inv);
+      } else {
+        const size_t at = token * p.out_ld + (size_t)(head0 + h) * p.vd_out;
+        const bool wide = p.out_dtype == RUAI_F32 && p.vd_out % 4 == 0 && p.out_ld % 4 == 0;
+#pragma unroll
+        for (int j = 0; j < OC; j += 4) {
+          if (wide) {
+            if (c0 + j < p.vd_out) *reinterpret_cast<float4*>(p.out + at + c0 + j) = make_float4(o[j] * inv, o[j + 1] * inv, o[j + 2] * inv, o[j + 3] * inv);
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (c0 + j + u < p.vd_out) store_from_f32(p.out, p.out_dtype, at + c0 + j + u, o[j + u] * inv);
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (s_abort && tid == 0 && p.status) atomicCAS(p.status, 0, 3);
+  if (warp == 1) tmem_dealloc(tmem, s.tmem);
+}
+
+// Two score maps per head: out_scale * rms_norm(map 1 - lambda map 2), a warp per (token, head).
+__global__ void __launch_bounds__(256) attn_maps_kernel(const AttnParams p, const Pieces s, uint32_t tokens, uint32_t heads) {
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const uint32_t lane = threadIdx.x & 31u, item = blockIdx.x * 8u + (threadIdx.x >> 5);
+  if (item >= tokens * heads || (uint32_t)*p.len + p.T > p.cap) return;
+  const size_t token = (size_t)s.b0 * p.T + item / heads;
+  const uint32_t head = item % heads;
+  const float lam = *p.lambda;
+  const float4* a = reinterpret_cast<const float4*>(s.maps + (size_t)item * 2 * p.vd);
+  float4 y[2];
+  float ss = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const uint32_t e = lane + 32u * j;
+    y[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (e < p.vd / 4) {
+      const float4 u = a[e], z = a[p.vd / 4 + e];
+      y[j] = make_float4(u.x - lam * z.x, u.y - lam * z.y, u.z - lam * z.z, u.w - lam * z.w);  // columns past vd_out are zero in both maps
+      ss = fmaf(y[j].x, y[j].x, ss); ss = fmaf(y[j].y, y[j].y, ss); ss = fmaf(y[j].z, y[j].z, ss); ss = fmaf(y[j].w, y[j].w, ss);
+    }
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
+  const float f = p.out_scale / sqrtf(ss / (float)p.vd_out + p.eps);
+  const size_t at = token * p.out_ld + (size_t)head * p.vd_out;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const uint32_t e = 4 * (lane + 32u * j);
+    const float v[4] = {y[j].x * f, y[j].y * f, y[j].z * f, y[j].w * f};
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i)
+      if (e + i < p.vd_out) store_from_f32(p.out, p.out_dtype, at + e + i, v[i]);
+  }
+}
+
+template <int CS, int OC>
+cudaError_t launch_tc(ruai_ctx* c, const AttnParams& p, const Pieces& s, dim3 grid, uint32_t smem) {
+  static bool done[64] = {};
+  if (!done[c->ordinal & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(attn_tc_kernel<CS, OC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemMax + 1024));
+    if (e != cudaSuccess) return e;
+    done[c->ordinal & 63] = true;
+  }
+  return ruai_launch(c, attn_tc_kernel<CS, OC>, grid, dim3((kControl + 4 * CS) * 32), smem, true, p, s);
+}
+
+constexpr size_t kScratchMost = 256u << 20;  // a step's pieces (and maps) at a time
+// Fewer tokens leave most of the 128 rows and of the tensor core's time to nothing while the splitting costs a launch.  Us of a whole prompt, here |
+// attn_prefill.cu: 64 tokens of the 8B shape's 2 layers 656 | 648, of the 135M shape's 10 718 | 687; 96 tokens 700 | 718, 768 | 796, of
+// the 1.1B shape's 6 803 | 836, of GPT-2 1056 | 1126; 160 tokens 1080 | 1123, 833 | 937, 1105 | 1197, 1226 | 1410.
+constexpr uint32_t kFromTokens = 96;
+
+}  // namespace
+
+// 1: launched; 0: this shape is not taken; < 0: error.  `p`: as ruai_attention_prefill has completed it.
+int ruai_attention_prefill_tc(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep) {
+  if (p.T < kFromTokens || rep > 64 || p.k_pos || p.sink || p.gate) return 0;
+  Pieces s = {};
+  s.rep = rep;
+  s.blocks = (p.hd + 63) / 64;
+  s.vdp = (p.vd + 15) / 16 * 16;
+  s.tiles = (p.cap + kKeys - 1) / kKeys;
+  s.tmem = s.vdp <= 64 ? 256 : 512;
+  const uint32_t q = 2 * s.blocks * kRows * 128, ks = 2 * s.blocks * kKeys * 128, vs = 2 * s.vdp * 128;
+  if (q + ks + vs > kSmemMax) return 0;
+  s.kslots = q + 2 * ks + vs <= kSmemMax ? 2 : 1;
+  s.vslots = q + s.kslots * ks + 2 * vs <= kSmemMax ? 2 : 1;
+  const uint32_t smem = q + s.kslots * ks + s.vslots * vs + 1024;
+  // sequences at a time: what their pieces take of the scratch
+  auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t k1 = (size_t)p.KV * s.tiles * p.maps * ks, v1 = (size_t)p.KV * s.tiles * vs, f1 = (size_t)p.KV * s.tiles * 2 * sizeof(float);
+  const size_t m1 = p.maps == 2 ? (size_t)p.T * p.KV * rep * 2 * p.vd * sizeof(float) : 0, one = k1 + v1 + f1 + m1 + 1024;
+  if (one > kScratchMost) return 0;
+  const uint32_t per = (uint32_t)std::min<size_t>(B, std::min<size_t>(kScratchMost / one, 65535u / p.KV));
+  if (!per) return 0;
+  const size_t held = c->partial_bytes;
+  if ((size_t)per * one > held) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return 0;  // nothing may be allocated
+    if (ruai_ctx_reserve(c, (size_t)per * one, 0) != RUAI_OK) {  // no memory for the pieces: the kernel without them, the scratch as it was
+      (void)cudaGetLastError();
+      return ruai_ctx_reserve(c, held, 0) == RUAI_OK ? 0 : -1;
+    }
+  }
+  unsigned char* at = reinterpret_cast<unsigned char*>(c->partial);
+  s.k = at; at += up(per * k1);
+  s.v = at; at += up(per * v1);
+  s.factor = reinterpret_cast<float*>(at); at += up(per * f1);
+  s.maps = reinterpret_cast<float*>(at);
+  static bool done[64] = {};
+  cudaError_t e = cudaSuccess;
+  if (!done[c->ordinal & 63]) {
+    e = cudaFuncSetAttribute(attn_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kKeys * 257 * 4);
+    done[c->ordinal & 63] = e == cudaSuccess;
+  }
+  const uint32_t qt = kRows / rep;
+  for (uint32_t b0 = 0; b0 < B && e == cudaSuccess; b0 += per) {
+    const uint32_t nb = std::min(per, B - b0);
+    s.b0 = b0;
+    e = ruai_launch(c, attn_split_kernel, dim3(s.tiles, nb * p.KV), dim3(kSplitThreads), (size_t)kKeys * (p.vd + 1) * 4, true, p, s);
+    const dim3 grid((p.T + qt - 1) / qt, nb * p.KV, p.maps);
+    if (e == cudaSuccess) e = p.vd <= 64 ? launch_tc<2, 32>(c, p, s, grid, smem) : p.vd <= 128 ? launch_tc<4, 32>(c, p, s, grid, smem) : launch_tc<4, 64>(c, p, s, grid, smem);
+    const uint32_t heads = p.KV * rep;
+    if (e == cudaSuccess && p.maps == 2)
+      e = ruai_launch(c, attn_maps_kernel, dim3((nb * p.T * heads + 7) / 8), dim3(256), 0, true, p, s, nb * p.T, heads);
+  }
+  if (e != cudaSuccess) { ruai_fail(c, RUAI_ERR_CUDA, "prefill attention launch: %s", cudaGetErrorString(e)); return -1; }
+  return 1;
+}

@@ -50,6 +50,8 @@ int ruai_rope_kv(ruai_ctx* c, float* qkv, uint32_t qkv_ld, uint32_t k_off, uint3
 int ruai_attention(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep);
 // Many query positions at once, queries in tiles (attn_prefill.cu).  1: launched; 0: not taken for this shape; < 0: error.
 int ruai_attention_prefill(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep);
+// The same on the tensor cores (attn_prefill_tc.cu), for what ruai_attention_prefill passes on to it.
+int ruai_attention_prefill_tc(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep);
 // Whether heads of these widths, each with keys of its own (rep 1, one map), fit it.
 bool ruai_attention_prefill_fits(uint32_t hd, uint32_t vd);
 int ruai_argmax(ruai_ctx* c, const float* logits, uint32_t ld, uint32_t rows, uint32_t n, int32_t* out, uint32_t out_offset);
