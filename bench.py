@@ -45,9 +45,9 @@ DEFAULT_CTX = {"llama3-8b": 1024, "tinyllama-1.1b": 512, "smollm2-135m": 64, "gp
 OTHER_WORKLOADS = ["llama3-8b-int8-b1", "llama3-8b-int4-b16", "llama3-8b-int8-b16", "llama3-8b-int4-b128", "llama3-8b-int4-prefill1024",
                    "tinyllama-1.1b-int4-b1", "tinyllama-1.1b-int4-b64", "tinyllama-1.1b-int4-prefill512",
                    "smollm2-135m-int8-b1", "smollm2-135m-int4-b16", "gpt2-small-int8-b1"]
-ARITHMETIC = ("f32 in and out; inside the GEMV the activations are block fixed point (int4 weights: 21 bits per group of 32; "
-              "int8 weights: 28 bits per row of a CTA's slice), products exact in tcgen05 kind::i8, one f32 scale multiply-add "
-              "per group, split-k sums met in 64-bit fixed point")
+ARITHMETIC = ("f32 in and out; inside the GEMV the activations are block fixed point (int4 weights: 23 bits per group of 32; "
+              "int8 weights: 28 bits per block of 128 k), products exact in dp4a, one f32 scale multiply-add per group or block (2 to 4 rows of "
+              "large weights: 21 bits, 28 per row of a CTA's slice, exact in tcgen05 kind::i8; the persistent step too, with split-k sums met in 64-bit fixed point)")
 # steps of 5..16 sequences and prefill-sized row counts: other arithmetics
 ARITHMETIC_WIDE = ("f32 in and out; inside the Linears the activations are two bf16 pieces x = hi + lo (16 significant bits; from 17 rows on "
                    "two fp16 pieces under a power of two per row, 22 bits), the int4 / int8 weights exact, products and sums in f32 in tcgen05 kind::f16, one f32 scale multiply-add per group "

@@ -553,8 +553,8 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
     hx = m->xl.as<float>();
   }
   GemvEpilogue eh;
-  // the pick rides in the head GEMV's epilogue where that runs as one row tile on a tensor-core kernel (up to 4 rows, or
-  // 5..16 on the 16-row tile); otherwise the separate argmax kernel beats the CUDA-core kernel that could fuse it
+  // the pick rides in the head GEMV's epilogue where that runs as one row tile (up to 8 rows on gemv_dot.cu and the tensor-core
+  // kernels, up to 16 on the 16-row tile); otherwise the separate argmax kernel beats the CUDA-core kernel that could fuse it
   const bool fused_pick = want_argmax && !tp && (out_rows <= kGemvDotPickRows || (c->use_bulk && c->use_tc && ruai_gemv_wide_eligible(c, m->head.w, out_rows)));
   if (fused_pick) {
     eh.argmax_out = m->d_ids.as<int32_t>(); eh.argmax_slots = m->arg_slots.as<int2>(); eh.argmax_counter = m->arg_counter.as<unsigned>();
