@@ -22,8 +22,8 @@
 // another width than the keys, and two score maps per head over the same values (MAPS = 2: half of the warps own the
 // rows of each map; the maps meet in shared memory at the end).
 //
-// Prompts of 96 tokens and more go to attn_prefill_tc.cu (the line is explained there); this one keeps shorter ones, keys that lie
-// apart, sinks and gates.
+// Prompts of 96 tokens and more of the quantized decoders go to attn_prefill_tc.cu (the line is explained there); this one keeps shorter
+// ones and the decoders built from a list of layers.
 #include "common.cuh"
 #include "decode_ops.cuh"
 #include "pipeline.cuh"

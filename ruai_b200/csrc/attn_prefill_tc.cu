@@ -8,23 +8,22 @@
 // score's head dimension) only: sums over tiles, the running softmax and its exponentials are f32 in registers.  Infinities and NaN
 // stay what they are in hi (lo is 0 there) and make the rows that see them non-finite.
 //
-// Keys that lie apart (latent attention spread out) stay on attn_prefill.cu: the decoder that has them may follow them with a choice of
-// experts, which the smallest change of rounding turns where two scores are close.
+// The decoders built from a list of layers (p.pieces is 0) stay on attn_prefill.cu.  They round every layer's output to bf16, and
+// sums in another order turn some of those roundings: their outputs would be others (2.3e-3 of a norm) without being nearer to 64 bits, and
+// where a choice of experts follows, other experts.
 //
 // attn_split_kernel writes the pieces of keys and values once, in the form the tensor core reads (K-major, 128-byte swizzle; values
 // transposed), so that a tile is one bulk copy for each of the query tiles that see it.
 //
-// attn_tc_kernel: a CTA owns 128 rows (queries x the query heads of a KV head, of one score map).  One thread copies tiles, one issues
+// attn_tc_kernel: a CTA owns 128 rows (queries x the query heads of a KV head).  One thread copies tiles, one issues
 // the MMAs (scores of tile t + 1 ahead of the values of tile t), and 4 CS warps are the softmax: thread = row and a CS-th of the
 // tile's keys, and of the output's columns.  Scores lie in tensor memory twice, probabilities (the A operand of the second product)
 // and a tile's weighted values once; the latter are read out and added up in registers while the next tile's scores are made.
-// Two score maps per head: a CTA each, their rows through scratch to attn_maps_kernel, which combines and norms them.
 // Every mbarrier wait is bounded.
 //
 // What bounds it: the softmax warps' issue slots (scores read out, scaled, exponentials, split into pieces, and a tile's values read out
 // and added up), not the MMAs, of which three f16 products of 128 x 64 x 128 take some 600 clocks a tile.  2000 tokens of the 8B shape
-// (32 heads of 128, 8 of keys): 180 to 200 us a layer and 23 for the split, where the f32 units took 1541; two maps of 128 with values of
-// 256, 2048 tokens: 227 us, 69 for the maps and 23 for the split, before 1843.  Two warps per row and tile (CS = 2) where the values are at
+// (32 heads of 128, 8 of keys): 180 to 200 us a layer and 23 for the split, where the f32 units took 1541.  Two warps per row and tile (CS = 2) where the values are at
 // most 64 wide, else four: the registers that hold the output then leave room for the products' read-out.
 #include <algorithm>
 
@@ -44,10 +43,9 @@ constexpr float kLoScale = 4096.0f;
 constexpr uint32_t kSmemMax = 227 * 1024 - 1024 - 5120;  // what a CTA can have, less the alignment of operands and the static part
 
 struct Pieces {
-  unsigned char* k;   // [B * KV][tiles][map][piece][block of 64 elements][64 keys][128 bytes]
+  unsigned char* k;   // [B * KV][tiles][piece][block of 64 elements][64 keys][128 bytes]
   unsigned char* v;   // [B * KV][tiles][piece][vdp][128 bytes: 64 keys]
   float* factor;      // [B * KV][tiles][2]: what a tile's scores and weighted values are multiplied by
-  float* maps;        // [B * T][heads][2][vd]: two score maps per head
   uint32_t tiles, blocks, vdp, kslots, vslots, tmem, rep, b0;
 };
 
@@ -92,25 +90,25 @@ constexpr int kSplitThreads = 256;
 
 // grid (tiles, sequences * KV): 64 keys and their values.
 __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const AttnParams p, const Pieces s) {
-  extern __shared__ float vs[];  // [64][vd + 1]
+  extern __shared__ float vs[];  // [64][hd + 1]
   __shared__ uint32_t red[kSplitThreads / 32];
   grid_dependency_wait();
   grid_launch_dependents();
   const uint32_t tile = blockIdx.x, k0 = tile * kKeys, tid = threadIdx.x, n = (uint32_t)*p.len + p.T;
   if (k0 >= n || n > p.cap) return;  // beyond the cache: the attention kernel reports it
-  const uint32_t nk = min((uint32_t)kKeys, n - k0), hd = p.hd, vd = p.vd, krow = p.maps * hd;
+  const uint32_t nk = min((uint32_t)kKeys, n - k0), hd = p.hd;
   const uint32_t b = s.b0 + blockIdx.y / p.KV, kvh = blockIdx.y % p.KV;
   const size_t bk = (size_t)b * p.KV + kvh;
-  const float* kbase = p.kcache + bk * p.cap * krow;
-  const float* vbase = p.vcache + bk * p.cap * vd;
-  auto key4 = [&](uint32_t k, uint32_t e) { return *reinterpret_cast<const float4*>(kbase + (size_t)(k0 + k) * krow + e); };  // of key k0 + k
+  const float* kbase = p.kcache + bk * p.cap * hd;
+  const float* vbase = p.vcache + bk * p.cap * hd;
+  auto key4 = [&](uint32_t k, uint32_t e) { return *reinterpret_cast<const float4*>(kbase + (size_t)(k0 + k) * hd + e); };  // of key k0 + k
   auto mag4 = [](const float4& v) { return max(max(magnitude(v.x), magnitude(v.y)), max(magnitude(v.z), magnitude(v.w))); };
   uint32_t km = 0, vm = 0;
-  for (uint32_t i = tid; i < nk * (krow / 4); i += kSplitThreads) km = max(km, mag4(key4(i / (krow / 4), 4 * (i % (krow / 4)))));
-  for (uint32_t i = tid; i < kKeys * (vd / 4); i += kSplitThreads) {
-    const uint32_t k = i / (vd / 4), e = 4 * (i % (vd / 4));
-    const float4 v = k < nk ? *reinterpret_cast<const float4*>(vbase + (size_t)(k0 + k) * vd + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-    float* d = vs + k * (vd + 1) + e;
+  for (uint32_t i = tid; i < nk * (hd / 4); i += kSplitThreads) km = max(km, mag4(key4(i / (hd / 4), 4 * (i % (hd / 4)))));
+  for (uint32_t i = tid; i < kKeys * (hd / 4); i += kSplitThreads) {
+    const uint32_t k = i / (hd / 4), e = 4 * (i % (hd / 4));
+    const float4 v = k < nk ? *reinterpret_cast<const float4*>(vbase + (size_t)(k0 + k) * hd + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float* d = vs + k * (hd + 1) + e;
     d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     vm = max(vm, mag4(v));
   }
@@ -125,18 +123,18 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const AttnPar
     s.factor[2 * at + 1] = vback * (1.0f / 16384.0f);
   }
   const uint32_t piece = s.blocks * (kKeys * 128);
-  unsigned char* kd = s.k + at * p.maps * 2 * piece;
-  for (uint32_t i = tid; i < p.maps * kKeys * s.blocks * 8; i += kSplitThreads) {  // (map, key, chunk of eight elements)
-    const uint32_t c = i % (s.blocks * 8), k = i / (s.blocks * 8) % kKeys, map = i / (kKeys * s.blocks * 8);
+  unsigned char* kd = s.k + at * 2 * piece;
+  for (uint32_t i = tid; i < kKeys * s.blocks * 8; i += kSplitThreads) {  // (key, chunk of eight elements)
+    const uint32_t c = i % (s.blocks * 8), k = i / (s.blocks * 8);
     uint32_t hi[4], lo[4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const uint32_t e = 8 * c + 4 * h;
-      const float4 v = k < nk && e < hd ? key4(k, map * hd + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 v = k < nk && e < hd ? key4(k, e) : make_float4(0.f, 0.f, 0.f, 0.f);
       split2_any(v.x * kf, v.y * kf, hi[2 * h], lo[2 * h]);
       split2_any(v.z * kf, v.w * kf, hi[2 * h + 1], lo[2 * h + 1]);
     }
-    unsigned char* dst = kd + map * 2 * piece + (c >> 3) * (kKeys * 128) + k * 128 + (((c ^ k) & 7u) << 4);
+    unsigned char* dst = kd + (c >> 3) * (kKeys * 128) + k * 128 + (((c ^ k) & 7u) << 4);
     *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4*>(dst + piece) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
@@ -146,7 +144,7 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const AttnPar
     uint32_t hi[4], lo[4];
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
-      const float a = r < vd ? vs[(8 * c + 2 * h) * (vd + 1) + r] : 0.0f, d = r < vd ? vs[(8 * c + 2 * h + 1) * (vd + 1) + r] : 0.0f;
+      const float a = r < hd ? vs[(8 * c + 2 * h) * (hd + 1) + r] : 0.0f, d = r < hd ? vs[(8 * c + 2 * h + 1) * (hd + 1) + r] : 0.0f;
       split2_any(a * vf, d * vf, hi[h], lo[h]);
     }
     unsigned char* dst = vdst + r * 128 + (((c ^ r) & 7u) << 4);
@@ -244,8 +242,8 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
   const uint32_t q_piece = s.blocks * (kRows * 128), k_piece = s.blocks * (kKeys * 128), k_slot = 2 * k_piece, v_piece = s.vdp * 128, v_slot = 2 * v_piece;
   const uint32_t off_k = 2 * q_piece, off_v = off_k + s.kslots * k_slot;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t hd = p.hd, vd = p.vd, rep = s.rep, qt = kRows / rep;  // queries per CTA
-  const uint32_t bk = blockIdx.y, b = s.b0 + bk / p.KV, kvh = bk % p.KV, map = blockIdx.z;
+  const uint32_t hd = p.hd, rep = s.rep, qt = kRows / rep;  // queries per CTA
+  const uint32_t bk = blockIdx.y, b = s.b0 + bk / p.KV, kvh = bk % p.KV;
   const uint32_t q0 = (gridDim.x - 1u - blockIdx.x) * qt;  // the tiles with the most keys first: they are the long ones
   const uint32_t head0 = kvh * rep;
 
@@ -273,17 +271,12 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
     kmax = 0;
     if (tid == 0 && p.status) atomicCAS(p.status, 0, 5);
   }
-  // tiles that hold a kept first position, then those from the first query's window on
-  const uint32_t all_tiles = (kmax + kKeys - 1) / kKeys, first = past + q0;
-  const uint32_t lo = p.window && first + 1u > p.window ? first + 1u - p.window : 0u;
-  const uint32_t kept_tiles = (min(p.keep, kmax) + kKeys - 1) / kKeys, lo_tile = min(max(lo / kKeys, kept_tiles), all_tiles);
-  const uint32_t ntiles = kept_tiles + all_tiles - lo_tile;
-  auto tile_at = [&](uint32_t i) { return i < kept_tiles ? i : lo_tile + (i - kept_tiles); };
+  const uint32_t ntiles = (kmax + kKeys - 1) / kKeys;
 
   if (warp < kControl) {
     if (warp == 0 && elect_one()) {
       // ===== copies =====
-      const unsigned char* kbase = s.k + (size_t)bk * s.tiles * p.maps * k_slot + map * k_slot;
+      const unsigned char* kbase = s.k + (size_t)bk * s.tiles * k_slot;
       const unsigned char* vbase = s.v + (size_t)bk * s.tiles * v_slot;
       // the keys of tile i, then the values of tile i - 1: keys are needed sooner and freed sooner
       uint32_t k = 0, v = 0;  // requested
@@ -292,14 +285,14 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
           const uint32_t slot = i % s.kslots;
           if (i >= s.kslots && !mbar_wait(&k_empty[slot], (i / s.kslots - 1u) & 1u)) { s_abort = 1; break; }
           mbar_expect_tx(&k_full[slot], k_slot);
-          bulk_load(smem + off_k + slot * k_slot, kbase + (size_t)tile_at(i) * p.maps * k_slot, k_slot, &k_full[slot]);
+          bulk_load(smem + off_k + slot * k_slot, kbase + (size_t)i * k_slot, k_slot, &k_full[slot]);
           ++k;
         }
         if (i > 0) {
           const uint32_t slot = v % s.vslots;
           if (v >= s.vslots && !mbar_wait(&v_empty[slot], (v / s.vslots - 1u) & 1u)) { s_abort = 1; break; }
           mbar_expect_tx(&v_full[slot], v_slot);
-          bulk_load(smem + off_v + slot * v_slot, vbase + (size_t)tile_at(v) * v_slot, v_slot, &v_full[slot]);
+          bulk_load(smem + off_v + slot * v_slot, vbase + (size_t)v * v_slot, v_slot, &v_full[slot]);
           ++v;
         }
       }
@@ -359,7 +352,7 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
     for (uint32_t r = warp - kControl; r < (uint32_t)kRows; r += kSoftWarps) {
       const uint32_t qi = r / rep, h = r % rep;
       const bool in = r < qt * rep && qi < nq;
-      const float* src = p.q + (size_t)(b * p.T + q0 + qi) * p.q_ld + (size_t)((head0 + h) * p.maps + map) * hd;
+      const float* src = p.q + (size_t)(b * p.T + q0 + qi) * p.q_ld + (size_t)(head0 + h) * hd;
       float4 v[2];
       uint32_t mx = 0;
 #pragma unroll
@@ -393,7 +386,6 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
     const float qback = s_qback[row];
     const uint32_t qi = row / rep, h = row % rep;
     const uint32_t qpos = past + q0 + min(qi, nq - 1u);  // the last key this row's query sees (rows without a query: any)
-    const uint32_t qlo = p.window && qpos + 1u > p.window ? qpos + 1u - p.window : 0u;  // the first but for the kept ones
     const uint32_t lanes = (quarter * 32u) << 16;
     float m_run = -INFINITY, l_run = 0.0f, corr_prev = 0.0f, vf_prev = 0.0f;
     unsigned long long sums[OC / 2];  // pairs of columns
@@ -423,11 +415,11 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
       }
     };
     const float* factor = s.factor + (size_t)bk * s.tiles * 2;
-    float2 fac = ntiles ? *reinterpret_cast<const float2*>(factor + 2 * tile_at(0)) : make_float2(0.f, 0.f);
+    float2 fac = ntiles ? *reinterpret_cast<const float2*>(factor) : make_float2(0.f, 0.f);
     for (uint32_t i = 0; i < ntiles; ++i) {
-      const uint32_t sb = i & 1u, key0 = tile_at(i) * kKeys + cp * SC;  // this thread's first key
+      const uint32_t sb = i & 1u, key0 = i * kKeys + cp * SC;  // this thread's first key
       const float2 cur = fac;
-      if (i + 1 < ntiles) fac = *reinterpret_cast<const float2*>(factor + 2 * tile_at(i + 1));
+      if (i + 1 < ntiles) fac = *reinterpret_cast<const float2*>(factor + 2 * (i + 1));
       wait(&s_full[sb], (i >> 1) & 1u);
       float sc[SC];
 #pragma unroll
@@ -440,10 +432,9 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_free[sb]);
-      // which of the keys the row sees: bit j = key0 + j in [qlo, qpos], or below keep
-      auto below = [&](uint32_t n) { return n <= key0 ? 0u : n - key0 >= 32u ? 0xFFFFFFFFu : (1u << (n - key0)) - 1u; };
+      // which of the keys the row sees: bit j = key0 + j <= qpos
       const uint32_t all = SC == 32 ? 0xFFFFFFFFu : (1u << (SC & 31)) - 1u;
-      const uint32_t seen = below(qpos + 1u) & (~below(qlo) | below(p.keep)) & all;
+      const uint32_t seen = qpos < key0 ? 0u : qpos - key0 >= 31u ? all : ((2u << (qpos - key0)) - 1u) & all;
       const bool whole = __all_sync(0xFFFFFFFFu, seen == all);
       if (!whole) {
 #pragma unroll
@@ -499,67 +490,16 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
       const size_t token = (size_t)b * p.T + q0 + qi;
       const uint32_t c0 = cp * OC;
       const float inv = 1.0f / l;
-      if (p.maps == 2) {
-        float* dst = s.maps + (((token - (size_t)s.b0 * p.T) * (p.KV * rep) + head0 + h) * 2 + map) * vd;
+      float* dst = p.out + token * p.out_ld + (size_t)(head0 + h) * hd;
 #pragma unroll
-        for (int j = 0; j < OC; j += 4)
-          if (c0 + j < vd) *reinterpret_cast<float4*>(dst + c0 + j) = make_float4(o[j] * inv, o[j + 1] * inv, o[j + 2] * inv, o[j + 3] * inv);
-      } else {
-        const size_t at = token * p.out_ld + (size_t)(head0 + h) * p.vd_out;
-        const bool wide = p.out_dtype == RUAI_F32 && p.vd_out % 4 == 0 && p.out_ld % 4 == 0;
-#pragma unroll
-        for (int j = 0; j < OC; j += 4) {
-          if (wide) {
-            if (c0 + j < p.vd_out) *reinterpret_cast<float4*>(p.out + at + c0 + j) = make_float4(o[j] * inv, o[j + 1] * inv, o[j + 2] * inv, o[j + 3] * inv);
-          } else {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (c0 + j + u < p.vd_out) store_from_f32(p.out, p.out_dtype, at + c0 + j + u, o[j + u] * inv);
-          }
-        }
-      }
+      for (int j = 0; j < OC; j += 4)
+        if (c0 + j < hd) *reinterpret_cast<float4*>(dst + c0 + j) = make_float4(o[j] * inv, o[j + 1] * inv, o[j + 2] * inv, o[j + 3] * inv);
     }
   }
   tc_fence_before_sync();
   __syncthreads();
   if (s_abort && tid == 0 && p.status) atomicCAS(p.status, 0, 3);
   if (warp == 1) tmem_dealloc(tmem, s.tmem);
-}
-
-// Two score maps per head: out_scale * rms_norm(map 1 - lambda map 2), a warp per (token, head).
-__global__ void __launch_bounds__(256) attn_maps_kernel(const AttnParams p, const Pieces s, uint32_t tokens, uint32_t heads) {
-  grid_dependency_wait();
-  grid_launch_dependents();
-  const uint32_t lane = threadIdx.x & 31u, item = blockIdx.x * 8u + (threadIdx.x >> 5);
-  if (item >= tokens * heads || (uint32_t)*p.len + p.T > p.cap) return;
-  const size_t token = (size_t)s.b0 * p.T + item / heads;
-  const uint32_t head = item % heads;
-  const float lam = *p.lambda;
-  const float4* a = reinterpret_cast<const float4*>(s.maps + (size_t)item * 2 * p.vd);
-  float4 y[2];
-  float ss = 0.0f;
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const uint32_t e = lane + 32u * j;
-    y[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (e < p.vd / 4) {
-      const float4 u = a[e], z = a[p.vd / 4 + e];
-      y[j] = make_float4(u.x - lam * z.x, u.y - lam * z.y, u.z - lam * z.z, u.w - lam * z.w);  // columns past vd_out are zero in both maps
-      ss = fmaf(y[j].x, y[j].x, ss); ss = fmaf(y[j].y, y[j].y, ss); ss = fmaf(y[j].z, y[j].z, ss); ss = fmaf(y[j].w, y[j].w, ss);
-    }
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
-  const float f = p.out_scale / sqrtf(ss / (float)p.vd_out + p.eps);
-  const size_t at = token * p.out_ld + (size_t)head * p.vd_out;
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const uint32_t e = 4 * (lane + 32u * j);
-    const float v[4] = {y[j].x * f, y[j].y * f, y[j].z * f, y[j].w * f};
-#pragma unroll
-    for (uint32_t i = 0; i < 4; ++i)
-      if (e + i < p.vd_out) store_from_f32(p.out, p.out_dtype, at + e + i, v[i]);
-  }
 }
 
 template <int CS, int OC>
@@ -573,7 +513,7 @@ cudaError_t launch_tc(ruai_ctx* c, const AttnParams& p, const Pieces& s, dim3 gr
   return ruai_launch(c, attn_tc_kernel<CS, OC>, grid, dim3((kControl + 4 * CS) * 32), smem, true, p, s);
 }
 
-constexpr size_t kScratchMost = 256u << 20;  // a step's pieces (and maps) at a time
+constexpr size_t kScratchMost = 256u << 20;  // a step's pieces at a time
 // Fewer tokens leave most of the 128 rows and of the tensor core's time to nothing while the splitting costs a launch.  Us of a whole prompt, here |
 // attn_prefill.cu: 64 tokens of the 8B shape's 2 layers 656 | 648, of the 135M shape's 10 718 | 687; 96 tokens 700 | 718, 768 | 796, of
 // the 1.1B shape's 6 803 | 836, of GPT-2 1056 | 1126; 160 tokens 1080 | 1123, 833 | 937, 1105 | 1197, 1226 | 1410.
@@ -583,11 +523,12 @@ constexpr uint32_t kFromTokens = 96;
 
 // 1: launched; 0: this shape is not taken; < 0: error.  `p`: as ruai_attention_prefill has completed it.
 int ruai_attention_prefill_tc(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep) {
-  if (p.T < kFromTokens || rep > 64 || p.k_pos || p.sink || p.gate) return 0;
+  if (!p.pieces || p.T < kFromTokens || rep > 64) return 0;
+  if (p.maps != 1 || p.window || p.keep || p.vd != p.hd || p.vd_out != p.hd || p.out_dtype != RUAI_F32 || p.k_pos || p.sink || p.gate) return 0;
   Pieces s = {};
   s.rep = rep;
   s.blocks = (p.hd + 63) / 64;
-  s.vdp = (p.vd + 15) / 16 * 16;
+  s.vdp = (p.hd + 15) / 16 * 16;
   s.tiles = (p.cap + kKeys - 1) / kKeys;
   s.tmem = s.vdp <= 64 ? 256 : 512;
   const uint32_t q = 2 * s.blocks * kRows * 128, ks = 2 * s.blocks * kKeys * 128, vs = 2 * s.vdp * 128;
@@ -597,8 +538,8 @@ int ruai_attention_prefill_tc(ruai_ctx* c, const AttnParams& p, uint32_t B, uint
   const uint32_t smem = q + s.kslots * ks + s.vslots * vs + 1024;
   // sequences at a time: what their pieces take of the scratch
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  const size_t k1 = (size_t)p.KV * s.tiles * p.maps * ks, v1 = (size_t)p.KV * s.tiles * vs, f1 = (size_t)p.KV * s.tiles * 2 * sizeof(float);
-  const size_t m1 = p.maps == 2 ? (size_t)p.T * p.KV * rep * 2 * p.vd * sizeof(float) : 0, one = k1 + v1 + f1 + m1 + 1024;
+  const size_t k1 = (size_t)p.KV * s.tiles * ks, v1 = (size_t)p.KV * s.tiles * vs, f1 = (size_t)p.KV * s.tiles * 2 * sizeof(float);
+  const size_t one = k1 + v1 + f1 + 1024;
   if (one > kScratchMost) return 0;
   const uint32_t per = (uint32_t)std::min<size_t>(B, std::min<size_t>(kScratchMost / one, 65535u / p.KV));
   if (!per) return 0;
@@ -614,8 +555,7 @@ int ruai_attention_prefill_tc(ruai_ctx* c, const AttnParams& p, uint32_t B, uint
   unsigned char* at = reinterpret_cast<unsigned char*>(c->partial);
   s.k = at; at += up(per * k1);
   s.v = at; at += up(per * v1);
-  s.factor = reinterpret_cast<float*>(at); at += up(per * f1);
-  s.maps = reinterpret_cast<float*>(at);
+  s.factor = reinterpret_cast<float*>(at);
   static bool done[64] = {};
   cudaError_t e = cudaSuccess;
   if (!done[c->ordinal & 63]) {
@@ -626,12 +566,9 @@ int ruai_attention_prefill_tc(ruai_ctx* c, const AttnParams& p, uint32_t B, uint
   for (uint32_t b0 = 0; b0 < B && e == cudaSuccess; b0 += per) {
     const uint32_t nb = std::min(per, B - b0);
     s.b0 = b0;
-    e = ruai_launch(c, attn_split_kernel, dim3(s.tiles, nb * p.KV), dim3(kSplitThreads), (size_t)kKeys * (p.vd + 1) * 4, true, p, s);
-    const dim3 grid((p.T + qt - 1) / qt, nb * p.KV, p.maps);
-    if (e == cudaSuccess) e = p.vd <= 64 ? launch_tc<2, 32>(c, p, s, grid, smem) : p.vd <= 128 ? launch_tc<4, 32>(c, p, s, grid, smem) : launch_tc<4, 64>(c, p, s, grid, smem);
-    const uint32_t heads = p.KV * rep;
-    if (e == cudaSuccess && p.maps == 2)
-      e = ruai_launch(c, attn_maps_kernel, dim3((nb * p.T * heads + 7) / 8), dim3(256), 0, true, p, s, nb * p.T, heads);
+    e = ruai_launch(c, attn_split_kernel, dim3(s.tiles, nb * p.KV), dim3(kSplitThreads), (size_t)kKeys * (p.hd + 1) * 4, true, p, s);
+    const dim3 grid((p.T + qt - 1) / qt, nb * p.KV);
+    if (e == cudaSuccess) e = p.hd <= 64 ? launch_tc<2, 32>(c, p, s, grid, smem) : p.hd <= 128 ? launch_tc<4, 32>(c, p, s, grid, smem) : launch_tc<4, 64>(c, p, s, grid, smem);
   }
   if (e != cudaSuccess) { ruai_fail(c, RUAI_ERR_CUDA, "prefill attention launch: %s", cudaGetErrorString(e)); return -1; }
   return 1;

@@ -19,10 +19,12 @@ struct AttnParams {
   uint32_t out_ld;
   int* status;          // context status word (bounded waits)
   unsigned long long* trace;  // debug timeline slot
-  // ruai_attention_prefill only.  Values of another width than the keys (0: as wide): rows of vd floats in the cache, of
+  // ruai_attention_prefill only.  pieces != 0: a long prompt's products may run on the tensor cores, in fp16 pieces of 22 bits
+  // (attn_prefill_tc.cu; f32 output, one map over all positions).  Values of another width than the keys (0: as wide): rows of vd floats in the cache, of
   // which vd_out reach the output.  Two score maps per head over the same values: key rows and query heads hold
   // [map 1 | map 2], hd each; the output is out_scale * rms_norm(map 1 - lambda map 2), over vd_out.
   // A position sees itself and the window - 1 ones before it (window 0: all), and of the earlier ones those below keep.
+  int pieces;
   uint32_t vd, vd_out, maps;
   uint32_t window, keep;
   const float* lambda;
@@ -50,7 +52,7 @@ int ruai_rope_kv(ruai_ctx* c, float* qkv, uint32_t qkv_ld, uint32_t k_off, uint3
 int ruai_attention(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep);
 // Many query positions at once, queries in tiles (attn_prefill.cu).  1: launched; 0: not taken for this shape; < 0: error.
 int ruai_attention_prefill(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep);
-// The same on the tensor cores (attn_prefill_tc.cu), for what ruai_attention_prefill passes on to it.
+// The same on the tensor cores (attn_prefill_tc.cu), for callers that set p.pieces.
 int ruai_attention_prefill_tc(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep);
 // Whether heads of these widths, each with keys of its own (rep 1, one map), fit it.
 bool ruai_attention_prefill_fits(uint32_t hd, uint32_t vd);

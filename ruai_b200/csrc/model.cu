@@ -501,7 +501,7 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
     ap.q = qkv; ap.q_ld = nqkv; ap.kcache = Ly.kc.as<float>(); ap.vcache = Ly.vc.as<float>(); ap.len = len;
     ap.fuse = fuse ? 1 : 0; ap.table = table; ap.k_off = nql; ap.v_off = nql + nkvl;
     ap.T = T; ap.KV = m->KVl; ap.hd = hd; ap.cap = m->cap; ap.scale = 1.0f / sqrtf((float)hd);
-    ap.out = att; ap.out_ld = nql; ap.status = c->status;
+    ap.out = att; ap.out_ld = nql; ap.status = c->status; ap.pieces = 1;
     {
       const int took = ruai_attention_prefill(c, ap, B, rep);  // many query positions: queries in tiles
       if (took < 0) return RUAI_ERR_CUDA;
