@@ -298,7 +298,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_kernel(const AttnPa
 #pragma unroll
       for (int off = kKeys; off < 32; off <<= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, off);
       const float s = valid ? a * p.scale : -INFINITY;
-      const float m_new = fmaxf(m[r], warp_max(s)), pr = valid ? expf(s - m_new) : 0.0f, corr = m[r] == -INFINITY ? 0.0f : expf(m[r] - m_new);
+      const float m_new = fmaxf(m[r], warp_max(s)), m_use = m_new == -INFINITY ? 0.0f : m_new;  // keys with scores of -inf weigh nothing beside others
+      const float pr = valid ? expf(s - m_use) : 0.0f, corr = m[r] == -INFINITY ? 0.0f : expf(m[r] - m_new);
       l[r] = fmaf(l[r], corr, lane < kKeys ? pr : 0.0f);
       m[r] = m_new;
 #pragma unroll

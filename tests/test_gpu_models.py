@@ -261,6 +261,32 @@ def test_attention_against_float64(dev, H, KV, hd, B, lengths):
             assert near(gm.forward_cached(ids[:, n // 3 + 1:], all_positions=True), want[:, n // 3 + 1:]), n
 
 
+@pytest.mark.parametrize("hd", [32, 128, 256])
+def test_scores_of_minus_infinity(dev, hd):
+    """Keys whose score overflows to -inf weigh nothing: a row that sees such keys (token A) and others (token B, all alike) is that of B alone.
+    The first 70 or 100 keys are A, so that whole shares of a step, chunks and tiles hold nothing else."""
+    d, V, rng = 256, 19, np.random.default_rng(hd)
+    H = d // hd
+    gm = nn.GPT2(dev, nn.GPT2Config(V, 400, d, 1, H))
+    A, B = np.tile([1.0, -1.0], d // 2), np.tile([1.0, 1.0, -1.0, -1.0], d // 4)  # LayerNorm leaves both as they are
+    u = np.ones(d)
+    qkv = np.concatenate([np.outer(B, 1e20 * u), np.outer(A, -1e20 * u), np.outer(B, rng.standard_normal(d)) + np.outer(A, rng.standard_normal(d))], 1) / d
+    embed = rng.standard_normal((V, d))
+    embed[0], embed[1] = A, B
+    for t, f in {7: qkv, 8: rng.standard_normal((d, d)) / 16, 9: rng.standard_normal((d, 4 * d)) / 16, 10: rng.standard_normal((4 * d, d)) / 32, 11: np.zeros(3 * d),
+                 12: np.zeros(d), 13: np.zeros(4 * d), 14: np.zeros(d), 0x10000000: embed, 0x10000002: np.zeros((400, d)), 0x40000000: np.ones(d), 0x40000001: np.zeros(d),
+                 0x50000000: np.ones(d), 0x51000000: np.zeros(d), 0x52000000: np.ones(d), 0x53000000: np.zeros(d)}.items():
+        gm.set_f32(t, f.astype(np.float32))
+    gm.quantize_int8()
+    want = gm.forward_cached(np.ones((1, 1), np.int32))[0]
+    assert np.isfinite(want).all()
+    for n in (70, 100):
+        gm.cache_clear()
+        got = [gm.forward_cached(np.array([[0] * n + [1] * 3], np.int32), all_positions=True)[0, n:]]
+        got += [gm.forward_cached(np.ones((1, t), np.int32), all_positions=True)[0] for t in (1, 2, 1, 9, 1)]
+        assert np.abs(np.concatenate(got) - want).max() <= 1e-4 * np.abs(want).max(), n
+
+
 def test_errors_mirror_the_reference_asserts(dev):
     _, gm = build(dev, llama_cfg(**dict(TINY_LLAMA, max_pos=8)), 5, 8)
     with pytest.raises(nn.RuaiError, match="exceeds max_position_embeddings"):
