@@ -274,7 +274,10 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_kernel(const AttnPa
       fetch(c0);
     }
     ok = __all_sync(0xFFFFFFFFu, pipe::mbar_wait(bar, phase & 1u));
-    if (!ok) break;
+    if (!ok) {
+      (void)pipe::mbar_wait(bar, phase & 1u);  // whoever gives up: no copy in flight into shared memory that another CTA may get
+      break;
+    }
     ++phase;
     const uint32_t nk = min((uint32_t)kKeys, k1 - c0);
     const bool valid = key < nk;
