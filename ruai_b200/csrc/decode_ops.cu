@@ -9,6 +9,7 @@
 // Positions and token ids are read from device memory so that a captured graph of
 // the step can be replayed without host involvement.
 #include <algorithm>
+#include <cmath>
 
 #include "decode_ops.cuh"
 #include "pipeline.cuh"
@@ -158,9 +159,9 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kv_kernel(float* __restrict
 // warp's lanes; values: a lane per four elements, all heads at once.  So a cached element is read from shared memory once per warp,
 // and nothing but the warps' results meets at a barrier.  Keys are split over a cluster of gridDim.z CTAs as well; the first one
 // merges the results, through distributed shared memory.
-// Bound by HBM where there are many sequences (64 of 260 keys, 4 key heads of 64 with 8 query heads each: 52 us a launch with the
-// warps of a CTA at 64 keys in turn, four barriers for them and every key and value read once per head; 25 us now, 5 at the
-// bandwidth), by latency where there is one (1024 keys: 8 to 9 us before and now).
+// Bound by its warps' latencies: a warp copies, waits, works (64 sequences of 256 keys, 4 key heads of 64 with 8 query heads each: 19 us alone
+// and 25 in a step, 5 at the bandwidth; attn_chunks.cu, whose CTAs read every key and value once per head and meet at four barriers a chunk, 36
+// and 52).  Where the keys of few items are many, or few query heads share a key, that one is the faster: ruai_attention_plan.
 template <int REP, int LPK>  // lanes per key: 1, 2 or 4 for head dimensions up to 64, 128, 256, so that a warp's copy stays below 17 KB
 __global__ void __launch_bounds__(kAttnWarps * 32) attention_kernel(const AttnParams p) {
   constexpr int kJ = LPK == 4 ? 2 : 1, kRepPad = REP == 3 ? 4 : REP, kKeys = 32 / LPK;
@@ -539,34 +540,84 @@ int ruai_rope_kv(ruai_ctx* c, float* qkv, uint32_t qkv_ld, uint32_t k_off, uint3
   return RUAI_OK;
 }
 
-int ruai_attention(ruai_ctx* c, const AttnParams& p_in, uint32_t B, uint32_t rep) {
+namespace {
+// The rounds that `ctas` take on `sms` SMs, per_sm at a time, and the CTAs that share an SM meanwhile.
+struct Waves { double rounds, together; };
+Waves waves(uint64_t ctas, uint64_t per_sm, double sms) {
+  const double q = ctas / (sms * per_sm);
+  return {q <= 1 ? 1.0 : q < 4 ? std::ceil(q) : q + 0.5, std::min((double)per_sm, std::max(1.0, std::ceil(ctas / sms)))};
+}
+double norm4(double a, double b, double c) { return std::sqrt(std::sqrt(a * a * a * a + b * b * b * b + c * c * c * c)); }
+
+// What a launch takes in microseconds, in chunks and with warps that work alone.  A chunk's (a step's) time is the CTA's own, the SM's
+// arithmetic or its share of the memory's rate, whichever is longest.  The constants are fitted to 2,300 launches: 13 head shapes (1 to 8 query heads per
+// key head, 32 to 256 wide), 1 to 64 sequences of 32 to 32768 positions, 1 to 7 queries; two in three are within 10 %.
+double chunks_us(const ruai_ctx* c, uint64_t items, uint32_t rep, uint32_t hd, uint32_t cap, uint32_t splits) {
+  const uint64_t ctas = items * splits, sub = ctas > 2u * (uint64_t)c->sm_count ? 1 : 2, threads = 64u * rep * sub;
+  const uint64_t per_sm = std::max<uint64_t>(1, std::min({2048 / threads, (uint64_t)(kAttnSmemMax / (ruai_attention_chunk_smem(rep, hd, (uint32_t)sub) + 1024)), 65536 / (80 * threads)}));
+  const Waves w = waves(ctas, per_sm, c->sm_count);
+  const uint32_t keys = (cap + splits - 1) / splits;
+  const double h = hd / 64.0;
+  const double chunk = norm4(0.81 + 0.049 * rep * h / sub + 0.2 * rep + 0.51 * h, w.together * 0.2 * (rep * h + 1.5), w.together * 0.54 * h * std::min(keys, 64u) / 64);
+  return 0.18 * rep + w.rounds * ((keys + 63) / 64 * chunk + 1.8) + (splits > 1 ? 2.6 + 0.0085 * splits * rep * h : 0.0);
+}
+double warps_us(const ruai_ctx* c, uint64_t items, uint32_t rep, uint32_t hd, uint32_t cap, uint32_t warps, uint32_t splits) {
+  const uint32_t registers = rep == 8 ? 144 : 64 + 8 * rep, shares = splits * warps * attn_keys(hd);
+  const uint64_t per_sm = std::max<uint64_t>(1, std::min<uint64_t>(kAttnSmemMax / (attn_smem(rep, hd, warps, splits) + 1024), 65536 / (registers * 32 * warps)));
+  // clusters lie within a group of SMs: of eight CTAs that fill an SM each there is room for 15, of four for 33
+  const Waves w = waves(items * splits, per_sm, c->sm_count * (splits == 8 ? 120 / 148.0 : splits == 4 ? 132 / 148.0 : 1.0));
+  const double h = hd / 64.0, f = attn_keys(hd) / 32.0, busy = w.together * warps;
+  const double step = norm4(1.2 + 0.37 * rep + 1.5 * h * f, busy * 0.073 * (rep * h * f + 0.27 * h + 1.5), busy * 0.23 * h * f);
+  return 0.18 * rep + w.rounds * ((cap + shares - 1) / shares * step + 2.0) + (splits > 1 ? 0.86 + 0.074 * splits : 0.0);
+}
+}  // namespace
+
+// The warps' numbers with the shortest launch, or chunks where that is not 13 % shorter by the formulas above (less 1 us with few query heads per
+// key: behind a step's other launches warps that work alone gain that much on chunks).  Of 489 steps measured (1 to 64 sequences of 40 to 32768
+// positions, six head shapes) none is more than 3 % slower than all in chunks, 5 % are shorter on average, and 1 in 40 is more than 5 % slower than all on
+// warps.  Us of a launch, chunks | warps:
+//   8 key heads of 128 with 4 query heads each: 1 sequence, 1024 positions 9.0 | 9.2, 8192 31 | 40, 32768 91 | 160; 16 sequences, 256 20 | 13,
+//   1024 42 | 47, 4096 129 | 163;  4 of 64 with 8 each: 1 sequence, 1024 10.2 | 10.7, 32768 77 | 101; 64 sequences, 256 36 | 19, 1024 126 | 65;
+//   3 of 64 with 3 each: 1 sequence, 8192 14 | 21; 64 sequences, 256 12.5 | 9.1, 4096 106 | 89;  12 of 64: 64 sequences, 1024 66 | 77
+// Up to 64 positions chunks always: one for all keys, and a CTA's warps share its arithmetic (4 of 64 with 8 each 6.7 | 8.3).
+AttnPlan ruai_attention_plan(const ruai_ctx* c, uint32_t B, uint32_t T, uint32_t KV, uint32_t rep, uint32_t hd, uint32_t cap) {
+  AttnPlan plan;
+  const uint64_t items = (uint64_t)B * KV * T;
+  // chunks: one per CTA where the capacity allows it; with many (sequence, KV head) items there are CTAs enough without it
+  const uint32_t by_len = (cap + 63) / 64;
+  if (T > 1) plan.splits = 1;
+  else if (items >= 512) plan.splits = std::max(1u, std::min(by_len, 2u));
+  else plan.splits = std::max(1u, std::min(B >= 5 ? (by_len + 1) / 2 : by_len, 64u));
+  if (cap <= 64) return plan;
+  double best = 0.87 * chunks_us(c, items, rep, hd, cap, plan.splits) + (rep < 4 ? 1.0 : 0.0);
+  for (uint32_t w = 4; w <= (uint32_t)kAttnWarps; w *= 2)
+    for (uint32_t s = 1; s <= 8; s *= 2) {
+      if (attn_smem(rep, hd, w, s) > kAttnSmemMax) break;
+      const double t = warps_us(c, items, rep, hd, cap, w, s);
+      if (t < best) { best = t; plan.warps = w; plan.splits = s; }
+    }
+  return plan;
+}
+
+int ruai_attention(ruai_ctx* c, const AttnParams& p_in, uint32_t B, uint32_t rep, const AttnPlan& plan) {
   AttnParams p = p_in;
   p.trace = ruai_trace_slot(c);
   if (p.hd % 4 || p.hd > 256) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "head_dim %u must be a multiple of 4 and at most 256", p.hd);
-  // Warps per CTA and CTAs per item: the numbers with the shortest launch, from the steps that a warp then takes one after the other
-  // and the rounds of CTAs that the grid takes.
-  uint32_t warps = 4, splits = 1;
-  double best = 1e30;
-  for (uint32_t w = 4; w <= (uint32_t)kAttnWarps; w *= 2)
-    for (uint32_t s = 1; s <= 8; s *= 2) {
-      const size_t smem = attn_smem(rep, p.hd, w, s);
-      if (smem > kAttnSmemMax) break;
-      const uint32_t shares = s * w * attn_keys(p.hd), steps = (p.cap + shares - 1) / shares;
-      const uint64_t places = (uint64_t)c->sm_count * std::max<size_t>(1, std::min<size_t>(32 / w, kAttnSmemMax / (smem + 1024)));
-      const uint64_t rounds = ((uint64_t)B * p.KV * p.T * s + places - 1) / places;
-      const double t = rounds * (2.0 + 1.2 * steps) + 0.1 * w + (s > 1 ? 0.6 + 0.1 * s : 0.0);
-      if (t < best) { best = t; splits = s; warps = w; }
-    }
-  const size_t smem = attn_smem(rep, p.hd, warps, splits);
-  const dim3 grid(B * p.KV, p.T, splits);
+  if (rep != 1 && rep != 2 && rep != 3 && rep != 4 && rep != 8) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "%u query heads per KV head (supported: 1, 2, 3, 4, 8)", rep);
   cudaError_t e;
-  switch (rep) {
-    case 1: e = launch_attn<1>(c, p, grid, warps, smem); break;
-    case 2: e = launch_attn<2>(c, p, grid, warps, smem); break;
-    case 3: e = launch_attn<3>(c, p, grid, warps, smem); break;
-    case 4: e = launch_attn<4>(c, p, grid, warps, smem); break;
-    case 8: e = launch_attn<8>(c, p, grid, warps, smem); break;
-    default: return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "%u query heads per KV head (supported: 1, 2, 3, 4, 8)", rep);
+  if (plan.warps == 0) {
+    if (plan.splits > 1 && (!p.scratch || !p.counters)) return ruai_fail(c, RUAI_ERR_ARG, "attention in chunks: no memory for %u splits", plan.splits);
+    e = ruai_attention_chunks(c, p, B, rep, plan.splits);
+  } else {
+    const size_t smem = attn_smem(rep, p.hd, plan.warps, plan.splits);
+    const dim3 grid(B * p.KV, p.T, plan.splits);
+    switch (rep) {
+      case 1: e = launch_attn<1>(c, p, grid, plan.warps, smem); break;
+      case 2: e = launch_attn<2>(c, p, grid, plan.warps, smem); break;
+      case 3: e = launch_attn<3>(c, p, grid, plan.warps, smem); break;
+      case 4: e = launch_attn<4>(c, p, grid, plan.warps, smem); break;
+      default: e = launch_attn<8>(c, p, grid, plan.warps, smem); break;
+    }
   }
   if (e != cudaSuccess) return ruai_fail(c, RUAI_ERR_CUDA, "attention launch: %s", cudaGetErrorString(e));
   return RUAI_OK;

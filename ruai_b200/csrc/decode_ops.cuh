@@ -17,6 +17,8 @@ struct AttnParams {
   float scale;          // 1/sqrt(hd)
   float* out;           // [B*T, out_ld]
   uint32_t out_ld;
+  float* scratch;       // attention in chunks, several splits: [B*KV*T][splits][rep][hd+4]
+  unsigned* counters;   // [B*KV*T], zero between launches
   int* status;          // context status word (bounded waits)
   unsigned long long* trace;  // debug timeline slot
   // ruai_attention_prefill only.  pieces != 0: a long prompt's products may run on the tensor cores, in fp16 pieces of 22 bits
@@ -49,7 +51,12 @@ int ruai_layer_norm(ruai_ctx* c, const float* x, const float* w, const float* b,
 int ruai_rope_table(ruai_ctx* c, const float* inv_freq, uint32_t half, uint32_t max_pos, float2* table);
 int ruai_rope_kv(ruai_ctx* c, float* qkv, uint32_t qkv_ld, uint32_t k_off, uint32_t v_off, const float2* table, const int32_t* len, uint32_t rows,
                  uint32_t T, uint32_t Hq, uint32_t KV, uint32_t hd, uint32_t cap, float* kcache, float* vcache);
-int ruai_attention(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep);
+// How ruai_attention runs: warps that work alone (their number per CTA), or 0: in chunks (attn_chunks.cu); and the CTAs that share an item's keys.
+struct AttnPlan { uint32_t warps = 0, splits = 1; };
+AttnPlan ruai_attention_plan(const ruai_ctx* c, uint32_t B, uint32_t T, uint32_t KV, uint32_t rep, uint32_t hd, uint32_t cap);
+int ruai_attention(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep, const AttnPlan& plan);
+size_t ruai_attention_chunk_smem(uint32_t rep, uint32_t hd, uint32_t sub);
+cudaError_t ruai_attention_chunks(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep, uint32_t splits);
 // Many query positions at once, queries in tiles (attn_prefill.cu).  1: launched; 0: not taken for this shape; < 0: error.
 int ruai_attention_prefill(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep);
 // The same on the tensor cores (attn_prefill_tc.cu), for callers that set p.pieces.

@@ -439,6 +439,20 @@ int ensure_activations(ruai_model* m, uint32_t rows, uint32_t out_rows, uint32_t
     m->logit_rows = out_rows;
     drop_graph(m);
   }
+  const uint32_t rep = m->Hl / m->KVl;
+  const AttnPlan plan = T == 1 ? ruai_attention_plan(c, B, T, m->KVl, rep, m->hd, m->cap) : AttnPlan();
+  if (plan.warps == 0 && plan.splits > 1) {
+    const size_t items = (size_t)B * m->KVl, need = items * plan.splits * rep * (m->hd + 4) * sizeof(float), cnt = items * sizeof(unsigned);
+    if (need > m->attn_scratch.bytes || cnt > m->attn_counters.bytes) {
+      RUAI_CUDA(c, cudaStreamSynchronize(c->stream));
+      RUAI_TRY(m->attn_scratch.reserve(c, need));
+      if (cnt > m->attn_counters.bytes) {
+        RUAI_TRY(m->attn_counters.alloc(c, cnt));
+        RUAI_CUDA(c, cudaMemsetAsync(m->attn_counters.p, 0, cnt, c->stream));
+      }
+      drop_graph(m);
+    }
+  }
   return RUAI_OK;
 }
 
@@ -502,10 +516,11 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
     ap.fuse = fuse ? 1 : 0; ap.table = table; ap.k_off = nql; ap.v_off = nql + nkvl;
     ap.T = T; ap.KV = m->KVl; ap.hd = hd; ap.cap = m->cap; ap.scale = 1.0f / sqrtf((float)hd);
     ap.out = att; ap.out_ld = nql; ap.status = c->status; ap.pieces = 1;
+    ap.scratch = m->attn_scratch.as<float>(); ap.counters = m->attn_counters.as<unsigned>();
     {
       const int took = ruai_attention_prefill(c, ap, B, rep);  // many query positions: queries in tiles
       if (took < 0) return RUAI_ERR_CUDA;
-      if (took == 0) RUAI_TRY(ruai_attention(c, ap, B, rep));
+      if (took == 0) RUAI_TRY(ruai_attention(c, ap, B, rep, ruai_attention_plan(c, B, T, m->KVl, rep, hd, m->cap)));
     }
     GemvEpilogue eo;
     eo.bias = Ly.o.bias.as<float>();
@@ -829,7 +844,7 @@ RUAI_API int ruai_model_destroy(ruai_model* m) {
   ruai_sweight_free(&m->head.sw);
   for (DevBuf* b : {&m->ps.layers, &m->ps.x, &m->ps.ss, &m->ps.acc, &m->ps.poison, &m->ps.att_part, &m->ps.arg_slots, &m->ps.sync}) b->release();
   for (DevBuf* b : {&m->embed, &m->wpe, &m->final_w, &m->final_b, &m->rope_table, &m->d_ids, &m->d_len, &m->d_err, &m->x, &m->xn, &m->qkv, &m->att,
-                    &m->hbuf, &m->xl, &m->logits, &m->sumsq, &m->arg_slots, &m->arg_counter})
+                    &m->hbuf, &m->xl, &m->logits, &m->attn_scratch, &m->attn_counters, &m->sumsq, &m->arg_slots, &m->arg_counter})
     b->release();
   m->d_rows.release();
   hybrid_destroy(m);

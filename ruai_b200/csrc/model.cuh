@@ -84,7 +84,7 @@ struct ruai_model {
   // cache state
   uint32_t B = 0, len = 0, cap = 0;
   // device state
-  DevBuf d_ids, d_rows, d_len, d_err, x, xn, qkv, att, hbuf, xl, logits, sumsq, arg_slots, arg_counter;
+  DevBuf d_ids, d_rows, d_len, d_err, x, xn, qkv, att, hbuf, xl, logits, attn_scratch, attn_counters, sumsq, arg_slots, arg_counter;
   uint32_t act_rows = 0, logit_rows = 0;
   // decode graph
   cudaGraphExec_t graph = nullptr;

@@ -59,3 +59,28 @@ def test_long_prompts_of_quantized_decoders_use_the_tensor_cores(dev):
     for T, tc in ((95, False), (96, True), (300, True)):
         names = kernels(dev, lambda: prompt(m, np.zeros((1, T), np.int32)))
         assert any("attn_tc_kernel" in n for n in names) == tc and any("attention_prefill_kernel" in n for n in names) != tc, (T, names)
+
+
+@pytest.mark.parametrize("B,H,KV,hd,positions,chunks", [(1, 8, 2, 128, 8192, True), (2, 4, 1, 256, 4096, True), (1, 3, 3, 64, 40, True), (64, 16, 2, 64, 300, False),
+                                                        (16, 8, 2, 128, 300, False)])
+def test_attention_of_a_step_long_caches_in_chunks(dev, B, H, KV, hd, positions, chunks):
+    """Few key heads over a long cache need more CTAs than a cluster has; many sequences, whose warps work alone, do not."""
+    m = llama(dev, H=H, KV=KV, hd=hd, positions=16384)
+    m.cache_reserve(B, positions)
+    m.forward_cached(np.zeros((B, 1), np.int32), want_logits=False)
+    names = kernels(dev, lambda: m.decode_step(B))
+    assert any("attention_chunk_kernel" in n for n in names) == chunks and any("attention_kernel" in n for n in names) != chunks, names
+
+
+@pytest.mark.parametrize("B,H,KV,hd", [(1, 8, 2, 128), (3, 8, 1, 64), (1, 2, 2, 256), (2, 3, 1, 80)])
+def test_steps_over_a_long_capacity_repeat_those_over_a_short_one(dev, B, H, KV, hd):
+    """The same tokens through the two attention kernels of a step (the capacity decides), and after growing from one to the other."""
+    ids = np.random.default_rng(hd).integers(0, 500, (B, 90)).astype(np.int32)
+    out = []
+    for reserve in (0, 16000):
+        m = llama(dev, H=H, KV=KV, hd=hd, positions=16384, L=2)
+        if reserve:
+            m.cache_reserve(B, reserve)
+        out.append([m.forward_cached(ids[:, :40])] + [m.forward_cached(ids[:, t:t + 1]) for t in range(40, 80)] + [m.forward_cached(ids[:, 80:83])])
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= 1e-5 * np.abs(a).max()
