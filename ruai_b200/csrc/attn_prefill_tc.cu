@@ -5,8 +5,9 @@
 // values; 2^14 for the probabilities) so that its largest magnitude lies below 2^15, and split into two fp16 pieces,
 // x = hi + 2^-12 lo: 22 bits down to 2^-28 of the largest, then a quantum of 2^-50 of it.  A product takes three of the four products
 // of pieces; the lo ones go first and the first hi one scales them by 2^-12 (exact).  The tensor core adds a tile's 64 keys (a
-// score's head dimension) only: sums over tiles, the running softmax and its exponentials are f32 in registers.  Infinities and NaN
-// stay what they are in hi (lo is 0 there) and make the rows that see them non-finite.
+// score's head dimension) only: sums over tiles, the running softmax and its exponentials are f32 in registers.  A tile with an
+// infinity or a NaN in it has a factor of NaN, and a CTA that meets one works its rows out again in f32, key by key: an infinite key may score
+// -inf, and what a row does not see does not reach it, whereas 0 x inf is NaN in a product of tiles.  (In a query they make its row NaN either way.)
 //
 // The decoders built from a list of layers (p.pieces is 0) stay on attn_prefill.cu.  They round every layer's output to bf16, and
 // sums in another order turn some of those roundings: their outputs would be others (2.3e-3 of a norm) without being nearer to 64 bits, and
@@ -70,11 +71,8 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
   const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
   lo = half2_bits((a - h.x) * kLoScale, (b - h.y) * kLoScale);
 }
-__device__ __forceinline__ void split2_any(float a, float b, uint32_t& hi, uint32_t& lo) {  // the same where infinities and NaN may come
-  hi = half2_bits(a, b);
-  const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-  const float x = magnitude(a) || a == 0.0f ? (a - h.x) * kLoScale : 0.0f, y = magnitude(b) || b == 0.0f ? (b - h.y) * kLoScale : 0.0f;
-  lo = half2_bits(x, y);
+__device__ __forceinline__ bool finite(const float4& v) {
+  return isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w);
 }
 
 __device__ __forceinline__ uint32_t block_max(uint32_t v, uint32_t* red) {
@@ -104,22 +102,29 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const AttnPar
   auto key4 = [&](uint32_t k, uint32_t e) { return *reinterpret_cast<const float4*>(kbase + (size_t)(k0 + k) * hd + e); };  // of key k0 + k
   auto mag4 = [](const float4& v) { return max(max(magnitude(v.x), magnitude(v.y)), max(magnitude(v.z), magnitude(v.w))); };
   uint32_t km = 0, vm = 0;
-  for (uint32_t i = tid; i < nk * (hd / 4); i += kSplitThreads) km = max(km, mag4(key4(i / (hd / 4), 4 * (i % (hd / 4)))));
+  bool odd = false;
+  for (uint32_t i = tid; i < nk * (hd / 4); i += kSplitThreads) {
+    const float4 v = key4(i / (hd / 4), 4 * (i % (hd / 4)));
+    km = max(km, mag4(v));
+    odd = odd || !finite(v);
+  }
   for (uint32_t i = tid; i < kKeys * (hd / 4); i += kSplitThreads) {
     const uint32_t k = i / (hd / 4), e = 4 * (i % (hd / 4));
     const float4 v = k < nk ? *reinterpret_cast<const float4*>(vbase + (size_t)(k0 + k) * hd + e) : make_float4(0.f, 0.f, 0.f, 0.f);
     float* d = vs + k * (hd + 1) + e;
     d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     vm = max(vm, mag4(v));
+    odd = odd || !finite(v);
   }
   km = block_max(km, red);
   vm = block_max(vm, red);
+  odd = __syncthreads_or(odd);
   float kf, kback, vf, vback;
   scale_of(km, kf, kback);
   scale_of(vm, vf, vback);
   const size_t at = (size_t)blockIdx.y * s.tiles + tile;
   if (tid == 0) {
-    s.factor[2 * at] = kback * (p.scale * 1.44269504088896341f);  // scores in powers of two
+    s.factor[2 * at] = odd ? __int_as_float(0x7fc00000) : kback * (p.scale * 1.44269504088896341f);  // scores in powers of two
     s.factor[2 * at + 1] = vback * (1.0f / 16384.0f);
   }
   const uint32_t piece = s.blocks * (kKeys * 128);
@@ -131,8 +136,8 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const AttnPar
     for (int h = 0; h < 2; ++h) {
       const uint32_t e = 8 * c + 4 * h;
       const float4 v = k < nk && e < hd ? key4(k, e) : make_float4(0.f, 0.f, 0.f, 0.f);
-      split2_any(v.x * kf, v.y * kf, hi[2 * h], lo[2 * h]);
-      split2_any(v.z * kf, v.w * kf, hi[2 * h + 1], lo[2 * h + 1]);
+      split2(v.x * kf, v.y * kf, hi[2 * h], lo[2 * h]);
+      split2(v.z * kf, v.w * kf, hi[2 * h + 1], lo[2 * h + 1]);
     }
     unsigned char* dst = kd + (c >> 3) * (kKeys * 128) + k * 128 + (((c ^ k) & 7u) << 4);
     *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -145,7 +150,7 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const AttnPar
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       const float a = r < hd ? vs[(8 * c + 2 * h) * (hd + 1) + r] : 0.0f, d = r < hd ? vs[(8 * c + 2 * h + 1) * (hd + 1) + r] : 0.0f;
-      split2_any(a * vf, d * vf, hi[h], lo[h]);
+      split2(a * vf, d * vf, hi[h], lo[h]);
     }
     unsigned char* dst = vdst + r * 128 + (((c ^ r) & 7u) << 4);
     *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -223,6 +228,50 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
   unsigned long long r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
+}
+
+// The rows of a CTA again where its tiles hold infinities or NaN: a warp per row, a key at a time, in f32.
+__device__ void rows_in_f32(const AttnParams& p, uint32_t b, uint32_t kvh, uint32_t rep, uint32_t past, uint32_t q0, uint32_t nq, uint32_t first, uint32_t step) {
+  constexpr int kMost = 6;  // elements of a head per lane: heads above 192 are not taken
+  const uint32_t lane = threadIdx.x & 31u, hd = p.hd;
+  const float* kbase = p.kcache + ((size_t)b * p.KV + kvh) * p.cap * hd;
+  const float* vbase = p.vcache + ((size_t)b * p.KV + kvh) * p.cap * hd;
+  for (uint32_t r = first; r < nq * rep; r += step) {
+    const size_t token = (size_t)b * p.T + q0 + r / rep;
+    const uint32_t head = kvh * rep + r % rep;
+    float q[kMost], o[kMost], m = -INFINITY, l = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kMost; ++j) {
+      const uint32_t e = lane + 32u * j;
+      q[j] = e < hd ? p.q[token * p.q_ld + (size_t)head * hd + e] : 0.0f;
+      o[j] = 0.0f;
+    }
+    for (uint32_t k = 0; k <= past + q0 + r / rep; ++k) {
+      float a = 0.0f;
+#pragma unroll
+      for (int j = 0; j < kMost; ++j) {
+        const uint32_t e = lane + 32u * j;
+        if (e < hd) a = fmaf(q[j], kbase[(size_t)k * hd + e], a);
+      }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, off);
+      a *= p.scale;
+      if (a == -INFINITY) continue;
+      const float m_new = fmaxf(m, a), corr = m == -INFINITY ? 0.0f : expf(m - m_new), pr = expf(a - m_new);
+      l = fmaf(l, corr, pr);
+      m = m_new;
+#pragma unroll
+      for (int j = 0; j < kMost; ++j) {
+        const uint32_t e = lane + 32u * j;
+        if (e < hd) o[j] = fmaf(pr, vbase[(size_t)k * hd + e], o[j] * corr);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kMost; ++j) {
+      const uint32_t e = lane + 32u * j;
+      if (e < hd) p.out[token * p.out_ld + (size_t)head * hd + e] = o[j] / l;
+    }
+  }
 }
 
 // Tensor memory: scores [2][64 columns], probabilities (hi 32 columns, lo 32), weighted values.
@@ -370,8 +419,8 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
         const uint32_t e = 4 * (lane + 32 * j);
         if (e < s.blocks * 64) {
           uint2 hi, lo2;
-          split2_any(v[j].x * f, v[j].y * f, hi.x, lo2.x);
-          split2_any(v[j].z * f, v[j].w * f, hi.y, lo2.y);
+          split2(v[j].x * f, v[j].y * f, hi.x, lo2.x);
+          split2(v[j].z * f, v[j].w * f, hi.y, lo2.y);
           unsigned char* dst = smem + (e >> 6) * (kRows * 128) + r * 128 + ((((e & 63u) >> 3) ^ (r & 7u)) << 4) + (e & 4u) * 2u;
           *reinterpret_cast<uint2*>(dst) = hi;
           *reinterpret_cast<uint2*>(dst + q_piece) = lo2;
@@ -388,6 +437,7 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
     const uint32_t qpos = past + q0 + min(qi, nq - 1u);  // the last key this row's query sees (rows without a query: any)
     const uint32_t lanes = (quarter * 32u) << 16;
     float m_run = -INFINITY, l_run = 0.0f, corr_prev = 0.0f, vf_prev = 0.0f;
+    bool odd = false;  // a tile's factor was NaN: the same for the whole CTA
     unsigned long long sums[OC / 2];  // pairs of columns
 #pragma unroll
     for (int j = 0; j < OC / 2; ++j) sums[j] = 0ull;
@@ -419,6 +469,7 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
     for (uint32_t i = 0; i < ntiles; ++i) {
       const uint32_t sb = i & 1u, key0 = i * kKeys + cp * SC;  // this thread's first key
       const float2 cur = fac;
+      odd = odd || cur.x != cur.x;
       if (i + 1 < ntiles) fac = *reinterpret_cast<const float2*>(factor + 2 * (i + 1));
       wait(&s_full[sb], (i >> 1) & 1u);
       float sc[SC];
@@ -486,7 +537,9 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
     for (int c = 0; c < CS; ++c) l += s_max[0][c][row];
 #pragma unroll
     for (int j = 0; j < OC; ++j) o[j] = __uint_as_float((uint32_t)(sums[j / 2] >> (32 * (j & 1))));
-    if (!over && !s_abort && row < qt * rep && qi < nq) {
+    if (odd) {
+      if (!over && !s_abort) rows_in_f32(p, b, kvh, rep, past, q0, nq, (uint32_t)(warp - kControl), kSoftWarps);
+    } else if (!over && !s_abort && row < qt * rep && qi < nq) {
       const size_t token = (size_t)b * p.T + q0 + qi;
       const uint32_t c0 = cp * OC;
       const float inv = 1.0f / l;

@@ -287,6 +287,61 @@ def test_scores_of_minus_infinity(dev, hd):
         assert np.abs(np.concatenate(got) - want).max() <= 1e-4 * np.abs(want).max(), n
 
 
+def _orthogonal_tokens(dev, hd, inf_keys, inf_values):
+    """A GPT-2 whose tokens are rows of a Hadamard matrix, so that LayerNorm makes them +-1 and their products with each other are 0 exactly.  Keys are 0
+    but for token 5's, and queries negative; token 5 has keys of +inf (scores of -inf), token 6 values of inf in a few columns."""
+    d, V, rng = 256, 40, np.random.default_rng(hd)
+    h = np.ones((1, 1))
+    while len(h) < d:
+        h = np.block([[h, h], [h, -h]])
+    h = h[1:V + 1]  # rows of sum 0
+    gm = nn.GPT2(dev, nn.GPT2Config(V, 500, d, 1, d // hd))
+    q, v = -h.T @ (0.5 + rng.random((V, d))) / d, h.T @ rng.standard_normal((V, d)) / d
+    k = np.outer(h[5], np.full(d, 3e38)) if inf_keys else np.zeros((d, d))
+    if inf_values:
+        v[:, ::16] = np.outer(h[6], np.full(d // 16, 3e38))
+    for t, f in {7: np.concatenate([q, k, v], 1), 8: rng.standard_normal((d, d)) / 4, 9: rng.standard_normal((d, 4 * d)) / 16, 10: rng.standard_normal((4 * d, d)) / 32,
+                 11: np.zeros(3 * d), 12: np.zeros(d), 13: np.zeros(4 * d), 14: np.zeros(d), 0x10000000: 1024 * h, 0x10000002: np.zeros((500, d)), 0x40000000: np.ones(d),
+                 0x40000001: np.zeros(d), 0x50000000: np.ones(d), 0x51000000: np.zeros(d), 0x52000000: np.ones(d), 0x53000000: np.zeros(d)}.items():
+        gm.set_f32(t, f.astype(np.float32))
+    gm.quantize_int8()
+    return gm, rng.permutation([t for t in range(V) if t not in (5, 6)])
+
+
+@pytest.mark.parametrize("n", [60, 130, 300])
+@pytest.mark.parametrize("hd", [32, 128])
+def test_infinite_keys_weigh_nothing(dev, hd, n):
+    """Token 5's scores are -inf: the other rows, of prompts and of steps, are those of the sequence without it."""
+    gm, others = _orthogonal_tokens(dev, hd, True, False)
+    ids = np.resize(others, n).astype(np.int32)
+    want = gm.forward_cached(ids[None], all_positions=True)[0]
+    assert np.isfinite(want).all()
+    for at in ([0], [7, 40], [0, 1, 2, 33, min(64, n - 10), n - 5]):
+        at = np.array(at)
+        with5 = np.insert(ids, at, 5)
+        rows = np.delete(np.arange(len(with5)), at + np.arange(len(at)))
+        gm.cache_clear()
+        got = [gm.forward_cached(with5[None, :-3], all_positions=True)[0]] + [gm.forward_cached(with5[None, i:i + 1]) for i in range(len(with5) - 3, len(with5))]
+        assert np.abs(np.concatenate(got)[rows] - want).max() <= 1e-4 * np.abs(want).max(), at
+
+
+@pytest.mark.parametrize("n", [60, 130, 300])
+@pytest.mark.parametrize("hd", [32, 128])
+def test_infinite_values_reach_only_the_rows_that_see_them(dev, hd, n):
+    gm, others = _orthogonal_tokens(dev, hd, False, True)
+    ids = np.resize(others, n).astype(np.int32)
+    want = gm.forward_cached(ids[None], all_positions=True)[0]
+    assert np.isfinite(want).all()
+    for at in (50, n - 1):
+        ids6 = ids.copy()
+        ids6[at] = 6
+        gm.cache_clear()
+        got = gm.forward_cached(ids6[None], all_positions=True)[0]
+        seen = at if n > 95 else at // 64 * 64  # (the kernel of short prompts multiplies weights of 0 within a tile of queries)
+        assert np.abs(got[:seen] - want[:seen]).max(initial=0.0) <= 1e-4 * np.abs(want).max() and not np.isfinite(got[at:]).all(-1).any(), at
+        assert not np.isfinite(gm.forward_cached(ids[None, :1])).any()
+
+
 def test_errors_mirror_the_reference_asserts(dev):
     _, gm = build(dev, llama_cfg(**dict(TINY_LLAMA, max_pos=8)), 5, 8)
     with pytest.raises(nn.RuaiError, match="exceeds max_position_embeddings"):
