@@ -576,7 +576,7 @@ constexpr uint32_t kFromTokens = 96;
 
 // 1: launched; 0: this shape is not taken; < 0: error.  `p`: as ruai_attention_prefill has completed it.
 int ruai_attention_prefill_tc(ruai_ctx* c, const AttnParams& p, uint32_t B, uint32_t rep) {
-  if (!p.pieces || p.T < kFromTokens || rep > 64) return 0;
+  if (!c->use_tc || !p.pieces || p.T < kFromTokens || rep > 64) return 0;
   if (p.maps != 1 || p.window || p.keep || p.vd != p.hd || p.vd_out != p.hd || p.out_dtype != RUAI_F32 || p.k_pos || p.sink || p.gate) return 0;
   Pieces s = {};
   s.rep = rep;

@@ -34,7 +34,7 @@ struct ruai_ctx {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool use_pdl = true;  // programmatic dependent launch between consecutive kernels
   bool use_bulk = true; // bulk-copy staged GEMV (gemv_bulk.cu) where the weight allows it
-  bool use_tc = true;   // tensor-core GEMV (gemv_tc.cu, gemv_tc8.cu) for chunk-layout weights and up to 16 rows
+  bool use_tc = true;   // tensor-core kernels of chunk-layout weights (GEMVs, GEMM), the dot-product GEMV, prompts' attention (RUAI_B200_TC=0: none of them)
   unsigned force_splits = 0;  // debug: overrides the split-K choice of the tensor-core GEMVs (0 = automatic)
   unsigned force_cols = 0, force_rows = 0;  // debug: the same for the prefill GEMM's tile
   unsigned long long* trace = nullptr;  // debug: per-launch [first entry, first past the dependency wait, last exit] in ns

@@ -84,3 +84,12 @@ def test_steps_over_a_long_capacity_repeat_those_over_a_short_one(dev, B, H, KV,
         out.append([m.forward_cached(ids[:, :40])] + [m.forward_cached(ids[:, t:t + 1]) for t in range(40, 80)] + [m.forward_cached(ids[:, 80:83])])
     for a, b in zip(*out):
         assert np.abs(a - b).max() <= 1e-5 * np.abs(a).max()
+
+
+def test_the_tensor_cores_can_be_turned_off_for_prompts(monkeypatch):
+    monkeypatch.setenv("RUAI_B200_TC", "0")
+    dev = nn.Device(0)
+    m = llama(dev)
+    names = kernels(dev, lambda: prompt(m, np.zeros((1, 200), np.int32)))
+    assert any("attention_prefill_kernel" in n for n in names) and not any("_tc" in n for n in names), names
+    m.close()
