@@ -17,8 +17,6 @@
 // Number of SMs of the target part; grids are sized in multiples of it.
 constexpr int kSmCountB200 = 148;
 
-constexpr uint32_t kPinnedWords = 1024;
-
 struct ruai_ctx {
   int ordinal = 0;
   cudaStream_t stream = nullptr;
@@ -40,7 +38,6 @@ struct ruai_ctx {
   unsigned long long* trace = nullptr;  // debug: per-launch [first entry, first past the dependency wait, last exit] in ns
   unsigned trace_slots = 0, trace_seq = 0;
   int* status = nullptr;  // device word: 0 ok, 3 / 4 = a bounded wait inside a kernel ran out (mbarrier / grid barrier), 5 = cache position out of range
-  int32_t* pinned = nullptr;  // kPinnedWords words of pinned host memory: what a step leaves for the host
   unsigned long long launches = 0;
   // persistent kernels (pstep.cu)
   unsigned spin_limit = 1u << 20;  // polls of a bounded device-side wait (about a second)

@@ -63,11 +63,6 @@ RUAI_API int ruai_ctx_create(int ordinal, void* stream_or_null, ruai_ctx** out) 
     delete c;
     return ruai_fail(nullptr, RUAI_ERR_CUDA, "cannot allocate the status word");
   }
-  if (cudaHostAlloc(&c->pinned, kPinnedWords * sizeof(int32_t), cudaHostAllocDefault) != cudaSuccess) {
-    cudaFree(c->status);
-    delete c;
-    return ruai_fail(nullptr, RUAI_ERR_CUDA, "cannot allocate pinned memory");
-  }
   int rc = ruai_ctx_reserve(c, kScratchBytes, 4096);
   if (rc != RUAI_OK) { g_ruai_global_err = c->err; delete c; return rc; }
   if (!block_pool::attach(c, ordinal, c->stream)) {
@@ -86,7 +81,6 @@ RUAI_API int ruai_ctx_destroy(ruai_ctx* c) {
   cudaFree(c->partial);
   cudaFree(c->counters);
   cudaFree(c->status);
-  cudaFreeHost(c->pinned);
   cudaFree(c->ps_sync);
   cudaFree(c->sample_buf);
   cudaEventDestroy(c->ev0);

@@ -317,11 +317,14 @@ int stage_fill(ruai_model* m, uint64_t id, float v) {
   return ruai_fill_dev(m->ctx, b->as<float>(), s.rows * s.cols, v);
 }
 
+constexpr uint32_t kPinnedWords = 1024;
+
 int finish_create(ruai_model* m) {
   ruai_ctx* c = m->ctx;
   m->layers.resize(m->L);
   RUAI_TRY(m->d_len.alloc(c, sizeof(int32_t)));
   RUAI_TRY(m->d_err.alloc(c, sizeof(int32_t)));
+  RUAI_CUDA(c, cudaHostAlloc((void**)&m->pinned, kPinnedWords * sizeof(int32_t), cudaHostAllocDefault));
   RUAI_CUDA(c, cudaMemsetAsync(m->d_len.p, 0, sizeof(int32_t), c->stream));
   RUAI_CUDA(c, cudaMemsetAsync(m->d_err.p, 0, sizeof(int32_t), c->stream));
   if (m->llama) {
@@ -595,10 +598,10 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
 int pstep_reset(ruai_model* m);
 
 // Waits for the step; its error words and the first n token ids come back with it, through pinned memory, so that the host waits once:
-// a copy into pageable memory is a wait of its own.
+// a copy into pageable memory is a wait of its own.  (The model's own: models of one context may be stepped by several threads.)
 int read_back(ruai_model* m, int32_t* ids_host, uint32_t n) {
   ruai_ctx* c = m->ctx;
-  int32_t* h = c->pinned;  // the model's error word, the context's, the ids
+  int32_t* h = m->pinned;  // the model's error word, the context's, the ids
   const bool staged = n + 2 <= kPinnedWords;
   RUAI_CUDA(c, cudaMemcpyAsync(h, m->d_err.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   RUAI_CUDA(c, cudaMemcpyAsync(h + 1, c->status, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
@@ -847,6 +850,7 @@ RUAI_API int ruai_model_destroy(ruai_model* m) {
                     &m->hbuf, &m->xl, &m->logits, &m->attn_scratch, &m->attn_counters, &m->sumsq, &m->arg_slots, &m->arg_counter})
     b->release();
   m->d_rows.release();
+  cudaFreeHost(m->pinned);
   hybrid_destroy(m);
   delete m;
   return RUAI_OK;

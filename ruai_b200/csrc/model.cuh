@@ -86,6 +86,7 @@ struct ruai_model {
   // device state
   DevBuf d_ids, d_rows, d_len, d_err, x, xn, qkv, att, hbuf, xl, logits, attn_scratch, attn_counters, sumsq, arg_slots, arg_counter;
   uint32_t act_rows = 0, logit_rows = 0;
+  int32_t* pinned = nullptr;  // kPinnedWords words of pinned host memory: what a step leaves for the host
   // decode graph
   cudaGraphExec_t graph = nullptr;
   uint32_t graph_B = 0, graph_cap = 0, graph_launches = 0;

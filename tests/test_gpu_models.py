@@ -342,6 +342,33 @@ def test_infinite_values_reach_only_the_rows_that_see_them(dev, hd, n):
         assert not np.isfinite(gm.forward_cached(ids[None, :1])).any()
 
 
+def test_models_of_one_context_in_threads(dev):
+    """Each gets its own ids back: what a step leaves for the host is the model's, not the context's."""
+    import threading
+    models = [build(dev, llama_cfg(**dict(TINY_LLAMA, V=V, max_pos=160)), seed, 8)[1] for seed, V in ((5, 41), (6, 37), (7, 39), (8, 43), (9, 35), (10, 33))]
+    first = np.arange(4, dtype=np.int32).reshape(4, 1)
+
+    def steps(m):
+        out = []
+        for _ in range(30):
+            m.cache_clear()
+            m.forward_cached(first, want_logits=False)
+            out += [m.decode_step(4) for _ in range(150)]
+        return np.array(out)
+
+    want, got = [steps(m) for m in models], [None] * len(models)
+
+    def work(i):
+        got[i] = steps(models[i])
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(models))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
 def test_errors_mirror_the_reference_asserts(dev):
     _, gm = build(dev, llama_cfg(**dict(TINY_LLAMA, max_pos=8)), 5, 8)
     with pytest.raises(nn.RuaiError, match="exceeds max_position_embeddings"):
