@@ -664,8 +664,8 @@ Shape shape_of(const ruai_ctx* c, const ruai_qweight* w, uint32_t m) {
 
 }  // namespace gemv_dot
 
-// One row of int4 whose columns are a multiple of four, and of int8: always.  Others of int4 are served by f32 multiply-adds (gemv.cu), whose
-// error is below that of 23 bits.  Several rows: as long as the dp4a of all of them cost less than the tensor cores' fixed parts, which is with short k
+// One row of int4 whose columns are a multiple of four, and of int8 with k up to 32768.  Others are served by f32 multiply-adds (gemv.cu, gemv_bulk.cu),
+// which keep what a block of one exponent rounds away.  Several rows: as long as the dp4a of all of them cost less than the tensor cores' fixed parts, which is with short k
 // (digits for all of k have to be made first) and few weights.  Us of a launch, here | gemv_tc.cu or gemv_tc8.cu:
 //   int4, 2 rows: 576 x 576 2.5 | 3.8, 768 x 3072 2.8 | 4.4;  2048 x 2560 4.6 | 4.8, 3072 x 768 5.2 | 4.6, 5632 x 2048 8.2 | 6.9
 //   int4, 4 rows: 576 x 576 3.2 | 5.0, 768 x 3072 3.7 | 5.5, 1536 x 576 4.0 | 5.2;  2048 x 2048 6.0 | 5.8, 3072 x 768 8.2 | 5.6
@@ -677,6 +677,7 @@ bool ruai_gemv_dot_takes(const ruai_ctx* c, const ruai_qweight* w, uint32_t m) {
   using namespace gemv_dot;
   if (!c->use_bulk || !c->use_tc || w->layout != QL_CHUNK16 || m == 0) return false;
   if (w->bits == 4 && (w->group != 32 || w->n % 4)) return false;
+  if (w->bits == 8 && w->k > 32768) return false;
   if (m > 1 && (m > 16 || w->k > 1536 || (uint64_t)w->k * w->n > (5u << 19))) return false;
   if (m > 2 && w->bits == 8 && w->n > 16u * (uint32_t)c->sm_count) return false;
   return shape_of(c, w, m).smem <= kSmemMax;

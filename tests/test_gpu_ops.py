@@ -415,6 +415,21 @@ def test_few_rows_against_float64(dev, k, n, rows, bits, dtype):
         assert (np.abs(got - want) <= bound).all(), (m, (np.abs(got - want) / bound).max())
 
 
+@pytest.mark.parametrize("k", [32769, 40000])
+def test_long_rows_of_int8_stay_f32(dev, k):
+    """Beyond k = 32768 the activations are multiplied as they are: small ones beside a large one whose weights are zero are not lost."""
+    n = 64
+    rng = np.random.default_rng(k)
+    q = rng.integers(1, 128, (k, n)).astype(np.int8)
+    q[::128] = 0
+    s = np.full(n, 0.01, np.float32)
+    x = np.ones((1, k), np.float32)
+    x[0, ::128] = 2.0 ** 30
+    _, got = run_matmul(dev, x, nn.QWeight.int8(dev, q, s), "f32", None)
+    want = x.astype(np.float64) @ (q.astype(np.float64) * s)
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
 # ---- the GEMM's tiles: edges of rows, columns and k, every split of k ----
 
 @pytest.mark.parametrize("bits", [8, 4])
