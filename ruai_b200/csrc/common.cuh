@@ -216,7 +216,7 @@ struct GemvEpilogue {
 // rstd = 1/sqrt(sum(x^2) * (1/k) + eps), the sum given as per-tile partial sums [tiles][m].
 struct GemvPrologue {
   const float* norm_w = nullptr;  // f32 [k]; NULL: x is used as it is
-  const float* norm_b = nullptr;  // f32 [k]: LayerNorm (functional.rs:137-146) in the place of RMSNorm; gemv_dot.cu only
+  const float* norm_b = nullptr;  // f32 [k]: LayerNorm (functional.rs:137-146) in the place of RMSNorm; gemv_dot.cu only, ruai_gemv_launch refuses it elsewhere
   const float* sumsq = nullptr;
   uint32_t tiles = 0;
   float eps = 0.0f;

@@ -381,6 +381,7 @@ int ruai_gemv_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x_dt
     return ruai_dense_launch(c, &d, 1, x_dtype, m);
   }
   if (ruai_gemv_dot_takes(c, w, m)) return ruai_gemv_dot_launch(c, w, x, x_dtype, x_ld, m, out, epi_in, pro);
+  if (pro.norm_b) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "LayerNorm in the prologue of %u rows of a %u x %u Linear", m, w->k, w->n);
   if (ruai_gemm_tc_takes(c, w, m, epi_in))
     return ruai_gemm_tc_launch(c, w, x, x_dtype, x_ld, m, out, epi_in, pro);
   if (c->use_bulk && c->use_tc && ruai_gemv_wide_eligible(c, w, m)) return ruai_gemv_wide_launch(c, w, x, x_dtype, x_ld, m, out, epi_in, pro);
