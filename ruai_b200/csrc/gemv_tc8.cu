@@ -418,20 +418,8 @@ cudaError_t launch_one(ruai_ctx* c, const Params& p, dim3 grid, uint32_t slice_k
 
 }  // namespace gemv_tc8
 
-bool ruai_gemv_tc8_eligible(const ruai_qweight* w, uint32_t m) {
-  return w->layout == QL_CHUNK16 && w->bits == 8 && m >= 1 && m <= 16 && w->k <= 8u * (uint32_t)gemv_tc8::kMaxSliceK;
-}
-
-int ruai_gemv_tc8_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x_dtype, uint32_t x_ld, uint32_t m, void* out,
-                         const GemvEpilogue& epi_in, const GemvPrologue& pro) {
-  using namespace gemv_tc8;
-  GemvEpilogue epi = epi_in;
-  if (epi.act == ACT_SWIGLU && (w->n & 1)) return ruai_fail(c, RUAI_ERR_SHAPE, "SwiGLU epilogue needs an even column count, got %u", w->n);
-  if (epi.out_ld == 0) epi.out_ld = epi.act == ACT_SWIGLU ? w->n / 2 : w->n;
-  if (epi.sumsq && epi.act == ACT_SWIGLU) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "sum of squares with the SwiGLU epilogue");
-  const int mt = m <= 2 ? 2 : m <= 4 ? 4 : 8;
-  const uint32_t row_tiles = (m + mt - 1) / mt;
-  if (epi.argmax_out && (row_tiles != 1 || epi.act == ACT_SWIGLU)) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "fused argmax needs a single row tile");
+namespace gemv_tc8 {
+uint32_t choose(const ruai_ctx* c, const ruai_qweight* w, int mt, uint32_t row_tiles) {  // the split of k
   const uint32_t col_tiles = (w->n + kCols - 1) / kCols;
   // the slice of k per CTA is bounded (digit buffer, 32-bit sums); beyond that, split over a cluster
   uint32_t splits = 1;
@@ -448,7 +436,37 @@ int ruai_gemv_tc8_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int 
     const double t = waves * (6.0 + 0.4 * stages + 0.15 * s2);
     if (t < best) { best = t; best_s = s2; }
   }
-  splits = best_s;
+  return best_s;
+}
+}  // namespace gemv_tc8
+
+double ruai_gemv_tc8_row_us(const ruai_ctx* c, const ruai_qweight* w) {
+  using namespace gemv_tc8;
+  const uint32_t splits = choose(c, w, 1, 1), ctas = (w->n + kCols - 1) / kCols * splits;
+  const uint32_t per = (w->chunks + splits - 1) / splits, stages = (per + kStageChunks - 1) / kStageChunks, slice_k = stages * kStageChunks * 16;
+  const size_t bytes = slice_k >= 4096 ? Smem<1, kStagesLong>::bytes(slice_k, splits) : Smem<1, kStagesShort>::bytes(slice_k, splits);
+  const uint32_t places = ruai_cluster_places(c, (uint32_t)std::max<size_t>(1, std::min<size_t>(3, 228 * 1024 / (bytes + 1024))), splits);
+  const double on_sm = (ctas + c->sm_count - 1) / c->sm_count, waves = (ctas + places - 1) / places;
+  const double t = (2.5 + stages * std::max(0.39, 0.083 * on_sm) + 0.62 * on_sm) * (waves > 1 ? 0.88 * waves : 1.0);
+  return std::max(t, 0.18e-6 * w->k * w->n);
+}
+
+bool ruai_gemv_tc8_eligible(const ruai_qweight* w, uint32_t m) {
+  return w->layout == QL_CHUNK16 && w->bits == 8 && m >= 1 && m <= 16 && w->k <= 8u * (uint32_t)gemv_tc8::kMaxSliceK;
+}
+
+int ruai_gemv_tc8_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x_dtype, uint32_t x_ld, uint32_t m, void* out,
+                         const GemvEpilogue& epi_in, const GemvPrologue& pro) {
+  using namespace gemv_tc8;
+  GemvEpilogue epi = epi_in;
+  if (epi.act == ACT_SWIGLU && (w->n & 1)) return ruai_fail(c, RUAI_ERR_SHAPE, "SwiGLU epilogue needs an even column count, got %u", w->n);
+  if (epi.out_ld == 0) epi.out_ld = epi.act == ACT_SWIGLU ? w->n / 2 : w->n;
+  if (epi.sumsq && epi.act == ACT_SWIGLU) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "sum of squares with the SwiGLU epilogue");
+  const int mt = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : 8;
+  const uint32_t row_tiles = (m + mt - 1) / mt;
+  if (epi.argmax_out && (row_tiles != 1 || epi.act == ACT_SWIGLU)) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "fused argmax needs a single row tile");
+  const uint32_t col_tiles = (w->n + kCols - 1) / kCols;
+  uint32_t splits = choose(c, w, mt, row_tiles);
   if ((c->force_splits & 255u) && (c->force_splits & 255u) >= splits && (c->force_splits & 255u) <= 8) splits = c->force_splits & 255u;
   uint32_t cpc = (w->chunks + splits - 1) / splits;
   cpc = (cpc + kStageChunks - 1) / kStageChunks * kStageChunks;
@@ -461,7 +479,8 @@ int ruai_gemv_tc8_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int 
   p.pro.trace = ruai_trace_slot(c);
   const dim3 grid(col_tiles, splits, row_tiles);
   const bool deep = mt <= 2 && slice_k >= 4096;  // a long slice of k and a small digit buffer: the deeper ring pays
-  cudaError_t e = mt == 2 ? (deep ? launch_one<2, kStagesLong>(c, p, grid, slice_k) : launch_one<2, kStagesShort>(c, p, grid, slice_k))
+  cudaError_t e = mt == 1 ? (deep ? launch_one<1, kStagesLong>(c, p, grid, slice_k) : launch_one<1, kStagesShort>(c, p, grid, slice_k))
+                : mt == 2 ? (deep ? launch_one<2, kStagesLong>(c, p, grid, slice_k) : launch_one<2, kStagesShort>(c, p, grid, slice_k))
                 : mt == 4 ? launch_one<4, kStagesShort>(c, p, grid, slice_k) : launch_one<8, kStagesShort>(c, p, grid, slice_k);
   if (e != cudaSuccess) return ruai_fail(c, RUAI_ERR_CUDA, "int8 tensor-core gemv launch failed: %s", cudaGetErrorString(e));
   return RUAI_OK;

@@ -133,6 +133,7 @@ static int make_qweight(ruai_ctx* c, const int8_t* q, const float* scale, uint32
   else if (group == 32) { w->layout = QL_CHUNK16; w->chunks = k / 32; }
   else { w->layout = QL_REFERENCE; w->chunks = 0; }
   w->data_bytes = w->layout == QL_CHUNK16 ? (size_t)w->chunks * n * 16 : q_bytes;
+  w->row_tc = ruai_gemv_row_tc(c, w);
   if (w->chunks > 65535) { delete w; return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "repack: k = %u too large", k); }
   void *qd = nullptr, *sd = nullptr;
   bool qo = false, so = false;

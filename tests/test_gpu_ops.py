@@ -393,7 +393,7 @@ def test_lora_forward_matches_checker(dev, m, k, n, rank, bits):
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("k,n,rows", [(32, 4, (1, 2, 8)), (64, 8, (1, 3, 16)), (96, 36, (1, 4, 9)), (544, 132, (1, 2, 3, 4, 8, 13, 16)), (1056, 1300, (1, 2, 5, 16)),
-                                      (1536, 1664, (2, 4, 8, 16)), (2080, 2500, (1,)), (4128, 4900, (1,)), (4096, 4736, (1,)), (14336, 96, (1,))])
+                                      (1536, 1664, (2, 4, 8, 16)), (2080, 2500, (1,)), (4128, 4900, (1,)), (4096, 4736, (1,)), (14336, 96, (1,)), (512, 28672, (1,))])
 def test_few_rows_against_float64(dev, k, n, rows, bits, dtype):
     """x is rounded to half of 2^-22 (int8: 2^-27) of the largest magnitude of its block of 32 (128) at the most, the sums are f32: errors
     below that, summed over the block's weights, and 2^-20 of the sum of the products' magnitudes."""

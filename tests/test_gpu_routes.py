@@ -93,3 +93,15 @@ def test_the_tensor_cores_can_be_turned_off_for_prompts(monkeypatch):
     names = kernels(dev, lambda: prompt(m, np.zeros((1, 200), np.int32)))
     assert any("attention_prefill_kernel" in n for n in names) and not any("_tc" in n for n in names), names
     m.close()
+
+
+@pytest.mark.parametrize("bits,k,n,tc", [(8, 2048, 2048, False), (8, 1024, 19456, True), (8, 4096, 5120, True), (4, 4096, 4096, False), (4, 512, 28672, True)])
+def test_one_row_by_itself_runs_on_the_shorter_kernel(dev, bits, k, n, tc):
+    if bits == 8:
+        w = nn.QWeight.int8(dev, np.ones((k, n), np.int8), np.ones(n, np.float32))
+    else:
+        w = nn.QWeight.int4(dev, np.full((k // 2, n), 0x11, np.int8), np.ones((k // 32, n), np.float32), 32)
+    x = nn.Tensor.from_numpy(dev, np.ones((1, k), np.float32))
+    names = kernels(dev, lambda: nn._matmul_q(x, w))
+    assert any("gemv_tc" in name for name in names) == tc and any("row_kernel" in name for name in names) != tc, names
+    assert np.array_equal(nn._matmul_q(x, w).numpy(), np.full((1, n), float(k), np.float32))
