@@ -579,7 +579,8 @@ double warps_us(const ruai_ctx* c, uint64_t items, uint32_t rep, uint32_t hd, ui
 //   8 key heads of 128 with 4 query heads each: 1 sequence, 1024 positions 9.0 | 9.2, 8192 31 | 40, 32768 91 | 160; 16 sequences, 256 20 | 13,
 //   1024 42 | 47, 4096 129 | 163;  4 of 64 with 8 each: 1 sequence, 1024 10.2 | 10.7, 32768 77 | 101; 64 sequences, 256 36 | 19, 1024 126 | 65;
 //   3 of 64 with 3 each: 1 sequence, 8192 14 | 21; 64 sequences, 256 12.5 | 9.1, 4096 106 | 89;  12 of 64: 64 sequences, 1024 66 | 77
-// Up to 64 positions chunks always: one for all keys, and a CTA's warps share its arithmetic (4 of 64 with 8 each 6.7 | 8.3).
+// Up to 64 positions chunks, one for all keys, whose arithmetic a CTA's warps share (4 of 64 with 8 each 6.7 | 8.3); but with one or two query heads
+// per key a step is 0.4 to 1.3 us a layer shorter on warps, up to some 500 items (32 sequences of 16 heads: 1.9 longer).
 AttnPlan ruai_attention_plan(const ruai_ctx* c, uint32_t B, uint32_t T, uint32_t KV, uint32_t rep, uint32_t hd, uint32_t cap) {
   AttnPlan plan;
   const uint64_t items = (uint64_t)B * KV * T;
@@ -588,7 +589,10 @@ AttnPlan ruai_attention_plan(const ruai_ctx* c, uint32_t B, uint32_t T, uint32_t
   if (T > 1) plan.splits = 1;
   else if (items >= 512) plan.splits = std::max(1u, std::min(by_len, 2u));
   else plan.splits = std::max(1u, std::min(B >= 5 ? (by_len + 1) / 2 : by_len, 64u));
-  if (cap <= 64) return plan;
+  if (cap <= 64) {
+    if (rep <= 2 && items < 512) { plan.warps = 4; plan.splits = 1; }
+    return plan;
+  }
   double best = 0.87 * chunks_us(c, items, rep, hd, cap, plan.splits) + (rep < 4 ? 1.0 : 0.0);
   for (uint32_t w = 4; w <= (uint32_t)kAttnWarps; w *= 2)
     for (uint32_t s = 1; s <= 8; s *= 2) {

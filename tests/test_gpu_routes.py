@@ -61,7 +61,7 @@ def test_long_prompts_of_quantized_decoders_use_the_tensor_cores(dev):
         assert any("attn_tc_kernel" in n for n in names) == tc and any("attention_prefill_kernel" in n for n in names) != tc, (T, names)
 
 
-@pytest.mark.parametrize("B,H,KV,hd,positions,chunks", [(1, 8, 2, 128, 8192, True), (2, 4, 1, 256, 4096, True), (1, 3, 3, 64, 40, True), (64, 16, 2, 64, 300, False),
+@pytest.mark.parametrize("B,H,KV,hd,positions,chunks", [(1, 8, 2, 128, 8192, True), (2, 4, 1, 256, 4096, True), (1, 12, 3, 64, 40, True), (1, 3, 3, 64, 40, False), (64, 16, 2, 64, 300, False),
                                                         (16, 8, 2, 128, 300, False)])
 def test_attention_of_a_step_long_caches_in_chunks(dev, B, H, KV, hd, positions, chunks):
     """Few key heads over a long cache need more CTAs than a cluster has; many sequences, whose warps work alone, do not."""
