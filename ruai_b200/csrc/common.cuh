@@ -67,7 +67,7 @@ struct ruai_qweight {
   uint8_t* data = nullptr;  // device
   float* scale = nullptr;   // device; int8 [n], int4 [k/group][n]
   size_t data_bytes = 0, scale_bytes = 0;
-  bool row_tc = false;      // a single row by itself (ruai_matmul_q) runs on the tensor-core kernels (ruai_gemv_row_tc)
+  bool row_tc = false;      // int8: a single row by itself (ruai_matmul_q) runs on the tensor cores (ruai_gemv_row_tc)
 };
 
 extern thread_local std::string g_ruai_global_err;
@@ -233,9 +233,8 @@ uint32_t ruai_gemv_tiles(const ruai_ctx* ctx, const ruai_qweight* w, uint32_t m)
 // The dot-product kernel (gemv_dot.cu): whether it runs m rows of w, and the sumsq tiles it then writes.  It works the norm of its
 // input out by itself (the prologue's sumsq is not used).
 bool ruai_gemv_dot_takes(const ruai_ctx* ctx, const ruai_qweight* w, uint32_t m);
-bool ruai_gemv_row_tc(const ruai_ctx* ctx, const ruai_qweight* w);  // whether a single row by itself is shorter on those: worked out once per weight
-// What one row takes on the tensor-core kernels, in microseconds (by the measurements that gemv_dot.cu cites).
-double ruai_gemv_tc_row_us(const ruai_ctx* ctx, const ruai_qweight* w);
+bool ruai_gemv_row_tc(const ruai_ctx* ctx, const ruai_qweight* w);  // whether a single row by itself is shorter on gemv_tc8.cu: worked out once per weight
+// What one row takes there, in microseconds (by the measurements that gemv_dot.cu cites).
 double ruai_gemv_tc8_row_us(const ruai_ctx* ctx, const ruai_qweight* w);
 // CTAs that find a place at once in clusters of `splits`, per_sm on an SM (1 to 3): clusters lie within a group of SMs and do not fill all of them.
 inline uint32_t ruai_cluster_places(const ruai_ctx* ctx, uint32_t per_sm, uint32_t splits) {

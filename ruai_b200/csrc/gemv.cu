@@ -446,8 +446,7 @@ RUAI_API int ruai_matmul_q(ruai_ctx* c, int x_dtype, const void* x, const ruai_q
   GemvEpilogue e;
   e.bias = bias;
   e.out_dtype = x_dtype;
-  if (m == 1 && w->row_tc && c->use_bulk && c->use_tc)
-    return w->bits == 8 ? ruai_gemv_tc8_launch(c, w, x, x_dtype, w->k, m, out, e, GemvPrologue()) : ruai_gemv_tc_launch(c, w, x, x_dtype, w->k, m, out, e, GemvPrologue());
+  if (m == 1 && w->row_tc && c->use_bulk && c->use_tc) return ruai_gemv_tc8_launch(c, w, x, x_dtype, w->k, m, out, e, GemvPrologue());
   return ruai_gemv_launch(c, w, x, x_dtype, w->k, m, out, e);
 }
 

@@ -21,7 +21,7 @@
 // cluster to launch and join, no tensor memory, no hand-over between warps.  Large ones: int4 the issue slots, 99 instructions of a warp per
 // 32 chunks of 16 bytes (4096 x 28672 17.4 | 22.0, 4.2 TB/s); int8 HBM's latency with four loads of a lane in flight (4096 x 28672 25.7 | 31.1,
 // 4.6 TB/s; 4096 x 128256 95 | 114, 5.5 TB/s).  Not won: long k with few columns, where the conversion of x in every
-// CTA shows, and tiles that do not share out over the SMs (192 of int8 4096 x 6144); ruai_gemv_row_tc leaves those to the other kernels.
+// CTA shows, and tiles that do not share out over the SMs (192 of int8 4096 x 6144): ruai_gemv_row_tc.
 // Two CTAs of 64 registers per SM, not one with more and eight loads ahead: alone that is the faster launch (4096 x 28672 18.9 for
 // 20.9 then), but a CTA that fills the register file keeps the next kernel's out until it ends, and with it the weights that this would
 // request: steps were 10 % slower.
@@ -662,30 +662,28 @@ Shape shape_of(const ruai_ctx* c, const ruai_qweight* w, uint32_t m) {
   return s;
 }
 
-// What one row takes, in microseconds: fitted to 426 shapes, k of 512 to 28672 and 512 to 32768 columns, in a chain of launches over weights that are
-// not in the L2 (one standard deviation 6 %, as that of the tensor-core kernels' formulas).
+// What one row of int8 takes, in microseconds: fitted to 213 shapes, k of 512 to 28672 and 512 to 32768 columns, in a chain of launches over weights that are
+// not in the L2 (one standard deviation 6 %, as that of the tensor-core kernel's formula).
 double row_us(const ruai_ctx* c, const ruai_qweight* w, const Shape& s) {
   const uint32_t sms = (uint32_t)c->sm_count, ctas = std::min(s.tiles, s.per_sm * sms);
   const double side = std::min<double>(s.per_sm, (s.tiles + sms - 1) / sms), rounds = (s.tiles + ctas - 1) / ctas;  // CTAs on an SM, tiles of a CTA
-  if (w->bits == 4)
-    return std::max(1.0 + 0.37 * s.passes * side + rounds * std::max(0.3 * s.steps + 0.64, 0.21 * s.steps * side) + 0.4 * (side - 1), 0.22e-6 * 0.625 * w->k * w->n);
   return std::max(0.37 + 0.35 * s.passes * side + rounds * std::max(0.25 * s.steps + 1.2, 0.15 * s.steps * side) + 0.65 * (side - 1), 0.19e-6 * w->k * w->n);
 }
 
 }  // namespace gemv_dot
 
-// One row by itself: the tensor-core kernels where their launch is the shorter one by the formulas, in one of six shapes: where the tiles of columns leave
-// SMs with one more than others while those kernels' CTAs all find a place.  Us, here | there:
-//   int4: 4096 x 4096 4.7 | 5.8, 4096 x 28672 17.4 | 22.0, 2048 x 11264 5.2 | 6.5;  11008 x 3072 10.3 | 9.5, 14336 x 4096 13.4 | 12.3, 28672 x 4096 24.7 | 21.9
-//   int8: 4096 x 4096 5.7 | 6.6, 4096 x 28672 25.7 | 31.1, 14336 x 2048 11.5 | 14.7;  4096 x 6144 8.3 | 7.5, 4096 x 12288 15.0 | 11.6, 11008 x 6144 20.7 | 14.8
-// Over all shapes the choice takes 0.81 (int4) and 0.79 (int8) of the tensor-core kernels' time, and 0.99 and 0.97 of this kernel's.
-// Not in a decoder's step, where the norm rides along here and a change of kernels costs their overlap: steps of the 8B shape (int8, 4 layers) 357 us, with the
-// choice 375; of the 3B shape (int4, 6 layers) 306, 315.
+// One row of int8 by itself: the tensor-core kernel where its launch is the shorter one by the formulas, in one of five shapes: where the tiles of columns
+// leave SMs with one more than others while that kernel's CTAs all find a place.  Us, here | there:  4096 x 4096 5.7 | 6.6, 4096 x 28672 25.7 | 31.1,
+// 14336 x 2048 11.5 | 14.7;  4096 x 6144 8.3 | 7.5, 4096 x 12288 15.0 | 11.6, 11008 x 6144 20.7 | 14.8.  Over all shapes the choice takes 0.79 of that
+// kernel's time and 0.97 of this one's; errors against 64 bits are equal (5.2e-8 to 9.0e-8 there, 6.5e-8 to 8.5e-8 here).
+// Not in a decoder's step, where the norm rides along here and a change of kernels costs their overlap: steps of the 8B shape (4 layers) 357 us, with the
+// choice 375.  Not int4: a few shapes are shorter on gemv_tc.cu (14336 x 4096 13.4 | 12.3, 28672 x 4096 24.7 | 21.9, 11008 x 3072 10.3 | 9.5), but its 21 bits
+// err by 1.0e-6 to 2.0e-6 where the 23 here do by 2.6e-7 to 5.1e-7.
 bool ruai_gemv_row_tc(const ruai_ctx* c, const ruai_qweight* w) {
   using namespace gemv_dot;
-  if (w->layout != QL_CHUNK16 || (w->bits == 4 && (w->group != 32 || w->n % 4)) || (w->bits == 8 && w->k > 32768)) return false;
+  if (w->layout != QL_CHUNK16 || w->bits != 8 || !ruai_gemv_tc8_eligible(w, 1)) return false;
   const Shape s = shape_of(c, w, 1);
-  return s.smem > kSmemMax || row_us(c, w, s) > (w->bits == 4 ? ruai_gemv_tc_row_us(c, w) : ruai_gemv_tc8_row_us(c, w));
+  return s.smem > kSmemMax || row_us(c, w, s) > ruai_gemv_tc8_row_us(c, w);
 }
 
 // One row of int4 whose columns are a multiple of four, and of int8 with k up to 32768.  Others are served by f32 multiply-adds (gemv.cu, gemv_bulk.cu),

@@ -1,5 +1,5 @@
 // Fused dequantize + GEMV on the tensor cores (tcgen05, accumulators in tensor memory) for
-// int4 group-32 weights and up to sixteen rows of activations (eight per CTA): what gemv_dot.cu leaves of the decode hot path.
+// int4 group-32 weights and two to sixteen rows of activations (eight per CTA): what gemv_dot.cu leaves of the decode hot path.
 //
 // Why tensor cores for a memory-bound kernel: at full HBM speed one SM has to consume about
 // 46 int4 weights per clock.  On the CUDA cores every weight costs a byte permute, a
@@ -520,15 +520,29 @@ cudaError_t launch_one(ruai_ctx* c, const Params& p, dim3 grid) {
 
 }  // namespace gemv_tc
 
-namespace gemv_tc {
-// Split k over a cluster of up to 8 CTAs.  A launch is a link in a chain of dependent kernels, so what counts is its
-// latency.  Measured on the 8B shapes, in microseconds: about 5.5 per wave of CTAs that is fixed, 0.45 per stage
-// (more with more rows) and 0.15 per CTA of the cluster for the reduction.
-struct Choice { uint32_t splits = 1, stages = 0; bool small = false; };  // small: the three-CTAs-per-SM variant
-Choice choose(const ruai_ctx* c, const ruai_qweight* w, int mt, uint32_t row_tiles) {
+bool ruai_gemv_tc_eligible(const ruai_qweight* w, uint32_t m) {
+  return w->layout == QL_CHUNK16 && w->bits == 4 && w->n % 4 == 0 && m >= 1 && m <= 16;
+}
+
+int ruai_gemv_tc_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x_dtype, uint32_t x_ld, uint32_t m, void* out,
+                        const GemvEpilogue& epi_in, const GemvPrologue& pro) {
+  using namespace gemv_tc;
+  GemvEpilogue epi = epi_in;
+  if (epi.act == ACT_SWIGLU && (w->n & 1)) return ruai_fail(c, RUAI_ERR_SHAPE, "SwiGLU epilogue needs an even column count, got %u", w->n);
+  if (epi.out_ld == 0) epi.out_ld = epi.act == ACT_SWIGLU ? w->n / 2 : w->n;
+  if (epi.sumsq && epi.act == ACT_SWIGLU) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "sum of squares with the SwiGLU epilogue");
+  if (epi.argmax_out && epi.act == ACT_SWIGLU) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "argmax with the SwiGLU epilogue");
+  // up to 8 rows per CTA; 9..16 rows run as two row tiles (the second pass over the weights mostly hits the L2)
+  const int mt = m <= 2 ? 2 : m <= 4 ? 4 : 8;
+  const uint32_t row_tiles = (m + mt - 1) / mt;
+  if (epi.argmax_out && row_tiles != 1) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "fused argmax needs a single row tile");
   const uint32_t col_tiles = (w->n + kCols - 1) / kCols;
-  const double per_stage = 0.45 * (mt == 1 ? 1.0 : mt == 2 ? 1.4 : mt == 4 ? 2.0 : 3.2);
-  Choice r;
+  // Split k over a cluster of up to 8 CTAs.  A launch is a link in a chain of dependent kernels, so what counts is its
+  // latency.  Measured on the 8B shapes, in microseconds: about 5.5 per wave of CTAs that is fixed, 0.45 per stage
+  // (more with more rows) and 0.15 per CTA of the cluster for the reduction.
+  const double per_stage = 0.45 * (mt == 2 ? 1.4 : mt == 4 ? 2.0 : 3.2);
+  uint32_t splits = 1;
+  bool small = false;  // the three-CTAs-per-SM variant
   double best = 1e30;
   for (int variant = 0; variant < (mt <= 2 ? 2 : 1); ++variant) {
     const uint32_t slots = (variant ? 3u : 2u) * (uint32_t)c->sm_count;
@@ -543,41 +557,9 @@ Choice choose(const ruai_ctx* c, const ruai_qweight* w, int mt, uint32_t row_til
       // 5.7 or 9.8 us from launch to launch; as 128 CTAs in clusters of 4 always 6.5)
       const double crowd = (s2 == 8 && (variant ? 10u * ctas > 9u * slots : 4u * ctas > 3u * slots)) ? 2.0 : 0.0;
       const double t = waves * (5.5 + per_stage * stages) + 0.15 * s2 + crowd + (variant ? 0.2 : 0.0);
-      if (t < best) { best = t; r.splits = s2; r.stages = stages; r.small = variant != 0; }
+      if (t < best) { best = t; splits = s2; small = variant != 0; }
     }
   }
-  return r;
-}
-}  // namespace gemv_tc
-
-double ruai_gemv_tc_row_us(const ruai_ctx* c, const ruai_qweight* w) {
-  const gemv_tc::Choice s = gemv_tc::choose(c, w, 1, 1);
-  const uint32_t ctas = (w->n + gemv_tc::kCols - 1) / gemv_tc::kCols * s.splits, places = ruai_cluster_places(c, s.small ? 3 : 2, s.splits);
-  const double on_sm = (ctas + c->sm_count - 1) / c->sm_count, waves = (ctas + places - 1) / places;
-  const double t = (1.8 + s.stages * std::max(0.55, 0.21 * on_sm) + 0.76 * on_sm) * (waves > 1 ? 0.88 * waves : 1.0);
-  return std::max(t, 0.24e-6 * 0.625 * w->k * w->n);
-}
-
-bool ruai_gemv_tc_eligible(const ruai_qweight* w, uint32_t m) {
-  return w->layout == QL_CHUNK16 && w->bits == 4 && w->n % 4 == 0 && m >= 1 && m <= 16;
-}
-
-int ruai_gemv_tc_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x_dtype, uint32_t x_ld, uint32_t m, void* out,
-                        const GemvEpilogue& epi_in, const GemvPrologue& pro) {
-  using namespace gemv_tc;
-  GemvEpilogue epi = epi_in;
-  if (epi.act == ACT_SWIGLU && (w->n & 1)) return ruai_fail(c, RUAI_ERR_SHAPE, "SwiGLU epilogue needs an even column count, got %u", w->n);
-  if (epi.out_ld == 0) epi.out_ld = epi.act == ACT_SWIGLU ? w->n / 2 : w->n;
-  if (epi.sumsq && epi.act == ACT_SWIGLU) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "sum of squares with the SwiGLU epilogue");
-  if (epi.argmax_out && epi.act == ACT_SWIGLU) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "argmax with the SwiGLU epilogue");
-  // up to 8 rows per CTA; 9..16 rows run as two row tiles (the second pass over the weights mostly hits the L2)
-  const int mt = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : 8;
-  const uint32_t row_tiles = (m + mt - 1) / mt;
-  if (epi.argmax_out && row_tiles != 1) return ruai_fail(c, RUAI_ERR_UNSUPPORTED, "fused argmax needs a single row tile");
-  const uint32_t col_tiles = (w->n + kCols - 1) / kCols;
-  const Choice chosen = choose(c, w, mt, row_tiles);
-  uint32_t splits = chosen.splits;
-  const bool small = chosen.small;
   uint32_t cpc = (w->chunks + splits - 1) / splits;
   cpc = (cpc + kStageGroups - 1) / kStageGroups * kStageGroups;
   Params p;
@@ -593,8 +575,7 @@ int ruai_gemv_tc_launch(ruai_ctx* c, const ruai_qweight* w, const void* x, int x
   const dim3 grid(col_tiles, splits, row_tiles);
   // few CTAs per SM: spend the free registers on a deeper weight queue
   const bool deep = !(c->force_splits & 256u);
-  cudaError_t e = mt == 1 ? (deep && !small ? launch_one<1, 4>(c, p, grid) : launch_one<1, 2>(c, p, grid))
-                : mt == 2 ? (deep && !small ? launch_one<2, 4>(c, p, grid) : launch_one<2, 2>(c, p, grid))
+  cudaError_t e = mt == 2 ? (deep && !small ? launch_one<2, 4>(c, p, grid) : launch_one<2, 2>(c, p, grid))
                 : mt == 4 ? launch_one<4, 2>(c, p, grid)
                           : launch_one<8, 2>(c, p, grid);
   if (e != cudaSuccess) return ruai_fail(c, RUAI_ERR_CUDA, "tensor-core gemv launch failed: %s", cudaGetErrorString(e));

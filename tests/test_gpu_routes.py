@@ -95,7 +95,7 @@ def test_the_tensor_cores_can_be_turned_off_for_prompts(monkeypatch):
     m.close()
 
 
-@pytest.mark.parametrize("bits,k,n,tc", [(8, 2048, 2048, False), (8, 1024, 19456, True), (8, 4096, 5120, True), (4, 4096, 4096, False), (4, 512, 28672, True)])
+@pytest.mark.parametrize("bits,k,n,tc", [(8, 2048, 2048, False), (8, 1024, 19456, True), (8, 4096, 5120, True), (4, 4096, 4096, False), (4, 14336, 4096, False)])
 def test_one_row_by_itself_runs_on_the_shorter_kernel(dev, bits, k, n, tc):
     if bits == 8:
         w = nn.QWeight.int8(dev, np.ones((k, n), np.int8), np.ones(n, np.float32))
