@@ -153,6 +153,27 @@ def test_steps_of_five_to_sixteen_sequences(dev, kind, bits, B):
     assert (got[decisive] == want[decisive]).all(), f"{kind} int{bits} B={B}: fused pick"
 
 
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("B", [2, 4, 5, 9, 16])
+def test_sums_of_squares_of_narrow_tiles_reach_wider_kernels(dev, bits, B):
+    """o_proj and down_proj of these widths run on the dot-product kernel, whose sums of squares lie in tiles of 8 to 32 columns, and the head
+    (int8, 9000 columns of 576) does not: it reads them in its prologue."""
+    om, gm = build(dev, llama_cfg(V=9000, d=576, ffn=1536, L=2, H=9, KV=3, hd=64, max_pos=64), 7, bits, 32)
+    prompts = np.stack([oracle.synth_tokens(7, 0x20000000 + b, 2, 9000) for b in range(B)])
+    lo = om.forward_cached(prompts)
+    close(lo, gm.forward_cached(prompts), "prefill")
+    for step in range(2):
+        nxt = np.array([oracle.argmax(r) for r in lo], np.int32)
+        lo = om.forward_cached(nxt[:, None])
+        close(lo, gm.forward_cached(nxt[:, None]), f"int{bits} B={B} step {step}")
+    nxt = np.array([oracle.argmax(r) for r in lo], np.int32)
+    lo = om.forward_cached(nxt[:, None])
+    got = gm.decode_step(B, nn.Tensor.from_numpy(dev, nxt).ptr)
+    srt = np.sort(lo, axis=1)
+    decisive = (srt[:, -1] - srt[:, -2]) > 1e-4
+    assert (got[decisive] == np.array([oracle.argmax(r) for r in lo])[decisive]).all()
+
+
 def test_decode_graph_survives_a_larger_scratch(dev):
     """The captured decode step holds the address of the context's scratch (split activations of the 16-row tile).  A
     later prefill of many rows needs a larger scratch, which moves it: the next decode step has to be captured anew, not
@@ -201,10 +222,10 @@ def test_attention_geometries(dev, H, KV, hd, B):
         tok = np.argmax(want, axis=1).astype(np.int32).reshape(B, 1)
 
 
-def _pointed(dev, H, KV, hd, B):
+def _pointed(dev, H, KV, hd, B, positions=700):
     """One layer whose queries and keys are large, so that few keys carry the weight of a row: the model, and its logits [B, T, V] in float64."""
     V, d, ff, rng = 41, 64, 32, np.random.default_rng(H * 1000 + hd + B)
-    gm = nn.Llama(dev, nn.LlamaConfig(V, d, ff, 1, H, KV, hd, 700, 1e-5, 10000.0, 0))
+    gm = nn.Llama(dev, nn.LlamaConfig(V, d, ff, 1, H, KV, hd, positions, 1e-5, 10000.0, 0))
     shapes = {0: (d, H * hd, 0.3), 1: (d, KV * hd, 0.3), 2: (d, KV * hd, 0.3), 3: (H * hd, d, 0.1), 4: (d, ff, 0.02), 5: (d, ff, 0.02), 6: (ff, d, 0.02), T_LMHEAD: (d, V, 0.1)}
     w = {}
     for t, (k, n, std) in shapes.items():
@@ -257,8 +278,32 @@ def test_attention_against_float64(dev, H, KV, hd, B, lengths):
         assert near(gm.forward_cached(ids[:, n:]), want[:, -1]), n
         gm.cache_clear()
         gm.forward_cached(ids[:, :n // 3 + 1], want_logits=False)
-        if n // 3 < n:
-            assert near(gm.forward_cached(ids[:, n // 3 + 1:], all_positions=True), want[:, n // 3 + 1:]), n
+        assert near(gm.forward_cached(ids[:, n // 3 + 1:], all_positions=True), want[:, n // 3 + 1:]), n
+
+
+@pytest.mark.parametrize("H,KV,hd", [(2, 1, 160), (3, 3, 192)])
+def test_wide_heads_of_long_prompts_against_float64(dev, H, KV, hd):
+    """Heads above 128 on the tensor cores: three blocks of 64 elements, one buffer of keys, 64 columns of the output per thread."""
+    gm, logits, rng = _pointed(dev, H, KV, hd, 1)
+    for n in (96, 129, 300):
+        ids = rng.integers(0, 41, (1, n)).astype(np.int32)
+        want = logits(ids)
+        gm.cache_clear()
+        assert np.abs(gm.forward_cached(ids, all_positions=True) - want).max() <= 2e-5 * np.abs(want).max(), n
+
+
+def test_prompts_whose_pieces_fill_the_scratch_run_in_portions(dev):
+    """8 key heads of 128 and room for 20000 positions: the pieces of one sequence take 164 MB of the 256, so that three run one after the other."""
+    gm, logits, rng = _pointed(dev, 8, 8, 128, 3)
+    ids = rng.integers(0, 41, (3, 200)).astype(np.int32)
+    want = logits(ids)
+    gm.close()
+    gm, _, _ = _pointed(dev, 8, 8, 128, 3, positions=20000)
+    gm.cache_reserve(3, 20000)
+    for cut in (200, 100):
+        gm.cache_clear()
+        got = [gm.forward_cached(ids[:, a:a + cut], all_positions=True) for a in range(0, 200, cut)]
+        assert np.abs(np.concatenate(got, 1) - want).max() <= 2e-5 * np.abs(want).max(), cut
 
 
 @pytest.mark.parametrize("hd", [32, 128, 256])

@@ -248,7 +248,7 @@ def test_matmul_five_to_sixteen_rows(dev, m, k, n, bits):
 
 
 @pytest.mark.parametrize("bits", [8, 4])
-@pytest.mark.parametrize("m", [1, 3, 9])
+@pytest.mark.parametrize("m", [1, 2, 3, 9])  # (one row has no splits)
 def test_fixed_split_counts_give_the_same_product(dev, bits, m):
     """ruai_ctx_force_splits: the product does not depend on how many CTAs share k beyond the order of a few f32 additions
     (more splits than stages of k leave some CTAs of the cluster without work)."""
@@ -428,6 +428,36 @@ def test_long_rows_of_int8_stay_f32(dev, k):
     _, got = run_matmul(dev, x, nn.QWeight.int8(dev, q, s), "f32", None)
     want = x.astype(np.float64) @ (q.astype(np.float64) * s)
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("k,n,rows", [(2080, 1100, (2, 3, 4, 8, 9, 16)), (1568, 132, (2, 4, 9, 16)), (4000, 900, (2, 3, 8, 16)), (1024, 19460, (1,))])
+def test_narrow_tensor_core_kernels_against_float64(dev, k, n, rows, bits):
+    """Just past the line where the dot-product kernel ends, below the 4M weights of the 16-row one (and one row of int8 that stays with the tensor
+    cores): ragged columns and k, every number of splits.  x is rounded to half of 2^-20 of the largest of its 32 (int4), 2^-27 of the largest
+    of its row (int8), and f32 sums leave 2^-20 of the products' magnitudes."""
+    if bits == 8:
+        k -= 5
+        n -= 1
+    q, s, qw = _qw(dev, bits, k, n, 53)
+    wd = q.astype(np.float64) * s if bits == 8 else qw.dequant().astype(np.float64)
+    bias = oracle.synth_normal(53, 1, (n,))
+    try:
+        for m in rows:
+            x = oracle.synth_normal(53, m, (m, k), 1.0) * np.exp2(np.arange(k) // 32 % 15 - 7).astype(np.float32)
+            want, mag = x.astype(np.float64) @ wd + bias, np.abs(x).astype(np.float64) @ np.abs(wd) + np.abs(bias)
+            if bits == 4:
+                top = np.abs(x).reshape(m, k // 32, 32).max(2)
+                rounding = np.repeat(top, 32, 1).astype(np.float64) @ np.abs(wd) * 2.0 ** -20
+            else:
+                rounding = np.abs(x).max(1, keepdims=True) * np.abs(wd).sum(0) * 2.0 ** -27
+            for splits in (0, 1, 2, 4, 8):
+                dev.force_splits(splits)
+                _, got = run_matmul(dev, x, qw, "f32", bias)
+                bound = rounding + 2.0 ** -20 * mag
+                assert (np.abs(got - want) <= bound).all(), (m, splits, (np.abs(got - want) / bound).max())
+    finally:
+        dev.force_splits(0)
 
 
 # ---- the GEMM's tiles: edges of rows, columns and k, every split of k ----
