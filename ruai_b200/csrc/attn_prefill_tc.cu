@@ -22,8 +22,13 @@
 // and a tile's weighted values once; the latter are read out and added up in registers while the next tile's scores are made.
 // Every mbarrier wait is bounded.
 //
-// What bounds it: the softmax warps' issue slots (scores read out, scaled, exponentials, split into pieces, and a tile's values read out
-// and added up), not the MMAs, of which three f16 products of 128 x 64 x 128 take some 600 clocks a tile.  2000 tokens of the 8B shape
+// Errors against 64 bits (norms over the output; heads of 16 to 192; f32 units | here): smaller nearly everywhere, as a row's sums are over tiles
+// (heads of 128, normal queries, keys and values: 128 keys 2.7e-7 | 2.2e-7, 1030 keys 6.9e-7 | 3.4e-7; scores of 40 1.3e-6 | 6.1e-7).  Larger with few
+// keys only: values around a common offset, 128 keys 1.4e-7 | 1.7e-7, 500 keys 2.4e-7 | 1.9e-7 (the tensor core's sums truncate); heads of 16 1.49e-7 | 1.55e-7.
+//
+// What bounds it: the softmax warps (scores read out, scaled, exponentials, split into pieces, and a tile's values read out and added up), whose
+// waits for tensor memory leave half of the issue slots empty; the MMAs keep the tensor pipe busy for 35 % (for heads of 128 six products of 128 x 64 x
+// 128 take 1540 clocks a tile at least, of some 6000).  attn_tc_kernel<4, 64> spills 100 bytes a thread.  2000 tokens of the 8B shape
 // (32 heads of 128, 8 of keys): 180 to 200 us a layer and 23 for the split, where the f32 units took 1541.  Two warps per row and tile (CS = 2) where the values are at
 // most 64 wide, else four: the registers that hold the output then leave room for the products' read-out.
 #include <algorithm>

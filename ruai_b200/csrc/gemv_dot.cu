@@ -6,8 +6,8 @@
 // x = f * 2^(e - F) with |f| <= 2^F, e from the block's largest magnitude, and f as balanced base-256 digits, each an int8
 // (int4: F = 22, three digits; int8: F = 27, four), so that a dp4a multiplies four weights with one digit of four activations,
 // exactly.  A block's integer is converted to f32 once and multiplied by its scales.  Stored int4 weights are u = q + 8
-// (pack.cu): 8 * sum f is taken off the integer.  The rounding of x to 23 (28) bits of its block's largest magnitude is the
-// only approximation; blocks below 2^-104 (2^-99) keep a quantum of 2^-126.
+// (pack.cu): 8 * sum f is taken off the integer.  Roundings: x to 23 (28) bits of its block's largest magnitude, a block's integer (of up to
+// 30 bits) to f32, and the f32 sums of blocks; blocks below 2^-104 (2^-99) keep a quantum of 2^-126.
 //
 // Organisation.  A CTA of sixteen warps owns TC columns at a time; every warp multiplies a range of k of its own with all of
 // them, lane = column (TC below 32: 32 / TC chunks of k side by side), and the warps meet once per tile of columns, to add their
@@ -22,7 +22,7 @@
 // 32 chunks of 16 bytes (4096 x 28672 17.4 | 22.0, 4.2 TB/s); int8 HBM's latency with four loads of a lane in flight (4096 x 28672 25.7 | 31.1,
 // 4.6 TB/s; 4096 x 128256 95 | 114, 5.5 TB/s).  Not won: long k with few columns, where the conversion of x in every
 // CTA shows, and tiles that do not share out over the SMs (192 of int8 4096 x 6144): ruai_gemv_row_tc.
-// Two CTAs of 64 registers per SM, not one with more and eight loads ahead: alone that is the faster launch (4096 x 28672 18.9 for
+// Two CTAs of 64 registers per SM (row_kernel spills 8 to 28 bytes a thread, rows_kernel<4, 16> 72 to 76), not one with more and eight loads ahead: alone that is the faster launch (4096 x 28672 18.9 for
 // 20.9 then), but a CTA that fills the register file keeps the next kernel's out until it ends, and with it the weights that this would
 // request: steps were 10 % slower.
 #include <algorithm>

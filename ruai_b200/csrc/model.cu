@@ -489,8 +489,8 @@ int issue_step(ruai_model* m, uint32_t B, uint32_t T, const HeadRows& head, bool
   float *x = m->x.as<float>(), *qkv = m->qkv.as<float>(), *att = m->att.as<float>(), *hb = m->hbuf.as<float>();
   const bool tp = m->world > 1;
   // RMSNorm rides in the prologue of the GEMV that consumes it: the producer of x (embedding, o_proj, down_proj)
-  // leaves per-tile sums of squares.  LayerNorm (GPT-2) and the sharded model (x is produced by the exchange
-  // kernel) keep the standalone norm kernels.
+  // leaves per-tile sums of squares; gemv_dot.cu works the norm out itself, LayerNorm (GPT-2) too (normed_linear).  Other Linears behind
+  // a LayerNorm, and the sharded model where the exchange kernel supplies no sums, keep the standalone norm kernels.
   // decode-sized steps on the chunk-layout kernels; sharded: only where the exchange kernel can supply the sum of squares
   const bool fold = m->llama && (m->bits == 8 || m->group == 32) && rows <= 16 && (!tp || ruai_tp_allreduce_gives_sumsq(rows, d));
   auto dot = [&](const Lin& l) { return ruai_gemv_dot_takes(c, l.w, rows); };
