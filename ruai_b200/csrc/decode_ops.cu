@@ -568,14 +568,16 @@ double warps_us(const ruai_ctx* c, uint64_t items, uint32_t rep, uint32_t hd, ui
   const Waves w = waves(items * splits, per_sm, c->sm_count * (splits == 8 ? 120 / 148.0 : splits == 4 ? 132 / 148.0 : 1.0));
   const double h = hd / 64.0, f = attn_keys(hd) / 32.0, busy = w.together * warps;
   const double step = norm4(1.2 + 0.37 * rep + 1.5 * h * f, busy * 0.073 * (rep * h * f + 0.27 * h + 1.5), busy * 0.23 * h * f);
-  return 0.18 * rep + w.rounds * ((cap + shares - 1) / shares * step + 2.0) + (splits > 1 ? 0.86 + 0.074 * splits : 0.0);
+  // a last step of few keys is a short one
+  const double full = cap / shares, part = (double)(cap % shares) / shares, steps = std::max(1.0, full + (part > 0 ? 0.2 + 0.8 * part : 0.0));
+  return 0.18 * rep + w.rounds * (steps * step + 2.0) + (splits > 1 ? 0.86 + 0.074 * splits : 0.0);
 }
 }  // namespace
 
-// The warps' numbers with the shortest launch, or chunks where that is not 13 % shorter by the formulas above (less 1 us with few query heads per
-// key: behind a step's other launches warps that work alone gain that much on chunks).  Of 489 steps measured (1 to 64 sequences of 40 to 32768
-// positions, six head shapes) none is more than 3 % slower than all in chunks, 5 % are shorter on average, and 1 in 40 is more than 5 % slower than all on
-// warps.  Us of a launch, chunks | warps:
+// The warps' numbers with the shortest launch, or chunks where that is not 13 % shorter by the formulas above (less 0.5 us, 1 with few query heads
+// per key: behind a step's other launches warps that work alone gain that much on chunks).  Of 489 steps measured (1 to 64 sequences of 40 to 32768
+// positions, six head shapes) none is more than 4 % slower than all in chunks, they are 5 % shorter on average, and 1 in 35 is more than 5 % slower than
+// all on warps; so are, by up to 24 %, steps of one or two sequences whose cache has room for twice the positions that it holds.  Us of a launch, chunks | warps:
 //   8 key heads of 128 with 4 query heads each: 1 sequence, 1024 positions 9.0 | 9.2, 8192 31 | 40, 32768 91 | 160; 16 sequences, 256 20 | 13,
 //   1024 42 | 47, 4096 129 | 163;  4 of 64 with 8 each: 1 sequence, 1024 10.2 | 10.7, 32768 77 | 101; 64 sequences, 256 36 | 19, 1024 126 | 65;
 //   3 of 64 with 3 each: 1 sequence, 8192 14 | 21; 64 sequences, 256 12.5 | 9.1, 4096 106 | 89;  12 of 64: 64 sequences, 1024 66 | 77
@@ -593,7 +595,7 @@ AttnPlan ruai_attention_plan(const ruai_ctx* c, uint32_t B, uint32_t T, uint32_t
     if (rep <= 2 && items < 512) { plan.warps = 4; plan.splits = 1; }
     return plan;
   }
-  double best = 0.87 * chunks_us(c, items, rep, hd, cap, plan.splits) + (rep < 4 ? 1.0 : 0.0);
+  double best = 0.87 * chunks_us(c, items, rep, hd, cap, plan.splits) + (rep < 4 ? 1.0 : 0.5);
   for (uint32_t w = 4; w <= (uint32_t)kAttnWarps; w *= 2)
     for (uint32_t s = 1; s <= 8; s *= 2) {
       if (attn_smem(rep, hd, w, s) > kAttnSmemMax) break;
