@@ -569,7 +569,7 @@ double warps_us(const ruai_ctx* c, uint64_t items, uint32_t rep, uint32_t hd, ui
   const double h = hd / 64.0, f = attn_keys(hd) / 32.0, busy = w.together * warps;
   const double step = norm4(1.2 + 0.37 * rep + 1.5 * h * f, busy * 0.073 * (rep * h * f + 0.27 * h + 1.5), busy * 0.23 * h * f);
   // a last step of few keys is a short one
-  const double full = cap / shares, part = (double)(cap % shares) / shares, steps = std::max(1.0, full + (part > 0 ? 0.2 + 0.8 * part : 0.0));
+  const double full = cap / shares, part = (double)(cap % shares) / shares, steps = std::max(1.0, full + (part > 0 ? 0.35 + 0.65 * part : 0.0));
   return 0.18 * rep + w.rounds * (steps * step + 2.0) + (splits > 1 ? 0.86 + 0.074 * splits : 0.0);
 }
 }  // namespace
