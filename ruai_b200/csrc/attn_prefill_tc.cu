@@ -163,50 +163,6 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const AttnPar
   }
 }
 
-__device__ __forceinline__ bool elect_one() {  // (a lane that the compiler knows to be one issues an MMA in 10 clocks, `lane == 0` in 45)
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {  // K-major, 128-byte swizzle, 1024 bytes between 8-row blocks
-  return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// D (+)= A B, fp16 x fp16 -> f32; A in shared memory (SS) or in tensor memory (TS).  after_lo: the sums so far are of lo pieces.
-__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
-               "r"(accumulate)
-               : "memory");
-}
-__device__ __forceinline__ void mma_ss_after_lo(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
-               "n"(kLoShift)
-               : "memory");
-}
-__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc),
-               "r"(accumulate)
-               : "memory");
-}
-__device__ __forceinline__ void mma_ts_after_lo(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc),
-               "n"(kLoShift)
-               : "memory");
-}
-// 16 consecutive 32-bit columns of this thread's lane of tensor memory.  The load writes its registers until the wait has returned, so
-// the wait takes them as operands.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]),
-                 "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-               :
-               : "memory");
-}
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
                "r"(v[5]), "r"(v[6]), "r"(v[7])
@@ -357,7 +313,7 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
       // ===== MMAs: the scores of tile i, then the weighted values of tile i - 1 =====
       const uint32_t idesc_s = (1u << 4) | ((uint32_t)(kKeys >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
       const uint32_t idesc_v = (1u << 4) | ((s.vdp >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
-      const uint64_t qd = desc_sw128(smem_u32(smem)), kd = desc_sw128(smem_u32(smem + off_k)), vd0 = desc_sw128(smem_u32(smem + off_v));
+      const uint64_t qd = umma_desc_sw128(smem_u32(smem)), kd = umma_desc_sw128(smem_u32(smem + off_k)), vd0 = umma_desc_sw128(smem_u32(smem + off_v));
       const uint32_t steps = (hd + 15) / 16;
       bool ok = ntiles == 0 || mbar_wait(&q_ready, 0);
       for (uint32_t i = 0; i <= ntiles && ok && ntiles; ++i) {
@@ -369,11 +325,11 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
           auto at_q = [&](uint32_t e) { return umma_desc_advance(qd, (e >> 2) * (kRows * 128) + (e & 3u) * 32u); };
           auto at_k = [&](uint32_t e) { return umma_desc_advance(kt, (e >> 2) * (kKeys * 128) + (e & 3u) * 32u); };
           for (uint32_t e = 0; e < steps; ++e) {
-            mma_ss(d, at_q(e), umma_desc_advance(at_k(e), k_piece), idesc_s, e != 0 ? 1u : 0u);
-            mma_ss(d, umma_desc_advance(at_q(e), q_piece), at_k(e), idesc_s, 1u);
+            umma_f16_ss(d, at_q(e), umma_desc_advance(at_k(e), k_piece), idesc_s, e != 0 ? 1u : 0u);
+            umma_f16_ss(d, umma_desc_advance(at_q(e), q_piece), at_k(e), idesc_s, 1u);
           }
-          mma_ss_after_lo(d, at_q(0), at_k(0), idesc_s);
-          for (uint32_t e = 1; e < steps; ++e) mma_ss(d, at_q(e), at_k(e), idesc_s, 1u);
+          umma_f16_ss_after<kLoShift>(d, at_q(0), at_k(0), idesc_s);
+          for (uint32_t e = 1; e < steps; ++e) umma_f16_ss(d, at_q(e), at_k(e), idesc_s, 1u);
           umma_commit(&k_empty[ks]);
           umma_commit(&s_full[sb]);
         }
@@ -384,12 +340,12 @@ __global__ void __launch_bounds__((kControl + 4 * CS) * 32, CS == 2 && OC == 32 
           const uint64_t vt = umma_desc_advance(vd0, vs * v_slot);
 #pragma unroll
           for (uint32_t e = 0; e < kKeys / 16; ++e) {
-            mma_ts(d, ph + e * 8, umma_desc_advance(vt, v_piece + e * 32u), idesc_v, e != 0 ? 1u : 0u);
-            mma_ts(d, pl + e * 8, umma_desc_advance(vt, e * 32u), idesc_v, 1u);
+            umma_f16_ts(d, ph + e * 8, umma_desc_advance(vt, v_piece + e * 32u), idesc_v, e != 0 ? 1u : 0u);
+            umma_f16_ts(d, pl + e * 8, umma_desc_advance(vt, e * 32u), idesc_v, 1u);
           }
-          mma_ts_after_lo(d, ph, vt, idesc_v);
+          umma_f16_ts_after<kLoShift>(d, ph, vt, idesc_v);
 #pragma unroll
-          for (uint32_t e = 1; e < kKeys / 16; ++e) mma_ts(d, ph + e * 8, umma_desc_advance(vt, e * 32u), idesc_v, 1u);
+          for (uint32_t e = 1; e < kKeys / 16; ++e) umma_f16_ts(d, ph + e * 8, umma_desc_advance(vt, e * 32u), idesc_v, 1u);
           umma_commit(&v_empty[vs]);
           umma_commit(&o_full);
         }

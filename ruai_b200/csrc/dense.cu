@@ -359,18 +359,9 @@ constexpr int stages_of(int nt) { return nt == 128 ? 3 : 4; }
 constexpr size_t stage_bytes(int nt) { return (size_t)(kTileN + nt) * kTileK * 2; }
 constexpr size_t gemm_smem(int nt) { return stages_of(nt) * stage_bytes(nt) + 1024; }
 
-// Operand descriptor: K-major, 128-byte swizzle, rows of 128 bytes, 1024 bytes between 8-row blocks.
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
-  return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
 __device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
                "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b),
-               "r"(idesc), "r"(accumulate)
                : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
@@ -462,10 +453,10 @@ __global__ void __launch_bounds__(kGThreads) dense_gemm_kernel(const __grid_cons
         const uint32_t s = i % S;
         if (s_abort || !mbar_wait(&full[s], (i / S) & 1u)) { s_abort = 1; break; }
         tc_fence_after_sync();
-        const uint64_t ad = desc_sw128(smem_u32(ring + s * (kABytes + kBBytes))), bd = desc_sw128(smem_u32(ring + s * (kABytes + kBBytes) + kABytes));
+        const uint64_t ad = umma_desc_sw128(smem_u32(ring + s * (kABytes + kBBytes))), bd = umma_desc_sw128(smem_u32(ring + s * (kABytes + kBBytes) + kABytes));
 #pragma unroll
         for (uint32_t q = 0; q < kTileK / 16; ++q)
-          mma_bf16(tmem, umma_desc_advance(ad, q * 32), umma_desc_advance(bd, q * 32), idesc, (i | q) != 0 ? 1u : 0u);
+          umma_f16_ss(tmem, umma_desc_advance(ad, q * 32), umma_desc_advance(bd, q * 32), idesc, (i | q) != 0 ? 1u : 0u);
         umma_commit(&empty[s]);
       }
       umma_commit(&done);

@@ -187,41 +187,6 @@ struct Params {
   GemvEpilogue epi;
 };
 
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {  // K-major, 128-byte swizzle, 1024 bytes between 8-row blocks
-  return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// A from tensor memory: lane = column of W, word c of a step holds its k positions 2 c and 2 c + 1.
-__device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b),
-               "r"(idesc), "r"(accumulate)
-               : "memory");
-}
-// The same onto sums of lo pieces, which it brings to the hi pieces' scale.
-__device__ __forceinline__ void mma_f16_after_lo(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t}" ::"r"(d), "r"(a), "l"(b),
-               "r"(idesc), "n"(kLoShift)
-               : "memory");
-}
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
-// 16 consecutive 32-bit columns of this thread's TMEM lane.  The load writes its registers until the wait has returned, so the wait
-// takes them as operands: nothing that uses them can be placed ahead of it, and nothing else can be put into them.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]),
-                 "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-               :
-               : "memory");
-}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "r"(v[0]),
@@ -453,7 +418,7 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
       // the tensor pipe has nothing to do), so two threads issue, each into its own sums: one per column block, or, with one
       // column block, every other stage each. =====
       constexpr uint32_t idesc = (1u << 4) | (BF ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(NT >> 3) << 17) | ((128u >> 4) << 24);  // fp16 x fp16 or bf16 x bf16 -> f32
-      const uint64_t xd0 = desc_sw128(smem_u32(smem));
+      const uint64_t xd0 = umma_desc_sw128(smem_u32(smem));
       const uint32_t pieces = (uint32_t)p.pieces, h = (uint32_t)warp - 1u, cb = CB == 2 ? h : 0u;
       uint32_t it = 0, unit = BITS == 4 && CB == 1 ? 0u : h;
       bool ok = true;
@@ -475,13 +440,13 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
                 const uint32_t d = tmem + (unit % 3) * NT, au = a + u * 16;
                 const uint64_t xu = umma_desc_advance(xd, u * 64u);
                 if (pieces == 2) {
-                  mma_f16(d, au, umma_desc_advance(xu, T::kPiece), idesc, 0u);
-                  mma_f16(d, au + 8, umma_desc_advance(xu, T::kPiece + 32u), idesc, 1u);
-                  mma_f16_after_lo(d, au, xu, idesc);
+                  umma_f16_ts(d, au, umma_desc_advance(xu, T::kPiece), idesc, 0u);
+                  umma_f16_ts(d, au + 8, umma_desc_advance(xu, T::kPiece + 32u), idesc, 1u);
+                  umma_f16_ts_after<kLoShift>(d, au, xu, idesc);
                 } else {
-                  mma_f16(d, au, xu, idesc, 0u);
+                  umma_f16_ts(d, au, xu, idesc, 0u);
                 }
-                mma_f16(d, au + 8, umma_desc_advance(xu, 32u), idesc, 1u);
+                umma_f16_ts(d, au + 8, umma_desc_advance(xu, 32u), idesc, 1u);
                 umma_commit(&acc_full[unit % T::kUnitBars]);
               }
             } else {
@@ -491,7 +456,7 @@ __global__ void __launch_bounds__(Tile<BITS, CB, NT>::kThreads, 1) gemm_tc_kerne
               const uint32_t d = tmem + (unit % 3) * NT;
               for (uint32_t pc = 0; pc < pieces; ++pc)
 #pragma unroll
-                for (uint32_t q = 0; q < 4; ++q) mma_f16(d, a + q * 8, umma_desc_advance(xd, pc * T::kPiece + q * 32u), idesc, !first || (pc | q) != 0 ? 1u : 0u);
+                for (uint32_t q = 0; q < 4; ++q) umma_f16_ts(d, a + q * 8, umma_desc_advance(xd, pc * T::kPiece + q * 32u), idesc, !first || (pc | q) != 0 ? 1u : 0u);
               if (last) { umma_commit(&acc_full[unit % T::kUnitBars]); unit += 2; }
             }
             umma_commit(&x_empty[slot]);
